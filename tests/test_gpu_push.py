@@ -1,0 +1,70 @@
+"""The extended solve's push factor at the ends of its fast range: pairs whose
+squared distance, root or quotient is where a short square root and division
+could round differently (coincident, denormal and tiny separations, roots
+whose significand is all ones, distances next to the minimum distance), and
+rows of candidates of every parity and length.  Compared bit for bit with the
+oracle."""
+import numpy as np
+import pytest
+
+from tests.helpers import assert_frame_equal
+
+pytestmark = pytest.mark.gpu
+
+
+def _separations(min_distance, rng):
+    """x and y separations of pairs, as float32."""
+    m = np.float32(min_distance)
+    ones = [np.nextafter(np.float32(2.0 ** k), np.float32(0)) for k in range(-52, 1)]
+    edge = [m, np.nextafter(m, np.float32(0)), np.nextafter(m, np.float32(9)), m / 2]
+    tiny = [0.0, 1e-45, 1e-38, 1e-30, 2.0 ** -30, 2.0 ** -31, np.nextafter(np.float32(2.0 ** -30), np.float32(0))]
+    x = np.array(ones + edge + tiny, np.float32)
+    pairs = [(a, 0.0) for a in x] + [(0.0, a) for a in x]
+    log = np.exp(rng.uniform(np.log(1e-7), np.log(min_distance), (100, 2)))
+    return np.concatenate([np.array(pairs, np.float32), log.astype(np.float32)])
+
+
+@pytest.mark.parametrize("min_distance", [1.0, 0.37, 2.5, 2.0 ** -22])
+def test_push_of_one_pair(W, O, min_distance):
+    # one pair per world, next to the origin, where float32 holds its separation
+    sep = _separations(min_distance, np.random.default_rng(3))
+    cfg = W.WrachConfig(cell_size=1, mode=1, iterations=2, gravity=0.0, min_distance=min_distance,
+                        capacity=4)
+    dims = (6.0, 6.0)
+    ph = O.Physics(1, 2, 0.0, min_distance, 1.0, 9)
+    w = O.world(dims[0], dims[1], 1)
+    vel = np.zeros((2, 2), np.float32)
+    with W.Simulation(cfg, worlds=[dims] * len(sep)) as sim:
+        for k, d in enumerate(sep):
+            sim.set_particles(np.array([(0, 0), d], np.float32), vel, world=k)
+        sim.step(1)
+        for k, d in enumerate(sep):
+            pos = np.array([(0, 0), d], np.float32)
+            ref = O.step(w, ph, *O.pack(w, pos, vel, 4), 1)[:3]
+            assert_frame_equal(sim.read_frame(world=k), ref, "separation %r" % (d,))
+
+
+@pytest.mark.parametrize("cap,cell_size", [(1, 1), (9, 1), (10, 2), (11, 2), (16, 2)])
+def test_rows_of_every_length(W, O, cap, cell_size):
+    # 0 .. cap + 2 particles per cell, so that rows start at odd and even
+    # places and have every length up to 3 * cap, at both ends of the table too
+    rng = np.random.default_rng(cap)
+    gx, gy = 23, 19
+    counts = rng.integers(0, cap + 3, gx * gy)
+    counts[:3] = counts[-3:] = cap + 2
+    cell = np.repeat(np.arange(gx * gy), counts)
+    pos = (np.stack([cell % gx, cell // gx], 1) + rng.uniform(0.01, 0.99, (len(cell), 2))) * cell_size
+    pos = pos.astype(np.float32)
+    vel = rng.normal(0, 0.5, pos.shape).astype(np.float32)
+    dims = (float(gx * cell_size) - 0.5, float(gy * cell_size) - 0.5)
+    cfg = W.WrachConfig(dimensions=dims, cell_size=cell_size, mode=1, iterations=4, gravity=0.1,
+                        cell_capacity=cap, capacity=len(pos))
+    ph = O.Physics(1, 4, 0.1, 1.0, 1.0, cap)
+    w = O.world(dims[0], dims[1], cell_size)
+    with W.Simulation(cfg) as sim:
+        sim.set_particles(pos, vel)
+        ref = O.pack(w, pos, vel, len(pos))
+        for frame in range(3):
+            sim.step(1)
+            ref = O.step(w, ph, ref[0], ref[1], ref[2], 1)[:3]
+            assert_frame_equal(sim.read_frame(), ref, "frame %d" % frame)

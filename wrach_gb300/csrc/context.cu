@@ -9,7 +9,7 @@
 //   pos, vel          binned state, float2 x capacity        (cell order)
 //   pos_o, vel_o      solve output, float2 x capacity        (same order)
 //   q1, q2            extended-mode Jacobi iterates
-//   rows              the iterations' neighbour-row ranges per compacted particle (4 planes)
+//   rows              the iterations' neighbour-row ranges per compacted particle
 //   cell_of[2]        cell of each binned particle (u32)
 //   cs[2]             cell-start table, cells + 1 u32 (ping-pong per frame)
 //   ct[2], tp_pos[2], tp_vel[2], tp_cell[2]
@@ -222,7 +222,6 @@ wrach::SolveArgs solve_args(WrachContext* ctx) {
   a.tp_vel = ctx->tp_vel[ctx->cur];
   a.sms = ctx->sms;
   a.rows = ctx->rows;
-  a.rows_stride = ctx->total_cap;
   return a;
 }
 
@@ -455,6 +454,9 @@ int create_impl(const WrachConfig* config, uint32_t nworlds, const float* dims,
   ctx->ph.vmax = c.max_velocity;
   ctx->ph.cap = c.cell_capacity;
   ctx->ph.skip_d2 = skip_threshold(c.min_distance);
+  // far from the ends of the exponent range every intermediate value of the
+  // fast push factor is normal; other distances take the general code
+  ctx->ph.slow_below = c.min_distance >= 0x1p-20f && c.min_distance <= 0x1p20f ? 0x1p-60f : INFINITY;
 
   ctx->nworlds = nworlds;
   ctx->worlds_h.resize(nworlds);
@@ -512,16 +514,16 @@ int create_impl(const WrachConfig* config, uint32_t nworlds, const float* dims,
   if ((e = dalloc(&ctx->pos_o, tc)) != cudaSuccess) return oom(e);
   if ((e = dalloc(&ctx->vel_o, tc)) != cudaSuccess) return oom(e);
   if (c.mode == WRACH_MODE_EXTENDED && ctx->ph.iterations >= 2) {
-    if ((e = dalloc(&ctx->q1, tc)) != cudaSuccess) return oom(e);
-    if ((e = dalloc(&ctx->q2, tc)) != cudaSuccess) return oom(e);
+    if ((e = dalloc(&ctx->q1, tc + wrach::kRowPad)) != cudaSuccess) return oom(e);
+    if ((e = dalloc(&ctx->q2, tc + wrach::kRowPad)) != cudaSuccess) return oom(e);
   }
   if (c.mode == WRACH_MODE_EXTENDED && ctx->ph.iterations >= 3)
-    if ((e = dalloc(&ctx->rows, 4 * tc)) != cudaSuccess) return oom(e);
+    if ((e = dalloc(&ctx->rows, tc)) != cudaSuccess) return oom(e);
   if (c.mode == WRACH_MODE_EXTENDED) {
     for (int i = 0; i < 2; ++i) {
       if ((e = dalloc(&ctx->ct[i], (size_t)ctx->ncells + 1)) != cudaSuccess) return oom(e);
       if ((e = cudaMemset(ctx->ct[i], 0, ((size_t)ctx->ncells + 1) * 4)) != cudaSuccess) return oom(e);
-      if ((e = dalloc(&ctx->tp_pos[i], tc)) != cudaSuccess) return oom(e);
+      if ((e = dalloc(&ctx->tp_pos[i], tc + wrach::kRowPad)) != cudaSuccess) return oom(e);
       if ((e = dalloc(&ctx->tp_vel[i], tc)) != cudaSuccess) return oom(e);
       if ((e = dalloc(&ctx->tp_cell[i], tc)) != cudaSuccess) return oom(e);
     }

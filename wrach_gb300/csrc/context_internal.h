@@ -46,7 +46,7 @@ struct WrachContext {
   wrach::WorldDev* worlds_d = nullptr;
   float2 *pos = nullptr, *vel = nullptr, *pos_o = nullptr, *vel_o = nullptr;
   float2 *q1 = nullptr, *q2 = nullptr;
-  uint32_t* rows = nullptr;  // the iterations' neighbour rows: 4 planes of total_cap u32
+  uint4* rows = nullptr;  // the iterations' neighbour rows per compacted particle
   uint32_t* cell_of[2] = {nullptr, nullptr};
   uint32_t* cs[2] = {nullptr, nullptr};
   int cur = 0;

@@ -97,28 +97,28 @@ k_solve_reference(const WorldDev* __restrict__ worlds, int nworlds,
 // The iterations run over the compacted taking-part particles (the capped
 // table ct of the rebin): there a neighbour row of the 3x3 search is one
 // contiguous range [ct[row + x0], ct[row + x1 + 1]) whatever the cells'
-// occupancy, and the particles that take no part cost nothing.  Per row, the
-// candidates within reach are marked with an exact squared-distance test
-// (cheap, every candidate), then the reference's push (IEEE square root and
-// division) is applied to the marked ones only, in candidate order, in one
-// loop over the three rows' marks, so that a lane moves on to its next row
-// without waiting for the warp's other lanes to finish the current one.
+// occupancy, and the particles that take no part cost nothing.
 
-__device__ __forceinline__ uint32_t low_bit(uint32_t m) { return __ffs((int)m) - 1; }
-__device__ __forceinline__ uint32_t low_bit(uint64_t m) { return __ffsll((long long)m) - 1; }
+// The candidates of one particle: the compacted starts of its three
+// neighbour rows, and packed their lengths (6 bits each, at most 3 * 16) and
+// the particle's own place in the middle row (6 bits).
+struct Rows {
+  uint32_t s0, s1, s2, len;
+  __device__ uint32_t start(int r) const { return r == 0 ? s0 : r == 1 ? s1 : s2; }
+  __device__ uint32_t length(int r) const { return (len >> (6 * r)) & 63u; }
+  __device__ uint32_t particle() const { return s1 + (len >> 18); }
+};
+static_assert(3 * kMaxCellCapacity < 64, "row lengths fit 6 bits");
 
-// The push sum (ax, ay) of the compacted particle t of cell c at q_t = qi2,
-// over the compacted iterate q.  Mask holds one bit per candidate of a row:
-// 3 * cap bits.  METRICS: pen = the deepest overlap min_d - distance with a
-// pushing neighbour.
-// The compacted ranges [rs[r], re[r]) of the three neighbour rows of cell c
-// (independent loads of the capped table).
-__device__ __forceinline__ void tp_rows(const WorldDev& w, const uint32_t* __restrict__ ct,
-                                        uint32_t c, uint32_t (&rs)[3], uint32_t (&re)[3]) {
+// The rows of the compacted particle t of cell c (independent loads of the
+// capped table).
+__device__ __forceinline__ Rows tp_rows(const WorldDev& w, const uint32_t* __restrict__ ct,
+                                        uint32_t c, uint32_t t) {
   uint32_t cx, cy;
   cell_xy(w, c - w.cell_off, cx, cy);
   const uint32_t x0 = cx > 0 ? cx - 1 : 0;
   const uint32_t x1 = cx + 1 < w.gx ? cx + 1 : w.gx - 1;
+  uint32_t rs[3], re[3];
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
     const int ny = (int)cy - 1 + r;
@@ -127,73 +127,118 @@ __device__ __forceinline__ void tp_rows(const WorldDev& w, const uint32_t* __res
     rs[r] = ok ? ct[rb + x0] : 0u;
     re[r] = ok ? ct[rb + x1 + 1] : 0u;
   }
+  return Rows{rs[0], rs[1], rs[2],
+              (re[0] - rs[0]) | ((re[1] - rs[1]) << 6) | ((re[2] - rs[2]) << 12) |
+                  ((t - rs[1]) << 18)};
 }
 
-// The push sum over the candidates of the rows [rs[r], re[r]) of the
-// compacted particle t (in the middle row).
-template <typename Mask, bool METRICS>
-__device__ __forceinline__ void tp_push_rows(const PhysDev& ph, const f32x2* __restrict__ q,
-                                             f32x2 qi2, uint32_t t, const uint32_t (&rs)[3],
-                                             const uint32_t (&re)[3], float& ax, float& ay,
-                                             float& pen) {
-  // the candidates within reach, three per step (a short last step tests
-  // its last candidate again and keeps the first result); a NaN distance
-  // counts as within reach, as in the reference's test
-  Mask rmask[3];
+// Candidates are read two per 16-byte load from an even index, kStep per
+// step: a row's marks have one bit per index from its start rounded down to
+// even, and up to kStep - 1 indices past its end are read (and unmarked).
+constexpr uint32_t kStep = 4;
+static_assert(kStep - 1 <= kRowPad, "the iterates are padded for the last step");
+
+// The candidates of row r within reach of the particle at qi2 (a NaN
+// distance counts, as in the reference's test).  Mask holds the bits of a
+// row: 3 * cap + 1.
+template <typename Mask>
+__device__ __forceinline__ Mask row_marks(const PhysDev& ph, const f32x2* __restrict__ q, f32x2 qi2,
+                                          const Rows& R, int r) {
+  const uint32_t s = R.start(r), n = R.length(r), odd = s & 1u;
+  const ulonglong2* p = reinterpret_cast<const ulonglong2*>(q + (s - odd));
+  Mask marks = 0;
+  for (uint32_t k = 0; k < (n ? odd + n : 0u); k += kStep) {
+    uint32_t in = 0;
 #pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    Mask close = 0;
-    const uint32_t s0 = rs[r], e = re[r];
-    for (uint32_t j = s0; j < e; j += 3) {
-      const uint32_t j1 = min(j + 1, e - 1), j2 = min(j + 2, e - 1);
-      const f32x2 da = f2_sub(q[j], qi2), db = f2_sub(q[j1], qi2), dc = f2_sub(q[j2], qi2);
-      const bool ca = !(f2_len2(da) >= ph.skip_d2);
-      const bool cb = j + 1 < e && !(f2_len2(db) >= ph.skip_d2);
-      const bool cc = j + 2 < e && !(f2_len2(dc) >= ph.skip_d2);
-      close |= (Mask)((ca ? 1u : 0u) | (cb ? 2u : 0u) | (cc ? 4u : 0u)) << (j - s0);
+    for (uint32_t u = 0; u < kStep / 2; ++u) {
+      const ulonglong2 c = p[k / 2 + u];
+      if (!(f2_len2(f2_sub(c.x, qi2)) >= ph.skip_d2)) in |= 1u << (2 * u);
+      if (!(f2_len2(f2_sub(c.y, qi2)) >= ph.skip_d2)) in |= 2u << (2 * u);
     }
-    // the particle itself (in the middle row) is not its own neighbour
-    if (r == 1) close &= ~((Mask)1 << (t - s0));
-    rmask[r] = close;
+    marks |= (Mask)in << k;
   }
-  // the reference's push for those, in candidate order
-  Mask cur = rmask[0];
-  uint32_t base = rs[0];
-  Mask next1 = rmask[1], next2 = rmask[2];
-  for (;;) {
-    if (cur == 0) {
-      if (next1) {
-        cur = next1;
-        next1 = 0;
-        base = rs[1];
-      } else if (next2) {
-        cur = next2;
-        next2 = 0;
-        base = rs[2];
-      } else {
-        break;
-      }
-    }
-    const uint32_t b = low_bit(cur);
-    cur &= cur - 1;
-    const f32x2 dd = f2_sub(q[base + b], qi2);
-    float d;
-    const float f = push_factor_within(f2_x(dd), f2_y(dd), ph.min_d, d);
-    if (METRICS) pen = fmaxf(pen, __fsub_rn(ph.min_d, d));
-    // scalar: a paired multiply feeding a paired add may be fused
-    ax = __fadd_rn(ax, __fmul_rn(f2_x(dd), f));
-    ay = __fadd_rn(ay, __fmul_rn(f2_y(dd), f));
-  }
+  // the row alone, without the particle itself
+  marks &= (((Mask)1 << n) - 1) << odd;
+  if (r == 1) marks &= ~((Mask)1 << (R.particle() - (s - odd)));
+  return marks;
 }
 
+template <typename Mask>
+struct Marks {
+  Mask m[3];
+};
+template <typename Mask>
+__device__ __forceinline__ Marks<Mask> all_marks(const PhysDev& ph, const f32x2* __restrict__ q,
+                                                 f32x2 qi2, const Rows& R) {
+  Marks<Mask> M;
+#pragma unroll
+  for (int r = 0; r < 3; ++r) M.m[r] = row_marks<Mask>(ph, q, qi2, R, r);
+  return M;
+}
+
+__device__ __forceinline__ uint32_t low_bit(uint32_t m) { return __ffs((int)m) - 1; }
+__device__ __forceinline__ uint32_t low_bit(uint64_t m) { return __ffsll((long long)m) - 1; }
+
+// The marked candidates in order, one after the other: `cur` holds the marks
+// left of the row at `base`, and is empty only when no marks are left.
+template <typename Mask>
+struct MarkWalk {
+  Mask cur, next1, next2;
+  uint32_t base, base1, base2;
+  __device__ __forceinline__ MarkWalk(const Rows& R, const Marks<Mask>& M)
+      : cur(M.m[0]), next1(M.m[1]), next2(M.m[2]), base(R.s0 & ~1u), base1(R.s1 & ~1u),
+        base2(R.s2 & ~1u) {
+    if (!next1) advance1();
+    if (!cur) advance();
+  }
+  __device__ __forceinline__ void advance1() {
+    next1 = next2;
+    base1 = base2;
+    next2 = 0;
+  }
+  __device__ __forceinline__ void advance() {
+    cur = next1;
+    base = base1;
+    advance1();
+  }
+  __device__ __forceinline__ uint32_t take() {
+    const uint32_t j = base + low_bit(cur);
+    cur &= cur - 1;
+    if (!cur) advance();
+    return j;
+  }
+};
+
+// The reference's push by the marked candidates, in candidate order, summed
+// into (ax, ay), in one loop over the three rows' marks, so that a lane moves
+// on to its next row without waiting for the warp's other lanes to finish the
+// current one.  Two marks a turn: their factors are paired arithmetic, and the
+// loop's own instructions serve both (4M particles in dense clusters, frame
+// 8: the three iterations 203, 176 and 227 us with one mark a turn and the
+// general square root and division, 181, 157 and 135 us now).  METRICS: pen =
+// the deepest overlap min_d - distance with a pushing neighbour.
 template <typename Mask, bool METRICS>
-__device__ __forceinline__ void tp_push(const WorldDev& w, const PhysDev& ph,
-                                        const uint32_t* __restrict__ ct,
-                                        const f32x2* __restrict__ q, f32x2 qi2, uint32_t c,
-                                        uint32_t t, float& ax, float& ay, float& pen) {
-  uint32_t rs[3], re[3];
-  tp_rows(w, ct, c, rs, re);
-  tp_push_rows<Mask, METRICS>(ph, q, qi2, t, rs, re, ax, ay, pen);
+__device__ __forceinline__ void push_marked(const PhysDev& ph, const f32x2* __restrict__ q,
+                                            f32x2 qi2, const Rows& R, const Marks<Mask>& M,
+                                            float& ax, float& ay, float& pen) {
+  MarkWalk<Mask> walk(R, M);
+  while (walk.cur) {
+    const uint32_t j0 = walk.take();
+    const bool two = walk.cur != 0;
+    const uint32_t j1 = two ? walk.take() : j0;
+    const f32x2 d0 = f2_sub(q[j0], qi2), d1 = f2_sub(q[j1], qi2);
+    float f0, f1, e0, e1;
+    push_factors_near(f2_len2(d0), f2_len2(d1), ph, f0, f1, e0, e1);
+    if (METRICS) pen = fmaxf(pen, __fsub_rn(ph.min_d, e0));
+    // scalar: a paired multiply feeding a paired add may be fused
+    ax = __fadd_rn(ax, __fmul_rn(f2_x(d0), f0));
+    ay = __fadd_rn(ay, __fmul_rn(f2_y(d0), f0));
+    if (two) {
+      if (METRICS) pen = fmaxf(pen, __fsub_rn(ph.min_d, e1));
+      ax = __fadd_rn(ax, __fmul_rn(f2_x(d1), f1));
+      ay = __fadd_rn(ay, __fmul_rn(f2_y(d1), f1));
+    }
+  }
 }
 
 // One Jacobi iteration but the last, one thread per compacted (taking-part)
@@ -202,39 +247,32 @@ __device__ __forceinline__ void tp_push(const WorldDev& w, const PhysDev& ph,
 // frame, so each thread takes one or none).  A launch whose `run_if` flag
 // reads 0 returns at once.
 // ROWS 0: the neighbour rows from the capped table; 1: also written to
-// `rows` (4 planes of `stride`); 2: read from `rows` (the cell and its
-// world are then not needed).
+// `rows`; 2: read from `rows` (the cell and its world are then not needed).
+// At most 42 registers (three blocks of 512): the loads' latency needs the
+// warps.  On the 1M lattice an iteration issues about 60% of the time and
+// waits for its gathers through L1 for the rest.
 template <typename Mask, int ROWS>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(512, 3)
 k_jacobi_tp(const WorldDev* __restrict__ worlds, int nworlds, PhysDev ph, uint32_t ncells,
             const uint32_t* __restrict__ ct, const uint32_t* __restrict__ tp_cell,
             const float2* __restrict__ qin, float2* __restrict__ qout,
-            const uint32_t* __restrict__ run_if, uint32_t* __restrict__ rows, uint32_t stride) {
+            const uint32_t* __restrict__ run_if, uint4* __restrict__ rows) {
   if (run_if && *run_if == 0u) return;
   const uint32_t ntp = __ldg(ct + ncells);
   const f32x2* __restrict__ q = reinterpret_cast<const f32x2*>(qin);
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ntp; t += gridDim.x * blockDim.x) {
-    uint32_t rs[3], re[3];
+    Rows R;
     if (ROWS == 2) {
-      const uint32_t len = rows[3 * (size_t)stride + t];
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        rs[r] = rows[(size_t)r * stride + t];
-        re[r] = rs[r] + ((len >> (8 * r)) & 0xFFu);
-      }
+      const uint4 u = rows[t];
+      R = Rows{u.x, u.y, u.z, u.w};
     } else {
       const uint32_t c = tp_cell[t];
-      tp_rows(worlds[world_of_cell(worlds, nworlds, c)], ct, c, rs, re);
-      if (ROWS == 1) {
-#pragma unroll
-        for (int r = 0; r < 3; ++r) rows[(size_t)r * stride + t] = rs[r];
-        rows[3 * (size_t)stride + t] =
-            (re[0] - rs[0]) | ((re[1] - rs[1]) << 8) | ((re[2] - rs[2]) << 16);
-      }
+      R = tp_rows(worlds[world_of_cell(worlds, nworlds, c)], ct, c, t);
+      if (ROWS == 1) rows[t] = make_uint4(R.s0, R.s1, R.s2, R.len);
     }
     const f32x2 qi2 = q[t];
     float ax = 0.f, ay = 0.f, pen = 0.f;
-    tp_push_rows<Mask, false>(ph, q, qi2, t, rs, re, ax, ay, pen);
+    push_marked<Mask, false>(ph, q, qi2, R, all_marks<Mask>(ph, q, qi2, R), ax, ay, pen);
     qout[t] = make_float2(__fsub_rn(f2_x(qi2), ax), __fsub_rn(f2_y(qi2), ay));
   }
 }
@@ -252,7 +290,7 @@ k_jacobi_tp(const WorldDev* __restrict__ worlds, int nworlds, PhysDev ph, uint32
 // reflections only change the velocity).  A launch whose `run_if` flag
 // reads 0 returns at once.
 template <typename Mask, bool METRICS>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(512, METRICS ? 1 : 3)
 k_jacobi_final(const WorldDev* __restrict__ worlds, int nworlds, PhysDev ph, uint32_t n,
                int do_push, const uint32_t* __restrict__ cell_start,
                const uint32_t* __restrict__ ct, const uint32_t* __restrict__ cell_of,
@@ -289,7 +327,10 @@ k_jacobi_final(const WorldDev* __restrict__ worlds, int nworlds, PhysDev ph, uin
         const f32x2* __restrict__ q = reinterpret_cast<const f32x2*>(qtp);
         const f32x2 qi2 = q[t];
         float ax = 0.f, ay = 0.f;
-        if (do_push) tp_push<Mask, METRICS>(w, ph, ct, q, qi2, c, t, ax, ay, pen);
+        if (do_push) {
+          const Rows R = tp_rows(w, ct, c, t);
+          push_marked<Mask, METRICS>(ph, q, qi2, R, all_marks<Mask>(ph, q, qi2, R), ax, ay, pen);
+        }
         qx = __fsub_rn(f2_x(qi2), ax);
         qy = __fsub_rn(f2_y(qi2), ay);
       } else {
@@ -368,6 +409,9 @@ uint32_t solve_blocks(const SolveArgs& a) {
   return a.run_if && blocks > few ? few : blocks;
 }
 
+// A row's marks fit 32 bits: its candidates and one more for an odd start.
+static bool narrow_marks(const PhysDev& ph) { return 3 * ph.cap + 1 <= 32; }
+
 cudaError_t launch_jacobi_iteration(const SolveArgs& a, const float2* qin, float2* qout,
                                     cudaStream_t st) {
   if (a.n == 0) return cudaSuccess;
@@ -376,9 +420,8 @@ cudaError_t launch_jacobi_iteration(const SolveArgs& a, const float2* qin, float
   const int mode = a.rows ? a.rows_mode : 0;
 #define WRACH_TP(MASK, ROWS)                                                                  \
   k_jacobi_tp<MASK, ROWS><<<blocks, threads, 0, st>>>(a.worlds, a.nworlds, a.ph, a.ncells, a.ct, \
-                                                      a.tp_cell, qin, qout, a.run_if, a.rows,  \
-                                                      a.rows_stride)
-  if (3 * a.ph.cap <= 32) {
+                                                      a.tp_cell, qin, qout, a.run_if, a.rows)
+  if (narrow_marks(a.ph)) {
     if (mode == 1) WRACH_TP(uint32_t, 1);
     else if (mode == 2) WRACH_TP(uint32_t, 2);
     else WRACH_TP(uint32_t, 0);
@@ -396,7 +439,7 @@ cudaError_t launch_jacobi_final(const SolveArgs& a, const float2* qtp, int do_pu
   if (a.n == 0) return cudaSuccess;
   const uint32_t threads = a.block ? a.block : 128;
   const uint32_t blocks = solve_blocks(a);
-  const bool narrow = 3 * a.ph.cap <= 32;
+  const bool narrow = narrow_marks(a.ph);
 #define WRACH_FINAL(MASK, METRICS, PART)                                                     \
   k_jacobi_final<MASK, METRICS><<<blocks, threads, 0, st>>>(                                 \
       a.worlds, a.nworlds, a.ph, a.n, do_push, a.cell_start, a.ct, a.cell_of, a.pos, qtp,    \

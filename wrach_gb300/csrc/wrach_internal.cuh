@@ -35,6 +35,7 @@ struct PhysDev {
   float vmax;
   uint32_t cap;         // reference cell capacity
   float skip_d2;        // smallest squared distance s with sqrt_rn(s) > min_d
+  float slow_below;     // push_factors_near's own code serves squared distances from here up
 };
 
 // Device control block: counters of the persistent rebin kernel and the
@@ -130,6 +131,53 @@ __device__ __forceinline__ void enforce_limits(const WorldDev& w, float vmax,
   if (vy > vmax) vy = vmax;
 }
 
+// Packed pairs of binary32 values (x in the low word, as float2 in memory)
+// and sm_100-family paired arithmetic: each half rounds to nearest even on
+// its own, exactly as two __fadd_rn / __fsub_rn / __fmul_rn do.  A paired
+// multiply whose result feeds a paired add can be fused into one rounding
+// by the compiler (measured on sm_103a despite the .rn modifiers), so chains
+// that must round twice use the scalar intrinsics, which are never fused;
+// f2_len2 (paired multiply, then a scalar add of the halves) measured exact.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 f2_pack(float x, float y) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float f2_x(f32x2 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float f2_y(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 f2_both(float v) { return f2_pack(v, v); }
+__device__ __forceinline__ float rsqrt_approx(float s) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
+  return y;
+}
+// Squared length of a packed (dx, dy): fl(fl(dx*dx) + fl(dy*dy)).
+__device__ __forceinline__ float f2_len2(f32x2 d) {
+  const f32x2 q = f2_mul(d, d);
+  return __fadd_rn(f2_x(q), f2_y(q));
+}
+
 // The reference's pair push factor (shaders/physics/src/particles.rs:62-93):
 // returns false when the pair is farther apart than min_d, otherwise the
 // force 0.5 * (min_d - d) / d with d == 0 replaced by 0.0001.
@@ -137,30 +185,56 @@ __device__ __forceinline__ void enforce_limits(const WorldDev& w, float vmax,
 // the host); since sqrt_rn is monotonic, s >= skip_d2 is exactly the
 // reference's `distance > MIN_DISTANCE`, decided without the square root.
 __device__ __forceinline__ bool push_factor(float ex, float ey, float min_d,
-                                            float skip_d2, float& f, float& dist) {
+                                            float skip_d2, float& f) {
   const float s = __fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey));
   if (s >= skip_d2) return false;
   float d = __fsqrt_rn(s);
-  dist = d;
   if (d > min_d) return false;
   if (d == 0.0f) d = 0.0001f;
   f = __fdiv_rn(__fmul_rn(0.5f, __fsub_rn(min_d, d)), d);
   return true;
 }
-__device__ __forceinline__ bool push_factor(float ex, float ey, float min_d,
-                                            float skip_d2, float& f) {
-  float d;
-  return push_factor(ex, ey, min_d, skip_d2, f, d);
-}
-// The same force for a pair already found within reach (s < skip_d2, or s
-// NaN): both tests of push_factor would pass, so they are left out.
-__device__ __forceinline__ float push_factor_within(float ex, float ey, float min_d,
-                                                    float& dist) {
-  const float s = __fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey));
+// The same force for two pairs already found within reach (s < skip_d2, or s
+// NaN), from their squared distances and without the special-case code of a
+// general square root and division: both are finished by one exact residual
+// each, so they round correctly (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34,
+// 1990).
+//   root      d = g + (s - g^2) h with g ~ sqrt(s), h ~ 1 / (2 sqrt(s))
+//   quotient  f = q + (a - d q) y with q ~ a / d and y = RN(1 / d)
+// y takes two Newton steps from the root's estimate and is RN(1 / d) for
+// every d whose significand is not all ones; those, and s below
+// ph.slow_below (zero among them) or NaN, take the general code.  d and y
+// were compared with the correctly rounded root and reciprocal for every
+// binary32 s in [2^-60, 2^60].
+__device__ __forceinline__ float push_factor_general(float s, const PhysDev& ph, float& dist) {
   float d = __fsqrt_rn(s);
   dist = d;
   if (d == 0.0f) d = 0.0001f;
-  return __fdiv_rn(__fmul_rn(0.5f, __fsub_rn(min_d, d)), d);
+  return __fdiv_rn(__fmul_rn(0.5f, __fsub_rn(ph.min_d, d)), d);
+}
+__device__ __forceinline__ bool push_special(float s, float d, const PhysDev& ph) {
+  return !(s >= ph.slow_below) || (__float_as_uint(d) | 0xFF800000u) == 0xFFFFFFFFu;
+}
+__device__ __forceinline__ void push_factors_near(float s0, float s1, const PhysDev& ph, float& f0,
+                                                  float& f1, float& dist0, float& dist1) {
+  const f32x2 s = f2_pack(s0, s1), y = f2_pack(rsqrt_approx(s0), rsqrt_approx(s1));
+  const f32x2 g = f2_mul(s, y), minus = f2_both(-1.0f), one = f2_both(1.0f);
+  const f32x2 d = f2_fma(f2_fma(g, g, f2_mul(s, minus)), f2_mul(y, f2_both(-0.5f)), g);
+  const f32x2 nd = f2_mul(d, minus);
+  const f32x2 y1 = f2_fma(y, f2_fma(nd, y, one), y);
+  const f32x2 y2 = f2_fma(y1, f2_fma(nd, y1, one), y1);
+  const f32x2 a = f2_mul(f2_add(f2_both(ph.min_d), nd), f2_both(0.5f));
+  const f32x2 q = f2_mul(a, y2);
+  const f32x2 f = f2_fma(f2_fma(nd, q, a), y2, q);
+  f0 = f2_x(f);
+  f1 = f2_y(f);
+  dist0 = f2_x(d);
+  dist1 = f2_y(d);
+  if (push_special(s0, dist0, ph) || push_special(s1, dist1, ph)) {
+    f0 = push_factor_general(s0, ph, dist0);
+    f1 = push_factor_general(s1, ph, dist1);
+  }
 }
 
 // Counting-sort ticket of a particle whose next cell is k (k >= ncells: no
@@ -223,42 +297,6 @@ __device__ __forceinline__ uint32_t tp_index(const uint32_t* __restrict__ cs,
                                              uint32_t i, uint32_t cap) {
   const uint32_t r = i - cs[c];
   return r < cap ? ct[c] + r : 0xFFFFFFFFu;
-}
-
-// Packed pairs of binary32 values (x in the low word, as float2 in memory)
-// and sm_100-family paired arithmetic: each half rounds to nearest even on
-// its own, exactly as two __fadd_rn / __fsub_rn / __fmul_rn do.  A paired
-// multiply whose result feeds a paired add can be fused into one rounding
-// by the compiler (measured on sm_103a despite the .rn modifiers), so chains
-// that must round twice use the scalar intrinsics, which are never fused;
-// f2_len2 (paired multiply, then a scalar add of the halves) measured exact.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 f2_pack(float x, float y) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ float f2_x(f32x2 v) { return __uint_as_float((uint32_t)v); }
-__device__ __forceinline__ float f2_y(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
-__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-// Squared length of a packed (dx, dy): fl(fl(dx*dx) + fl(dy*dy)).
-__device__ __forceinline__ float f2_len2(f32x2 d) {
-  const f32x2 q = f2_mul(d, d);
-  return __fadd_rn(f2_x(q), f2_y(q));
 }
 
 __device__ __forceinline__ uint64_t ld_acquire_u64(const uint64_t* p) {

@@ -8,6 +8,10 @@
 
 namespace wrach {
 
+// Entries past their particle count that the compacted positions and the
+// iterates have room for (the iterations read candidates several at a time).
+constexpr uint32_t kRowPad = 4;
+
 struct SolveArgs {
   const WorldDev* worlds;
   int nworlds;
@@ -34,11 +38,10 @@ struct SolveArgs {
   const float2* tp_vel;         // compacted velocities of the binned state
   int sms;                      // SMs of the device
   // extended iterations (optional): each compacted taking-part particle's
-  // three neighbour rows, as 4 planes of rows_stride u32 (the rows' compacted
-  // starts, then their lengths packed one byte each); rows_mode 0 computes
-  // the rows from the capped table, 1 also writes them, 2 reads them
-  uint32_t* rows;
-  uint32_t rows_stride;
+  // three neighbour rows (total_cap entries); rows_mode 0 computes the rows
+  // from the capped table, 1 also writes them, 2 reads them (the launches of
+  // a frame have the same block size)
+  uint4* rows;
   int rows_mode;
 };
 

@@ -280,7 +280,7 @@ def launch_bytes(kind, n, c, n_tp=None):
 
 
 # the launches of the rebin (a stable counting sort), in order; the first is
-# left out of extended-physics frames, whose last Jacobi pass takes the tickets
+# left out of frames, whose last solve launch takes the tickets
 REBIN_STEPS = ["count", "scan", "scatter", "place", "large_cells"]
 
 
@@ -352,8 +352,8 @@ def run_ours(args):
     # (frames 1..K of the trajectory), the frames the line's value covers
     solve_kinds = (["jacobi"] * (cfg["iterations"] - 1) + ["jacobi_final"] if cfg["mode"] else
                    ["solve_reference"])
-    # extended frames take the rebin's tickets in their last Jacobi pass
-    rebin_kinds = REBIN_STEPS[1:] if cfg["mode"] else REBIN_STEPS
+    # frames take the rebin's tickets in their last solve launch
+    rebin_kinds = REBIN_STEPS[1:]
     kinds = solve_kinds + ["rebin_" + s for s in rebin_kinds]
     sim.set_particles(pos, vel)
     window = min(args.steps, args.trajectory)

@@ -276,14 +276,14 @@ int enqueue_frame(WrachContext* ctx) {
   wrach::SolveArgs a = solve_args(ctx);
   cudaStream_t st = ctx->stream;
   mark(ctx);
+  // the last solve launch takes the rebin's tickets (it computes the keys)
+  wrach::SolveArgs fin = a;
+  fin.count = ticket_args(ctx);
   if (ctx->ph.mode == WRACH_MODE_REFERENCE) {
-    CK(wrach::launch_solve_reference(a, st));
+    CK(wrach::launch_solve_reference(fin, st));
     mark(ctx);
-    ctx->launches += 1;
+    ctx->launches += ctx->n ? 1 : 0;
   } else {
-    // the last pass takes the rebin's tickets (it computes the keys)
-    wrach::SolveArgs fin = a;
-    fin.count = ticket_args(ctx);
     const uint32_t K = ctx->ph.iterations;
     const float2* q = nullptr;
     CK(enqueue_iterations(ctx, a, K > 0 ? K - 1 : 0, st, &q, [&]() { mark(ctx); }));
@@ -291,7 +291,6 @@ int enqueue_frame(WrachContext* ctx) {
     mark(ctx);
     ctx->launches += ctx->n ? std::max<uint32_t>(K, 1) : 0u;
   }
-  const bool tickets_taken = ctx->ph.mode != WRACH_MODE_REFERENCE;
   wrach::RebinArgs r = rebin_args(ctx);
   r.n = ctx->n;
   r.dst_capacity = ctx->total_cap;
@@ -306,7 +305,7 @@ int enqueue_frame(WrachContext* ctx) {
   // cells' pass before it, so outside per-launch profiling it runs on the
   // auxiliary stream at the same time, joined back before the frame ends
   const bool fork = !ctx->event_hook && r.n;
-  for (int step = tickets_taken ? 1 : 0; step < wrach::kCountSortSteps; ++step) {
+  for (int step = 1; step < wrach::kCountSortSteps; ++step) {
     bool launched;
     if (fork && step == wrach::kCountSortSteps - 2) {
       CK(cudaEventRecord(ctx->fork_ev, st));
@@ -320,24 +319,23 @@ int enqueue_frame(WrachContext* ctx) {
     CK(wrach::launch_count_sort_step(r, step, ctx->big_blocks, st, &launched));
     if (launched) mark(ctx);
   }
-  ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells) - (tickets_taken && r.n ? 1 : 0);
+  ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells) - (r.n ? 1 : 0);
   ctx->cur ^= 1;
   return WRACH_OK;
 }
 
 // Steps wrach_profile_frame times in one frame: each solve launch, then
-// each rebin launch (an empty frame's extended solve launches nothing, but
-// still marks its steps).
+// each rebin launch (an empty frame's solve launches nothing, but still marks
+// its steps).
 uint32_t frame_steps(const WrachContext* ctx) {
   const uint32_t rebin = wrach::count_sort_steps(ctx->n);
-  if (ctx->ph.mode == WRACH_MODE_REFERENCE) return 1 + rebin;
   return std::max<uint32_t>(ctx->ph.iterations, 1) + rebin - (ctx->n ? 1 : 0);
 }
 
 // Kernel launches of one frame.
 uint32_t frame_launches(const WrachContext* ctx) {
   const uint32_t extra = wrach::count_sort_launches(ctx->n, ctx->ncells) - wrach::count_sort_steps(ctx->n);
-  if (ctx->ph.mode == WRACH_MODE_EXTENDED && !ctx->n) return wrach::count_sort_launches(0, ctx->ncells);
+  if (!ctx->n) return wrach::count_sort_launches(0, ctx->ncells);
   return frame_steps(ctx) + extra;
 }
 

@@ -275,7 +275,7 @@ __device__ __forceinline__ uint32_t warp_ticket(uint32_t k, uint32_t ncells, uin
   return ticket;
 }
 
-// What the last Jacobi pass needs to take the counting sort's tickets.
+// What the last solve launch needs to take the counting sort's tickets.
 struct CountDev {
   uint32_t* counts;         // ncells, zero on entry
   uint32_t* tile_sums;      // one per tile of 2^tile_shift cells, zero on entry

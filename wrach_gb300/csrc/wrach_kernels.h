@@ -30,7 +30,7 @@ struct SolveArgs {
   uint32_t per_thread;          // extended solve: particles per thread in turn (0 = 1)
   const uint32_t* run_if;       // extended solve: skip the launch when *run_if == 0 (optional)
   float* part;                  // final extended pass: per-block metrics, 8 floats a block (optional)
-  CountDev count;               // final extended pass: take the rebin's tickets (count.ticket set)
+  CountDev count;               // last solve launch: the rebin's tickets (extended: if count.ticket is set)
   // the frame's taking-part particles, compacted (extended physics)
   const uint32_t* ct;           // ncells + 1: capped table
   const uint32_t* tp_cell;      // cell of each compacted particle
@@ -130,7 +130,7 @@ cudaError_t launch_count_sort(const RebinArgs& a, uint32_t big_blocks, cudaStrea
 // The same, one step at a time (steps 0 .. kCountSortSteps - 1: count, scan,
 // scatter, place, large cells); *launched is false for a step that has
 // nothing to do.  Step 0 may be left out when the tickets were taken by the
-// last Jacobi pass (SolveArgs::count).
+// last solve launch (SolveArgs::count).
 constexpr int kCountSortSteps = 5;
 cudaError_t launch_count_sort_step(const RebinArgs& a, int step, uint32_t big_blocks,
                                    cudaStream_t st, bool* launched);

@@ -83,6 +83,33 @@ def test_forward_and_gradients_match_oracle(W):
             assert err < 3e-2, (name, err)
 
 
+@pytest.mark.parametrize("n,shift", [(1, 0), (17, 0), (128, 0), (129, 2), (300, 4), (20011, 0), (40001, 2)])
+def test_gradients_over_tiles(W, n, shift):
+    # tiles of 128 rows, one or several per block, ragged last tiles, and rows
+    # that start at 16-, 8- and 4-byte boundaries.  Tolerance: the gradients
+    # are products of at most three BF16-rounded factors of each kind (weight,
+    # activation, gradient; relative error 2^-9 each) and the derivative's
+    # hardware tanh (2^-11): below 9 * 2^-9 = 1.8e-2 of their norm
+    torch = _torch()
+    rng = np.random.default_rng(11 + n)
+    with _sim(W, (30.0, 30.0), 100) as sim:
+        sim.surrogate_init(0, 16)
+        params = _random_net(rng)
+        sim.surrogate_set_params(params)
+        x = M.bf16(rng.normal(0, 0.7, (n, 64)).astype(np.float32))
+        t = rng.normal(0, 0.3, (n, 2)).astype(np.float32)
+        flat = torch.zeros(n * 64 + shift, dtype=torch.int16, device="cuda")
+        flat[shift:] = torch.from_numpy(M.bf16_bits(x).astype(np.uint16).view(np.int16)).cuda().flatten()
+        dt = torch.from_numpy(t).cuda()
+        torch.cuda.synchronize()
+        g_gpu, l_gpu = sim.surrogate_gradients(flat.data_ptr() + 2 * shift, dt.data_ptr(), n)
+        g_cpu, l_cpu = M.gradients(params, x, t)
+        assert abs(l_gpu - l_cpu) <= 1.8e-2 * l_cpu
+        for name, a, b in zip(("w1", "b1", "w2", "b2", "w3", "b3"), M.unpack(g_gpu), M.unpack(g_cpu)):
+            err = np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-12)
+            assert err < 1.8e-2, (name, err)
+
+
 @pytest.mark.parametrize("n", [1, 127, 128, 129, 70001, 400009])
 def test_tcgen05_forward_matches_mma_forward(W, n):
     # the tcgen05 kernel (tiles of 128 rows in two slots per CTA, accumulators

@@ -100,7 +100,7 @@ void drop_graphs(WrachContext* ctx) {
 void release(WrachContext* ctx) {
   drop_graphs(ctx);
   {
-    void* sp[] = {ctx->sur.params, ctx->sur.grad, ctx->sur.mom1, ctx->sur.mom2, ctx->sur.loss,
+    void* sp[] = {ctx->sur.params, ctx->sur.grad, ctx->sur.mom1, ctx->sur.mom2,
                   ctx->sur.metrics, ctx->sur.bf16, ctx->sur.x, ctx->sur.corr, ctx->sur.tx,
                   ctx->sur.tt, ctx->sur.part, ctx->sur.gate};
     for (void* p : sp) dfree(p);
@@ -119,6 +119,7 @@ void release(WrachContext* ctx) {
     dfree(s.vel);
   }
   if (ctx->gather_h) cudaFreeHost(ctx->gather_h);
+  if (ctx->sur.grad_h) cudaFreeHost(ctx->sur.grad_h);
   if (ctx->fork_ev) cudaEventDestroy(ctx->fork_ev);
   if (ctx->join_ev) cudaEventDestroy(ctx->join_ev);
   if (ctx->counts_ev) cudaEventDestroy(ctx->counts_ev);

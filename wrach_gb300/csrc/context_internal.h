@@ -91,7 +91,9 @@ struct WrachContext {
     bool ready = false;
     wrach::MlpDev m{};
     float *params = nullptr, *grad = nullptr, *mom1 = nullptr, *mom2 = nullptr;
-    float *loss = nullptr, *metrics = nullptr;
+    float *loss = nullptr;           // behind the gradients, in their allocation
+    float *grad_h = nullptr;         // pinned: the gradients and the loss read back
+    float *metrics = nullptr;
     float* part = nullptr;           // per-block metrics of a solve launch (8 floats a block)
     wrach::GateState* gate = nullptr;
     uint16_t* bf16 = nullptr;        // the six BF16 weight arrays

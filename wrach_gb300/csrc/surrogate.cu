@@ -55,15 +55,13 @@ __device__ __forceinline__ float tanh_hw(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float gelu(float x) {
-  const float t = tanh_hw(kGeluC * x * (1.0f + kGeluA * x * x));
-  return 0.5f * x * (1.0f + t);
-}
-// d/dx: 0.5 (1 + t) + 0.5 x (1 - t^2) c (1 + 3 a x^2)
-__device__ __forceinline__ float gelu_grad(float x) {
-  const float x2 = x * x;
+// Returns GELU(x) and turns x into the derivative there,
+// 0.5 (1 + t) + 0.5 x (1 - t^2) c (1 + 3 a x^2).
+__device__ __forceinline__ float gelu_and_grad(float& x) {
+  const float x2 = x * x, h = 0.5f * x;
   const float t = tanh_hw(kGeluC * x * (1.0f + kGeluA * x2));
-  return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * kGeluC * (1.0f + 3.0f * kGeluA * x2);
+  x = 0.5f * (1.0f + t) + h * (1.0f - t * t) * kGeluC * (1.0f + 3.0f * kGeluA * x2);
+  return h * (1.0f + t);
 }
 
 // Shared-memory copy of the network for the forward pass: the weights as
@@ -73,20 +71,21 @@ __device__ __forceinline__ float gelu_grad(float x) {
 // 0..3) fall in 32 distinct banks: (36 g + t) mod 32 = 4 g + t.
 constexpr uint32_t kRow = kIn / 2 + 4;
 static_assert(kIn == kHid, "one padded row length serves every layer");
-struct SmemNet {
+struct alignas(16) SmemNet {
   uint32_t w1t[kHid * kRow], w2t[kHid * kRow], w3t[kOutPad * kRow];
   float b1[kHid], b2[kHid], b3[kOutPad];
 };
 // The [in][out] copies the backward pass multiplies the gradients by.
-struct SmemNetT {
-  uint32_t w1[kIn * kRow], w2[kHid * kRow], w3[kHid * kOutPad / 2];
+struct alignas(16) SmemNetT {
+  uint32_t w2[kHid * kRow], w3[kHid * kOutPad / 2];
 };
 
-// rows x 32 words from a packed global array into padded shared rows
+// rows x 64 BF16 from a packed global array into padded shared rows, 16
+// bytes at a time (both sides are 16-byte aligned: kRow words are 144 bytes)
 __device__ __forceinline__ void load_rows(uint32_t* dst, const uint16_t* src, uint32_t rows) {
-  const uint32_t* s = reinterpret_cast<const uint32_t*>(src);
-  for (uint32_t i = threadIdx.x; i < rows * (kIn / 2); i += blockDim.x)
-    dst[(i / (kIn / 2)) * kRow + i % (kIn / 2)] = s[i];
+  const uint4* s = reinterpret_cast<const uint4*>(src);
+  for (uint32_t i = threadIdx.x; i < rows * (kIn / 8); i += blockDim.x)
+    *reinterpret_cast<uint4*>(dst + (i / (kIn / 8)) * kRow + (i % (kIn / 8)) * 4) = s[i];
 }
 
 __device__ void load_net(const MlpDev& m, SmemNet& s, SmemNetT* st) {
@@ -94,7 +93,6 @@ __device__ void load_net(const MlpDev& m, SmemNet& s, SmemNetT* st) {
   load_rows(s.w2t, m.w2t, kHid);
   load_rows(s.w3t, m.w3t, kOutPad);
   if (st) {
-    load_rows(st->w1, m.w1, kIn);
     load_rows(st->w2, m.w2, kHid);
     for (uint32_t i = threadIdx.x; i < kHid * kOutPad / 2; i += blockDim.x)
       st->w3[i] = reinterpret_cast<const uint32_t*>(m.w3)[i];
@@ -117,61 +115,48 @@ __device__ __forceinline__ void bfrag(const uint32_t* wt, uint32_t kk, uint32_t 
   b1 = wt[row + kk * 8 + 4 + t];
 }
 
-// Forward pass of one 16-row tile held by a warp.  `ax` is the A fragment of
-// the input (4 k-tiles).  Writes the pre-activations z1, z2 (C layout, 8
-// n-tiles), the A fragments h1, h2 of the activations and the output y
-// (one n-tile).
+// Forward pass of one 16-row tile held by a warp, for training.  `ax` is the A
+// fragment of the input (4 k-tiles).  Writes the A fragments h1, h2 of the
+// activations, the GELU's derivatives z1, z2 at the pre-activations (C
+// layout, 8 n-tiles) and the output y (one n-tile).
+__device__ __forceinline__ void hidden_layer(const uint32_t* wt, const float* b, uint32_t lane,
+                                             const uint32_t (&in)[4][4], float (&z)[8][4],
+                                             uint32_t (&h)[4][4]) {
+  const uint32_t t = lane & 3;
+#pragma unroll
+  for (uint32_t nt = 0; nt < 8; ++nt) {
+    const float bl = b[nt * 8 + 2 * t], bh = b[nt * 8 + 2 * t + 1];
+    z[nt][0] = bl; z[nt][1] = bh; z[nt][2] = bl; z[nt][3] = bh;
+#pragma unroll
+    for (uint32_t kk = 0; kk < 4; ++kk) {
+      uint32_t b0, b1;
+      bfrag(wt, kk, nt, lane, b0, b1);
+      mma_bf16(z[nt], in[kk], b0, b1);
+    }
+  }
+#pragma unroll
+  for (uint32_t nt = 0; nt < 8; ++nt) {
+    const float g0 = gelu_and_grad(z[nt][0]), g1 = gelu_and_grad(z[nt][1]);
+    const float g2 = gelu_and_grad(z[nt][2]), g3 = gelu_and_grad(z[nt][3]);
+    h[nt / 2][2 * (nt & 1)] = pack_bf16(g0, g1);
+    h[nt / 2][2 * (nt & 1) + 1] = pack_bf16(g2, g3);
+  }
+}
 __device__ __forceinline__ void mlp_tile_forward(const SmemNet& s, uint32_t lane,
                                                  const uint32_t (&ax)[4][4],
                                                  float (&z1)[8][4], uint32_t (&h1)[4][4],
                                                  float (&z2)[8][4], uint32_t (&h2)[4][4],
                                                  float (&y)[4]) {
   const uint32_t t = lane & 3;
-#pragma unroll
-  for (uint32_t nt = 0; nt < 8; ++nt) {
-    const float bl = s.b1[nt * 8 + 2 * t], bh = s.b1[nt * 8 + 2 * t + 1];
-    z1[nt][0] = bl; z1[nt][1] = bh; z1[nt][2] = bl; z1[nt][3] = bh;
-#pragma unroll
-    for (uint32_t kk = 0; kk < 4; ++kk) {
-      uint32_t b0, b1;
-      bfrag(s.w1t, kk, nt, lane, b0, b1);
-      mma_bf16(z1[nt], ax[kk], b0, b1);
-    }
-  }
+  hidden_layer(s.w1t, s.b1, lane, ax, z1, h1);
+  hidden_layer(s.w2t, s.b2, lane, h1, z2, h2);
+  const float bl = s.b3[2 * t], bh = s.b3[2 * t + 1];
+  y[0] = bl; y[1] = bh; y[2] = bl; y[3] = bh;
 #pragma unroll
   for (uint32_t kk = 0; kk < 4; ++kk) {
-    h1[kk][0] = pack_bf16(gelu(z1[2 * kk][0]), gelu(z1[2 * kk][1]));
-    h1[kk][1] = pack_bf16(gelu(z1[2 * kk][2]), gelu(z1[2 * kk][3]));
-    h1[kk][2] = pack_bf16(gelu(z1[2 * kk + 1][0]), gelu(z1[2 * kk + 1][1]));
-    h1[kk][3] = pack_bf16(gelu(z1[2 * kk + 1][2]), gelu(z1[2 * kk + 1][3]));
-  }
-#pragma unroll
-  for (uint32_t nt = 0; nt < 8; ++nt) {
-    const float bl = s.b2[nt * 8 + 2 * t], bh = s.b2[nt * 8 + 2 * t + 1];
-    z2[nt][0] = bl; z2[nt][1] = bh; z2[nt][2] = bl; z2[nt][3] = bh;
-#pragma unroll
-    for (uint32_t kk = 0; kk < 4; ++kk) {
-      uint32_t b0, b1;
-      bfrag(s.w2t, kk, nt, lane, b0, b1);
-      mma_bf16(z2[nt], h1[kk], b0, b1);
-    }
-  }
-#pragma unroll
-  for (uint32_t kk = 0; kk < 4; ++kk) {
-    h2[kk][0] = pack_bf16(gelu(z2[2 * kk][0]), gelu(z2[2 * kk][1]));
-    h2[kk][1] = pack_bf16(gelu(z2[2 * kk][2]), gelu(z2[2 * kk][3]));
-    h2[kk][2] = pack_bf16(gelu(z2[2 * kk + 1][0]), gelu(z2[2 * kk + 1][1]));
-    h2[kk][3] = pack_bf16(gelu(z2[2 * kk + 1][2]), gelu(z2[2 * kk + 1][3]));
-  }
-  {
-    const float bl = s.b3[2 * t], bh = s.b3[2 * t + 1];
-    y[0] = bl; y[1] = bh; y[2] = bl; y[3] = bh;
-#pragma unroll
-    for (uint32_t kk = 0; kk < 4; ++kk) {
-      uint32_t b0, b1;
-      bfrag(s.w3t, kk, 0, lane, b0, b1);
-      mma_bf16(y, h2[kk], b0, b1);
-    }
+    uint32_t b0, b1;
+    bfrag(s.w3t, kk, 0, lane, b0, b1);
+    mma_bf16(y, h2[kk], b0, b1);
   }
 }
 
@@ -275,246 +260,270 @@ __global__ void __launch_bounds__(128) k_mlp_forward(MlpDev m, const uint16_t* _
   }
 }
 
-// Per-warp scratch of the backward pass: activations and gradients of one
-// tile stored transposed ([feature][row], rows contiguous) as BF16 pairs, the
-// A operand layout of the weight-gradient products X^T dZ1, H1^T dZ2, H2^T dY.
-struct SmemBack {
-  uint16_t xt[kIn][16], h1t[kHid][16], h2t[kHid][16];
-  uint16_t dz1t[kHid][16], dz2t[kHid][16], dyt[kOutPad][16];
-};
+// ---------------------------------------------------------------------------
+// Training
+// ---------------------------------------------------------------------------
 
-// Accumulators of the block: FP32 gradients, in the parameter order.
-struct SmemGrad {
-  float w1[kIn * kHid], b1[kHid], w2[kHid * kHid], b2[kHid], w3[kHid * kOutPad], b3[kOutPad];
-};
-static_assert(sizeof(SmemGrad) == kMlpParams * sizeof(float), "gradient order = parameters");
+// A block of 8 warps takes tiles of 128 rows.  First each warp runs 16 of the
+// rows forward and backward and leaves their activations and gradients in
+// shared memory as BF16, [row][feature] in padded rows.  Then the warps share
+// out the weight gradients X^T dZ1, H1^T dZ2 and H2^T dY, contractions over
+// the tile's rows: warp w owns input features 16 (w mod 4) .. + 15 and one
+// half of the outputs of each product, and keeps those sums in its registers
+// over all of the block's tiles (the transposed operands come from
+// ldmatrix.trans).  What it waits for is latency (of the weights' loads, the
+// two layers and the final sums into global memory): 16,384 rows are 128
+// blocks of one tile.  Before, each warp added every 16-row product into
+// shared memory with atomics, 272 of them a tile, and 4 warps filled an SM's
+// shared memory: 61 us then, 15 us now (16,384 rows).
+constexpr uint32_t kTrainRows = 128, kTrainThreads = 256;
 
-__device__ __forceinline__ uint16_t bf16_bits(float v) {
-  __nv_bfloat16 b = __float2bfloat16_rn(v);
-  return *reinterpret_cast<uint16_t*>(&b);
+struct SmemTile {
+  uint32_t x[kTrainRows * kRow], h1[kTrainRows * kRow], h2[kTrainRows * kRow];
+  uint32_t dz1[kTrainRows * kRow], dz2[kTrainRows * kRow];
+  uint32_t dy[kTrainRows * kOutPad / 2];
+};
+struct SmemTrain {
+  SmemNet net;
+  SmemNetT t;
+  SmemTile tile;
+};
+static_assert(sizeof(SmemNet) % 16 == 0 && sizeof(SmemNetT) % 16 == 0, "16-byte rows");
+
+// Four (two) 8x8 BF16 matrices from shared memory; lane l gives the address of
+// row l mod 8 of matrix l / 8.
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm2t(uint32_t& r0, uint32_t& r1, const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
+               : "=r"(r0), "=r"(r1)
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
 }
 
-// Scatter a C-layout tile (8 n-tiles of 16x8) into a transposed BF16 array.
-__device__ __forceinline__ void store_ct(uint16_t (*dst)[16], const float (&c)[8][4],
-                                         uint32_t lane) {
+// A fragments of 16 rows (4 k-tiles) into padded rows, row0 the first.
+__device__ __forceinline__ void store_a(uint32_t* dst, uint32_t row0, uint32_t lane,
+                                        const uint32_t (&a)[4][4]) {
   const uint32_t g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (uint32_t nt = 0; nt < 8; ++nt) {
-    const uint32_t col = nt * 8 + 2 * t;
-    dst[col][g] = bf16_bits(c[nt][0]);
-    dst[col + 1][g] = bf16_bits(c[nt][1]);
-    dst[col][g + 8] = bf16_bits(c[nt][2]);
-    dst[col + 1][g + 8] = bf16_bits(c[nt][3]);
-  }
-}
-
-// Scatter an A-layout BF16 tile (4 k-tiles) into a transposed array.
-__device__ __forceinline__ void store_at(uint16_t (*dst)[16], const uint32_t (&a)[4][4],
-                                         uint32_t lane) {
-  const uint32_t g = lane >> 2, t = lane & 3;
+  uint32_t* p0 = dst + (row0 + g) * kRow + t;
+  uint32_t* p1 = p0 + 8 * kRow;
 #pragma unroll
   for (uint32_t kk = 0; kk < 4; ++kk) {
-    const uint32_t c0 = kk * 16 + 2 * t, c1 = c0 + 8;
-    dst[c0][g] = (uint16_t)(a[kk][0] & 0xFFFF);
-    dst[c0 + 1][g] = (uint16_t)(a[kk][0] >> 16);
-    dst[c0][g + 8] = (uint16_t)(a[kk][1] & 0xFFFF);
-    dst[c0 + 1][g + 8] = (uint16_t)(a[kk][1] >> 16);
-    dst[c1][g] = (uint16_t)(a[kk][2] & 0xFFFF);
-    dst[c1 + 1][g] = (uint16_t)(a[kk][2] >> 16);
-    dst[c1][g + 8] = (uint16_t)(a[kk][3] & 0xFFFF);
-    dst[c1 + 1][g + 8] = (uint16_t)(a[kk][3] >> 16);
+    p0[kk * 8] = a[kk][0];
+    p1[kk * 8] = a[kk][1];
+    p0[kk * 8 + 4] = a[kk][2];
+    p1[kk * 8 + 4] = a[kk][3];
   }
 }
 
-// dW[m][n] += sum over the 16 rows of AT[m][row] * BT[n][row] for m in
-// [0, mdim), n in [0, ndim): the tile's weight-gradient product on the
-// tensor cores (K = 16 rows), added into the block's FP32 accumulator.
-__device__ __forceinline__ void grad_product(const uint16_t (*at)[16], uint32_t mdim,
-                                             const uint16_t (*bt)[16], uint32_t ndim,
-                                             float* acc, uint32_t lane) {
-  const uint32_t g = lane >> 2, t = lane & 3;
-  for (uint32_t mt = 0; mt < mdim / 16; ++mt) {
-    uint32_t a[4];
-    a[0] = *reinterpret_cast<const uint32_t*>(&at[mt * 16 + g][2 * t]);
-    a[1] = *reinterpret_cast<const uint32_t*>(&at[mt * 16 + g + 8][2 * t]);
-    a[2] = *reinterpret_cast<const uint32_t*>(&at[mt * 16 + g][2 * t + 8]);
-    a[3] = *reinterpret_cast<const uint32_t*>(&at[mt * 16 + g + 8][2 * t + 8]);
-    for (uint32_t nt = 0; nt < ndim / 8; ++nt) {
-      const uint32_t b0 = *reinterpret_cast<const uint32_t*>(&bt[nt * 8 + g][2 * t]);
-      const uint32_t b1 = *reinterpret_cast<const uint32_t*>(&bt[nt * 8 + g][2 * t + 8]);
-      float d[4] = {0.f, 0.f, 0.f, 0.f};
-      mma_bf16(d, a, b0, b1);
-      const uint32_t m0 = mt * 16 + g, n0 = nt * 8 + 2 * t;
-      atomicAdd(&acc[m0 * ndim + n0], d[0]);
-      atomicAdd(&acc[m0 * ndim + n0 + 1], d[1]);
-      atomicAdd(&acc[(m0 + 8) * ndim + n0], d[2]);
-      atomicAdd(&acc[(m0 + 8) * ndim + n0 + 1], d[3]);
-    }
+// A C-layout tile (8 n-tiles of 16x8) as the A fragment of the next product.
+__device__ __forceinline__ void to_a(uint32_t (&a)[4][4], const float (&c)[8][4]) {
+#pragma unroll
+  for (uint32_t kk = 0; kk < 4; ++kk) {
+    a[kk][0] = pack_bf16(c[2 * kk][0], c[2 * kk][1]);
+    a[kk][1] = pack_bf16(c[2 * kk][2], c[2 * kk][3]);
+    a[kk][2] = pack_bf16(c[2 * kk + 1][0], c[2 * kk + 1][1]);
+    a[kk][3] = pack_bf16(c[2 * kk + 1][2], c[2 * kk + 1][3]);
   }
+}
+
+// acc (4 n-tiles from column n0) += AT^T BT over the tile's rows, AT the
+// columns m0 .. m0 + 15 of `at`.
+__device__ __forceinline__ void rows_product(float (&acc)[4][4], const uint32_t* at,
+                                             const uint32_t* bt, uint32_t m0, uint32_t n0,
+                                             uint32_t lane) {
+  const uint32_t mi = lane >> 3, r = lane & 7;
+  // A: matrices (k 0-7, m 0-7), (k 0-7, m 8-15), (k 8-15, m 0-7), (k 8-15, m 8-15)
+  const uint32_t* pa = at + ((mi >> 1) * 8 + r) * kRow + (m0 + (mi & 1) * 8) / 2;
+  // B: matrices (k 0-7, n 0-7), (k 8-15, n 0-7), (k 0-7, n 8-15), (k 8-15, n 8-15)
+  const uint32_t* pb = bt + ((mi & 1) * 8 + r) * kRow + (n0 + (mi >> 1) * 8) / 2;
+#pragma unroll
+  for (uint32_t ks = 0; ks < kTrainRows / 16; ++ks) {
+    uint32_t a[4], b[4], c[4];
+    ldsm4t(a, pa + ks * 16 * kRow);
+    ldsm4t(b, pb + ks * 16 * kRow);
+    ldsm4t(c, pb + ks * 16 * kRow + 8);
+    mma_bf16(acc[0], a, b[0], b[1]);
+    mma_bf16(acc[1], a, b[2], b[3]);
+    mma_bf16(acc[2], a, c[0], c[1]);
+    mma_bf16(acc[3], a, c[2], c[3]);
+  }
+}
+
+// A 16x8 tile of sums (C layout) into the row-major matrix w of `ld` columns.
+__device__ __forceinline__ void add_tile(float* w, uint32_t ld, uint32_t m0, uint32_t n0,
+                                         const float (&c)[4], uint32_t lane) {
+  const uint32_t g = lane >> 2, t = lane & 3;
+  float* p = w + (m0 + g) * ld + n0 + 2 * t;
+  atomicAdd(reinterpret_cast<float2*>(p), make_float2(c[0], c[1]));
+  atomicAdd(reinterpret_cast<float2*>(p + 8 * ld), make_float2(c[2], c[3]));
 }
 
 // Gradients of L = 0.5 * sum over rows and the 2 outputs of (y - target)^2 /
 // `scale_rows` with respect to every parameter, added into `grad` (FP32,
 // the MlpDev parameter order: w1 [in][out], b1, w2, b2, w3 [in][8], b3).
 // Also adds the loss into *loss.
-__global__ void __launch_bounds__(128) k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x,
-                                                      const float2* __restrict__ target,
-                                                      uint32_t n, float inv_rows,
-                                                      float* __restrict__ grad,
-                                                      float* __restrict__ loss) {
+__global__ void __launch_bounds__(kTrainThreads, 1)
+k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restrict__ target,
+               uint32_t n, float inv_rows, float* __restrict__ grad, float* __restrict__ loss) {
   extern __shared__ __align__(16) uint8_t dyn[];
-  SmemNet& s = *reinterpret_cast<SmemNet*>(dyn);
-  SmemNetT& st = *reinterpret_cast<SmemNetT*>(dyn + sizeof(SmemNet));
-  SmemGrad& acc = *reinterpret_cast<SmemGrad*>(dyn + sizeof(SmemNet) + sizeof(SmemNetT));
-  SmemBack* back =
-      reinterpret_cast<SmemBack*>(dyn + sizeof(SmemNet) + sizeof(SmemNetT) + sizeof(SmemGrad));
-  load_net(m, s, &st);
-  float* accf = reinterpret_cast<float*>(&acc);
-  for (uint32_t i = threadIdx.x; i < sizeof(SmemGrad) / 4; i += blockDim.x) accf[i] = 0.f;
-  __syncthreads();
+  SmemTrain& sm = *reinterpret_cast<SmemTrain*>(dyn);
+  SmemTile& st = sm.tile;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t g = lane >> 2, t = lane & 3;
-  SmemBack& sb = back[warp];
-  float lsum = 0.f;
-  const uint32_t tiles = (n + 15) / 16;
-  for (uint32_t tile = blockIdx.x * 4 + warp; tile < tiles; tile += gridDim.x * 4) {
-    uint32_t ax[4][4], h1[4][4], h2[4][4];
+  const uint32_t row0 = warp * 16, m0 = (warp & 3) * 16, n0 = (warp >> 2) * 32;
+  float acc1[4][4] = {}, acc2[4][4] = {}, acc3[4] = {};
+  float sb1[8][2] = {}, sb2[8][2] = {}, sb3[2] = {}, lsum = 0.f;
+  const uint32_t tiles = (n + kTrainRows - 1) / kTrainRows;
+  // a caller's rows may start at any 4-byte boundary
+  const bool x16 = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+  for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    // the tile's features (rows past n are zero); the network with the first
+    const uint32_t base = tile * kTrainRows;
+    for (uint32_t i = threadIdx.x; i < kTrainRows * (kIn / 8); i += kTrainThreads) {
+      const uint32_t r = i / (kIn / 8), c = i % (kIn / 8);
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (base + r < n) {
+        const uint16_t* p = x + (size_t)(base + r) * kIn + c * 8;
+        if (x16) {
+          v = *reinterpret_cast<const uint4*>(p);
+        } else {
+          const uint32_t* w = reinterpret_cast<const uint32_t*>(p);
+          v = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
+      *reinterpret_cast<uint4*>(st.x + r * kRow + c * 4) = v;
+    }
+    const uint32_t r0 = base + row0 + g, r1 = r0 + 8;
+    float2 tg0 = make_float2(0.f, 0.f), tg1 = tg0;
+    if (t == 0 && r0 < n) tg0 = target[r0];
+    if (t == 0 && r1 < n) tg1 = target[r1];
+    if (tile == blockIdx.x)
+      load_net(m, sm.net, &sm.t);
+    else
+      __syncthreads();
+
+    uint32_t a[4][4], h1[4][4], h2[4][4];
     float z1[8][4], z2[8][4], y[4];
-    load_x_tile(x, tile * 16, n, lane, ax);
-    mlp_tile_forward(s, lane, ax, z1, h1, z2, h2, y);
+#pragma unroll
+    for (uint32_t kk = 0; kk < 4; ++kk)
+      ldsm4(a[kk], st.x + (row0 + (lane & 15)) * kRow + kk * 8 + (lane >> 4) * 4);
+    mlp_tile_forward(sm.net, lane, a, z1, h1, z2, h2, y);
+    store_a(st.h1, row0, lane, h1);
+    store_a(st.h2, row0, lane, h2);
     // dY (C layout, one n-tile; only columns 0 and 1 are real outputs)
-    const uint32_t r0 = tile * 16 + g, r1 = r0 + 8;
     float dy[4] = {0.f, 0.f, 0.f, 0.f};
     if (t == 0) {
       if (r0 < n) {
-        const float2 tg = target[r0];
-        const float e0 = y[0] - tg.x, e1 = y[1] - tg.y;
+        const float e0 = y[0] - tg0.x, e1 = y[1] - tg0.y;
         lsum += 0.5f * (e0 * e0 + e1 * e1);
         dy[0] = e0 * inv_rows;
         dy[1] = e1 * inv_rows;
       }
       if (r1 < n) {
-        const float2 tg = target[r1];
-        const float e0 = y[2] - tg.x, e1 = y[3] - tg.y;
+        const float e0 = y[2] - tg1.x, e1 = y[3] - tg1.y;
         lsum += 0.5f * (e0 * e0 + e1 * e1);
         dy[2] = e0 * inv_rows;
         dy[3] = e1 * inv_rows;
       }
     }
+    sb3[0] += dy[0] + dy[2];
+    sb3[1] += dy[1] + dy[3];
     // dH2 = dY W3^T  (K = 8 outputs padded to 16 with zeros)
-    uint32_t ady[4];
-    ady[0] = pack_bf16(dy[0], dy[1]);
-    ady[1] = pack_bf16(dy[2], dy[3]);
-    ady[2] = 0u;
-    ady[3] = 0u;
-    float dz2[8][4];
+    const uint32_t ady[4] = {pack_bf16(dy[0], dy[1]), pack_bf16(dy[2], dy[3]), 0u, 0u};
+    st.dy[(row0 + g) * (kOutPad / 2) + t] = ady[0];
+    st.dy[(row0 + g + 8) * (kOutPad / 2) + t] = ady[1];
 #pragma unroll
     for (uint32_t nt = 0; nt < 8; ++nt) {
-      dz2[nt][0] = dz2[nt][1] = dz2[nt][2] = dz2[nt][3] = 0.f;
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
       // B(k = out, n = in) = W3[in][out]; W3 stored [in][8]
-      const uint32_t b0 = st.w3[(nt * 8 + g) * (kOutPad / 2) + t];
-      mma_bf16(dz2[nt], ady, b0, 0u);
+      mma_bf16(d, ady, sm.t.w3[(nt * 8 + g) * (kOutPad / 2) + t], 0u);
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) z2[nt][q] = d[q] * z2[nt][q];
+      sb2[nt][0] += z2[nt][0] + z2[nt][2];
+      sb2[nt][1] += z2[nt][1] + z2[nt][3];
     }
-#pragma unroll
-    for (uint32_t nt = 0; nt < 8; ++nt)
-#pragma unroll
-      for (uint32_t q = 0; q < 4; ++q) dz2[nt][q] *= gelu_grad(z2[nt][q]);
     // dH1 = dZ2 W2^T
-    uint32_t adz2[4][4];
-#pragma unroll
-    for (uint32_t kk = 0; kk < 4; ++kk) {
-      adz2[kk][0] = pack_bf16(dz2[2 * kk][0], dz2[2 * kk][1]);
-      adz2[kk][1] = pack_bf16(dz2[2 * kk][2], dz2[2 * kk][3]);
-      adz2[kk][2] = pack_bf16(dz2[2 * kk + 1][0], dz2[2 * kk + 1][1]);
-      adz2[kk][3] = pack_bf16(dz2[2 * kk + 1][2], dz2[2 * kk + 1][3]);
-    }
-    float dz1[8][4];
+    to_a(a, z2);
+    store_a(st.dz2, row0, lane, a);
 #pragma unroll
     for (uint32_t nt = 0; nt < 8; ++nt) {
-      dz1[nt][0] = dz1[nt][1] = dz1[nt][2] = dz1[nt][3] = 0.f;
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (uint32_t kk = 0; kk < 4; ++kk) {
         uint32_t b0, b1;
-        bfrag(st.w2, kk, nt, lane, b0, b1);  // W2 [in][out]: B(k=out, n=in)
-        mma_bf16(dz1[nt], adz2[kk], b0, b1);
+        bfrag(sm.t.w2, kk, nt, lane, b0, b1);  // W2 [in][out]: B(k=out, n=in)
+        mma_bf16(d, a[kk], b0, b1);
+      }
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) z1[nt][q] = d[q] * z1[nt][q];
+      sb1[nt][0] += z1[nt][0] + z1[nt][2];
+      sb1[nt][1] += z1[nt][1] + z1[nt][3];
+    }
+    to_a(a, z1);
+    store_a(st.dz1, row0, lane, a);
+    __syncthreads();
+    // the weight gradients' products over the tile's rows
+    rows_product(acc1, st.x, st.dz1, m0, n0, lane);
+    rows_product(acc2, st.h1, st.dz2, m0, n0, lane);
+    if (n0 == 0) {
+      const uint32_t mi = lane >> 3, r = lane & 7;
+#pragma unroll
+      for (uint32_t ks = 0; ks < kTrainRows / 16; ++ks) {
+        uint32_t b[4], b0, b1;
+        ldsm4t(b, st.h2 + (ks * 16 + (mi >> 1) * 8 + r) * kRow + (m0 + (mi & 1) * 8) / 2);
+        ldsm2t(b0, b1, st.dy + (ks * 16 + (mi & 1) * 8 + r) * (kOutPad / 2));
+        mma_bf16(acc3, b, b0, b1);
       }
     }
+    __syncthreads();
+  }
+  // the block's sums into global memory
+  const uint32_t o_b1 = kIn * kHid, o_w2 = o_b1 + kHid, o_b2 = o_w2 + kHid * kHid;
+  const uint32_t o_w3 = o_b2 + kHid, o_b3 = o_w3 + kHid * kOutPad;
+#pragma unroll
+  for (uint32_t u = 0; u < 4; ++u) {
+    add_tile(grad, kHid, m0, n0 + u * 8, acc1[u], lane);
+    add_tile(grad + o_w2, kHid, m0, n0 + u * 8, acc2[u], lane);
+  }
+  if (n0 == 0) add_tile(grad + o_w3, kOutPad, m0, 0, acc3, lane);
+  // bias gradients: the columns' sums over the rows a warp's lanes hold
+#pragma unroll
+  for (uint32_t o = 4; o < 32; o <<= 1) {
 #pragma unroll
     for (uint32_t nt = 0; nt < 8; ++nt)
 #pragma unroll
-      for (uint32_t q = 0; q < 4; ++q) dz1[nt][q] *= gelu_grad(z1[nt][q]);
-
-    // bias gradients: column sums over the tile's rows
+      for (uint32_t u = 0; u < 2; ++u) {
+        sb1[nt][u] += __shfl_xor_sync(0xffffffffu, sb1[nt][u], o);
+        sb2[nt][u] += __shfl_xor_sync(0xffffffffu, sb2[nt][u], o);
+      }
+#pragma unroll
+    for (uint32_t u = 0; u < 2; ++u) sb3[u] += __shfl_xor_sync(0xffffffffu, sb3[u], o);
+    lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+  }
+  if (g == 0) {
 #pragma unroll
     for (uint32_t nt = 0; nt < 8; ++nt) {
-      float s2a = dz2[nt][0] + dz2[nt][2], s2b = dz2[nt][1] + dz2[nt][3];
-      float s1a = dz1[nt][0] + dz1[nt][2], s1b = dz1[nt][1] + dz1[nt][3];
-#pragma unroll
-      for (uint32_t o = 4; o < 32; o <<= 1) {
-        s2a += __shfl_xor_sync(0xffffffffu, s2a, o);
-        s2b += __shfl_xor_sync(0xffffffffu, s2b, o);
-        s1a += __shfl_xor_sync(0xffffffffu, s1a, o);
-        s1b += __shfl_xor_sync(0xffffffffu, s1b, o);
-      }
-      if (g == 0) {
-        atomicAdd(&acc.b2[nt * 8 + 2 * t], s2a);
-        atomicAdd(&acc.b2[nt * 8 + 2 * t + 1], s2b);
-        atomicAdd(&acc.b1[nt * 8 + 2 * t], s1a);
-        atomicAdd(&acc.b1[nt * 8 + 2 * t + 1], s1b);
-      }
+      atomicAdd(reinterpret_cast<float2*>(grad + o_b1 + nt * 8 + 2 * t),
+                make_float2(sb1[nt][0], sb1[nt][1]));
+      atomicAdd(reinterpret_cast<float2*>(grad + o_b2 + nt * 8 + 2 * t),
+                make_float2(sb2[nt][0], sb2[nt][1]));
     }
-    {
-      float a0 = dy[0] + dy[2], a1 = dy[1] + dy[3];
-#pragma unroll
-      for (uint32_t o = 4; o < 32; o <<= 1) {
-        a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-      }
-      if (g == 0 && t == 0) {
-        atomicAdd(&acc.b3[0], a0);
-        atomicAdd(&acc.b3[1], a1);
-      }
-    }
-    // weight gradients: X^T dZ1, H1^T dZ2, H2^T dY (K = the tile's 16 rows)
-    store_at(sb.xt, ax, lane);
-    store_at(sb.h1t, h1, lane);
-    store_at(sb.h2t, h2, lane);
-    store_ct(sb.dz1t, dz1, lane);
-    store_ct(sb.dz2t, dz2, lane);
-    {
-      // dY transposed: 8 output columns x 16 rows
-      for (uint32_t c = 0; c < kOutPad; ++c) {
-        sb.dyt[c][g] = 0;
-        sb.dyt[c][g + 8] = 0;
-      }
-      __syncwarp();
-      if (t == 0) {
-        sb.dyt[0][g] = bf16_bits(dy[0]);
-        sb.dyt[1][g] = bf16_bits(dy[1]);
-        sb.dyt[0][g + 8] = bf16_bits(dy[2]);
-        sb.dyt[1][g + 8] = bf16_bits(dy[3]);
-      }
-    }
-    __syncwarp();
-    grad_product(sb.xt, kIn, sb.dz1t, kHid, acc.w1, lane);
-    grad_product(sb.h1t, kHid, sb.dz2t, kHid, acc.w2, lane);
-    grad_product(sb.h2t, kHid, sb.dyt, kOutPad, acc.w3, lane);
-    __syncwarp();
   }
-  // the tile losses of the warp, then the block's gradients into global
-#pragma unroll
-  for (uint32_t o = 1; o < 32; o <<= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-  if (lane == 0 && lsum != 0.f) atomicAdd(loss, lsum * inv_rows);
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < sizeof(SmemGrad) / 4; i += blockDim.x)
-    if (accf[i] != 0.f) atomicAdd(&grad[i], accf[i]);
+  if (lane == 0) {
+    atomicAdd(reinterpret_cast<float2*>(grad + o_b3), make_float2(sb3[0], sb3[1]));
+    if (lsum != 0.f) atomicAdd(loss, lsum * inv_rows);
+  }
 }
 
-size_t backward_smem() {
-  return sizeof(SmemNet) + sizeof(SmemNetT) + sizeof(SmemGrad) + 4 * sizeof(SmemBack);
-}
-
-// Adam on the FP32 master parameters (the SmemGrad order), then the BF16
+// Adam on the FP32 master parameters (the order above), then the BF16
 // copies in both layouts.
 __global__ void k_adam(MlpDev m, const float* __restrict__ grad, float* __restrict__ mom1,
                        float* __restrict__ mom2, float lr, float b1, float b2, float eps,
@@ -995,17 +1004,18 @@ cudaError_t launch_mlp_forward(const MlpDev& m, const uint16_t* x, uint32_t n, f
   return cudaGetLastError();
 }
 
+bool train_setup() {
+  return cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)sizeof(SmemTrain)) == cudaSuccess;
+}
+
 cudaError_t launch_mlp_backward(const MlpDev& m, const uint16_t* x, const float2* target,
-                                uint32_t n, float inv_rows, float* grad, float* loss, int blocks,
+                                uint32_t n, float inv_rows, float* grad, float* loss, int sms,
                                 cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  const size_t smem = backward_smem();
-  cudaError_t e = cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
-  if (e != cudaSuccess) return e;
-  const int need = (int)((n + 63) / 64);
-  k_mlp_backward<<<need < blocks ? need : blocks, 128, smem, st>>>(m, x, target, n, inv_rows,
-                                                                   grad, loss);
+  const uint32_t tiles = (n + kTrainRows - 1) / kTrainRows, most = sms > 0 ? sms : 1;
+  k_mlp_backward<<<tiles < most ? tiles : most, kTrainThreads, sizeof(SmemTrain), st>>>(
+      m, x, target, n, inv_rows, grad, loss);
   return cudaGetLastError();
 }
 

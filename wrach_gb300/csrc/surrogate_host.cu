@@ -143,10 +143,12 @@ int wrach_surrogate_init(WrachContext* ctx, uint32_t seed, uint32_t max_samples)
   if (!S.ready) {
     const size_t nbf = (size_t)2 * (2 * kMlpIn * kMlpHidden + kMlpHidden * kMlpOutPad);
     CK(dalloc(&S.params, kMlpParams));
-    CK(dalloc(&S.grad, kMlpParams));
+    // the gradients and, behind them, the loss: cleared and read back as one
+    CK(dalloc(&S.grad, kMlpParams + 1));
+    S.loss = S.grad + kMlpParams;
+    CK(cudaMallocHost(reinterpret_cast<void**>(&S.grad_h), (kMlpParams + 1) * sizeof(float)));
     CK(dalloc(&S.mom1, kMlpParams));
     CK(dalloc(&S.mom2, kMlpParams));
-    CK(dalloc(&S.loss, 1));
     CK(dalloc(&S.metrics, 8));
     CK(dalloc(&S.bf16, nbf));
     CK(dalloc(&S.x, (size_t)ctx->total_cap * kMlpIn));
@@ -165,7 +167,7 @@ int wrach_surrogate_init(WrachContext* ctx, uint32_t seed, uint32_t max_samples)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     S.blocks = sms > 0 ? 4 * sms : 64;
     S.correct_blocks = wrach::surrogate_correct_blocks(ctx->device);
-    if (S.correct_blocks <= 0) return fail(ctx, WRACH_ERR_CUDA, "surrogate kernel set-up failed");
+    if (S.correct_blocks <= 0 || !wrach::train_setup()) return fail(ctx, WRACH_ERR_CUDA, "surrogate kernel set-up failed");
   }
   if (max_samples > S.max_samples) {
     dfree(S.tx);
@@ -260,14 +262,15 @@ int wrach_surrogate_gradients(WrachContext* ctx, const uint16_t* d_x, const floa
   if (!n || !d_x || !d_t || !grad || !loss) return WRACH_ERR_INVALID_ARGUMENT;
   DeviceGuard guard(ctx->device);
   auto& S = ctx->sur;
-  CK(cudaMemsetAsync(S.grad, 0, wrach::kMlpParams * 4, ctx->stream));
-  CK(cudaMemsetAsync(S.loss, 0, 4, ctx->stream));
+  CK(cudaMemsetAsync(S.grad, 0, (wrach::kMlpParams + 1) * 4, ctx->stream));
   CK(wrach::launch_mlp_backward(S.m, d_x, reinterpret_cast<const float2*>(d_t), n, 1.0f / n, S.grad,
-                                S.loss, S.blocks, ctx->stream));
+                                S.loss, ctx->sms, ctx->stream));
   ctx->launches += 1;
-  CK(cudaMemcpyAsync(grad, S.grad, wrach::kMlpParams * 4, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(loss, S.loss, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaMemcpyAsync(S.grad_h, S.grad, (wrach::kMlpParams + 1) * 4, cudaMemcpyDeviceToHost,
+                     ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
+  std::memcpy(grad, S.grad_h, wrach::kMlpParams * 4);
+  *loss = S.grad_h[wrach::kMlpParams];
   return WRACH_OK;
 }
 
@@ -369,10 +372,9 @@ int wrach_surrogate_train(WrachContext* ctx, uint32_t steps, uint32_t batch, flo
     // a window of the sample buffer, spread over it by a multiplicative hash
     const uint32_t span = S.nsamples - b + 1;
     const uint32_t off = (uint32_t)(((uint64_t)(S.step + 1) * 2654435761ull) % span);
-    CK(cudaMemsetAsync(S.grad, 0, wrach::kMlpParams * 4, ctx->stream));
-    CK(cudaMemsetAsync(S.loss, 0, 4, ctx->stream));
+    CK(cudaMemsetAsync(S.grad, 0, (wrach::kMlpParams + 1) * 4, ctx->stream));
     CK(wrach::launch_mlp_backward(S.m, S.tx + (size_t)off * wrach::kMlpIn, S.tt + off, b, 1.0f / b,
-                                  S.grad, S.loss, S.blocks, ctx->stream));
+                                  S.grad, S.loss, ctx->sms, ctx->stream));
     ++S.step;
     CK(wrach::launch_adam(S.m, S.grad, S.mom1, S.mom2, lr, S.step, ctx->stream));
     ctx->launches += 2;

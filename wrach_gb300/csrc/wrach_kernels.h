@@ -227,9 +227,12 @@ cudaError_t launch_mlp_forward(const MlpDev& m, const uint16_t* x, uint32_t n, f
 // kFlagTimeout in *flags.
 cudaError_t launch_mlp_forward_tc(const MlpDev& m, const uint16_t* x, uint32_t n, float2* y,
                                   uint32_t* flags, int sms, cudaStream_t st);
+// One-time set-up of the training kernel on the current device (its shared
+// memory size).
+bool train_setup();
 cudaError_t launch_mlp_backward(const MlpDev& m, const uint16_t* x, const float2* target,
                                 uint32_t n, float inv_rows, float* grad, float* loss,
-                                int blocks, cudaStream_t st);
+                                int sms, cudaStream_t st);
 cudaError_t launch_adam(const MlpDev& m, const float* grad, float* mom1, float* mom2, float lr,
                         uint32_t step, cudaStream_t st);
 // target[i] = q_t - p_i for the first n frame particles, q compacted (zero

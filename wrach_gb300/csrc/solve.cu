@@ -166,31 +166,28 @@ __device__ __forceinline__ Rows tp_rows(const WorldDev& w, const uint32_t* __res
 constexpr uint32_t kStep = 4;
 static_assert(kStep - 1 <= kRowPad, "the iterates are padded for the last step");
 
-// The candidates of row r within reach of the particle at qi2 (a NaN
-// distance counts, as in the reference's test).  Mask holds the bits of a
-// row: 3 * cap + 1.
-template <typename Mask>
-__device__ __forceinline__ Mask row_marks(const PhysDev& ph, const f32x2* __restrict__ q, f32x2 qi2,
-                                          const Rows& R, int r) {
-  const uint32_t s = R.start(r), n = R.length(r), odd = s & 1u;
-  const ulonglong2* p = reinterpret_cast<const ulonglong2*>(q + (s - odd));
-  Mask marks = 0;
-  for (uint32_t k = 0; k < (n ? odd + n : 0u); k += kStep) {
+// One step of a row: the candidates c[0 .. kStep - 1] within reach of the
+// particle at qi2 (a NaN distance counts, as in the reference's test).
+struct RowStep {
+  ulonglong2 c[kStep / 2];
+  __device__ __forceinline__ void load(const f32x2* __restrict__ p) {
+#pragma unroll
+    for (uint32_t u = 0; u < kStep / 2; ++u) c[u] = reinterpret_cast<const ulonglong2*>(p)[u];
+  }
+  __device__ __forceinline__ uint32_t marks(const PhysDev& ph, f32x2 qi2) const {
     uint32_t in = 0;
 #pragma unroll
     for (uint32_t u = 0; u < kStep / 2; ++u) {
-      const ulonglong2 c = p[k / 2 + u];
-      if (!(f2_len2(f2_sub(c.x, qi2)) >= ph.skip_d2)) in |= 1u << (2 * u);
-      if (!(f2_len2(f2_sub(c.y, qi2)) >= ph.skip_d2)) in |= 2u << (2 * u);
+      if (!(f2_len2(f2_sub(c[u].x, qi2)) >= ph.skip_d2)) in |= 1u << (2 * u);
+      if (!(f2_len2(f2_sub(c[u].y, qi2)) >= ph.skip_d2)) in |= 2u << (2 * u);
     }
-    marks |= (Mask)in << k;
+    return in;
   }
-  // the row alone, without the particle itself
-  marks &= (((Mask)1 << n) - 1) << odd;
-  if (r == 1) marks &= ~((Mask)1 << (R.particle() - (s - odd)));
-  return marks;
-}
+};
 
+// The marks of the three rows' candidates.  Mask holds the bits of a row:
+// 3 * cap + 1.  The rows' first steps are loaded together; few rows of sparse
+// frames need a second.
 template <typename Mask>
 struct Marks {
   Mask m[3];
@@ -199,8 +196,23 @@ template <typename Mask>
 __device__ __forceinline__ Marks<Mask> all_marks(const PhysDev& ph, const f32x2* __restrict__ q,
                                                  f32x2 qi2, const Rows& R) {
   Marks<Mask> M;
+  RowStep first[3];
 #pragma unroll
-  for (int r = 0; r < 3; ++r) M.m[r] = row_marks<Mask>(ph, q, qi2, R, r);
+  for (int r = 0; r < 3; ++r) first[r].load(q + (R.start(r) & ~1u));
+#pragma unroll
+  for (int r = 0; r < 3; ++r) M.m[r] = first[r].marks(ph, qi2);
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    const uint32_t s = R.start(r), n = R.length(r), odd = s & 1u;
+    for (uint32_t k = kStep; k < odd + n; k += kStep) {
+      RowStep more;
+      more.load(q + (s - odd + k));
+      M.m[r] |= (Mask)more.marks(ph, qi2) << k;
+    }
+    // the row alone, without the particle itself
+    M.m[r] &= (((Mask)1 << n) - 1) << odd;
+    if (r == 1) M.m[r] &= ~((Mask)1 << (R.particle() - (s - odd)));
+  }
   return M;
 }
 

@@ -204,6 +204,7 @@ wrach::SolveArgs solve_args(WrachContext* ctx) {
   wrach::SolveArgs a{};
   a.worlds = ctx->worlds_d;
   a.nworlds = (int)ctx->nworlds;
+  a.world = ctx->worlds_h[0];
   a.ph = ctx->ph;
   a.ncells = ctx->ncells;
   a.n = ctx->n;
@@ -967,6 +968,7 @@ int wrach_set_viewport(WrachContext* ctx, uint32_t world, float anchor_x, float 
   if (rc) return rc;
   w.cell_off = old.cell_off;
   ctx->worlds_h[world] = w;
+  drop_graphs(ctx);  // a single world's settings are among its launches' arguments
   CK(cudaMemcpyAsync(ctx->worlds_d + world, &ctx->worlds_h[world], sizeof(WorldDev),
                      cudaMemcpyHostToDevice, ctx->stream));
   // the frame, packed from the store under the new viewport

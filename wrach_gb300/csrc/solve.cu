@@ -14,6 +14,25 @@ namespace wrach {
 
 namespace {
 
+// The worlds as a kernel's argument.  With one world (ONE) its settings come
+// with the launch, in the constant bank: no loads ahead of the first use and no
+// registers held.
+template <bool ONE>
+struct Worlds;
+template <>
+struct Worlds<true> {
+  WorldDev w;
+  __device__ __forceinline__ const WorldDev& of(uint32_t) const { return w; }
+};
+template <>
+struct Worlds<false> {
+  const WorldDev* all;
+  int n;
+  __device__ __forceinline__ const WorldDev& of(uint32_t c) const {
+    return all[world_of_cell(all, n, c)];
+  }
+};
+
 // Next cell of a solved particle (assets/shaders/particles_per_cell.wgsl:
 // 14-27), the key the rebin sorts by.
 __device__ __forceinline__ uint32_t next_key(const WorldDev& w, float px,
@@ -53,8 +72,9 @@ __device__ __forceinline__ void publish_flags(Ctrl* ctrl, uint32_t flags) {
 // its lanes), and integrates the particles past a cell's capacity among its
 // first W.  1M particles, cell size 1: 36 us and a separate ticket launch of
 // 14 us before, 23 us with the tickets now.
+template <bool ONE>
 __global__ void __launch_bounds__(512, 3)
-k_solve_reference(const WorldDev* __restrict__ worlds, int nworlds, PhysDev ph, uint32_t n,
+k_solve_reference(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t n,
                   const uint32_t* __restrict__ cell_start, const uint32_t* __restrict__ cell_of,
                   const float2* __restrict__ pin, const float2* __restrict__ vin,
                   float2* __restrict__ pout, float2* __restrict__ vout,
@@ -67,11 +87,11 @@ k_solve_reference(const WorldDev* __restrict__ worlds, int nworlds, PhysDev ph, 
   uint32_t flags = 0, key = count.ncells, rank = 0, m = 0;
   float px = 0.f, py = 0.f;
   float2 v = make_float2(0.f, 0.f);
-  WorldDev w;
   bool mine = i < n;
+  const uint32_t c = mine ? cell_of[i] : 0u;
+  const WorldDev& w = worlds.of(c);
   if (mine) {
-    const uint32_t c = cell_of[i], s = cell_start[c], e = cell_start[c + 1];
-    w = worlds[world_of_cell(worlds, nworlds, c)];
+    const uint32_t s = cell_start[c], e = cell_start[c + 1];
     rank = i - s;
     m = min(e - s, ph.cap);
     mine = rank < m ? s >= first && s - first < own : lane < own;
@@ -291,9 +311,9 @@ __device__ __forceinline__ void push_marked(const PhysDev& ph, const f32x2* __re
 // At most 42 registers (three blocks of 512): the loads' latency needs the
 // warps.  On the 1M lattice an iteration issues about 60% of the time and
 // waits for its gathers through L1 for the rest.
-template <typename Mask, int ROWS>
+template <typename Mask, int ROWS, bool ONE>
 __global__ void __launch_bounds__(512, 3)
-k_jacobi_tp(const WorldDev* __restrict__ worlds, int nworlds, PhysDev ph, uint32_t ncells,
+k_jacobi_tp(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t ncells,
             const uint32_t* __restrict__ ct, const uint32_t* __restrict__ tp_cell,
             const float2* __restrict__ qin, float2* __restrict__ qout,
             const uint32_t* __restrict__ run_if, uint4* __restrict__ rows) {
@@ -307,7 +327,7 @@ k_jacobi_tp(const WorldDev* __restrict__ worlds, int nworlds, PhysDev ph, uint32
       R = Rows{u.x, u.y, u.z, u.w};
     } else {
       const uint32_t c = tp_cell[t];
-      R = tp_rows(worlds[world_of_cell(worlds, nworlds, c)], ct, c, t);
+      R = tp_rows(worlds.of(c), ct, c, t);
       if (ROWS == 1) rows[t] = make_uint4(R.s0, R.s1, R.s2, R.len);
     }
     const f32x2 qi2 = q[t];
@@ -329,9 +349,9 @@ k_jacobi_tp(const WorldDev* __restrict__ worlds, int nworlds, PhysDev ph, uint32
 // kinetic energy a plain frame gives (gravity, the clamp and wall
 // reflections only change the velocity).  A launch whose `run_if` flag
 // reads 0 returns at once.
-template <typename Mask, bool METRICS>
-__global__ void __launch_bounds__(512, METRICS ? 1 : 3)
-k_jacobi_final(const WorldDev* __restrict__ worlds, int nworlds, PhysDev ph, uint32_t n,
+template <typename Mask, bool METRICS, bool ONE>
+__global__ void __launch_bounds__(512, METRICS ? 2 : 3)
+k_jacobi_final(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t n,
                int do_push, const uint32_t* __restrict__ cell_start,
                const uint32_t* __restrict__ ct, const uint32_t* __restrict__ cell_of,
                const float2* __restrict__ pin, const float2* __restrict__ qtp,
@@ -350,7 +370,7 @@ k_jacobi_final(const WorldDev* __restrict__ worlds, int nworlds, PhysDev ph, uin
     uint32_t key = count.ncells;  // no cell
     if (live) {
       const uint32_t c = cell_of[i];
-      const WorldDev w = worlds[world_of_cell(worlds, nworlds, c)];
+      const WorldDev& w = worlds.of(c);
       // the velocity and, for the tickets' atomics, the counters of the
       // particle's cell and of the cells above and below it (its next cell
       // is almost always among their lines) are fetched before the push
@@ -433,9 +453,15 @@ cudaError_t launch_solve_reference(const SolveArgs& a, cudaStream_t st) {
   if (a.n == 0) return cudaSuccess;
   const uint32_t threads = a.block ? a.block : 128;
   const uint32_t own = (33u - a.ph.cap) * (threads / 32);
-  k_solve_reference<<<(a.n + own - 1) / own, threads, 0, st>>>(
-      a.worlds, a.nworlds, a.ph, a.n, a.cell_start, a.cell_of, a.pos, a.vel, a.pos_out, a.vel_out,
-      a.keys, a.ctrl, a.count);
+  const uint32_t blocks = (a.n + own - 1) / own;
+  if (a.nworlds == 1)
+    k_solve_reference<true><<<blocks, threads, 0, st>>>(
+        Worlds<true>{a.world}, a.ph, a.n, a.cell_start, a.cell_of, a.pos, a.vel, a.pos_out,
+        a.vel_out, a.keys, a.ctrl, a.count);
+  else
+    k_solve_reference<false><<<blocks, threads, 0, st>>>(
+        Worlds<false>{a.worlds, a.nworlds}, a.ph, a.n, a.cell_start, a.cell_of, a.pos, a.vel,
+        a.pos_out, a.vel_out, a.keys, a.ctrl, a.count);
   return cudaGetLastError();
 }
 
@@ -452,26 +478,54 @@ uint32_t solve_blocks(const SolveArgs& a) {
 // A row's marks fit 32 bits: its candidates and one more for an odd start.
 static bool narrow_marks(const PhysDev& ph) { return 3 * ph.cap + 1 <= 32; }
 
+template <typename Mask, int ROWS>
+static void launch_iteration(const SolveArgs& a, uint32_t blocks, uint32_t threads,
+                             const float2* qin, float2* qout, cudaStream_t st) {
+  if (ROWS == 2 || a.nworlds == 1) {  // the rows read back need no world
+    k_jacobi_tp<Mask, ROWS, true><<<blocks, threads, 0, st>>>(
+        Worlds<true>{a.world}, a.ph, a.ncells, a.ct, a.tp_cell, qin, qout, a.run_if, a.rows);
+  } else if constexpr (ROWS != 2) {
+    k_jacobi_tp<Mask, ROWS, false><<<blocks, threads, 0, st>>>(
+        Worlds<false>{a.worlds, a.nworlds}, a.ph, a.ncells, a.ct, a.tp_cell, qin, qout, a.run_if,
+        a.rows);
+  }
+}
+
+template <typename Mask>
+static void launch_iteration(const SolveArgs& a, uint32_t blocks, uint32_t threads,
+                             const float2* qin, float2* qout, cudaStream_t st) {
+  const int mode = a.rows ? a.rows_mode : 0;
+  if (mode == 1)
+    launch_iteration<Mask, 1>(a, blocks, threads, qin, qout, st);
+  else if (mode == 2)
+    launch_iteration<Mask, 2>(a, blocks, threads, qin, qout, st);
+  else
+    launch_iteration<Mask, 0>(a, blocks, threads, qin, qout, st);
+}
+
 cudaError_t launch_jacobi_iteration(const SolveArgs& a, const float2* qin, float2* qout,
                                     cudaStream_t st) {
   if (a.n == 0) return cudaSuccess;
   const uint32_t threads = a.block ? a.block : 128;
   const uint32_t blocks = solve_blocks(a);
-  const int mode = a.rows ? a.rows_mode : 0;
-#define WRACH_TP(MASK, ROWS)                                                                  \
-  k_jacobi_tp<MASK, ROWS><<<blocks, threads, 0, st>>>(a.worlds, a.nworlds, a.ph, a.ncells, a.ct, \
-                                                      a.tp_cell, qin, qout, a.run_if, a.rows)
-  if (narrow_marks(a.ph)) {
-    if (mode == 1) WRACH_TP(uint32_t, 1);
-    else if (mode == 2) WRACH_TP(uint32_t, 2);
-    else WRACH_TP(uint32_t, 0);
-  } else {
-    if (mode == 1) WRACH_TP(uint64_t, 1);
-    else if (mode == 2) WRACH_TP(uint64_t, 2);
-    else WRACH_TP(uint64_t, 0);
-  }
-#undef WRACH_TP
+  if (narrow_marks(a.ph))
+    launch_iteration<uint32_t>(a, blocks, threads, qin, qout, st);
+  else
+    launch_iteration<uint64_t>(a, blocks, threads, qin, qout, st);
   return cudaGetLastError();
+}
+
+template <typename Mask, bool METRICS>
+static void launch_final(const SolveArgs& a, uint32_t blocks, uint32_t threads, const float2* qtp,
+                         int do_push, cudaStream_t st) {
+  if (a.nworlds == 1)
+    k_jacobi_final<Mask, METRICS, true><<<blocks, threads, 0, st>>>(
+        Worlds<true>{a.world}, a.ph, a.n, do_push, a.cell_start, a.ct, a.cell_of, a.pos, qtp,
+        a.pos_out, a.vel, a.vel_out, a.keys, a.ctrl, a.run_if, a.part, a.count);
+  else
+    k_jacobi_final<Mask, METRICS, false><<<blocks, threads, 0, st>>>(
+        Worlds<false>{a.worlds, a.nworlds}, a.ph, a.n, do_push, a.cell_start, a.ct, a.cell_of,
+        a.pos, qtp, a.pos_out, a.vel, a.vel_out, a.keys, a.ctrl, a.run_if, a.part, a.count);
 }
 
 cudaError_t launch_jacobi_final(const SolveArgs& a, const float2* qtp, int do_push,
@@ -480,19 +534,14 @@ cudaError_t launch_jacobi_final(const SolveArgs& a, const float2* qtp, int do_pu
   const uint32_t threads = a.block ? a.block : 128;
   const uint32_t blocks = solve_blocks(a);
   const bool narrow = narrow_marks(a.ph);
-#define WRACH_FINAL(MASK, METRICS, PART)                                                     \
-  k_jacobi_final<MASK, METRICS><<<blocks, threads, 0, st>>>(                                 \
-      a.worlds, a.nworlds, a.ph, a.n, do_push, a.cell_start, a.ct, a.cell_of, a.pos, qtp,    \
-      a.pos_out, a.vel, a.vel_out, a.keys, a.ctrl, a.run_if, PART, a.count)
   if (a.part && narrow)
-    WRACH_FINAL(uint32_t, true, a.part);
+    launch_final<uint32_t, true>(a, blocks, threads, qtp, do_push, st);
   else if (a.part)
-    WRACH_FINAL(uint64_t, true, a.part);
+    launch_final<uint64_t, true>(a, blocks, threads, qtp, do_push, st);
   else if (narrow)
-    WRACH_FINAL(uint32_t, false, nullptr);
+    launch_final<uint32_t, false>(a, blocks, threads, qtp, do_push, st);
   else
-    WRACH_FINAL(uint64_t, false, nullptr);
-#undef WRACH_FINAL
+    launch_final<uint64_t, false>(a, blocks, threads, qtp, do_push, st);
   return cudaGetLastError();
 }
 

@@ -15,6 +15,7 @@ constexpr uint32_t kRowPad = 4;
 struct SolveArgs {
   const WorldDev* worlds;
   int nworlds;
+  WorldDev world;               // the settings when there is one world
   PhysDev ph;
   uint32_t ncells;              // cells over all worlds
   uint32_t n;                   // particles over all worlds

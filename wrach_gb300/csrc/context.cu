@@ -12,11 +12,11 @@
 //   rows              the iterations' neighbour-row ranges per compacted particle
 //   cell_of[2]        cell of each binned particle (u32)
 //   cs[2]             cell-start table, cells + 1 u32 (ping-pong per frame)
-//   ct[2], tp_pos[2], tp_vel[2], tp_cell[2]
+//   ct[2], tp_pos[2], tp_vel[2], tp_cell[2], tp_of[2]
 //                     extended physics: the capped table (start of each
-//                     cell's taking-part particles among them all) and those
+//                     cell's taking-part particles among them all), those
 //                     particles' positions, velocities and cells, compacted in
-//                     cell order
+//                     cell order, and each frame particle's place among them
 //   keys              next cell of each solve output (u32)
 //   kA kB iA iB       rebin scratch (tickets, slot cells, slot sources, sort ping-pong)
 //   tile_sums         rebin: particles per tile of 2048 cells (zero between frames)
@@ -110,7 +110,7 @@ void release(WrachContext* ctx) {
                   ctx->cs[0], ctx->cs[1], ctx->keys, ctx->kA, ctx->kB,
                   ctx->iA, ctx->iB, ctx->tile_sums, ctx->ctrl, ctx->big_list,
                   ctx->ct[0], ctx->ct[1], ctx->tp_pos[0], ctx->tp_pos[1], ctx->tp_cell[0],
-                  ctx->tp_cell[1], ctx->tile_sums_cap, ctx->tp_vel[0], ctx->tp_vel[1],
+                  ctx->tp_cell[1], ctx->tp_of[0], ctx->tp_of[1], ctx->tile_sums_cap, ctx->tp_vel[0], ctx->tp_vel[1],
                   ctx->stage_pos, ctx->stage_vel, ctx->table_tmp, ctx->counts, ctx->render_cover, ctx->render_image,
                   ctx->gather_idx, ctx->gather_out, ctx->compact_sums};
   for (void* p : ptrs) dfree(p);
@@ -220,6 +220,7 @@ wrach::SolveArgs solve_args(WrachContext* ctx) {
   a.per_thread = ctx->cfg.solve_per_thread;
   a.ct = ctx->ct[ctx->cur];
   a.tp_cell = ctx->tp_cell[ctx->cur];
+  a.tp_of = ctx->tp_of[ctx->cur];
   a.tp_pos = ctx->tp_pos[ctx->cur];
   a.tp_vel = ctx->tp_vel[ctx->cur];
   a.sms = ctx->sms;
@@ -260,6 +261,7 @@ wrach::RebinArgs rebin_args(WrachContext* ctx) {
     r.tp_pos = ctx->tp_pos[ctx->cur ^ 1];
     r.tp_vel = ctx->tp_vel[ctx->cur ^ 1];
     r.tp_cell = ctx->tp_cell[ctx->cur ^ 1];
+    r.tp_of = ctx->tp_of[ctx->cur ^ 1];
   }
   return r;
 }
@@ -289,6 +291,7 @@ int enqueue_frame(WrachContext* ctx) {
     const uint32_t K = ctx->ph.iterations;
     const float2* q = nullptr;
     CK(enqueue_iterations(ctx, a, K > 0 ? K - 1 : 0, st, &q, [&]() { mark(ctx); }));
+    fin.rows_mode = K > 1 ? 2 : 0;
     CK(wrach::launch_jacobi_final(fin, q, K > 0 ? 1 : 0, st));
     mark(ctx);
     ctx->launches += ctx->n ? std::max<uint32_t>(K, 1) : 0u;
@@ -517,7 +520,7 @@ int create_impl(const WrachConfig* config, uint32_t nworlds, const float* dims,
     if ((e = dalloc(&ctx->q1, tc + wrach::kRowPad)) != cudaSuccess) return oom(e);
     if ((e = dalloc(&ctx->q2, tc + wrach::kRowPad)) != cudaSuccess) return oom(e);
   }
-  if (c.mode == WRACH_MODE_EXTENDED && ctx->ph.iterations >= 3)
+  if (c.mode == WRACH_MODE_EXTENDED && ctx->ph.iterations >= 2)
     if ((e = dalloc(&ctx->rows, tc)) != cudaSuccess) return oom(e);
   if (c.mode == WRACH_MODE_EXTENDED) {
     for (int i = 0; i < 2; ++i) {
@@ -526,6 +529,7 @@ int create_impl(const WrachConfig* config, uint32_t nworlds, const float* dims,
       if ((e = dalloc(&ctx->tp_pos[i], tc + wrach::kRowPad)) != cudaSuccess) return oom(e);
       if ((e = dalloc(&ctx->tp_vel[i], tc)) != cudaSuccess) return oom(e);
       if ((e = dalloc(&ctx->tp_cell[i], tc)) != cudaSuccess) return oom(e);
+      if ((e = dalloc(&ctx->tp_of[i], tc)) != cudaSuccess) return oom(e);
     }
   }
   for (int i = 0; i < 2; ++i) {

@@ -59,6 +59,7 @@ struct WrachContext {
   float2* tp_pos[2] = {nullptr, nullptr};     // compacted positions
   float2* tp_vel[2] = {nullptr, nullptr};     // compacted velocities
   uint32_t* tp_cell[2] = {nullptr, nullptr};  // compacted cells
+  uint32_t* tp_of[2] = {nullptr, nullptr};    // compacted index of each frame particle
   uint32_t* tile_sums_cap = nullptr;          // per scan tile, taking-part particles
   uint32_t ntiles = 0;
   uint32_t* big_list = nullptr;               // counting sort: large-cell work list
@@ -158,9 +159,9 @@ cudaError_t enqueue_iterations(WrachContext* ctx, const wrach::SolveArgs& a, uin
   for (uint32_t it = 0; it < count; ++it) {
     float2* dst = (it & 1) ? ctx->q2 : ctx->q1;
     // the first iteration writes the particles' neighbour rows, the later
-    // ones read them
+    // ones and the last pass read them
     wrach::SolveArgs ai = a;
-    ai.rows_mode = count > 1 ? (it == 0 ? 1 : 2) : 0;
+    ai.rows_mode = it == 0 ? 1 : 2;
     const cudaError_t e = wrach::launch_jacobi_iteration(ai, src, dst, st);
     if (e != cudaSuccess) return e;
     after();

@@ -273,9 +273,10 @@ __device__ __forceinline__ void place_one(const RebinArgs& a, uint32_t slot, uin
     a.pos_dst[slot] = p;
     a.vel_dst[slot] = v;
     a.cell_dst[slot] = cell;
-    if (rank < a.tp_cap) {
-      const uint32_t t = a.ct_new[cell] + rank;
-      if (t < a.dst_capacity) {  // always true unless the scan timed out
+    if (a.tp_cap) {
+      const uint32_t t = rank < a.tp_cap ? a.ct_new[cell] + rank : kNoTp;
+      a.tp_of[slot] = t;
+      if (t < a.dst_capacity) {
         a.tp_pos[t] = p;
         a.tp_vel[t] = v;
         a.tp_cell[t] = cell;
@@ -316,9 +317,10 @@ __global__ void __launch_bounds__(256) k_cs_place(RebinArgs a) {
       a.pos_dst[slot] = p;
       a.vel_dst[slot] = v;
       a.cell_dst[slot] = k;
-      if (rank < a.tp_cap) {
-        const uint32_t t = tp0 + rank;
-        if (t < a.dst_capacity) {  // always true unless the scan timed out
+      if (a.tp_cap) {
+        const uint32_t t = rank < a.tp_cap ? tp0 + rank : kNoTp;
+        a.tp_of[slot] = t;
+        if (t < a.dst_capacity) {
           a.tp_pos[t] = p;
           a.tp_vel[t] = v;
           a.tp_cell[t] = k;

@@ -339,21 +339,22 @@ k_jacobi_tp(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t nce
 
 // The last iteration, one thread per frame particle (a grid-stride loop
 // over whole blocks of particles; the plain frames' grid covers them all):
-// the push (taking-part particles, from the compacted iterate q), then
-// gravity, integration, boundaries, the velocity clamp and the key emission,
-// and the rebin's tickets.  METRICS also writes the block's sums for the
-// surrogate's fallback gate to part[blockIdx.x * 8 + k]: [0] sum and [1] max
-// over taking-part particles of the deepest overlap max(0, min_d - distance)
-// with a pushing neighbour (measured on the pass's input), [2] the number of
-// taking-part particles, [3] the kinetic energy of the output and [4] the
-// kinetic energy a plain frame gives (gravity, the clamp and wall
-// reflections only change the velocity).  A launch whose `run_if` flag
-// reads 0 returns at once.
-template <typename Mask, bool METRICS, bool ONE>
+// the push (taking-part particles, from the compacted iterate q; ROWS 2: by
+// the neighbour rows that the iterations wrote, 0: from the capped table),
+// then gravity, integration, boundaries, the velocity clamp and the key
+// emission, and the rebin's tickets.  METRICS also writes the block's sums
+// for the surrogate's fallback gate to part[blockIdx.x * 8 + k]: [0] sum and
+// [1] max over taking-part particles of the deepest overlap max(0, min_d -
+// distance) with a pushing neighbour (measured on the pass's input), [2] the
+// number of taking-part particles, [3] the kinetic energy of the output and
+// [4] the kinetic energy a plain frame gives (gravity, the clamp and wall
+// reflections only change the velocity).  A launch whose `run_if` flag reads
+// 0 returns at once.
+template <typename Mask, int ROWS, bool METRICS, bool ONE>
 __global__ void __launch_bounds__(512, METRICS ? 2 : 3)
 k_jacobi_final(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t n,
-               int do_push, const uint32_t* __restrict__ cell_start,
-               const uint32_t* __restrict__ ct, const uint32_t* __restrict__ cell_of,
+               int do_push, const uint32_t* __restrict__ ct, const uint32_t* __restrict__ tp_of,
+               const uint32_t* __restrict__ cell_of, const uint4* __restrict__ rows,
                const float2* __restrict__ pin, const float2* __restrict__ qtp,
                float2* __restrict__ pout, const float2* __restrict__ vin,
                float2* __restrict__ vout, uint32_t* __restrict__ keys, Ctrl* ctrl,
@@ -369,7 +370,7 @@ k_jacobi_final(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t 
     const bool live = i < n;
     uint32_t key = count.ncells;  // no cell
     if (live) {
-      const uint32_t c = cell_of[i];
+      const uint32_t t = tp_of[i], c = cell_of[i];
       const WorldDev& w = worlds.of(c);
       // the velocity and, for the tickets' atomics, the counters of the
       // particle's cell and of the cells above and below it (its next cell
@@ -380,15 +381,20 @@ k_jacobi_final(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t 
         prefetch_l2(count.counts + (c >= w.gx ? c - w.gx : c));
         prefetch_l2(count.counts + min(c + w.gx, count.ncells - 1));
       }
-      const uint32_t t = tp_index(cell_start, ct, c, i, ph.cap);
       float qx, qy;
-      if (t != 0xFFFFFFFFu) {
+      if (t != kNoTp) {
         if (METRICS) taking = __fadd_rn(taking, 1.f);
         const f32x2* __restrict__ q = reinterpret_cast<const f32x2*>(qtp);
         const f32x2 qi2 = q[t];
         float ax = 0.f, ay = 0.f;
         if (do_push) {
-          const Rows R = tp_rows(w, ct, c, t);
+          Rows R;
+          if (ROWS == 2) {
+            const uint4 u = rows[t];
+            R = Rows{u.x, u.y, u.z, u.w};
+          } else {
+            R = tp_rows(w, ct, c, t);
+          }
           push_marked<Mask, METRICS>(ph, q, qi2, R, all_marks<Mask>(ph, q, qi2, R), ax, ay, pen);
         }
         qx = __fsub_rn(f2_x(qi2), ax);
@@ -515,17 +521,31 @@ cudaError_t launch_jacobi_iteration(const SolveArgs& a, const float2* qin, float
   return cudaGetLastError();
 }
 
-template <typename Mask, bool METRICS>
+template <typename Mask, int ROWS, bool METRICS>
 static void launch_final(const SolveArgs& a, uint32_t blocks, uint32_t threads, const float2* qtp,
                          int do_push, cudaStream_t st) {
   if (a.nworlds == 1)
-    k_jacobi_final<Mask, METRICS, true><<<blocks, threads, 0, st>>>(
-        Worlds<true>{a.world}, a.ph, a.n, do_push, a.cell_start, a.ct, a.cell_of, a.pos, qtp,
+    k_jacobi_final<Mask, ROWS, METRICS, true><<<blocks, threads, 0, st>>>(
+        Worlds<true>{a.world}, a.ph, a.n, do_push, a.ct, a.tp_of, a.cell_of, a.rows, a.pos, qtp,
         a.pos_out, a.vel, a.vel_out, a.keys, a.ctrl, a.run_if, a.part, a.count);
   else
-    k_jacobi_final<Mask, METRICS, false><<<blocks, threads, 0, st>>>(
-        Worlds<false>{a.worlds, a.nworlds}, a.ph, a.n, do_push, a.cell_start, a.ct, a.cell_of,
+    k_jacobi_final<Mask, ROWS, METRICS, false><<<blocks, threads, 0, st>>>(
+        Worlds<false>{a.worlds, a.nworlds}, a.ph, a.n, do_push, a.ct, a.tp_of, a.cell_of, a.rows,
         a.pos, qtp, a.pos_out, a.vel, a.vel_out, a.keys, a.ctrl, a.run_if, a.part, a.count);
+}
+
+template <typename Mask>
+static void launch_final(const SolveArgs& a, uint32_t blocks, uint32_t threads, const float2* qtp,
+                         int do_push, cudaStream_t st) {
+  const bool rows = a.rows && a.rows_mode == 2;
+  if (a.part && rows)
+    launch_final<Mask, 2, true>(a, blocks, threads, qtp, do_push, st);
+  else if (a.part)
+    launch_final<Mask, 0, true>(a, blocks, threads, qtp, do_push, st);
+  else if (rows)
+    launch_final<Mask, 2, false>(a, blocks, threads, qtp, do_push, st);
+  else
+    launch_final<Mask, 0, false>(a, blocks, threads, qtp, do_push, st);
 }
 
 cudaError_t launch_jacobi_final(const SolveArgs& a, const float2* qtp, int do_push,
@@ -533,15 +553,10 @@ cudaError_t launch_jacobi_final(const SolveArgs& a, const float2* qtp, int do_pu
   if (a.n == 0) return cudaSuccess;
   const uint32_t threads = a.block ? a.block : 128;
   const uint32_t blocks = solve_blocks(a);
-  const bool narrow = narrow_marks(a.ph);
-  if (a.part && narrow)
-    launch_final<uint32_t, true>(a, blocks, threads, qtp, do_push, st);
-  else if (a.part)
-    launch_final<uint64_t, true>(a, blocks, threads, qtp, do_push, st);
-  else if (narrow)
-    launch_final<uint32_t, false>(a, blocks, threads, qtp, do_push, st);
+  if (narrow_marks(a.ph))
+    launch_final<uint32_t>(a, blocks, threads, qtp, do_push, st);
   else
-    launch_final<uint64_t, false>(a, blocks, threads, qtp, do_push, st);
+    launch_final<uint64_t>(a, blocks, threads, qtp, do_push, st);
   return cudaGetLastError();
 }
 

@@ -658,16 +658,16 @@ __device__ __forceinline__ void zero_row(uint32_t* row) {
 // particle; a particle that does not take part (past the capacity of its
 // cell) gets all zeros.
 __global__ void __launch_bounds__(256)
-k_knn_features(const WorldDev* __restrict__ worlds, int nworlds, PhysDev ph, uint32_t n,
-               const uint32_t* __restrict__ cell_start, const uint32_t* __restrict__ ct,
+k_knn_features(const WorldDev* __restrict__ worlds, int nworlds, uint32_t n,
+               const uint32_t* __restrict__ tp_of, const uint32_t* __restrict__ ct,
                const uint32_t* __restrict__ cell_of, const float2* __restrict__ tpp,
                const float2* __restrict__ tpv, uint16_t* __restrict__ x) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint32_t* row = reinterpret_cast<uint32_t*>(x + (size_t)i * kIn);
   const uint32_t c = cell_of[i];
-  const uint32_t t = tp_index(cell_start, ct, c, i, ph.cap);
-  if (t == 0xFFFFFFFFu) {
+  const uint32_t t = tp_of[i];
+  if (t == kNoTp) {
     zero_row(row);
     return;
   }
@@ -766,14 +766,13 @@ size_t correct_smem() { return sizeof(SmemNet) + (size_t)kFuseThreads * kRow * 4
 
 // target = q - p, the first K-1 iterations' correction of frame particle i
 // (q compacted: zero for a particle that takes no part)
-__global__ void k_target(uint32_t n, PhysDev ph, const uint32_t* __restrict__ cell_start,
-                         const uint32_t* __restrict__ ct, const uint32_t* __restrict__ cell_of,
+__global__ void k_target(uint32_t n, const uint32_t* __restrict__ tp_of,
                          const float2* __restrict__ pos, const float2* __restrict__ q,
                          float2* __restrict__ target) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const uint32_t t = tp_index(cell_start, ct, cell_of[i], i, ph.cap);
-  if (t == 0xFFFFFFFFu) {
+  const uint32_t t = tp_of[i];
+  if (t == kNoTp) {
     target[i] = make_float2(0.f, 0.f);
     return;
   }
@@ -952,8 +951,8 @@ cudaError_t launch_errors(const SolveArgs& a, const float2* corr, const float2* 
 
 cudaError_t launch_knn_features(const SolveArgs& a, uint16_t* x, cudaStream_t st) {
   if (a.n == 0) return cudaSuccess;
-  k_knn_features<<<(a.n + 255) / 256, 256, 0, st>>>(a.worlds, a.nworlds, a.ph, a.n, a.cell_start,
-                                                    a.ct, a.cell_of, a.tp_pos, a.tp_vel, x);
+  k_knn_features<<<(a.n + 255) / 256, 256, 0, st>>>(a.worlds, a.nworlds, a.n, a.tp_of, a.ct,
+                                                    a.cell_of, a.tp_pos, a.tp_vel, x);
   return cudaGetLastError();
 }
 
@@ -1031,8 +1030,7 @@ cudaError_t launch_adam(const MlpDev& m, const float* grad, float* mom1, float* 
 cudaError_t launch_target(const SolveArgs& a, uint32_t n, const float2* q, float2* target,
                           cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  k_target<<<(n + 255) / 256, 256, 0, st>>>(n, a.ph, a.cell_start, a.ct, a.cell_of, a.pos, q,
-                                            target);
+  k_target<<<(n + 255) / 256, 256, 0, st>>>(n, a.tp_of, a.pos, q, target);
   return cudaGetLastError();
 }
 

@@ -89,7 +89,9 @@ int enqueue_plain_solve(WrachContext* ctx, const wrach::SolveArgs& a) {
   inner.part = nullptr;
   const float2* q = nullptr;
   CK(enqueue_iterations(ctx, inner, ctx->ph.iterations - 1, ctx->stream, &q, []() {}));
-  CK(wrach::launch_jacobi_final(a, q, 1, ctx->stream));
+  wrach::SolveArgs fin = a;
+  fin.rows_mode = 2;  // at least one iteration has written the rows
+  CK(wrach::launch_jacobi_final(fin, q, 1, ctx->stream));
   ctx->launches += ctx->n ? ctx->ph.iterations : 0u;
   return WRACH_OK;
 }

@@ -290,14 +290,10 @@ struct CountDev {
 // cell order) are also kept compacted: cell c's taking-part particles are
 // compacted entries [ct[c], ct[c + 1]) (the capped table, ct[ncells] = their
 // number), frame particle i of cell c takes part when i - cs[c] < cap, and
-// its compacted index is then ct[c] + i - cs[c].  Every neighbour row of the
-// 3x3 search is then one contiguous compacted range, over-full cells or not.
-__device__ __forceinline__ uint32_t tp_index(const uint32_t* __restrict__ cs,
-                                             const uint32_t* __restrict__ ct, uint32_t c,
-                                             uint32_t i, uint32_t cap) {
-  const uint32_t r = i - cs[c];
-  return r < cap ? ct[c] + r : 0xFFFFFFFFu;
-}
+// its compacted index is then ct[c] + i - cs[c], which the rebin keeps as
+// tp_of[i] (kNoTp: takes no part).  Every neighbour row of the 3x3 search is
+// then one contiguous compacted range, over-full cells or not.
+constexpr uint32_t kNoTp = 0xFFFFFFFFu;
 
 __device__ __forceinline__ uint64_t ld_acquire_u64(const uint64_t* p) {
   uint64_t v;

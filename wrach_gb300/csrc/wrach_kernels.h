@@ -34,14 +34,14 @@ struct SolveArgs {
   CountDev count;               // last solve launch: the rebin's tickets (extended: if count.ticket is set)
   // the frame's taking-part particles, compacted (extended physics)
   const uint32_t* ct;           // ncells + 1: capped table
+  const uint32_t* tp_of;        // n: compacted index of each frame particle (kNoTp: none)
   const uint32_t* tp_cell;      // cell of each compacted particle
   const float2* tp_pos;         // compacted positions of the binned state
   const float2* tp_vel;         // compacted velocities of the binned state
   int sms;                      // SMs of the device
   // extended iterations (optional): each compacted taking-part particle's
   // three neighbour rows (total_cap entries); rows_mode 0 computes the rows
-  // from the capped table, 1 also writes them, 2 reads them (the launches of
-  // a frame have the same block size)
+  // from the capped table, 1 also writes them, 2 reads them
   uint4* rows;
   int rows_mode;
 };
@@ -99,6 +99,7 @@ struct RebinArgs {
   float2* tp_pos;               // compacted positions
   float2* tp_vel;               // compacted velocities
   uint32_t* tp_cell;            // compacted cells
+  uint32_t* tp_of;              // compacted index of each slot (kNoTp: takes no part)
   uint32_t tiles_prefixed;      // scan step: tile sums already turned into prefixes (set by it)
 };
 

@@ -650,7 +650,8 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
     src_vel = ctx->stage_vel;
   }
   CK(wrach::launch_upload_keys(ctx->worlds_d, (int)ctx->nworlds, ctx->ncells, world, n_keep,
-                               ctx->cell_of[ctx->cur], n_new, s.pos, ctx->keys, ctx->stream));
+                               ctx->cell_of[ctx->cur], n_new, s.pos, ctx->keys, ctx->ctrl,
+                               ticket_args(ctx), ctx->stream));
   ctx->launches += nsrc ? 1 : 0;
   wrach::RebinArgs r = rebin_args(ctx);
   r.n = (uint32_t)nsrc;
@@ -665,7 +666,7 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
   // per-world counts from the new table, read back as soon as the scan has
   // written it
   const uint32_t nw = ctx->nworlds;
-  for (int step = 0; step < wrach::kCountSortSteps; ++step) {
+  for (int step = 1; step < wrach::kCountSortSteps; ++step) {
     // the place steps (3, 4) are the first to read the velocities
     if (vel_aside && step == 3) CK(cudaStreamWaitEvent(ctx->stream, ctx->join_ev, 0));
     bool launched;
@@ -680,7 +681,7 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
       CK(cudaEventRecord(ctx->counts_ev, ctx->stream));
     }
   }
-  ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells) + 1;
+  ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells) + (r.n ? 0 : 1);
   if (direct) {
     // the call returns once the counts are known and both host arrays have
     // been read; the place steps are still running, ahead of whatever the
@@ -741,7 +742,8 @@ int write_back_impl(WrachContext* ctx, uint32_t world) {
   uint32_t kept = 0;
   if (s.n) {
     CK(wrach::launch_upload_keys(ctx->worlds_d, (int)ctx->nworlds, ctx->ncells, world, 0, nullptr,
-                                 s.n, s.pos, ctx->keys, ctx->stream));
+                                 s.n, s.pos, ctx->keys, ctx->ctrl, wrach::CountDev{},
+                                 ctx->stream));
     CK(wrach::launch_keep_outside(ctx->keys, ctx->ncells, s.n, s.pos, s.vel, ctx->stage_pos,
                                   ctx->stage_vel, ctx->compact_sums, ctx->compact_sums + ntiles,
                                   ctx->stream));

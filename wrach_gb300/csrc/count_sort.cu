@@ -8,8 +8,8 @@
 //            inside the cell, arrival order) is the returned base plus its
 //            rank among the warp's particles of that cell; per warp one more
 //            atomic adds the particles of each tile of 2048 cells to the
-//            tile's sum.  A frame takes the tickets in its last solve launch
-//            instead (the keys are computed there)
+//            tile's sum.  Plain frames and uploads take the tickets where
+//            they compute the keys instead
 //   scan     exclusive scan of the per-cell counts, one block per tile of
 //            2048 cells; a tile's prefix is the sum of the earlier tiles'
 //            sums (already final, so no block waits): each block adds them

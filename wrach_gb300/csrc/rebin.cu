@@ -384,32 +384,43 @@ namespace {
 __device__ __forceinline__ int32_t cell_coord_euclid(float x, uint32_t cs) {
   const float d = (float)cs;
   float q = truncf(__fdiv_rn(x, d));
-  if (fmodf(x, d) < 0.0f) q = __fsub_rn(q, 1.0f);
+  // the remainder has the sign of x
+  if (x < 0.0f && fmodf(x, d) < 0.0f) q = __fsub_rn(q, 1.0f);
   if (q != q) return 0;
   if (q >= 2147483648.0f) return INT_MAX;
   if (q <= -2147483648.0f) return INT_MIN;
   return (int32_t)q;
 }
 
-__global__ void k_upload_keys(const WorldDev* __restrict__ worlds, int nworlds,
-                              uint32_t ncells, uint32_t target,
-                              uint32_t n_keep,
-                              const uint32_t* __restrict__ cell_of,
-                              uint32_t n_new,
-                              const float2* __restrict__ new_pos,
-                              uint32_t* __restrict__ keys) {
+// Keys of the sources, and the counting sort's tickets with them when
+// count.ticket is set (every lane of a warp takes part): the keys never wait
+// in memory for a launch of their own (1M particles: 7.4 us + 16.6 us apart,
+// 18 us together).
+__global__ void __launch_bounds__(256)
+k_upload_keys(const WorldDev* __restrict__ worlds, int nworlds, uint32_t ncells, uint32_t target,
+              uint32_t n_keep, const uint32_t* __restrict__ cell_of, uint32_t n_new,
+              const float2* __restrict__ new_pos, uint32_t* __restrict__ keys, Ctrl* ctrl,
+              CountDev count) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = i < n_keep + n_new;
+  uint32_t key = ncells;
   if (i < n_keep) {
     const uint32_t k = cell_of[i];
-    keys[i] = (uint32_t)world_of_cell(worlds, nworlds, k) == target ? ncells : k;
-  } else if (i < n_keep + n_new) {
+    if ((uint32_t)world_of_cell(worlds, nworlds, k) != target) key = k;
+  } else if (live) {
     const WorldDev w = worlds[target];
     const float2 p = new_pos[i - n_keep];
     const int64_t cx = (int64_t)cell_coord_euclid(p.x, w.cs) - w.blx;
     const int64_t cy = (int64_t)cell_coord_euclid(p.y, w.cs) - w.bly;
-    keys[i] = (cx < 0 || cy < 0 || cx >= (int64_t)w.gx || cy >= (int64_t)w.gy)
-                  ? ncells
-                  : w.cell_off + (uint32_t)cy * w.gx + (uint32_t)cx;
+    if (!(cx < 0 || cy < 0 || cx >= (int64_t)w.gx || cy >= (int64_t)w.gy))
+      key = w.cell_off + (uint32_t)cy * w.gx + (uint32_t)cx;
+  }
+  if (live) keys[i] = key;
+  if (count.ticket) {
+    if (i == 0) ctrl->big_count = 0u;  // the scan lists this rebin's large cells
+    const uint32_t t = warp_ticket(key, ncells, count.counts, count.tile_sums, count.tile_shift,
+                                   count.cap, count.tile_sums_cap);
+    if (live) count.ticket[i] = t;
   }
 }
 
@@ -448,11 +459,12 @@ cudaError_t launch_upload_keys(const WorldDev* worlds, int nworlds,
                                uint32_t ncells, uint32_t target,
                                uint32_t n_keep, const uint32_t* cell_of,
                                uint32_t n_new, const float2* new_pos,
-                               uint32_t* keys, cudaStream_t st) {
+                               uint32_t* keys, Ctrl* ctrl, const CountDev& count,
+                               cudaStream_t st) {
   const uint32_t n = n_keep + n_new;
   if (n == 0) return cudaSuccess;
-  k_upload_keys<<<(n + 255) / 256, 256, 0, st>>>(
-      worlds, nworlds, ncells, target, n_keep, cell_of, n_new, new_pos, keys);
+  k_upload_keys<<<(n + 255) / 256, 256, 0, st>>>(worlds, nworlds, ncells, target, n_keep, cell_of,
+                                                 n_new, new_pos, keys, ctrl, count);
   return cudaGetLastError();
 }
 

@@ -131,8 +131,8 @@ constexpr uint32_t kBigBlocksPerSm = 8;
 cudaError_t launch_count_sort(const RebinArgs& a, uint32_t big_blocks, cudaStream_t st);
 // The same, one step at a time (steps 0 .. kCountSortSteps - 1: count, scan,
 // scatter, place, large cells); *launched is false for a step that has
-// nothing to do.  Step 0 may be left out when the tickets were taken by the
-// last solve launch (SolveArgs::count).
+// nothing to do.  Step 0 is left out when the tickets were taken with the
+// keys (SolveArgs::count, launch_upload_keys).
 constexpr int kCountSortSteps = 5;
 cudaError_t launch_count_sort_step(const RebinArgs& a, int step, uint32_t big_blocks,
                                    cudaStream_t st, bool* launched);
@@ -145,12 +145,14 @@ uint32_t count_sort_launches(uint32_t n, uint32_t ncells);
 // Keys for an upload re-pack: the first n_keep sources are particles of the
 // current frame (their cell, or `ncells` if they belong to world `target`),
 // the next n_new are store particles of world `target` binned as
-// SpatialBin::get_cell_coord does (ncells if outside the grid).
+// SpatialBin::get_cell_coord does (ncells if outside the grid).  With
+// count.ticket set, also the counting sort's tickets (its step 0).
 cudaError_t launch_upload_keys(const WorldDev* worlds, int nworlds,
                                uint32_t ncells, uint32_t target,
                                uint32_t n_keep, const uint32_t* cell_of,
                                uint32_t n_new, const float2* new_pos,
-                               uint32_t* keys, cudaStream_t st);
+                               uint32_t* keys, Ctrl* ctrl, const CountDev& count,
+                               cudaStream_t st);
 
 // One thread waits (bounded) while *word == value: out[0] = 1 if the wait
 // gave up, out[1] = microseconds waited.  The wait every device-side wait

@@ -122,10 +122,10 @@ int wrach_add_particles(WrachContext *ctx, uint32_t world, const float *pos,
  * from them (ParticleStore::add_particles_to_cell followed by
  * create_packed_data, runners/bevy/src/particle_store.rs:62-65,103-149,
  * for the whole store at once).  The host arrays are read before the call
- * returns (pinned memory makes the copies faster).  With one world and no
- * more particles than the frame capacity, the last steps of the re-pack may
- * still be running on the context's stream when it returns; every later call
- * on the context is ordered after them. */
+ * returns (pinned memory makes the copies faster).  The last steps of the
+ * re-pack may still be running on the context's stream when it (or
+ * wrach_add_particles, wrach_add_particles_device, wrach_set_viewport)
+ * returns; every later call on the context is ordered after them. */
 int wrach_set_particles(WrachContext *ctx, uint32_t world, const float *pos,
                         const float *vel, uint32_t n);
 
@@ -245,7 +245,8 @@ int wrach_write_back(WrachContext *ctx, uint32_t world);
  * store under the new viewport (its walls move with it).  The grid size must
  * stay the same (always so for a move by whole cells, or for a viewport whose
  * sides are multiples of the cell size); otherwise
- * WRACH_ERR_INVALID_ARGUMENT.  Blocks.  No counterpart in the reference. */
+ * WRACH_ERR_INVALID_ARGUMENT.  Blocks until the new frame's particles are
+ * counted.  No counterpart in the reference. */
 int wrach_set_viewport(WrachContext *ctx, uint32_t world, float anchor_x,
                        float anchor_y);
 /* Number of particles in the world's store. */

@@ -124,6 +124,7 @@ void release(WrachContext* ctx) {
   if (ctx->join_ev) cudaEventDestroy(ctx->join_ev);
   if (ctx->counts_ev) cudaEventDestroy(ctx->counts_ev);
   if (ctx->aux) cudaStreamDestroy(ctx->aux);
+  if (ctx->back) cudaStreamDestroy(ctx->back);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
 }
 
@@ -345,7 +346,7 @@ uint32_t frame_launches(const WrachContext* ctx) {
 }
 
 // One frame captured as a CUDA graph, instantiated once per table parity
-// (the frame reads cs[parity] and writes cs[parity ^ 1]).
+// (the frame reads cs[parity] and writes cs[parity ^ 1]) and particle count.
 int build_graph(WrachContext* ctx) {
   const int parity = ctx->cur;
   const uint64_t launches = ctx->launches;
@@ -500,6 +501,7 @@ int create_impl(const WrachConfig* config, uint32_t nworlds, const float* dims,
   cudaError_t e;
   if ((e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess) return oom(e);
   if ((e = cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking)) != cudaSuccess) return oom(e);
+  if ((e = cudaStreamCreateWithFlags(&ctx->back, cudaStreamNonBlocking)) != cudaSuccess) return oom(e);
   if ((e = cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming)) != cudaSuccess) return oom(e);
   if ((e = cudaEventCreateWithFlags(&ctx->join_ev, cudaEventDisableTiming)) != cudaSuccess) return oom(e);
   if ((e = cudaEventCreateWithFlags(&ctx->counts_ev, cudaEventDisableTiming)) != cudaSuccess) return oom(e);
@@ -605,11 +607,12 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
   if (replace) s.n = 0;
   int rc = ensure_store(ctx, s, (size_t)s.n + n_add);
   if (rc) return rc;
-  // One world re-packed from a store that holds no more particles than its
-  // frame: the capacity check below cannot fail, so the sort places straight
-  // into the frame buffers, and the velocities are copied on the second
-  // stream while the positions' keys are counted, scanned and scattered
-  // (only the place steps read them).
+  // The sort places straight into the frame buffers.  For one world re-packed
+  // from a store that holds no more particles than its frame (`direct`) the
+  // capacity check below cannot fail, so the place steps follow the scan at
+  // once, and the velocities are copied on the second stream while the
+  // positions' keys are counted, scanned and scattered (only the place steps
+  // read them); otherwise the place steps wait for the counts.
   const bool direct = ctx->nworlds == 1 && replace && n_add <= ctx->cap_h[world];
   const bool vel_aside = direct && n_add;
   if (n_add) {
@@ -659,61 +662,59 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
   r.pos_src = src_pos;
   r.vel_src = src_vel;
   r.cs_new = ctx->cs[ctx->cur ^ 1];
-  r.pos_dst = direct ? ctx->pos : ctx->pos_o;
-  r.vel_dst = direct ? ctx->vel : ctx->vel_o;
+  r.pos_dst = ctx->pos;
+  r.vel_dst = ctx->vel;
   r.cell_dst = ctx->cell_of[ctx->cur ^ 1];
   r.force_general = 1;
-  // per-world counts from the new table, read back as soon as the scan has
-  // written it
+  bool launched;
+  CK(wrach::launch_count_sort_step(r, 1, ctx->big_blocks, ctx->stream, &launched));
+  // per-world counts from the new table, written to the host on a stream of
+  // their own beside the place steps and the velocities' copy
   const uint32_t nw = ctx->nworlds;
-  for (int step = 1; step < wrach::kCountSortSteps; ++step) {
-    // the place steps (3, 4) are the first to read the velocities
-    if (vel_aside && step == 3) CK(cudaStreamWaitEvent(ctx->stream, ctx->join_ev, 0));
-    bool launched;
-    CK(wrach::launch_count_sort_step(r, step, ctx->big_blocks, ctx->stream, &launched));
-    if (step == 1) {
-      k_gather_u32<<<(nw + 1 + 255) / 256, 256, 0, ctx->stream>>>(ctx->cs[ctx->cur ^ 1],
-                                                                   ctx->gather_idx, nw + 1,
-                                                                   ctx->gather_out);
-      CK(cudaGetLastError());
-      CK(cudaMemcpyAsync(ctx->gather_h, ctx->gather_out, (nw + 1) * 4, cudaMemcpyDeviceToHost,
-                         ctx->stream));
-      CK(cudaEventRecord(ctx->counts_ev, ctx->stream));
-    }
-  }
+  CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
+  CK(cudaStreamWaitEvent(ctx->back, ctx->fork_ev, 0));
+  k_gather_u32<<<(nw + 1 + 255) / 256, 256, 0, ctx->back>>>(ctx->cs[ctx->cur ^ 1], ctx->gather_idx,
+                                                            nw + 1, ctx->gather_h);
+  CK(cudaGetLastError());
+  CK(cudaEventRecord(ctx->counts_ev, ctx->back));
   ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells) + (r.n ? 0 : 1);
-  if (direct) {
-    // the call returns once the counts are known and both host arrays have
-    // been read; the place steps are still running, ahead of whatever the
-    // caller enqueues next on the context's stream
-    CK(cudaEventSynchronize(ctx->counts_ev));
-    if (vel_aside) CK(cudaEventSynchronize(ctx->join_ev));
-  } else {
-    CK(cudaStreamSynchronize(ctx->stream));
-  }
+  auto place = [&]() {
+    for (int step = 2; step < wrach::kCountSortSteps; ++step) {
+      // the place steps (3, 4) are the first to read the velocities
+      if (vel_aside && step == 3) CK(cudaStreamWaitEvent(ctx->stream, ctx->join_ev, 0));
+      CK(wrach::launch_count_sort_step(r, step, ctx->big_blocks, ctx->stream, &launched));
+    }
+    return (int)WRACH_OK;
+  };
+  if (direct && (rc = place())) return rc;
+  // the call returns once the counts are known and the source arrays have
+  // been read; the place steps may still be running, ahead of whatever the
+  // caller enqueues next on the context's stream
+  CK(cudaEventSynchronize(ctx->counts_ev));
+  if (vel_aside) CK(cudaEventSynchronize(ctx->join_ev));
   const std::vector<uint32_t> starts(ctx->gather_h, ctx->gather_h + nw + 1);
   for (uint32_t w = 0; w < nw; ++w) {
     const uint32_t cnt = starts[w + 1] - starts[w];
     if (cnt > ctx->cap_h[w]) {
+      // nothing is placed; the counters are left as the place steps leave them
       s.n = old_n;
+      CK(cudaMemsetAsync(ctx->counts, 0, ((size_t)ctx->ncells + 1) * 4, ctx->stream));
+      CK(cudaMemsetAsync(ctx->tile_sums, 0, (size_t)ctx->ntiles * 4, ctx->stream));
+      if (ctx->tile_sums_cap)
+        CK(cudaMemsetAsync(ctx->tile_sums_cap, 0, (size_t)ctx->ntiles * 4, ctx->stream));
       return fail(ctx, WRACH_ERR_CAPACITY,
                   "world " + std::to_string(w) + ": " + std::to_string(cnt) +
                       " particles in the frame exceed its capacity " + std::to_string(ctx->cap_h[w]));
     }
   }
-  const uint32_t total = starts[nw];
-  if (total && !direct) {
-    CK(cudaMemcpyAsync(ctx->pos, ctx->pos_o, (size_t)total * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->vel, ctx->vel_o, (size_t)total * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
-  }
+  if (!direct && (rc = place())) return rc;
   ctx->cur ^= 1;
-  ctx->n = total;
+  ctx->n = starts[nw];
   for (uint32_t w = 0; w < nw; ++w) {
     ctx->n_h[w] = starts[w + 1] - starts[w];
     ctx->poff_h[w] = starts[w];
   }
   ctx->graph_ok = true;
-  if (!direct) CK(cudaStreamSynchronize(ctx->stream));
   return WRACH_OK;
 }
 
@@ -748,14 +749,28 @@ int write_back_impl(WrachContext* ctx, uint32_t world) {
                                   ctx->stage_vel, ctx->compact_sums, ctx->compact_sums + ntiles,
                                   ctx->stream));
     ctx->launches += ntiles ? 4 : 2;
-    CK(cudaMemcpyAsync(&kept, ctx->compact_sums + ntiles, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->gather_h, ctx->compact_sums + ntiles, 4, cudaMemcpyDeviceToHost,
+                       ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    kept = ctx->gather_h[0];
   }
   if (nf) {
     CK(cudaMemcpyAsync(ctx->stage_pos + kept, ctx->pos + off, (size_t)nf * sizeof(float2),
                        cudaMemcpyDeviceToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->stage_vel + kept, ctx->vel + off, (size_t)nf * sizeof(float2),
                        cudaMemcpyDeviceToDevice, ctx->stream));
+  }
+  if (ctx->nworlds == 1) {
+    // the rebuilt store takes the place of the old one, whose buffers serve
+    // the next rebuild (with more worlds the staging buffers are larger than
+    // any world's store)
+    std::swap(s.pos, ctx->stage_pos);
+    std::swap(s.vel, ctx->stage_vel);
+    const size_t cap = s.cap;
+    s.cap = (uint32_t)std::min<size_t>(ctx->stage_cap, 0xFFFFFFF0u);
+    ctx->stage_cap = cap;
+    s.n = kept + nf;
+    return WRACH_OK;
   }
   if ((rc = ensure_store(ctx, s, (size_t)kept + nf))) return rc;
   if (kept + nf) {
@@ -765,7 +780,6 @@ int write_back_impl(WrachContext* ctx, uint32_t world) {
                        cudaMemcpyDeviceToDevice, ctx->stream));
   }
   s.n = kept + nf;
-  CK(cudaStreamSynchronize(ctx->stream));
   return WRACH_OK;
 }
 
@@ -815,6 +829,7 @@ int wrach_destroy(WrachContext* ctx) {
     // a frame's work on `aux` is joined into `stream`, unless its enqueue
     // failed between the fork and the join
     if (ctx->aux) cudaStreamSynchronize(ctx->aux);
+    if (ctx->back) cudaStreamSynchronize(ctx->back);
     release(ctx);
   }
   delete ctx;
@@ -841,17 +856,20 @@ int wrach_step(WrachContext* ctx, uint32_t nsteps) {
   DeviceGuard guard(ctx->device);
   for (uint32_t s = 0; s < nsteps; ++s) {
     // a graph holds the particle count (grid sizes) it was captured with;
-    // buffer reallocations drop the graphs
-    if (ctx->graph[ctx->cur] && ctx->graph_n[ctx->cur] != ctx->n) {
-      cudaGraphExecDestroy(ctx->graph[ctx->cur]);
-      ctx->graph[ctx->cur] = nullptr;
-    }
-    if (ctx->graph_ok && !ctx->graph[ctx->cur]) {
+    // buffer reallocations drop the graphs.  Capturing one takes about as long
+    // as a 1M-particle frame, so the first frame of a new count runs eagerly
+    // (a viewport on the move never steps a count twice).
+    cudaGraphExec_t& graph = ctx->graph[ctx->cur];
+    const bool again = ctx->last_n == ctx->n;
+    ctx->last_n = ctx->n;
+    if (ctx->graph_ok && again && (!graph || ctx->graph_n[ctx->cur] != ctx->n)) {
+      if (graph) cudaGraphExecDestroy(graph);
+      graph = nullptr;
       int rc = build_graph(ctx);
       if (rc) return rc;
     }
-    if (ctx->graph_ok && ctx->graph[ctx->cur]) {
-      CK(cudaGraphLaunch(ctx->graph[ctx->cur], ctx->stream));
+    if (ctx->graph_ok && graph && ctx->graph_n[ctx->cur] == ctx->n) {
+      CK(cudaGraphLaunch(graph, ctx->stream));
       ctx->launches += frame_launches(ctx);
       ctx->cur ^= 1;
     } else {
@@ -956,7 +974,10 @@ int wrach_write_back(WrachContext* ctx, uint32_t world) {
   if (!ctx) return WRACH_ERR_INVALID_ARGUMENT;
   if (world >= ctx->nworlds) return fail(ctx, WRACH_ERR_INVALID_ARGUMENT, "world out of range");
   DeviceGuard guard(ctx->device);
-  return write_back_impl(ctx, world);
+  const int rc = write_back_impl(ctx, world);
+  if (rc) return rc;
+  CK(cudaStreamSynchronize(ctx->stream));
+  return WRACH_OK;
 }
 
 int wrach_set_viewport(WrachContext* ctx, uint32_t world, float anchor_x, float anchor_y) {

@@ -29,6 +29,8 @@ struct WrachContext {
   cudaStream_t stream = nullptr;
   // a frame's large-cell sort runs on `aux`, beside the small cells' pass
   cudaStream_t aux = nullptr;
+  // uploads: the counts' way to the host
+  cudaStream_t back = nullptr;
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   // uploads: the per-world counts read back (the call waits for them only)
   cudaEvent_t counts_ev = nullptr;
@@ -76,12 +78,13 @@ struct WrachContext {
   uint32_t* table_tmp = nullptr;  // one world's reference-layout table
   uint32_t* gather_idx = nullptr; // nworlds + 1
   uint32_t* gather_out = nullptr;
-  uint32_t* gather_h = nullptr;   // pinned host copy of gather_out (nworlds + 1)
+  uint32_t* gather_h = nullptr;   // pinned, written by the device (nworlds + 1)
   std::string err;
   uint64_t launches = 0;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   uint32_t graph_n[2] = {0, 0};       // particle count each graph was captured with
   bool graph_ok = true;
+  uint32_t last_n = 0xFFFFFFFFu;      // particle count of the last frame stepped
   uint32_t* render_cover = nullptr;   // wrach_render scratch and image
   uint8_t* render_image = nullptr;
   size_t render_cap = 0;

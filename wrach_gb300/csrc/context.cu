@@ -5,18 +5,18 @@
 //
 // Device layout of a context (all worlds concatenated; world w owns the
 // global cells [cell_off_w, cell_off_w + gx_w * gy_w) and, in the frame, the
-// particles [cell_start[cell_off_w], cell_start[cell_off_w + cells_w])):
+// particles [start(cell_off_w), start(cell_off_w + cells_w))):
 //   pos, vel          binned state, float2 x capacity        (cell order)
 //   pos_o, vel_o      solve output, float2 x capacity        (same order)
 //   q1, q2            extended-mode Jacobi iterates
 //   rows              the iterations' neighbour-row ranges per compacted particle
 //   cell_of[2]        cell of each binned particle (u32)
-//   cs[2]             cell-start table, cells + 1 u32 (ping-pong per frame)
-//   ct[2], tp_pos[2], tp_vel[2], tp_cell[2], tp_of[2]
-//                     extended physics: the capped table (start of each
-//                     cell's taking-part particles among them all), those
-//                     particles' positions, velocities and cells, compacted in
-//                     cell order, and each frame particle's place among them
+//   cs[2], ct[2] or groups[2]
+//                     the cell table (CellTable; ping-pong per frame)
+//   tp_pos[2], tp_vel[2], tp_cell[2], tp_of[2]
+//                     extended physics: the taking-part particles' positions,
+//                     velocities and cells, compacted in cell order, and each
+//                     frame particle's place among them
 //   keys              next cell of each solve output (u32)
 //   kA kB iA iB       rebin scratch (tickets, slot cells, slot sources, sort ping-pong)
 //   tile_sums         rebin: particles per tile of 2048 cells (zero between frames)
@@ -54,11 +54,11 @@ int32_t cell_coord(float x, uint32_t cs) {
   return sat_i32(q);
 }
 
-__global__ void k_gather_u32(const uint32_t* __restrict__ src,
-                             const uint32_t* __restrict__ idx, uint32_t n,
-                             uint32_t* __restrict__ out) {
+__global__ void k_gather_starts(const wrach::CellTable table,
+                                const uint32_t* __restrict__ cells, uint32_t n,
+                                uint32_t* __restrict__ out) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = src[idx[i]];
+  if (i < n) out[i] = table.start(cells[i]);
 }
 
 // The smallest binary32 s with sqrt_rn(s) > min_d.  Correctly rounded
@@ -109,7 +109,7 @@ void release(WrachContext* ctx) {
                   ctx->q1, ctx->q2, ctx->rows, ctx->cell_of[0], ctx->cell_of[1],
                   ctx->cs[0], ctx->cs[1], ctx->keys, ctx->kA, ctx->kB,
                   ctx->iA, ctx->iB, ctx->tile_sums, ctx->ctrl, ctx->big_list,
-                  ctx->ct[0], ctx->ct[1], ctx->tp_pos[0], ctx->tp_pos[1], ctx->tp_cell[0],
+                  ctx->groups[0], ctx->groups[1], ctx->ct[0], ctx->ct[1], ctx->tp_pos[0], ctx->tp_pos[1], ctx->tp_cell[0],
                   ctx->tp_cell[1], ctx->tp_of[0], ctx->tp_of[1], ctx->tile_sums_cap, ctx->tp_vel[0], ctx->tp_vel[1],
                   ctx->stage_pos, ctx->stage_vel, ctx->table_tmp, ctx->counts, ctx->render_cover, ctx->render_image,
                   ctx->gather_idx, ctx->gather_out, ctx->compact_sums};
@@ -209,7 +209,7 @@ wrach::SolveArgs solve_args(WrachContext* ctx) {
   a.ph = ctx->ph;
   a.ncells = ctx->ncells;
   a.n = ctx->n;
-  a.cell_start = ctx->cs[ctx->cur];
+  a.table = ctx->table(ctx->cur);
   a.cell_of = ctx->cell_of[ctx->cur];
   a.pos = ctx->pos;
   a.vel = ctx->vel;
@@ -219,7 +219,6 @@ wrach::SolveArgs solve_args(WrachContext* ctx) {
   a.ctrl = ctx->ctrl;
   a.block = ctx->cfg.solve_block;
   a.per_thread = ctx->cfg.solve_per_thread;
-  a.ct = ctx->ct[ctx->cur];
   a.tp_cell = ctx->tp_cell[ctx->cur];
   a.tp_of = ctx->tp_of[ctx->cur];
   a.tp_pos = ctx->tp_pos[ctx->cur];
@@ -255,10 +254,12 @@ wrach::RebinArgs rebin_args(WrachContext* ctx) {
   r.big_cap = ctx->big_cap;
   // every rebin writes the next table parity; extended physics also the
   // compacted taking-part particles
+  r.cs_new = ctx->cs[ctx->cur ^ 1];
+  r.groups_new = ctx->groups[ctx->cur ^ 1];
+  r.ct_new = ctx->ct[ctx->cur ^ 1];
   if (ctx->ph.mode == WRACH_MODE_EXTENDED) {
     r.tp_cap = ctx->ph.cap;
     r.tile_sums_cap = ctx->tile_sums_cap;
-    r.ct_new = ctx->ct[ctx->cur ^ 1];
     r.tp_pos = ctx->tp_pos[ctx->cur ^ 1];
     r.tp_vel = ctx->tp_vel[ctx->cur ^ 1];
     r.tp_cell = ctx->tp_cell[ctx->cur ^ 1];
@@ -302,7 +303,6 @@ int enqueue_frame(WrachContext* ctx) {
   r.dst_capacity = ctx->total_cap;
   r.pos_src = ctx->pos_o;
   r.vel_src = ctx->vel_o;
-  r.cs_new = ctx->cs[ctx->cur ^ 1];
   r.pos_dst = ctx->pos;
   r.vel_dst = ctx->vel;
   r.cell_dst = ctx->cell_of[ctx->cur ^ 1];
@@ -526,8 +526,6 @@ int create_impl(const WrachConfig* config, uint32_t nworlds, const float* dims,
     if ((e = dalloc(&ctx->rows, tc)) != cudaSuccess) return oom(e);
   if (c.mode == WRACH_MODE_EXTENDED) {
     for (int i = 0; i < 2; ++i) {
-      if ((e = dalloc(&ctx->ct[i], (size_t)ctx->ncells + 1)) != cudaSuccess) return oom(e);
-      if ((e = cudaMemset(ctx->ct[i], 0, ((size_t)ctx->ncells + 1) * 4)) != cudaSuccess) return oom(e);
       if ((e = dalloc(&ctx->tp_pos[i], tc + wrach::kRowPad)) != cudaSuccess) return oom(e);
       if ((e = dalloc(&ctx->tp_vel[i], tc)) != cudaSuccess) return oom(e);
       if ((e = dalloc(&ctx->tp_cell[i], tc)) != cudaSuccess) return oom(e);
@@ -536,6 +534,14 @@ int create_impl(const WrachConfig* config, uint32_t nworlds, const float* dims,
   }
   for (int i = 0; i < 2; ++i) {
     if ((e = dalloc(&ctx->cell_of[i], tc)) != cudaSuccess) return oom(e);
+    if (ctx->ncells > wrach::kDenseCells) {
+      const size_t ngroups = ctx->ncells / wrach::kGroup + 1;
+      if ((e = dalloc(&ctx->groups[i], ngroups)) != cudaSuccess) return oom(e);
+      if ((e = cudaMemset(ctx->groups[i], 0, ngroups * sizeof(uint4))) != cudaSuccess) return oom(e);
+    } else if (c.mode == WRACH_MODE_EXTENDED) {
+      if ((e = dalloc(&ctx->ct[i], (size_t)ctx->ncells + 1)) != cudaSuccess) return oom(e);
+      if ((e = cudaMemset(ctx->ct[i], 0, ((size_t)ctx->ncells + 1) * 4)) != cudaSuccess) return oom(e);
+    }
     if ((e = dalloc(&ctx->cs[i], (size_t)ctx->ncells + 1)) != cudaSuccess) return oom(e);
     if ((e = cudaMemset(ctx->cs[i], 0, ((size_t)ctx->ncells + 1) * 4)) != cudaSuccess) return oom(e);
   }
@@ -661,7 +667,6 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
   r.dst_capacity = ctx->total_cap;
   r.pos_src = src_pos;
   r.vel_src = src_vel;
-  r.cs_new = ctx->cs[ctx->cur ^ 1];
   r.pos_dst = ctx->pos;
   r.vel_dst = ctx->vel;
   r.cell_dst = ctx->cell_of[ctx->cur ^ 1];
@@ -673,8 +678,8 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
   const uint32_t nw = ctx->nworlds;
   CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
   CK(cudaStreamWaitEvent(ctx->back, ctx->fork_ev, 0));
-  k_gather_u32<<<(nw + 1 + 255) / 256, 256, 0, ctx->back>>>(ctx->cs[ctx->cur ^ 1], ctx->gather_idx,
-                                                            nw + 1, ctx->gather_h);
+  k_gather_starts<<<(nw + 1 + 255) / 256, 256, 0, ctx->back>>>(
+      ctx->table(ctx->cur ^ 1), ctx->gather_idx, nw + 1, ctx->gather_h);
   CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->counts_ev, ctx->back));
   ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells) + (r.n ? 0 : 1);
@@ -914,19 +919,21 @@ int wrach_read(WrachContext* ctx, uint32_t world, float* positions, float* veloc
     CK(cudaMemcpyAsync(velocities, ctx->vel + off, (size_t)n * 8, cudaMemcpyDeviceToHost, ctx->stream));
   const WorldDev& w = ctx->worlds_h[world];
   const uint32_t cells = w.gx * w.gy;
+  // a dense table's starts are the reference's table from its second entry on
+  const bool whole = ctx->nworlds == 1 && !ctx->groups[0];
   if (indices) {
-    if (ctx->nworlds == 1) {
+    if (whole) {
       CK(cudaMemcpyAsync(indices + 1, ctx->cs[ctx->cur], ((size_t)cells + 1) * 4,
                          cudaMemcpyDeviceToHost, ctx->stream));
     } else {
-      CK(wrach::launch_world_table(ctx->cs[ctx->cur], w.cell_off, cells, ctx->table_tmp, ctx->stream));
+      CK(wrach::launch_world_table(ctx->table(ctx->cur), w.cell_off, cells, ctx->table_tmp, ctx->stream));
       ctx->launches += 1;
       CK(cudaMemcpyAsync(indices, ctx->table_tmp, ((size_t)cells + 2) * 4, cudaMemcpyDeviceToHost,
                          ctx->stream));
     }
   }
   CK(cudaStreamSynchronize(ctx->stream));
-  if (indices && ctx->nworlds == 1) indices[0] = 0;
+  if (indices && whole) indices[0] = 0;
   return WRACH_OK;
 }
 

@@ -50,14 +50,19 @@ struct WrachContext {
   float2 *q1 = nullptr, *q2 = nullptr;
   uint4* rows = nullptr;  // the iterations' neighbour rows per compacted particle
   uint32_t* cell_of[2] = {nullptr, nullptr};
-  uint32_t* cs[2] = {nullptr, nullptr};
+  // the cell table (CellTable), grouped on grids of more than kDenseCells
+  uint4* groups[2] = {nullptr, nullptr};  // cells / 8 + 1
+  uint32_t* cs[2] = {nullptr, nullptr};   // starts, cells + 1
+  uint32_t* ct[2] = {nullptr, nullptr};   // dense, extended physics: cells + 1
+  wrach::CellTable table(int parity) const {
+    return wrach::CellTable{groups[parity], cs[parity], ct[parity]};
+  }
   int cur = 0;
   uint32_t* keys = nullptr;
   uint32_t *kA = nullptr, *kB = nullptr, *iA = nullptr, *iB = nullptr;
   size_t sort_cap = 0;
   uint32_t* tile_sums = nullptr;  // one word per tile of the cell table
   // extended physics: the taking-part particles compacted (ping-pong with cs)
-  uint32_t* ct[2] = {nullptr, nullptr};       // capped table, cells + 1
   float2* tp_pos[2] = {nullptr, nullptr};     // compacted positions
   float2* tp_vel[2] = {nullptr, nullptr};     // compacted velocities
   uint32_t* tp_cell[2] = {nullptr, nullptr};  // compacted cells

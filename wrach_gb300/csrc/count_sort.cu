@@ -14,11 +14,11 @@
 //            2048 cells; a tile's prefix is the sum of the earlier tiles'
 //            sums (already final, so no block waits): each block adds them
 //            up itself, or, past kPrefixTiles tiles (where that sum grows
-//            with the square of the grid), a one-block launch first turns
-//            the tile sums into their prefixes; it writes the
-//            cell-start table and (extended physics) the capped table of the
-//            taking-part particles from the counts capped at the cell
-//            capacity, and lists the cells of more than kSmallCell particles
+//            with the square of the grid), a launch first turns runs of tile
+//            sums into their prefixes; it writes the cell table
+//            (CellTable: starts, and the starts among the taking-part
+//            particles from the counts capped at the cell capacity) and
+//            lists the cells of more than kSmallCell particles
 //            (the pass that takes the tickets empties that list first); the
 //            place steps clear the counts of the non-empty cells afterwards
 //   scatter  source index and cell of every particle to table start + ticket
@@ -46,6 +46,19 @@ namespace wrach {
 namespace {
 
 constexpr uint32_t kScanThreads = 256, kScanPer = 8;
+// Without taking-part particles (reference physics) a grouped table's records
+// count up to this many particles of a cell; cells with more are wide.
+constexpr uint32_t kPlainCap = 31;
+static_assert(kDenseCells / kCountScanTile >= 2048, "grouped tables' tiles are prefixed");
+static_assert(kGroup * kPlainCap < 256 && kPlainCap < kSmallCell && kMaxCellCapacity < kSmallCell,
+              "a record's bytes; large cells are wide");
+
+// The new cell table; GROUPED as a constant, so that a dense table's lookups
+// are plain loads.
+template <bool GROUPED>
+__device__ __forceinline__ CellTable new_table(const RebinArgs& a) {
+  return CellTable{GROUPED ? a.groups_new : nullptr, a.cs_new, a.ct_new};
+}
 constexpr uint32_t kScanTile = kScanThreads * kScanPer;
 static_assert(kScanTile == kCountScanTile, "tile size shared with the tickets' tile sums");
 
@@ -76,26 +89,23 @@ __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* red) {
   return s;
 }
 
-// One block per tile of 2048 cells.  The tile's prefix is the sum of the
+// Scans: one block per tile of 2048 cells.  The tile's prefix is the sum of the
 // earlier tiles' counts, which the tickets' pass has already totalled, so no
 // block waits for another.
-// Past this many tiles of the table, the tile sums are turned into prefixes
-// by k_cs_tile_prefix first.
-constexpr uint32_t kPrefixTiles = 2048;
+// Past this many tiles of the table, k_cs_tile_prefix first turns the tile
+// sums into prefixes, one block per kRun tiles: a tile's sum becomes that of
+// the run's earlier tiles, and the run's own sum goes behind the tile sums.
+// A scan block then adds up the earlier runs instead of the earlier tiles (one
+// block that scanned all tiles by itself took 134 us for the 44,775 tiles of
+// 92M cells; 2.5 us now).
+constexpr uint32_t kPrefixTiles = 2048, kRun = 256;
 
-// One block of 1024 threads: the tile sums (and the capped ones) replaced by
-// their exclusive prefixes, in place; each thread scans a contiguous run.
-__global__ void __launch_bounds__(1024) k_cs_tile_prefix(RebinArgs a, uint32_t ntiles) {
-  __shared__ uint32_t ws[32], wc[32];
+__global__ void __launch_bounds__(kRun) k_cs_tile_prefix(RebinArgs a, uint32_t ntiles) {
+  __shared__ uint32_t ws[kRun / 32], wc[kRun / 32];
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const uint32_t per = (ntiles + 1023) / 1024;
-  const uint32_t i0 = min(t * per, ntiles), i1 = min(i0 + per, ntiles);
-  const bool cap = a.tp_cap != 0u;
-  uint32_t s = 0, c = 0;
-  for (uint32_t i = i0; i < i1; ++i) {
-    s += __ldcg(a.tile_sums + i);
-    if (cap) c += __ldcg(a.tile_sums_cap + i);
-  }
+  const uint32_t i = blockIdx.x * kRun + t;
+  const uint32_t s = i < ntiles ? a.tile_sums[i] : 0u;
+  const uint32_t c = i < ntiles && a.tp_cap ? a.tile_sums_cap[i] : 0u;
   uint32_t x = s, y = c;
 #pragma unroll
   for (uint32_t o = 1; o < 32; o <<= 1) {
@@ -110,22 +120,34 @@ __global__ void __launch_bounds__(1024) k_cs_tile_prefix(RebinArgs a, uint32_t n
     wc[warp] = y;
   }
   __syncthreads();
-  uint32_t bs = 0, bc = 0;
   for (uint32_t w = 0; w < warp; ++w) {
-    bs += ws[w];
-    bc += wc[w];
+    x += ws[w];
+    y += wc[w];
   }
-  uint32_t run = bs + x - s, crun = bc + y - c;
-  for (uint32_t i = i0; i < i1; ++i) {
-    const uint32_t v = __ldcg(a.tile_sums + i);
-    a.tile_sums[i] = run;
-    run += v;
-    if (cap) {
-      const uint32_t w = __ldcg(a.tile_sums_cap + i);
-      a.tile_sums_cap[i] = crun;
-      crun += w;
-    }
+  if (i < ntiles) {
+    a.tile_sums[i] = x - s;
+    if (a.tp_cap) a.tile_sums_cap[i] = y - c;
   }
+  if (t == kRun - 1) {
+    a.tile_sums[ntiles + blockIdx.x] = x;
+    if (a.tp_cap) a.tile_sums_cap[ntiles + blockIdx.x] = y;
+  }
+}
+
+// The particles (sums: tile_sums or tile_sums_cap) before a tile; the warp's
+// lanes call it together.
+__device__ __forceinline__ uint32_t before_tile(const uint32_t* sums, uint32_t tile,
+                                                uint32_t ntiles) {
+  uint32_t s = 0;
+  for (uint32_t r = threadIdx.x & 31; r < tile / kRun; r += 32) s += sums[ntiles + r];
+  return __reduce_add_sync(0xffffffffu, s) + sums[tile];
+}
+
+// The large cells' work list (at most n / (kSmallCell + 1) cells qualify, and
+// big_cap is larger).
+__device__ __forceinline__ void list_large(const RebinArgs& a, uint32_t cell) {
+  const uint32_t w = atomicAdd(&a.ctrl->big_count, 1u);
+  if (w < a.big_cap) a.big_list[w] = cell;
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_cs_scan(RebinArgs a) {
@@ -157,9 +179,9 @@ __global__ void __launch_bounds__(kScanThreads) k_cs_scan(RebinArgs a) {
   }
   // the earlier tiles' totals
   uint32_t prefix, cprefix;
-  if (a.tiles_prefixed) {
-    prefix = __ldcg(a.tile_sums + tile);
-    cprefix = cap ? __ldcg(a.tile_sums_cap + tile) : 0u;
+  if (a.prefixed_tiles) {
+    prefix = before_tile(a.tile_sums, tile, a.prefixed_tiles);
+    cprefix = cap ? before_tile(a.tile_sums_cap, tile, a.prefixed_tiles) : 0u;
   } else {
     uint32_t pre = 0, cpre = 0;
     for (uint32_t u = t; u < tile; u += kScanThreads) {
@@ -195,17 +217,10 @@ __global__ void __launch_bounds__(kScanThreads) k_cs_scan(RebinArgs a) {
   }
   uint32_t run = prefix + before + x - sum;
   uint32_t crun = cprefix + cbefore + cx - csum;
-  // the large cells' work list (at most n / (kSmallCell + 1) cells qualify,
-  // and big_cap is larger)
 #pragma unroll
-  for (uint32_t u = 0; u < kScanPer; ++u) {
-    if (v[u] > kSmallCell) {
-      const uint32_t w = atomicAdd(&a.ctrl->big_count, 1u);
-      if (w < a.big_cap) a.big_list[w] = c0 + u;
-    }
-  }
+  for (uint32_t u = 0; u < kScanPer; ++u)
+    if (v[u] > kSmallCell) list_large(a, c0 + u);
   if (cap) {
-    // the capped table (compacted starts of the cells' taking-part particles)
     if (c0 + kScanPer <= n) {
       uint4* dst = reinterpret_cast<uint4*>(a.ct_new + c0);
 #pragma unroll
@@ -247,6 +262,95 @@ __global__ void __launch_bounds__(kScanThreads) k_cs_scan(RebinArgs a) {
   if (t == 0 && (tile + 1) * kScanTile >= n) a.cs_new[n] = prefix + total;
 }
 
+// The same for a grouped table: a thread takes 16 cells, two records.  It
+// reads 4 bytes per cell and writes 2 where the dense scan writes 8 (92M
+// cells: 181 us dense, 82 us).
+constexpr uint32_t kGroupThreads = kScanTile / (2 * kGroup);
+
+__global__ void __launch_bounds__(kGroupThreads) k_cs_scan_groups(RebinArgs a) {
+  __shared__ uint32_t warp_sum[kGroupThreads / 32], warp_cap[kGroupThreads / 32];
+  constexpr uint32_t per = 2 * kGroup;
+  const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint32_t tile = blockIdx.x, n = a.ncells;
+  if (tile == 0 && t == 0 && !a.force_general) a.ctrl->frames += 1;
+  const uint32_t c0 = tile * kScanTile + t * per;
+  uint32_t v[per];
+  if (c0 + per <= n) {
+    const uint4* src = reinterpret_cast<const uint4*>(a.counts + c0);
+#pragma unroll
+    for (uint32_t u = 0; u < per / 4; ++u) {
+      const uint4 q = src[u];
+      v[4 * u] = q.x; v[4 * u + 1] = q.y; v[4 * u + 2] = q.z; v[4 * u + 3] = q.w;
+    }
+  } else {
+#pragma unroll
+    for (uint32_t u = 0; u < per; ++u) v[u] = c0 + u < n ? a.counts[c0 + u] : 0u;
+  }
+  const uint32_t prefix = before_tile(a.tile_sums, tile, a.prefixed_tiles);
+  const uint32_t cprefix = a.tp_cap ? before_tile(a.tile_sums_cap, tile, a.prefixed_tiles) : 0u;
+  // the capped counts: the taking-part particles (extended physics)
+  const uint32_t cap = a.tp_cap ? a.tp_cap : kPlainCap;
+  uint32_t sum[2], csum[2], low[2], high[2];
+  bool wide[2];
+#pragma unroll
+  for (uint32_t h = 0; h < 2; ++h) {
+    sum[h] = csum[h] = low[h] = high[h] = 0u;
+    wide[h] = false;
+#pragma unroll
+    for (uint32_t u = 0; u < kGroup; ++u) {
+      const uint32_t x = v[h * kGroup + u];
+      if (u < 4) low[h] |= csum[h] << (8 * u);
+      else high[h] |= csum[h] << (8 * (u - 4));
+      sum[h] += x;
+      csum[h] += min(x, cap);
+      wide[h] = wide[h] || x > cap;
+    }
+  }
+  uint32_t x = sum[0] + sum[1], cx = csum[0] + csum[1];
+#pragma unroll
+  for (uint32_t o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    const uint32_t cy = __shfl_up_sync(0xffffffffu, cx, o);
+    if (lane >= o) {
+      x += y;
+      cx += cy;
+    }
+  }
+  if (lane == 31) {
+    warp_sum[warp] = x;
+    warp_cap[warp] = cx;
+  }
+  __syncthreads();
+  uint32_t run = prefix + x - sum[0] - sum[1], crun = cprefix + cx - csum[0] - csum[1];
+#pragma unroll
+  for (uint32_t w = 0; w < kGroupThreads / 32 - 1; ++w) {
+    run += w < warp ? warp_sum[w] : 0u;
+    crun += w < warp ? warp_cap[w] : 0u;
+  }
+#pragma unroll
+  for (uint32_t h = 0; h < 2; ++h) {
+    // the record past the last cell holds the totals
+    const uint32_t c = c0 + h * kGroup;
+    if (c <= n)
+      a.groups_new[c / kGroup] = make_uint4(run, crun | (wide[h] ? kWide : 0u), low[h], high[h]);
+    if (wide[h]) {
+      uint32_t at = run;
+#pragma unroll
+      for (uint32_t u = 0; u < kGroup; ++u) {
+        const uint32_t k = v[h * kGroup + u];
+        if (c + u <= n) a.cs_new[c + u] = at;
+        at += k;
+        if (k > kSmallCell) list_large(a, c + u);
+      }
+    }
+    run += sum[h];
+    crun += csum[h];
+  }
+  if (t == kGroupThreads - 1 && (tile + 1) * kScanTile == n)
+    a.groups_new[n / kGroup] = make_uint4(run, crun, 0u, 0u);
+}
+
+template <bool GROUPED>
 __global__ void __launch_bounds__(256) k_cs_scatter(RebinArgs a, uint32_t ntiles) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   // the scan has read the tile sums: clear them for the next rebin
@@ -257,7 +361,7 @@ __global__ void __launch_bounds__(256) k_cs_scatter(RebinArgs a, uint32_t ntiles
   if (i >= a.n) return;
   const uint32_t k = a.keys[i];
   if (k >= a.ncells) return;
-  const uint32_t dst = a.cs_new[k] + a.ticket[i];
+  const uint32_t dst = new_table<GROUPED>(a).start(k) + a.ticket[i];
   if (dst < a.n) {  // always true unless the scan timed out
     a.idx_tmp[dst] = i;
     a.cell_tmp[dst] = k;
@@ -266,6 +370,7 @@ __global__ void __launch_bounds__(256) k_cs_scatter(RebinArgs a, uint32_t ntiles
 
 // The particle of source index `src` into `slot`, rank `rank` inside its
 // cell; a taking-part one (rank < tp_cap) also into the compacted arrays.
+template <bool GROUPED>
 __device__ __forceinline__ void place_one(const RebinArgs& a, uint32_t slot, uint32_t rank,
                                           uint32_t src, uint32_t cell, uint32_t& overflow) {
   if (slot < a.dst_capacity && src < a.n) {
@@ -274,7 +379,7 @@ __device__ __forceinline__ void place_one(const RebinArgs& a, uint32_t slot, uin
     a.vel_dst[slot] = v;
     a.cell_dst[slot] = cell;
     if (a.tp_cap) {
-      const uint32_t t = rank < a.tp_cap ? a.ct_new[cell] + rank : kNoTp;
+      const uint32_t t = rank < a.tp_cap ? new_table<GROUPED>(a).taking(cell) + rank : kNoTp;
       a.tp_of[slot] = t;
       if (t < a.dst_capacity) {
         a.tp_pos[t] = p;
@@ -292,14 +397,16 @@ __device__ __forceinline__ void add_overflow(const RebinArgs& a, uint32_t overfl
   if ((threadIdx.x & 31) == 0 && wo) atomicAdd(&a.ctrl->overflow, wo);
 }
 
+template <bool GROUPED>
 __global__ void __launch_bounds__(256) k_cs_place(RebinArgs a) {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t total = a.cs_new[a.ncells];
+  const CellTable table = new_table<GROUPED>(a);
+  const uint32_t total = table.start(a.ncells);
   uint32_t overflow = 0;
   // the guards below only matter if the scan timed out (table inconsistent)
   const uint32_t k = q < total && q < a.n ? a.cell_tmp[q] : a.ncells;
-  const uint32_t c0 = k < a.ncells ? a.cs_new[k] : 0u;
-  const uint32_t c1 = k < a.ncells ? a.cs_new[k + 1] : 0u;
+  uint32_t c0 = 0u, c1 = 0u;
+  if (k < a.ncells) table.span(k, c0, c1);
   // larger cells are the scan's work list, placed by k_cs_big
   if (k < a.ncells && c1 - c0 <= kSmallCell) {
     const uint32_t s1 = min(c1, min(total, a.n));
@@ -309,7 +416,7 @@ __global__ void __launch_bounds__(256) k_cs_place(RebinArgs a) {
     const bool src_ok = me < a.n;
     const float2 p = src_ok ? a.pos_src[me] : make_float2(0.f, 0.f);
     const float2 v = src_ok ? a.vel_src[me] : make_float2(0.f, 0.f);
-    const uint32_t tp0 = a.tp_cap ? a.ct_new[k] : 0u;
+    const uint32_t tp0 = a.tp_cap ? table.taking(k) : 0u;
     uint32_t rank = 0;
     for (uint32_t m = c0; m < s1; ++m) rank += a.idx_tmp[m] < me ? 1u : 0u;
     const uint32_t slot = c0 + rank;
@@ -401,19 +508,24 @@ __device__ uint32_t* block_radix_sort(uint32_t* src, uint32_t* alt, uint32_t m, 
 // indices sorted in shared memory (bitonic, padded to a power of two, one
 // compare-exchange per pair index and stage), larger cells by the block-wide
 // radix sort in global memory; then the gather.
-__global__ void __launch_bounds__(kBigThreads) k_cs_big(RebinArgs a) {
+// Eight blocks per SM (its grid), so at most 32 registers.
+template <bool GROUPED>
+__global__ void __launch_bounds__(kBigThreads, 8) k_cs_big(RebinArgs a) {
   __shared__ uint32_t sv[kBigCell];
   const uint32_t nb = min(a.ctrl->big_count, a.big_cap);
+  const CellTable table = new_table<GROUPED>(a);
   uint32_t overflow = 0;
   const uint32_t key_bits = a.n > 1 ? 32u - __clz(a.n - 1) : 1u;
   for (uint32_t w = blockIdx.x; w < nb; w += gridDim.x) {
     const uint32_t k = a.big_list[w];
-    const uint32_t s0 = a.cs_new[k], s1 = min(a.cs_new[k + 1], a.n);
+    uint32_t s0, s1;
+    table.span(k, s0, s1);
+    s1 = min(s1, a.n);
     if (threadIdx.x == 0) a.counts[k] = 0u;  // read by the scan; zero for the next rebin
     const uint32_t s = s1 > s0 ? s1 - s0 : 0u;
     if (s > kBigCell) {
       const uint32_t* sorted = block_radix_sort(a.idx_tmp + s0, a.idx_alt + s0, s, key_bits);
-      for (uint32_t r = threadIdx.x; r < s; r += kBigThreads) place_one(a, s0 + r, r, sorted[r], k, overflow);
+      for (uint32_t r = threadIdx.x; r < s; r += kBigThreads) place_one<GROUPED>(a, s0 + r, r, sorted[r], k, overflow);
       if (threadIdx.x == 0) atomicAdd(&a.ctrl->huge_cells, 1u);
       __syncthreads();
       continue;
@@ -437,7 +549,7 @@ __global__ void __launch_bounds__(kBigThreads) k_cs_big(RebinArgs a) {
         __syncthreads();
       }
     }
-    for (uint32_t r = threadIdx.x; r < s; r += kBigThreads) place_one(a, s0 + r, r, sv[r], k, overflow);
+    for (uint32_t r = threadIdx.x; r < s; r += kBigThreads) place_one<GROUPED>(a, s0 + r, r, sv[r], k, overflow);
     __syncthreads();
   }
   add_overflow(a, overflow);
@@ -458,22 +570,34 @@ cudaError_t launch_count_sort_step(const RebinArgs& a, int step, uint32_t big_bl
     k_cs_count<<<nblk, 256, 0, st>>>(a);
   } else if (step == 1) {
     RebinArgs b = a;
-    b.tiles_prefixed = ntiles > kPrefixTiles ? 1u : 0u;
-    if (b.tiles_prefixed) {
-      k_cs_tile_prefix<<<1, 1024, 0, st>>>(b, ntiles);
+    b.prefixed_tiles = ntiles > kPrefixTiles ? ntiles : 0u;
+    if (b.prefixed_tiles) {
+      k_cs_tile_prefix<<<(ntiles + kRun - 1) / kRun, kRun, 0, st>>>(b, ntiles);
       const cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return e;
     }
-    k_cs_scan<<<ntiles ? ntiles : 1u, kScanThreads, 0, st>>>(b);
+    if (a.groups_new)
+      k_cs_scan_groups<<<ntiles, kGroupThreads, 0, st>>>(b);
+    else
+      k_cs_scan<<<ntiles ? ntiles : 1u, kScanThreads, 0, st>>>(b);
   } else if (!nblk) {
     *launched = false;
     return cudaSuccess;
   } else if (step == 2) {
-    k_cs_scatter<<<nblk, 256, 0, st>>>(a, ntiles);
+    if (a.groups_new)
+      k_cs_scatter<true><<<nblk, 256, 0, st>>>(a, ntiles);
+    else
+      k_cs_scatter<false><<<nblk, 256, 0, st>>>(a, ntiles);
   } else if (step == 3) {
-    k_cs_place<<<nblk, 256, 0, st>>>(a);
+    if (a.groups_new)
+      k_cs_place<true><<<nblk, 256, 0, st>>>(a);
+    else
+      k_cs_place<false><<<nblk, 256, 0, st>>>(a);
   } else {
-    k_cs_big<<<big_blocks ? big_blocks : 1u, kBigThreads, 0, st>>>(a);
+    if (a.groups_new)
+      k_cs_big<true><<<big_blocks ? big_blocks : 1u, kBigThreads, 0, st>>>(a);
+    else
+      k_cs_big<false><<<big_blocks ? big_blocks : 1u, kBigThreads, 0, st>>>(a);
   }
   return cudaGetLastError();
 }

@@ -424,13 +424,12 @@ k_upload_keys(const WorldDev* __restrict__ worlds, int nworlds, uint32_t ncells,
   }
 }
 
-__global__ void k_world_table(const uint32_t* __restrict__ cell_start,
-                              uint32_t cell_off, uint32_t cells,
+__global__ void k_world_table(const CellTable table, uint32_t cell_off, uint32_t cells,
                               uint32_t* __restrict__ out) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t base = cell_start[cell_off];
+  const uint32_t base = table.start(cell_off);
   if (i == 0) out[0] = 0;
-  if (i <= cells) out[i + 1] = cell_start[cell_off + i] - base;
+  if (i <= cells) out[i + 1] = table.start(cell_off + i) - base;
 }
 
 }  // namespace
@@ -485,10 +484,10 @@ cudaError_t launch_local_keys(const uint32_t* cell_of, uint32_t n, uint32_t cell
   return cudaGetLastError();
 }
 
-cudaError_t launch_world_table(const uint32_t* cell_start, uint32_t cell_off,
+cudaError_t launch_world_table(const CellTable& table, uint32_t cell_off,
                                uint32_t cells, uint32_t* out, cudaStream_t st) {
   const uint32_t n = cells + 1;
-  k_world_table<<<(n + 255) / 256, 256, 0, st>>>(cell_start, cell_off, cells,
+  k_world_table<<<(n + 255) / 256, 256, 0, st>>>(table, cell_off, cells,
                                                   out);
   return cudaGetLastError();
 }

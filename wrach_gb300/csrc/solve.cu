@@ -75,7 +75,7 @@ __device__ __forceinline__ void publish_flags(Ctrl* ctrl, uint32_t flags) {
 template <bool ONE>
 __global__ void __launch_bounds__(512, 3)
 k_solve_reference(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t n,
-                  const uint32_t* __restrict__ cell_start, const uint32_t* __restrict__ cell_of,
+                  const CellTable table, const uint32_t* __restrict__ cell_of,
                   const float2* __restrict__ pin, const float2* __restrict__ vin,
                   float2* __restrict__ pout, float2* __restrict__ vout,
                   uint32_t* __restrict__ keys, Ctrl* ctrl, CountDev count) {
@@ -91,7 +91,8 @@ k_solve_reference(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32
   const uint32_t c = mine ? cell_of[i] : 0u;
   const WorldDev& w = worlds.of(c);
   if (mine) {
-    const uint32_t s = cell_start[c], e = cell_start[c + 1];
+    uint32_t s, e;
+    table.span(c, s, e);
     rank = i - s;
     m = min(e - s, ph.cap);
     mine = rank < m ? s >= first && s - first < own : lane < own;
@@ -142,10 +143,10 @@ k_solve_reference(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32
 // 3x3 cells in row-major order, table order inside a cell), so each
 // particle's push sum is deterministic.
 //
-// The iterations run over the compacted taking-part particles (the capped
-// table ct of the rebin): there a neighbour row of the 3x3 search is one
-// contiguous range [ct[row + x0], ct[row + x1 + 1]) whatever the cells'
-// occupancy, and the particles that take no part cost nothing.
+// The iterations run over the compacted taking-part particles: there a
+// neighbour row of the 3x3 search is one contiguous range [taking(row + x0),
+// taking(row + x1 + 1)) whatever the cells' occupancy, and the particles that
+// take no part cost nothing.
 
 // The candidates of one particle: the compacted starts of its three
 // neighbour rows, and packed their lengths (6 bits each, at most 3 * 16) and
@@ -158,23 +159,11 @@ struct Rows {
 };
 static_assert(3 * kMaxCellCapacity < 64, "row lengths fit 6 bits");
 
-// The rows of the compacted particle t of cell c (independent loads of the
-// capped table).
-__device__ __forceinline__ Rows tp_rows(const WorldDev& w, const uint32_t* __restrict__ ct,
-                                        uint32_t c, uint32_t t) {
-  uint32_t cx, cy;
-  cell_xy(w, c - w.cell_off, cx, cy);
-  const uint32_t x0 = cx > 0 ? cx - 1 : 0;
-  const uint32_t x1 = cx + 1 < w.gx ? cx + 1 : w.gx - 1;
+// The rows of the compacted particle t of cell c.
+__device__ __forceinline__ Rows tp_rows(const WorldDev& w, const CellTable& table, uint32_t c,
+                                        uint32_t t) {
   uint32_t rs[3], re[3];
-#pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    const int ny = (int)cy - 1 + r;
-    const bool ok = ny >= 0 && ny < (int)w.gy;
-    const uint32_t rb = w.cell_off + (uint32_t)(ok ? ny : 0) * w.gx;
-    rs[r] = ok ? ct[rb + x0] : 0u;
-    re[r] = ok ? ct[rb + x1 + 1] : 0u;
-  }
+  neighbour_rows(w, table, c, rs, re);
   return Rows{rs[0], rs[1], rs[2],
               (re[0] - rs[0]) | ((re[1] - rs[1]) << 6) | ((re[2] - rs[2]) << 12) |
                   ((t - rs[1]) << 18)};
@@ -302,11 +291,11 @@ __device__ __forceinline__ void push_marked(const PhysDev& ph, const f32x2* __re
 }
 
 // One Jacobi iteration but the last, one thread per compacted (taking-part)
-// particle: q' = q - push sum, over the compacted count ct[ncells] (a
+// particle: q' = q - push sum, over the compacted count (a
 // grid-stride loop; the plain frames' grid covers every particle of the
 // frame, so each thread takes one or none).  A launch whose `run_if` flag
 // reads 0 returns at once.
-// ROWS 0: the neighbour rows from the capped table; 1: also written to
+// ROWS 0: the neighbour rows from the cell table; 1: also written to
 // `rows`; 2: read from `rows` (the cell and its world are then not needed).
 // At most 42 registers (three blocks of 512): the loads' latency needs the
 // warps.  On the 1M lattice an iteration issues about 60% of the time and
@@ -314,11 +303,11 @@ __device__ __forceinline__ void push_marked(const PhysDev& ph, const f32x2* __re
 template <typename Mask, int ROWS, bool ONE>
 __global__ void __launch_bounds__(512, 3)
 k_jacobi_tp(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t ncells,
-            const uint32_t* __restrict__ ct, const uint32_t* __restrict__ tp_cell,
+            const CellTable table, const uint32_t* __restrict__ tp_cell,
             const float2* __restrict__ qin, float2* __restrict__ qout,
             const uint32_t* __restrict__ run_if, uint4* __restrict__ rows) {
   if (run_if && *run_if == 0u) return;
-  const uint32_t ntp = __ldg(ct + ncells);
+  const uint32_t ntp = table.taking(ncells);
   const f32x2* __restrict__ q = reinterpret_cast<const f32x2*>(qin);
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ntp; t += gridDim.x * blockDim.x) {
     Rows R;
@@ -327,7 +316,7 @@ k_jacobi_tp(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t nce
       R = Rows{u.x, u.y, u.z, u.w};
     } else {
       const uint32_t c = tp_cell[t];
-      R = tp_rows(worlds.of(c), ct, c, t);
+      R = tp_rows(worlds.of(c), table, c, t);
       if (ROWS == 1) rows[t] = make_uint4(R.s0, R.s1, R.s2, R.len);
     }
     const f32x2 qi2 = q[t];
@@ -340,7 +329,7 @@ k_jacobi_tp(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t nce
 // The last iteration, one thread per frame particle (a grid-stride loop
 // over whole blocks of particles; the plain frames' grid covers them all):
 // the push (taking-part particles, from the compacted iterate q; ROWS 2: by
-// the neighbour rows that the iterations wrote, 0: from the capped table),
+// the neighbour rows that the iterations wrote, 0: from the cell table),
 // then gravity, integration, boundaries, the velocity clamp and the key
 // emission, and the rebin's tickets.  METRICS also writes the block's sums
 // for the surrogate's fallback gate to part[blockIdx.x * 8 + k]: [0] sum and
@@ -353,7 +342,7 @@ k_jacobi_tp(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t nce
 template <typename Mask, int ROWS, bool METRICS, bool ONE>
 __global__ void __launch_bounds__(512, METRICS ? 2 : 3)
 k_jacobi_final(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t n,
-               int do_push, const uint32_t* __restrict__ ct, const uint32_t* __restrict__ tp_of,
+               int do_push, const CellTable table, const uint32_t* __restrict__ tp_of,
                const uint32_t* __restrict__ cell_of, const uint4* __restrict__ rows,
                const float2* __restrict__ pin, const float2* __restrict__ qtp,
                float2* __restrict__ pout, const float2* __restrict__ vin,
@@ -393,7 +382,7 @@ k_jacobi_final(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t 
             const uint4 u = rows[t];
             R = Rows{u.x, u.y, u.z, u.w};
           } else {
-            R = tp_rows(w, ct, c, t);
+            R = tp_rows(w, table, c, t);
           }
           push_marked<Mask, METRICS>(ph, q, qi2, R, all_marks<Mask>(ph, q, qi2, R), ax, ay, pen);
         }
@@ -462,11 +451,11 @@ cudaError_t launch_solve_reference(const SolveArgs& a, cudaStream_t st) {
   const uint32_t blocks = (a.n + own - 1) / own;
   if (a.nworlds == 1)
     k_solve_reference<true><<<blocks, threads, 0, st>>>(
-        Worlds<true>{a.world}, a.ph, a.n, a.cell_start, a.cell_of, a.pos, a.vel, a.pos_out,
+        Worlds<true>{a.world}, a.ph, a.n, a.table, a.cell_of, a.pos, a.vel, a.pos_out,
         a.vel_out, a.keys, a.ctrl, a.count);
   else
     k_solve_reference<false><<<blocks, threads, 0, st>>>(
-        Worlds<false>{a.worlds, a.nworlds}, a.ph, a.n, a.cell_start, a.cell_of, a.pos, a.vel,
+        Worlds<false>{a.worlds, a.nworlds}, a.ph, a.n, a.table, a.cell_of, a.pos, a.vel,
         a.pos_out, a.vel_out, a.keys, a.ctrl, a.count);
   return cudaGetLastError();
 }
@@ -489,10 +478,10 @@ static void launch_iteration(const SolveArgs& a, uint32_t blocks, uint32_t threa
                              const float2* qin, float2* qout, cudaStream_t st) {
   if (ROWS == 2 || a.nworlds == 1) {  // the rows read back need no world
     k_jacobi_tp<Mask, ROWS, true><<<blocks, threads, 0, st>>>(
-        Worlds<true>{a.world}, a.ph, a.ncells, a.ct, a.tp_cell, qin, qout, a.run_if, a.rows);
+        Worlds<true>{a.world}, a.ph, a.ncells, a.table, a.tp_cell, qin, qout, a.run_if, a.rows);
   } else if constexpr (ROWS != 2) {
     k_jacobi_tp<Mask, ROWS, false><<<blocks, threads, 0, st>>>(
-        Worlds<false>{a.worlds, a.nworlds}, a.ph, a.ncells, a.ct, a.tp_cell, qin, qout, a.run_if,
+        Worlds<false>{a.worlds, a.nworlds}, a.ph, a.ncells, a.table, a.tp_cell, qin, qout, a.run_if,
         a.rows);
   }
 }
@@ -526,11 +515,11 @@ static void launch_final(const SolveArgs& a, uint32_t blocks, uint32_t threads, 
                          int do_push, cudaStream_t st) {
   if (a.nworlds == 1)
     k_jacobi_final<Mask, ROWS, METRICS, true><<<blocks, threads, 0, st>>>(
-        Worlds<true>{a.world}, a.ph, a.n, do_push, a.ct, a.tp_of, a.cell_of, a.rows, a.pos, qtp,
+        Worlds<true>{a.world}, a.ph, a.n, do_push, a.table, a.tp_of, a.cell_of, a.rows, a.pos, qtp,
         a.pos_out, a.vel, a.vel_out, a.keys, a.ctrl, a.run_if, a.part, a.count);
   else
     k_jacobi_final<Mask, ROWS, METRICS, false><<<blocks, threads, 0, st>>>(
-        Worlds<false>{a.worlds, a.nworlds}, a.ph, a.n, do_push, a.ct, a.tp_of, a.cell_of, a.rows,
+        Worlds<false>{a.worlds, a.nworlds}, a.ph, a.n, do_push, a.table, a.tp_of, a.cell_of, a.rows,
         a.pos, qtp, a.pos_out, a.vel, a.vel_out, a.keys, a.ctrl, a.run_if, a.part, a.count);
 }
 

@@ -584,23 +584,12 @@ constexpr uint32_t kK = kKnn;
 // each as (dx, dy, dvx, dvy) relative to the particle; then the own
 // velocity; zero padding to 64.  Positions and velocities are the frame's
 // binned state, compacted (tpp, tpv).
-__device__ __forceinline__ void knn_row(const WorldDev& w, const uint32_t* __restrict__ ct,
+__device__ __forceinline__ void knn_row(const WorldDev& w, const CellTable& table,
                                         const float2* __restrict__ tpp,
                                         const float2* __restrict__ tpv, uint32_t c, uint32_t t,
                                         uint32_t* row) {
-  uint32_t cx, cy;
-  cell_xy(w, c - w.cell_off, cx, cy);
-  const uint32_t x0 = cx > 0 ? cx - 1 : 0;
-  const uint32_t x1 = cx + 1 < w.gx ? cx + 1 : w.gx - 1;
   uint32_t rs[3], re[3];
-#pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    const int ny = (int)cy - 1 + r;
-    const bool ok = ny >= 0 && ny < (int)w.gy;
-    const uint32_t rb = w.cell_off + (uint32_t)(ok ? ny : 0) * w.gx;
-    rs[r] = ok ? ct[rb + x0] : 0u;
-    re[r] = ok ? ct[rb + x1 + 1] : 0u;
-  }
+  neighbour_rows(w, table, c, rs, re);
   const float2 pi = tpp[t], vi = tpv[t];
   float bd[kK];
   uint32_t bj[kK];
@@ -659,7 +648,7 @@ __device__ __forceinline__ void zero_row(uint32_t* row) {
 // cell) gets all zeros.
 __global__ void __launch_bounds__(256)
 k_knn_features(const WorldDev* __restrict__ worlds, int nworlds, uint32_t n,
-               const uint32_t* __restrict__ tp_of, const uint32_t* __restrict__ ct,
+               const uint32_t* __restrict__ tp_of, const CellTable table,
                const uint32_t* __restrict__ cell_of, const float2* __restrict__ tpp,
                const float2* __restrict__ tpv, uint16_t* __restrict__ x) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -671,7 +660,7 @@ k_knn_features(const WorldDev* __restrict__ worlds, int nworlds, uint32_t n,
     zero_row(row);
     return;
   }
-  knn_row(worlds[world_of_cell(worlds, nworlds, c)], ct, tpp, tpv, c, t, row);
+  knn_row(worlds[world_of_cell(worlds, nworlds, c)], table, tpp, tpv, c, t, row);
 }
 
 // Training samples of the binned frame: the features of the taking-part
@@ -680,15 +669,15 @@ k_knn_features(const WorldDev* __restrict__ worlds, int nworlds, uint32_t n,
 // plain solver's first iterations) into target.
 __global__ void __launch_bounds__(256)
 k_samples(const WorldDev* __restrict__ worlds, int nworlds, uint32_t ncells,
-          const uint32_t* __restrict__ ct, const uint32_t* __restrict__ tp_cell,
+          const CellTable table, const uint32_t* __restrict__ tp_cell,
           const float2* __restrict__ tpp, const float2* __restrict__ tpv,
           const float2* __restrict__ q, uint32_t stride, uint32_t phase, uint32_t rows,
           uint16_t* __restrict__ x, float2* __restrict__ target) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t t = phase + k * stride;
-  if (k >= rows || t >= __ldg(ct + ncells)) return;
+  if (k >= rows || t >= table.taking(ncells)) return;
   const uint32_t c = tp_cell[t];
-  knn_row(worlds[world_of_cell(worlds, nworlds, c)], ct, tpp, tpv, c, t,
+  knn_row(worlds[world_of_cell(worlds, nworlds, c)], table, tpp, tpv, c, t,
           reinterpret_cast<uint32_t*>(x + (size_t)k * kIn));
   const float2 p = tpp[t], v = q[t];
   target[k] = make_float2(v.x - p.x, v.y - p.y);
@@ -706,15 +695,14 @@ constexpr uint32_t kFuseThreads = 256;
 
 __global__ void __launch_bounds__(kFuseThreads, 3)
 k_surrogate_correct(MlpDev m, const WorldDev* __restrict__ worlds, int nworlds,
-                    uint32_t ncells, const uint32_t* __restrict__ cell_start,
-                    const uint32_t* __restrict__ ct, const uint32_t* __restrict__ tp_cell,
+                    uint32_t ncells, const CellTable table, const uint32_t* __restrict__ tp_cell,
                     const float2* __restrict__ tpp, const float2* __restrict__ tpv,
                     float2* __restrict__ q, float2* __restrict__ corr) {
   extern __shared__ __align__(16) uint8_t dyn[];
   SmemNet& s = *reinterpret_cast<SmemNet*>(dyn);
   uint32_t* sx = reinterpret_cast<uint32_t*>(dyn + sizeof(SmemNet));  // [256][kRow]
   load_net(m, s, nullptr);
-  const uint32_t ntp = __ldg(ct + ncells);
+  const uint32_t ntp = table.taking(ncells);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t g = lane >> 2, t4 = lane & 3;
   for (uint32_t base = blockIdx.x * kFuseThreads; base < ntp; base += gridDim.x * kFuseThreads) {
@@ -722,7 +710,7 @@ k_surrogate_correct(MlpDev m, const WorldDev* __restrict__ worlds, int nworlds,
     uint32_t* row = sx + threadIdx.x * kRow;
     if (t < ntp) {
       const uint32_t c = tp_cell[t];
-      knn_row(worlds[world_of_cell(worlds, nworlds, c)], ct, tpp, tpv, c, t, row);
+      knn_row(worlds[world_of_cell(worlds, nworlds, c)], table, tpp, tpv, c, t, row);
     } else {
       zero_row(row);
     }
@@ -752,7 +740,7 @@ k_surrogate_correct(MlpDev m, const WorldDev* __restrict__ worlds, int nworlds,
             q[idx] = make_float2(__fadd_rn(p.x, cxv), __fadd_rn(p.y, cyv));
             if (corr) {
               const uint32_t c = tp_cell[idx];
-              corr[cell_start[c] + (idx - ct[c])] = make_float2(cxv, cyv);
+              corr[table.start(c) + (idx - table.taking(c))] = make_float2(cxv, cyv);
             }
           }
         }
@@ -811,7 +799,7 @@ __device__ __forceinline__ void block_partials(float (&v)[5], float* __restrict_
 // of taking-part particles, [3] kinetic energy, [4] 0.
 __global__ void __launch_bounds__(256)
 k_penetration(const WorldDev* __restrict__ worlds, int nworlds, PhysDev ph, uint32_t n,
-              const uint32_t* __restrict__ cell_start, const uint32_t* __restrict__ cell_of,
+              const CellTable table, const uint32_t* __restrict__ cell_of,
               const float2* __restrict__ pos, const float2* __restrict__ vel,
               float* __restrict__ part) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -820,7 +808,7 @@ k_penetration(const WorldDev* __restrict__ worlds, int nworlds, PhysDev ph, uint
     const float2 v = vel[i];
     ke = __fmul_rn(0.5f, __fadd_rn(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y)));
     const uint32_t c = cell_of[i];
-    if (i - cell_start[c] < ph.cap) {
+    if (i - table.start(c) < ph.cap) {
       cnt = 1.f;
       const WorldDev w = worlds[world_of_cell(worlds, nworlds, c)];
       uint32_t cx, cy;
@@ -831,8 +819,9 @@ k_penetration(const WorldDev* __restrict__ worlds, int nworlds, PhysDev ph, uint
       for (int ny = y0; ny <= y1; ++ny) {
         const uint32_t rb = w.cell_off + (uint32_t)ny * w.gx;
         for (int nx = x0; nx <= x1; ++nx) {
-          const uint32_t js = cell_start[rb + nx];
-          const uint32_t je = min(cell_start[rb + nx + 1], js + ph.cap);
+          uint32_t js, je;
+          table.span(rb + nx, js, je);
+          je = min(je, js + ph.cap);
           for (uint32_t j = js; j < je; ++j) {
             if (j == i) continue;
             const float2 pj = pos[j];
@@ -915,12 +904,12 @@ k_gate(const float* __restrict__ part, uint32_t nparts, GateState* __restrict__ 
 // Squared errors of the correction against the target, and of zero against
 // the target, over taking-part particles: out[0] += |corr - t|^2,
 // out[1] += |t|^2, out[2] += count.
-__global__ void k_errors(PhysDev ph, uint32_t n, const uint32_t* __restrict__ cell_start,
-                         const uint32_t* __restrict__ cell_of, const float2* __restrict__ corr,
-                         const float2* __restrict__ target, float* __restrict__ out) {
+__global__ void k_errors(uint32_t n, const uint32_t* __restrict__ tp_of,
+                         const float2* __restrict__ corr, const float2* __restrict__ target,
+                         float* __restrict__ out) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   float e = 0.f, z = 0.f, c = 0.f;
-  if (i < n && i - cell_start[cell_of[i]] < ph.cap) {
+  if (i < n && tp_of[i] != kNoTp) {
     const float2 a = corr[i], t = target[i];
     e = (a.x - t.x) * (a.x - t.x) + (a.y - t.y) * (a.y - t.y);
     z = t.x * t.x + t.y * t.y;
@@ -944,14 +933,13 @@ __global__ void k_errors(PhysDev ph, uint32_t n, const uint32_t* __restrict__ ce
 cudaError_t launch_errors(const SolveArgs& a, const float2* corr, const float2* target, float* out,
                           cudaStream_t st) {
   if (a.n == 0) return cudaSuccess;
-  k_errors<<<(a.n + 255) / 256, 256, 0, st>>>(a.ph, a.n, a.cell_start, a.cell_of, corr, target,
-                                              out);
+  k_errors<<<(a.n + 255) / 256, 256, 0, st>>>(a.n, a.tp_of, corr, target, out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_knn_features(const SolveArgs& a, uint16_t* x, cudaStream_t st) {
   if (a.n == 0) return cudaSuccess;
-  k_knn_features<<<(a.n + 255) / 256, 256, 0, st>>>(a.worlds, a.nworlds, a.n, a.tp_of, a.ct,
+  k_knn_features<<<(a.n + 255) / 256, 256, 0, st>>>(a.worlds, a.nworlds, a.n, a.tp_of, a.table,
                                                     a.cell_of, a.tp_pos, a.tp_vel, x);
   return cudaGetLastError();
 }
@@ -959,7 +947,7 @@ cudaError_t launch_knn_features(const SolveArgs& a, uint16_t* x, cudaStream_t st
 cudaError_t launch_samples(const SolveArgs& a, const float2* q, uint32_t stride, uint32_t phase,
                            uint32_t rows, uint16_t* x, float2* target, cudaStream_t st) {
   if (rows == 0) return cudaSuccess;
-  k_samples<<<(rows + 255) / 256, 256, 0, st>>>(a.worlds, a.nworlds, a.ncells, a.ct, a.tp_cell,
+  k_samples<<<(rows + 255) / 256, 256, 0, st>>>(a.worlds, a.nworlds, a.ncells, a.table, a.tp_cell,
                                                 a.tp_pos, a.tp_vel, q, stride, phase, rows, x,
                                                 target);
   return cudaGetLastError();
@@ -984,7 +972,7 @@ cudaError_t launch_surrogate_correct(const MlpDev& m, const SolveArgs& a, float2
   if (a.n == 0) return cudaSuccess;
   const int need = (int)((a.n + kFuseThreads - 1) / kFuseThreads);
   k_surrogate_correct<<<need < blocks ? need : blocks, kFuseThreads, correct_smem(), st>>>(
-      m, a.worlds, a.nworlds, a.ncells, a.cell_start, a.ct, a.tp_cell, a.tp_pos, a.tp_vel, q,
+      m, a.worlds, a.nworlds, a.ncells, a.table, a.tp_cell, a.tp_pos, a.tp_vel, q,
       corr);
   return cudaGetLastError();
 }
@@ -1038,7 +1026,7 @@ cudaError_t launch_penetration(const SolveArgs& a, const float2* pos, const floa
                                float* part, float* out, cudaStream_t st) {
   const uint32_t blocks = (a.n + 255) / 256;
   if (blocks) {
-    k_penetration<<<blocks, 256, 0, st>>>(a.worlds, a.nworlds, a.ph, a.n, a.cell_start, a.cell_of,
+    k_penetration<<<blocks, 256, 0, st>>>(a.worlds, a.nworlds, a.ph, a.n, a.table, a.cell_of,
                                           pos, vel, part);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;

@@ -71,7 +71,6 @@ int enqueue_rebin(WrachContext* ctx) {
   r.dst_capacity = ctx->total_cap;
   r.pos_src = ctx->pos_o;
   r.vel_src = ctx->vel_o;
-  r.cs_new = ctx->cs[ctx->cur ^ 1];
   r.pos_dst = ctx->pos;
   r.vel_dst = ctx->vel;
   r.cell_dst = ctx->cell_of[ctx->cur ^ 1];
@@ -287,8 +286,15 @@ int wrach_surrogate_collect(WrachContext* ctx, uint32_t stride, uint32_t* total)
   // offset that turns with each call, so that consecutive frames give others
   uint32_t ntp = 0;
   if (ctx->n) {
-    CK(cudaMemcpyAsync(&ntp, a.ct + ctx->ncells, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    // taking(ncells)
+    uint32_t g[4] = {0u, 0u, 0u, 0u};
+    const bool grouped = a.table.groups != nullptr;
+    CK(cudaMemcpyAsync(g, grouped ? (const void*)(a.table.groups + ctx->ncells / wrach::kGroup)
+                                  : (const void*)(a.table.takes + ctx->ncells),
+                       grouped ? sizeof(g) : 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    const uint32_t j = ctx->ncells % wrach::kGroup;
+    ntp = grouped ? (g[1] & ~wrach::kWide) + ((g[2 + j / 4] >> (8 * (j % 4))) & 0xFFu) : g[0];
   }
   const uint32_t phase = S.collects++ % stride;
   const uint32_t rows = ntp > phase ? (ntp - phase + stride - 1) / stride : 0u;

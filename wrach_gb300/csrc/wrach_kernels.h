@@ -19,7 +19,7 @@ struct SolveArgs {
   PhysDev ph;
   uint32_t ncells;              // cells over all worlds
   uint32_t n;                   // particles over all worlds
-  const uint32_t* cell_start;   // ncells + 1
+  CellTable table;              // of the binned frame
   const uint32_t* cell_of;      // n, cell of each binned particle
   const float2* pos;            // binned state
   const float2* vel;
@@ -33,7 +33,6 @@ struct SolveArgs {
   float* part;                  // final extended pass: per-block metrics, 8 floats a block (optional)
   CountDev count;               // last solve launch: the rebin's tickets (extended: if count.ticket is set)
   // the frame's taking-part particles, compacted (extended physics)
-  const uint32_t* ct;           // ncells + 1: capped table
   const uint32_t* tp_of;        // n: compacted index of each frame particle (kNoTp: none)
   const uint32_t* tp_cell;      // cell of each compacted particle
   const float2* tp_pos;         // compacted positions of the binned state
@@ -41,7 +40,7 @@ struct SolveArgs {
   int sms;                      // SMs of the device
   // extended iterations (optional): each compacted taking-part particle's
   // three neighbour rows (total_cap entries); rows_mode 0 computes the rows
-  // from the capped table, 1 also writes them, 2 reads them
+  // from the cell table, 1 also writes them, 2 reads them
   uint4* rows;
   int rows_mode;
 };
@@ -70,7 +69,7 @@ struct RebinArgs {
   const uint32_t* keys;         // n source keys, ncells = leave out
   const float2* pos_src;
   const float2* vel_src;
-  uint32_t* cs_new;             // ncells + 1
+  uint32_t* cs_new;             // ncells + 1: cell starts
   float2* pos_dst;
   float2* vel_dst;
   uint32_t* cell_dst;
@@ -92,15 +91,18 @@ struct RebinArgs {
   uint32_t* idx_alt;            // n: scratch of the in-memory sort of very large cells
   uint32_t* big_list;           // big_cap: cells of more than kSmallCell particles
   uint32_t big_cap;
+  // the cell table: the records of a grouped one (null: dense; cs_new holds
+  // the starts), the taking-part particles' starts of a dense one
+  uint4* groups_new;
+  uint32_t* ct_new;
+  uint32_t prefixed_tiles;      // scan step: tiles whose sums are prefixes (set by it; 0: none)
   // the taking-part particles, compacted (extended physics; tp_cap == 0: none)
   uint32_t tp_cap;              // cell capacity: the first tp_cap of a cell take part
   uint32_t* tile_sums_cap;      // per scan tile, its taking-part particles (zero between rebins)
-  uint32_t* ct_new;             // ncells + 1: capped table (compacted start of each cell)
   float2* tp_pos;               // compacted positions
   float2* tp_vel;               // compacted velocities
   uint32_t* tp_cell;            // compacted cells
   uint32_t* tp_of;              // compacted index of each slot (kNoTp: takes no part)
-  uint32_t tiles_prefixed;      // scan step: tile sums already turned into prefixes (set by it)
 };
 
 constexpr uint32_t kRebinThreads = 256;
@@ -164,9 +166,9 @@ cudaError_t launch_wait_probe(const uint32_t* word, uint32_t value, uint64_t lim
 cudaError_t launch_local_keys(const uint32_t* cell_of, uint32_t n, uint32_t cell_off,
                               uint32_t* out, cudaStream_t st);
 
-// Reference-layout table of one world (cells + 2 entries) from the global
-// cell-start table.
-cudaError_t launch_world_table(const uint32_t* cell_start, uint32_t cell_off,
+// Reference-layout table of one world (cells + 2 entries) from the cell
+// table.
+cudaError_t launch_world_table(const CellTable& table, uint32_t cell_off,
                                uint32_t cells, uint32_t* out, cudaStream_t st);
 
 // The surrogate network (surrogate.cu): FP32 master parameters in the order

@@ -13,9 +13,9 @@
 //   cell_of[2]        cell of each binned particle (u32)
 //   cs[2], ct[2] or groups[2]
 //                     the cell table (CellTable; ping-pong per frame)
-//   tp_pos[2], tp_vel[2], tp_cell[2], tp_of[2]
+//   tp_pos[2], tp_cell[2], tp_of[2]; tp_vel[2] with a surrogate
 //                     extended physics: the taking-part particles' positions,
-//                     velocities and cells, compacted in cell order, and each
+//                     cells and velocities, compacted in cell order, and each
 //                     frame particle's place among them
 //   keys              next cell of each solve output (u32)
 //   kA kB iA iB       rebin scratch (tickets, slot cells, slot sources, sort ping-pong)
@@ -82,20 +82,6 @@ uint32_t bits_for(uint32_t v) {
 
 
 namespace {
-
-void drop_graphs(WrachContext* ctx) {
-  for (auto& g : ctx->graph)
-    if (g) {
-      cudaGraphExecDestroy(g);
-      g = nullptr;
-    }
-  for (auto& row : ctx->sur.graph)
-    for (auto& g : row)
-      if (g) {
-        cudaGraphExecDestroy(g);
-        g = nullptr;
-      }
-}
 
 void release(WrachContext* ctx) {
   drop_graphs(ctx);
@@ -191,6 +177,20 @@ int ensure_store(WrachContext* ctx, Store& s, size_t need) {
 
 namespace wrach {
 namespace host {
+
+void drop_graphs(WrachContext* ctx) {
+  for (auto& g : ctx->graph)
+    if (g) {
+      cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
+  for (auto& row : ctx->sur.graph)
+    for (auto& g : row)
+      if (g) {
+        cudaGraphExecDestroy(g);
+        g = nullptr;
+      }
+}
 
 int fail(WrachContext* c, int code, const std::string& msg) {
   if (c) c->err = msg;
@@ -527,7 +527,6 @@ int create_impl(const WrachConfig* config, uint32_t nworlds, const float* dims,
   if (c.mode == WRACH_MODE_EXTENDED) {
     for (int i = 0; i < 2; ++i) {
       if ((e = dalloc(&ctx->tp_pos[i], tc + wrach::kRowPad)) != cudaSuccess) return oom(e);
-      if ((e = dalloc(&ctx->tp_vel[i], tc)) != cudaSuccess) return oom(e);
       if ((e = dalloc(&ctx->tp_cell[i], tc)) != cudaSuccess) return oom(e);
       if ((e = dalloc(&ctx->tp_of[i], tc)) != cudaSuccess) return oom(e);
     }

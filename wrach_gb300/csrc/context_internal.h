@@ -64,7 +64,7 @@ struct WrachContext {
   uint32_t* tile_sums = nullptr;  // one word per tile of the cell table
   // extended physics: the taking-part particles compacted (ping-pong with cs)
   float2* tp_pos[2] = {nullptr, nullptr};     // compacted positions
-  float2* tp_vel[2] = {nullptr, nullptr};     // compacted velocities
+  float2* tp_vel[2] = {nullptr, nullptr};     // compacted velocities (with a surrogate)
   uint32_t* tp_cell[2] = {nullptr, nullptr};  // compacted cells
   uint32_t* tp_of[2] = {nullptr, nullptr};    // compacted index of each frame particle
   uint32_t* tile_sums_cap = nullptr;          // per scan tile, taking-part particles
@@ -135,6 +135,9 @@ cudaError_t dalloc(T** p, size_t count) {
 }
 
 void dfree(void* p);
+
+// Destroys the captured frames (their launches' arguments are out of date).
+void drop_graphs(WrachContext* ctx);
 
 // Makes `dev` current for the scope of a C ABI call.
 struct DeviceGuard {

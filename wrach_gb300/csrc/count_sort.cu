@@ -26,8 +26,8 @@
 //   place    the stable order: inside a cell, a particle's rank is the number
 //            of the cell's particles with a smaller source index; then the
 //            gather of positions, velocities and cells into that slot, and of
-//            the taking-part particles' positions, velocities and cells into
-//            the compacted arrays.  Cells of up to kSmallCell particles are
+//            the taking-part particles' positions, cells and (for the learned
+//            surrogate) velocities into the compacted arrays.  Cells of up to kSmallCell particles are
 //            ranked by one thread per slot
 //   cells    one block per listed cell: up to kBigCell particles a bitonic
 //            sort of the source indices in shared memory, more than that a
@@ -383,7 +383,7 @@ __device__ __forceinline__ void place_one(const RebinArgs& a, uint32_t slot, uin
       a.tp_of[slot] = t;
       if (t < a.dst_capacity) {
         a.tp_pos[t] = p;
-        a.tp_vel[t] = v;
+        if (a.tp_vel) a.tp_vel[t] = v;
         a.tp_cell[t] = cell;
       }
     }
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(256) k_cs_place(RebinArgs a) {
         a.tp_of[slot] = t;
         if (t < a.dst_capacity) {
           a.tp_pos[t] = p;
-          a.tp_vel[t] = v;
+          if (a.tp_vel) a.tp_vel[t] = v;
           a.tp_cell[t] = k;
         }
       }

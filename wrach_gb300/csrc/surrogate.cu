@@ -638,6 +638,13 @@ __device__ __forceinline__ void knn_row(const WorldDev& w, const CellTable& tabl
   for (uint32_t k = 2 * kK + 1; k < kIn / 2; ++k) row[k] = 0u;
 }
 
+__global__ void k_compact_velocities(uint32_t n, const uint32_t* __restrict__ tp_of,
+                                     const float2* __restrict__ vel,
+                                     float2* __restrict__ tp_vel) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n && tp_of[i] != kNoTp) tp_vel[tp_of[i]] = vel[i];
+}
+
 __device__ __forceinline__ void zero_row(uint32_t* row) {
 #pragma unroll
   for (uint32_t k = 0; k < kIn / 2; ++k) row[k] = 0u;
@@ -934,6 +941,13 @@ cudaError_t launch_errors(const SolveArgs& a, const float2* corr, const float2* 
                           cudaStream_t st) {
   if (a.n == 0) return cudaSuccess;
   k_errors<<<(a.n + 255) / 256, 256, 0, st>>>(a.n, a.tp_of, corr, target, out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_compact_velocities(uint32_t n, const uint32_t* tp_of, const float2* vel,
+                                      float2* tp_vel, cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  k_compact_velocities<<<(n + 255) / 256, 256, 0, st>>>(n, tp_of, vel, tp_vel);
   return cudaGetLastError();
 }
 

@@ -141,6 +141,22 @@ int wrach_surrogate_init(WrachContext* ctx, uint32_t seed, uint32_t max_samples)
                 "the surrogate replaces iterations of the extended solve: mode EXTENDED, iterations >= 2");
   DeviceGuard guard(ctx->device);
   auto& S = ctx->sur;
+  if (!ctx->tp_vel[0]) {
+    // from here on the rebins also write the taking-part particles' velocities
+    float2* tv[2] = {nullptr, nullptr};
+    CK(dalloc(&tv[0], ctx->total_cap));
+    const cudaError_t e = dalloc(&tv[1], ctx->total_cap);
+    if (e != cudaSuccess) {
+      dfree(tv[0]);
+      CK(e);
+    }
+    ctx->tp_vel[0] = tv[0];
+    ctx->tp_vel[1] = tv[1];
+    drop_graphs(ctx);
+    CK(launch_compact_velocities(ctx->n, ctx->tp_of[ctx->cur], ctx->vel, ctx->tp_vel[ctx->cur],
+                                 ctx->stream));
+    ctx->launches += ctx->n ? 1 : 0;
+  }
   if (!S.ready) {
     const size_t nbf = (size_t)2 * (2 * kMlpIn * kMlpHidden + kMlpHidden * kMlpOutPad);
     CK(dalloc(&S.params, kMlpParams));

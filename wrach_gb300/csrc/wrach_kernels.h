@@ -36,7 +36,7 @@ struct SolveArgs {
   const uint32_t* tp_of;        // n: compacted index of each frame particle (kNoTp: none)
   const uint32_t* tp_cell;      // cell of each compacted particle
   const float2* tp_pos;         // compacted positions of the binned state
-  const float2* tp_vel;         // compacted velocities of the binned state
+  const float2* tp_vel;         // compacted velocities of the binned state (with a surrogate)
   int sms;                      // SMs of the device
   // extended iterations (optional): each compacted taking-part particle's
   // three neighbour rows (total_cap entries); rows_mode 0 computes the rows
@@ -100,7 +100,7 @@ struct RebinArgs {
   uint32_t tp_cap;              // cell capacity: the first tp_cap of a cell take part
   uint32_t* tile_sums_cap;      // per scan tile, its taking-part particles (zero between rebins)
   float2* tp_pos;               // compacted positions
-  float2* tp_vel;               // compacted velocities
+  float2* tp_vel;               // compacted velocities (optional)
   uint32_t* tp_cell;            // compacted cells
   uint32_t* tp_of;              // compacted index of each slot (kNoTp: takes no part)
 };
@@ -205,6 +205,10 @@ struct GateState {
   uint32_t pad[6];
 };
 
+// The compacted velocities of the n particles of the binned frame, for a
+// surrogate set up between rebins (which write them from then on).
+cudaError_t launch_compact_velocities(uint32_t n, const uint32_t* tp_of, const float2* vel,
+                                      float2* tp_vel, cudaStream_t st);
 cudaError_t launch_knn_features(const SolveArgs& a, uint16_t* x, cudaStream_t st);
 // Training rows of the binned frame: the features of the taking-part
 // particles t = phase + k * stride into rows k of x (at most `rows`) and

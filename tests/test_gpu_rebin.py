@@ -70,6 +70,29 @@ def test_floor_pile(W, O):
     assert st["huge_cells"] == 0
 
 
+@pytest.mark.parametrize("count", [65, 255, 256, 257, 513, 2048])
+@pytest.mark.parametrize("pages", [2, 3, 31, 32, 33, 60])
+def test_large_cell_sources_over_pages(W, O, count, pages):
+    # the sources of one large cell spread over `pages` runs of 1024 indices
+    # (up to 32 of them are ranked by a bitmap, more are sorted), at both ends
+    # and in the middle of each, and a second large cell after it
+    rng = np.random.default_rng(count + pages)
+    n = pages * 1024
+    pos = np.column_stack([rng.uniform(8, 60, n), rng.uniform(8, 40, n)]).astype(np.float32)
+    per = np.full(pages, count // pages)
+    per[: count % pages] += 1
+    for p, m in enumerate(per):
+        ends = [0, 1023, 31, 32]
+        pick = np.concatenate([ends, rng.permutation(np.setdiff1d(np.arange(1024), ends))])[:m]
+        pos[p * 1024 + pick] = np.column_stack([rng.uniform(3, 3.9, m), rng.uniform(2, 2.9, m)])
+    free = np.nonzero(pos[:, 0] >= 8)[0]
+    free = free[:90]
+    pos[free] = np.column_stack([rng.uniform(5, 5.9, len(free)), rng.uniform(2, 2.9, len(free))])
+    vel = rng.normal(0, 0.2, pos.shape).astype(np.float32)
+    st = _run(W, O, (64.0, 48.0), pos, vel, 1, 2, gravity=0.1)
+    assert st["huge_cells"] == 0
+
+
 def test_profiled_frames_match_graph_frames(W, O):
     # a profiled frame runs its launches one at a time on the frame's stream
     # (the large cells' sort included); graph frames run that sort on a

@@ -302,3 +302,50 @@ def test_surrogate_frames_hold_the_error_bounds(W):
     assert drift <= 0.01
     assert ms[:, 0].mean() - mp[:, 0].mean() <= 0.05
     assert abs(ms[:, 2].mean() / mp[:, 2].mean() - 1.0) <= 0.01
+
+
+def test_features_of_few_and_many_candidates(W):
+    # 0 .. 30 candidates around a particle (listed up to 12, inserted from 13
+    # on), equal distances and a candidate at a NaN distance, against the
+    # oracle; the fused pass reads the same rows through the network
+    torch = _torch()
+    rng = np.random.default_rng(31)
+    dims = (96.0, 60.0)
+    parts = []
+    for k in range(32):  # groups of k + 1, away from one another
+        at = np.array([6.0 * (k % 8) + 2, 6.0 * (k // 8) + 2])
+        parts.append(at + rng.uniform(-0.9, 0.9, (k + 1, 2)))
+    grid = np.stack(np.meshgrid(np.arange(5), np.arange(5)), -1).reshape(-1, 2) * 0.5 + (60.25, 30.25)
+    parts += [grid, rng.uniform((50, 40), (95, 59), (300, 2))]
+    pos = np.concatenate(parts).astype(np.float32)
+    vel = rng.normal(0, 0.7, pos.shape).astype(np.float32)
+    # one candidate whose distance is NaN (binned into cell 0)
+    pos[-2:] = [(np.nan, 0.4), (0.5, 0.6)]
+    with _sim(W, dims, 4000) as sim:
+        sim.set_particles(pos, vel)
+        sim.surrogate_init(0, 16)
+        p, v, table = sim.read_frame()
+        n = len(p)
+        x = torch.zeros((n, 64), dtype=torch.int16, device="cuda")
+        torch.cuda.synchronize()
+        sim.surrogate_features(x.data_ptr(), n)
+        sim.sync()
+        s = sim.settings()
+        corner = (p < 3.2).all(1) | np.isnan(p).any(1)  # where the NaN is a candidate
+        want = M.bf16_bits(M.features(s.grid_dimensions[0], s.grid_dimensions[1], 9, table, p, v))
+        got = x.cpu().numpy().view(np.uint16)
+        keep = ~corner
+        assert keep.sum() > 400
+        assert np.array_equal(got[keep], want[keep])
+        # the NaN candidate is left out: no neighbours, then the own velocity
+        lone = np.nonzero((p == np.float32([0.5, 0.6])).all(1))[0][0]
+        assert not got[lone, :48].any()
+        assert np.array_equal(got[lone, 48:50], M.bf16_bits(v[lone]))
+        corr = torch.zeros((n, 2), dtype=torch.float32, device="cuda")
+        y = torch.zeros((n, 2), dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
+        sim.surrogate_correction(corr.data_ptr())
+        sim.surrogate_forward(x.data_ptr(), n, y.data_ptr(), kernel="mma")
+        sim.sync()
+        taking = (got != 0).any(1) & keep
+        assert np.array_equal(corr.cpu().numpy()[taking], y.cpu().numpy()[taking])

@@ -507,7 +507,7 @@ __device__ uint32_t* block_radix_sort(uint32_t* src, uint32_t* alt, uint32_t m, 
 // The ranks of a large cell's source indices from a bitmap.  A pile's
 // particles come from its own cell and those around it, so their sources lie
 // in few pages of kPageBits indices, one word of bits per 32: the rank of an
-// index is the number of bits before its own.  Nine barriers for a cell of
+// index is the number of bits before its own.  Seven barriers for a cell of
 // any size, where the bitonic sort takes 45 for 512 indices (the collapsed 1M
 // lattice: 33 us sorting, 16 us now; 4M particles: 122 and 49 us).  Cells whose indices lie in more than
 // kPages pages (uploads in any order) are sorted.

@@ -171,56 +171,67 @@ __device__ __forceinline__ uint32_t lds_keep(const uint32_t* p) {
   return v;
 }
 
-// The forward pass of a 16-row tile for inference only: the same products in
-// the same order as mlp_tile_forward, computed two n-tiles at a time so that
-// no pre-activation array stays live, with the GELU on packed FP16 pairs
+// The forward pass of TILES 16-row tiles for inference only: the same products
+// in the same order as mlp_tile_forward, computed two n-tiles at a time so
+// that no pre-activation array stays live, with the GELU on packed FP16 pairs
 // (gelu2_bf16; the training pass keeps the FP32 GELU and its derivative).
-__device__ __forceinline__ void mlp_tile_infer(const SmemNet& s, uint32_t lane,
-                                               const uint32_t (&ax)[4][4], float (&y)[4]) {
+// Each weight fragment read from shared memory serves all TILES tiles: with
+// one tile the 17 KB of fragments per 16 rows bound the kernels by shared
+// memory's bandwidth.
+template <uint32_t TILES>
+__device__ __forceinline__ void infer_layer(const uint32_t* wt, const float* b, uint32_t lane,
+                                            const uint32_t (&in)[TILES][4][4],
+                                            uint32_t (&out)[TILES][4][4]) {
   const uint32_t g = lane >> 2, t = lane & 3;
-  uint32_t h1[4][4], h2[4][4];
 #pragma unroll
   for (uint32_t kq = 0; kq < 4; ++kq) {
-    float z[2][4];
+    float z[TILES][2][4];
 #pragma unroll
     for (uint32_t u = 0; u < 2; ++u) {
       const uint32_t nt = 2 * kq + u;
-      const float bl = s.b1[nt * 8 + 2 * t], bh = s.b1[nt * 8 + 2 * t + 1];
-      z[u][0] = bl; z[u][1] = bh; z[u][2] = bl; z[u][3] = bh;
-      const uint32_t* row = s.w1t + (nt * 8 + g) * kRow + t;
+      const float bl = b[nt * 8 + 2 * t], bh = b[nt * 8 + 2 * t + 1];
 #pragma unroll
-      for (uint32_t kk = 0; kk < 4; ++kk)
-        mma_bf16(z[u], ax[kk], lds_keep(row + kk * 8), lds_keep(row + kk * 8 + 4));
+      for (uint32_t r = 0; r < TILES; ++r) {
+        z[r][u][0] = bl; z[r][u][1] = bh; z[r][u][2] = bl; z[r][u][3] = bh;
+      }
+      const uint32_t* row = wt + (nt * 8 + g) * kRow + t;
+#pragma unroll
+      for (uint32_t kk = 0; kk < 4; ++kk) {
+        const uint32_t b0 = lds_keep(row + kk * 8), b1 = lds_keep(row + kk * 8 + 4);
+#pragma unroll
+        for (uint32_t r = 0; r < TILES; ++r) mma_bf16(z[r][u], in[r][kk], b0, b1);
+      }
     }
-    h1[kq][0] = gelu2_bf16(z[0][0], z[0][1]);
-    h1[kq][1] = gelu2_bf16(z[0][2], z[0][3]);
-    h1[kq][2] = gelu2_bf16(z[1][0], z[1][1]);
-    h1[kq][3] = gelu2_bf16(z[1][2], z[1][3]);
-  }
 #pragma unroll
-  for (uint32_t kq = 0; kq < 4; ++kq) {
-    float z[2][4];
-#pragma unroll
-    for (uint32_t u = 0; u < 2; ++u) {
-      const uint32_t nt = 2 * kq + u;
-      const float bl = s.b2[nt * 8 + 2 * t], bh = s.b2[nt * 8 + 2 * t + 1];
-      z[u][0] = bl; z[u][1] = bh; z[u][2] = bl; z[u][3] = bh;
-      const uint32_t* row = s.w2t + (nt * 8 + g) * kRow + t;
-#pragma unroll
-      for (uint32_t kk = 0; kk < 4; ++kk)
-        mma_bf16(z[u], h1[kk], lds_keep(row + kk * 8), lds_keep(row + kk * 8 + 4));
+    for (uint32_t r = 0; r < TILES; ++r) {
+      out[r][kq][0] = gelu2_bf16(z[r][0][0], z[r][0][1]);
+      out[r][kq][1] = gelu2_bf16(z[r][0][2], z[r][0][3]);
+      out[r][kq][2] = gelu2_bf16(z[r][1][0], z[r][1][1]);
+      out[r][kq][3] = gelu2_bf16(z[r][1][2], z[r][1][3]);
     }
-    h2[kq][0] = gelu2_bf16(z[0][0], z[0][1]);
-    h2[kq][1] = gelu2_bf16(z[0][2], z[0][3]);
-    h2[kq][2] = gelu2_bf16(z[1][0], z[1][1]);
-    h2[kq][3] = gelu2_bf16(z[1][2], z[1][3]);
   }
+}
+
+template <uint32_t TILES>
+__device__ __forceinline__ void mlp_infer(const SmemNet& s, uint32_t lane,
+                                          const uint32_t (&ax)[TILES][4][4],
+                                          float (&y)[TILES][4]) {
+  const uint32_t g = lane >> 2, t = lane & 3;
+  uint32_t h1[TILES][4][4], h2[TILES][4][4];
+  infer_layer<TILES>(s.w1t, s.b1, lane, ax, h1);
+  infer_layer<TILES>(s.w2t, s.b2, lane, h1, h2);
   const float bl = s.b3[2 * t], bh = s.b3[2 * t + 1];
-  y[0] = bl; y[1] = bh; y[2] = bl; y[3] = bh;
+#pragma unroll
+  for (uint32_t r = 0; r < TILES; ++r) {
+    y[r][0] = bl; y[r][1] = bh; y[r][2] = bl; y[r][3] = bh;
+  }
   const uint32_t* row = s.w3t + g * kRow + t;
 #pragma unroll
-  for (uint32_t kk = 0; kk < 4; ++kk)
-    mma_bf16(y, h2[kk], lds_keep(row + kk * 8), lds_keep(row + kk * 8 + 4));
+  for (uint32_t kk = 0; kk < 4; ++kk) {
+    const uint32_t b0 = lds_keep(row + kk * 8), b1 = lds_keep(row + kk * 8 + 4);
+#pragma unroll
+    for (uint32_t r = 0; r < TILES; ++r) mma_bf16(y[r], h2[r][kk], b0, b1);
+  }
 }
 
 // A fragment (4 k-tiles) of 16 rows of X (BF16 [rows][64]); rows past n read
@@ -246,16 +257,22 @@ __global__ void __launch_bounds__(128) k_mlp_forward(MlpDev m, const uint16_t* _
   load_net(m, s, nullptr);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t g = lane >> 2, t = lane & 3;
-  const uint32_t tiles = (n + 15) / 16;
-  for (uint32_t tile = blockIdx.x * 4 + warp; tile < tiles; tile += gridDim.x * 4) {
-    uint32_t ax[4][4];
-    float out[4];
-    load_x_tile(x, tile * 16, n, lane, ax);
-    mlp_tile_infer(s, lane, ax, out);
+  constexpr uint32_t kTiles = 2;
+  const uint32_t groups = (n + 16 * kTiles - 1) / (16 * kTiles);
+  for (uint32_t group = blockIdx.x * 4 + warp; group < groups; group += gridDim.x * 4) {
+    uint32_t ax[kTiles][4][4];
+    float out[kTiles][4];
+#pragma unroll
+    for (uint32_t r = 0; r < kTiles; ++r)
+      load_x_tile(x, (group * kTiles + r) * 16, n, lane, ax[r]);
+    mlp_infer<kTiles>(s, lane, ax, out);
     if (t == 0) {
-      const uint32_t r0 = tile * 16 + g, r1 = r0 + 8;
-      if (r0 < n) y[r0] = make_float2(out[0], out[1]);
-      if (r1 < n) y[r1] = make_float2(out[2], out[3]);
+#pragma unroll
+      for (uint32_t r = 0; r < kTiles; ++r) {
+        const uint32_t r0 = (group * kTiles + r) * 16 + g, r1 = r0 + 8;
+        if (r0 < n) y[r0] = make_float2(out[r][0], out[r][1]);
+        if (r1 < n) y[r1] = make_float2(out[r][2], out[r][3]);
+      }
     }
   }
 }
@@ -574,16 +591,44 @@ __global__ void k_adam(MlpDev m, const float* __restrict__ grad, float* __restri
 // Features
 // ---------------------------------------------------------------------------
 
-constexpr uint32_t kK = kKnn;
+constexpr uint32_t kK = kKnn, kBatch = 4;
+static_assert(kK % kBatch == 0, "whole batches");
+
+// 32 words of a feature row, from registers: 16 bytes at a time into shared
+// memory, where 8 lanes' rows (144 bytes apart) then cover all banks, and 4
+// into a caller's global buffer, which may start anywhere.
+template <bool SHARED>
+__device__ __forceinline__ void set_row(uint32_t* row, const uint32_t (&w)[kIn / 2]) {
+  if (SHARED) {
+#pragma unroll
+    for (uint32_t k = 0; k < kIn / 8; ++k)
+      reinterpret_cast<uint4*>(row)[k] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+  } else {
+#pragma unroll
+    for (uint32_t k = 0; k < kIn / 2; ++k) row[k] = w[k];
+  }
+}
+
+template <bool SHARED>
+__device__ __forceinline__ void zero_row(uint32_t* row) {
+  const uint32_t w[kIn / 2] = {};
+  set_row<SHARED>(row, w);
+}
 
 // Features of the taking-part particle of compacted index t (cell c) into
-// `row` (32 words, global or shared memory): the 12 nearest taking-part
-// particles in the 3x3 cells around its cell -- the candidates of its Jacobi
-// iterations, one contiguous compacted range per neighbour row -- by binary32
-// squared distance (each product and sum rounded on its own), ties by index;
-// each as (dx, dy, dvx, dvy) relative to the particle; then the own
-// velocity; zero padding to 64.  Positions and velocities are the frame's
-// binned state, compacted (tpp, tpv).
+// `row` (32 words): the 12 nearest taking-part particles in the 3x3 cells
+// around its cell -- the candidates of its Jacobi iterations, one contiguous
+// compacted range per neighbour row -- by binary32 squared distance (each
+// product and sum rounded on its own), ties by index; each as (dx, dy, dvx,
+// dvy) relative to the particle; then the own velocity; zero padding to 64.
+// A candidate at a NaN or infinite distance is left out.  Positions and
+// velocities are the frame's binned state, compacted (tpp, tpv).
+//
+// With at most 12 candidates (sparse frames: 4.2 of them on average) all are
+// listed, and each one's place is the number of nearer ones, counted pair by
+// pair; more are inserted into an ascending list, which moves 12 entries per
+// candidate.
+template <bool SHARED>
 __device__ __forceinline__ void knn_row(const WorldDev& w, const CellTable& table,
                                         const float2* __restrict__ tpp,
                                         const float2* __restrict__ tpv, uint32_t c, uint32_t t,
@@ -591,6 +636,58 @@ __device__ __forceinline__ void knn_row(const WorldDev& w, const CellTable& tabl
   uint32_t rs[3], re[3];
   neighbour_rows(w, table, c, rs, re);
   const float2 pi = tpp[t], vi = tpv[t];
+  uint32_t out[kIn / 2] = {};
+  out[2 * kK] = pack_bf16(vi.x, vi.y);
+  const uint32_t b0 = re[0] - rs[0], b1 = b0 + t - rs[1], b2 = b0 + re[1] - rs[1] - 1u;
+  const uint32_t others = b2 + re[2] - rs[2];
+  if (others <= kK) {
+    // candidate m is t's m-th in index order: first row, middle row before
+    // and after t, last row
+    const uint32_t o0 = rs[0], o1 = rs[1] - b0, o2 = o1 + 1u, o3 = rs[2] - b2;
+    set_row<SHARED>(row, out);
+    float d[kK];
+    uint32_t place[kK], dp[kK], dv[kK];
+#pragma unroll
+    for (uint32_t m0 = 0; m0 < kK; m0 += kBatch) {
+      // a batch's loads go out together (past the last candidate: t itself)
+      float2 p[kBatch], v[kBatch];
+      if (m0 < others) {
+#pragma unroll
+        for (uint32_t u = 0; u < kBatch; ++u) {
+          const uint32_t m = m0 + u;
+          const uint32_t j = m < others ? m + (m < b0 ? o0 : m < b1 ? o1 : m < b2 ? o2 : o3) : t;
+          p[u] = tpp[j];
+          v[u] = tpv[j];
+        }
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < kBatch; ++u) {
+        const uint32_t m = m0 + u;
+        d[m] = INFINITY;
+        place[m] = 0u;
+        if (m0 < others) {
+          const float dx = __fsub_rn(p[u].x, pi.x), dy = __fsub_rn(p[u].y, pi.y);
+          const float s = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+          dp[m] = pack_bf16(dx, dy);
+          dv[m] = pack_bf16(__fsub_rn(v[u].x, vi.x), __fsub_rn(v[u].y, vi.y));
+          if (m < others && s < INFINITY) d[m] = s;
+          // a tie keeps the earlier one nearer
+#pragma unroll
+          for (uint32_t k = 0; k < m; ++k) {
+            if (d[m] < d[k]) ++place[k];
+            else ++place[m];
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (uint32_t m = 0; m < kK; ++m)
+      if (d[m] < INFINITY) {
+        row[2 * place[m]] = dp[m];
+        row[2 * place[m] + 1] = dv[m];
+      }
+    return;
+  }
   float bd[kK];
   uint32_t bj[kK];
 #pragma unroll
@@ -626,16 +723,11 @@ __device__ __forceinline__ void knn_row(const WorldDev& w, const CellTable& tabl
   for (uint32_t k = 0; k < kK; ++k) {
     if (bj[k] != 0xFFFFFFFFu) {
       const float2 pj = tpp[bj[k]], vj = tpv[bj[k]];
-      row[2 * k] = pack_bf16(__fsub_rn(pj.x, pi.x), __fsub_rn(pj.y, pi.y));
-      row[2 * k + 1] = pack_bf16(__fsub_rn(vj.x, vi.x), __fsub_rn(vj.y, vi.y));
-    } else {
-      row[2 * k] = 0u;
-      row[2 * k + 1] = 0u;
+      out[2 * k] = pack_bf16(__fsub_rn(pj.x, pi.x), __fsub_rn(pj.y, pi.y));
+      out[2 * k + 1] = pack_bf16(__fsub_rn(vj.x, vi.x), __fsub_rn(vj.y, vi.y));
     }
   }
-  row[2 * kK] = pack_bf16(vi.x, vi.y);
-#pragma unroll
-  for (uint32_t k = 2 * kK + 1; k < kIn / 2; ++k) row[k] = 0u;
+  set_row<SHARED>(row, out);
 }
 
 __global__ void k_compact_velocities(uint32_t n, const uint32_t* __restrict__ tp_of,
@@ -643,11 +735,6 @@ __global__ void k_compact_velocities(uint32_t n, const uint32_t* __restrict__ tp
                                      float2* __restrict__ tp_vel) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n && tp_of[i] != kNoTp) tp_vel[tp_of[i]] = vel[i];
-}
-
-__device__ __forceinline__ void zero_row(uint32_t* row) {
-#pragma unroll
-  for (uint32_t k = 0; k < kIn / 2; ++k) row[k] = 0u;
 }
 
 // Features of the binned frame into x (BF16 [n][64]), one thread per frame
@@ -664,10 +751,10 @@ k_knn_features(const WorldDev* __restrict__ worlds, int nworlds, uint32_t n,
   const uint32_t c = cell_of[i];
   const uint32_t t = tp_of[i];
   if (t == kNoTp) {
-    zero_row(row);
+    zero_row<false>(row);
     return;
   }
-  knn_row(worlds[world_of_cell(worlds, nworlds, c)], table, tpp, tpv, c, t, row);
+  knn_row<false>(worlds[world_of_cell(worlds, nworlds, c)], table, tpp, tpv, c, t, row);
 }
 
 // Training samples of the binned frame: the features of the taking-part
@@ -684,8 +771,8 @@ k_samples(const WorldDev* __restrict__ worlds, int nworlds, uint32_t ncells,
   const uint32_t t = phase + k * stride;
   if (k >= rows || t >= table.taking(ncells)) return;
   const uint32_t c = tp_cell[t];
-  knn_row(worlds[world_of_cell(worlds, nworlds, c)], table, tpp, tpv, c, t,
-          reinterpret_cast<uint32_t*>(x + (size_t)k * kIn));
+  knn_row<false>(worlds[world_of_cell(worlds, nworlds, c)], table, tpp, tpv, c, t,
+                 reinterpret_cast<uint32_t*>(x + (size_t)k * kIn));
   const float2 p = tpp[t], v = q[t];
   target[k] = make_float2(v.x - p.x, v.y - p.y);
 }
@@ -697,10 +784,14 @@ k_samples(const WorldDev* __restrict__ worlds, int nworlds, uint32_t ncells,
 // correction is applied on the spot: the compacted iterate q_t = p_t +
 // correction.  `corr` (optional) receives the correction at the frame index
 // of each taking-part particle.  Persistent: the network is loaded once per
-// block.
+// block, and a warp waits for none of the others afterwards (its rows are its
+// own lanes').  1M lattice: 130 us with one 16-row tile at a time, 4-byte row
+// stores (8 lanes to a bank) and every candidate inserted, 95 us now; it
+// issues 43% of the time and waits for the candidates' loads for most of the
+// rest, with 4 warps a scheduler (128 registers; 3 blocks an SM spill: 118).
 constexpr uint32_t kFuseThreads = 256;
 
-__global__ void __launch_bounds__(kFuseThreads, 3)
+__global__ void __launch_bounds__(kFuseThreads, 2)
 k_surrogate_correct(MlpDev m, const WorldDev* __restrict__ worlds, int nworlds,
                     uint32_t ncells, const CellTable table, const uint32_t* __restrict__ tp_cell,
                     const float2* __restrict__ tpp, const float2* __restrict__ tpv,
@@ -717,32 +808,34 @@ k_surrogate_correct(MlpDev m, const WorldDev* __restrict__ worlds, int nworlds,
     uint32_t* row = sx + threadIdx.x * kRow;
     if (t < ntp) {
       const uint32_t c = tp_cell[t];
-      knn_row(worlds[world_of_cell(worlds, nworlds, c)], table, tpp, tpv, c, t, row);
+      knn_row<true>(worlds[world_of_cell(worlds, nworlds, c)], table, tpp, tpv, c, t, row);
     } else {
-      zero_row(row);
+      zero_row<true>(row);
     }
-    __syncthreads();
-#pragma unroll 1
+    __syncwarp();  // a warp's 32 rows are its own lanes'
+    uint32_t ax[2][4][4];
+    float out[2][4];
+#pragma unroll
     for (uint32_t rt = 0; rt < 2; ++rt) {
-      const uint32_t r0 = warp * 32 + rt * 16;
-      uint32_t ax[4][4];
-      float out[4];
-      const uint32_t* p0 = sx + (r0 + g) * kRow;
-      const uint32_t* p1 = sx + (r0 + g + 8) * kRow;
+      const uint32_t* p0 = sx + (warp * 32 + rt * 16 + g) * kRow;
+      const uint32_t* p1 = p0 + 8 * kRow;
 #pragma unroll
       for (uint32_t kk = 0; kk < 4; ++kk) {
-        ax[kk][0] = p0[kk * 8 + t4];
-        ax[kk][1] = p1[kk * 8 + t4];
-        ax[kk][2] = p0[kk * 8 + 4 + t4];
-        ax[kk][3] = p1[kk * 8 + 4 + t4];
+        ax[rt][kk][0] = p0[kk * 8 + t4];
+        ax[rt][kk][1] = p1[kk * 8 + t4];
+        ax[rt][kk][2] = p0[kk * 8 + 4 + t4];
+        ax[rt][kk][3] = p1[kk * 8 + 4 + t4];
       }
-      mlp_tile_infer(s, lane, ax, out);
-      if (t4 == 0) {
+    }
+    mlp_infer<2>(s, lane, ax, out);
+    if (t4 == 0) {
+#pragma unroll
+      for (uint32_t rt = 0; rt < 2; ++rt) {
 #pragma unroll
         for (uint32_t h = 0; h < 2; ++h) {
-          const uint32_t idx = base + r0 + g + 8 * h;
+          const uint32_t idx = base + warp * 32 + rt * 16 + g + 8 * h;
           if (idx < ntp) {
-            const float cxv = out[2 * h], cyv = out[2 * h + 1];
+            const float cxv = out[rt][2 * h], cyv = out[rt][2 * h + 1];
             const float2 p = tpp[idx];
             q[idx] = make_float2(__fadd_rn(p.x, cxv), __fadd_rn(p.y, cyv));
             if (corr) {
@@ -753,7 +846,7 @@ k_surrogate_correct(MlpDev m, const WorldDev* __restrict__ worlds, int nworlds,
         }
       }
     }
-    __syncthreads();
+    __syncwarp();
   }
 }
 

@@ -298,35 +298,8 @@ int enqueue_frame(WrachContext* ctx) {
     mark(ctx);
     ctx->launches += ctx->n ? std::max<uint32_t>(K, 1) : 0u;
   }
-  wrach::RebinArgs r = rebin_args(ctx);
-  r.n = ctx->n;
-  r.dst_capacity = ctx->total_cap;
-  r.pos_src = ctx->pos_o;
-  r.vel_src = ctx->vel_o;
-  r.pos_dst = ctx->pos;
-  r.vel_dst = ctx->vel;
-  r.cell_dst = ctx->cell_of[ctx->cur ^ 1];
-  r.force_general = 0;
-  // the large cells' sort (the last step) writes other slots than the small
-  // cells' pass before it, so outside per-launch profiling it runs on the
-  // auxiliary stream at the same time, joined back before the frame ends
-  const bool fork = !ctx->event_hook && r.n;
-  for (int step = 1; step < wrach::kCountSortSteps; ++step) {
-    bool launched;
-    if (fork && step == wrach::kCountSortSteps - 2) {
-      CK(cudaEventRecord(ctx->fork_ev, st));
-      CK(cudaStreamWaitEvent(ctx->aux, ctx->fork_ev, 0));
-      CK(wrach::launch_count_sort_step(r, step + 1, ctx->big_blocks, ctx->aux, &launched));
-      CK(cudaEventRecord(ctx->join_ev, ctx->aux));
-      CK(wrach::launch_count_sort_step(r, step, ctx->big_blocks, st, &launched));
-      CK(cudaStreamWaitEvent(st, ctx->join_ev, 0));
-      break;
-    }
-    CK(wrach::launch_count_sort_step(r, step, ctx->big_blocks, st, &launched));
-    if (launched) mark(ctx);
-  }
-  ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells) - (r.n ? 1 : 0);
-  ctx->cur ^= 1;
+  // outside per-launch profiling the large cells' sort runs aside
+  CK(enqueue_rebin(ctx, !ctx->event_hook, [&]() { mark(ctx); }));
   return WRACH_OK;
 }
 

@@ -156,8 +156,48 @@ struct DeviceGuard {
 // The launch arguments of the context's current binned frame.
 wrach::SolveArgs solve_args(WrachContext* ctx);
 wrach::RebinArgs rebin_args(WrachContext* ctx);
-// What a frame's last extended pass needs to take the rebin's tickets.
+// What a frame's last solve launch needs to take the rebin's tickets.
 wrach::CountDev ticket_args(WrachContext* ctx);
+// The rebin of a frame whose solve output is in pos_o / vel_o / keys and
+// whose tickets are taken.  `after` runs after each launch; with `fork` the
+// large cells' step runs on the second stream beside the small cells'.
+template <typename After>
+cudaError_t enqueue_rebin(WrachContext* ctx, bool fork, After after) {
+  wrach::RebinArgs r = rebin_args(ctx);
+  r.n = ctx->n;
+  r.dst_capacity = ctx->total_cap;
+  r.pos_src = ctx->pos_o;
+  r.vel_src = ctx->vel_o;
+  r.pos_dst = ctx->pos;
+  r.vel_dst = ctx->vel;
+  r.cell_dst = ctx->cell_of[ctx->cur ^ 1];
+  r.force_general = 0;
+  cudaStream_t st = ctx->stream;
+  cudaError_t e;
+  bool launched;
+  for (int step = 1; step < wrach::kCountSortSteps; ++step) {
+    // the large cells' sort (the last step) writes other slots than the
+    // small cells' pass before it
+    if (fork && r.n && step == wrach::kCountSortSteps - 2) {
+      if ((e = cudaEventRecord(ctx->fork_ev, st)) != cudaSuccess ||
+          (e = cudaStreamWaitEvent(ctx->aux, ctx->fork_ev, 0)) != cudaSuccess ||
+          (e = wrach::launch_count_sort_step(r, step + 1, ctx->big_blocks, ctx->aux, &launched)) !=
+              cudaSuccess ||
+          (e = cudaEventRecord(ctx->join_ev, ctx->aux)) != cudaSuccess ||
+          (e = wrach::launch_count_sort_step(r, step, ctx->big_blocks, st, &launched)) !=
+              cudaSuccess ||
+          (e = cudaStreamWaitEvent(st, ctx->join_ev, 0)) != cudaSuccess)
+        return e;
+      break;
+    }
+    if ((e = wrach::launch_count_sort_step(r, step, ctx->big_blocks, st, &launched)) != cudaSuccess)
+      return e;
+    if (launched) after();
+  }
+  ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells) - (r.n ? 1 : 0);
+  ctx->cur ^= 1;
+  return cudaSuccess;
+}
 
 // The first `count` extended iterations of the binned frame over the
 // compacted taking-part particles, from a.tp_pos through the iterates q1 and

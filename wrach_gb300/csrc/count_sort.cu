@@ -1,15 +1,15 @@
 // Rebin as a stable counting sort over the cells: the count, scan and pack
 // passes of a frame (assets/shaders/particles_per_cell.wgsl, prefix_sum.wgsl,
 // pack_new_particle_data.wgsl; dispatched by runners/bevy/src/compute/
-// builder.rs:86-89) as a chain of five short launches.
+// builder.rs:86-89) as a chain of short launches.
 //
-//   count    per warp, the particles of one cell (__match_any_sync) take one
-//            atomic on the cell's counter; each particle's ticket (its slot
-//            inside the cell, arrival order) is the returned base plus its
-//            rank among the warp's particles of that cell; per warp one more
-//            atomic adds the particles of each tile of 2048 cells to the
-//            tile's sum.  Plain frames and uploads take the tickets where
-//            they compute the keys instead
+//   count    (warp_ticket, in the launch that computes the keys: a frame's
+//            last solve launch, an upload's keys) per warp, the particles of
+//            one cell (__match_any_sync) take one atomic on the cell's
+//            counter; each particle's ticket (its slot inside the cell,
+//            arrival order) is the returned base plus its rank among the
+//            warp's particles of that cell; per warp one more atomic adds the
+//            particles of each tile of 2048 cells to the tile's sum
 //   scan     exclusive scan of the per-cell counts, one block per tile of
 //            2048 cells; a tile's prefix is the sum of the earlier tiles'
 //            sums (already final, so no block waits): each block adds them
@@ -62,18 +62,18 @@ __device__ __forceinline__ CellTable new_table(const RebinArgs& a) {
 constexpr uint32_t kScanTile = kScanThreads * kScanPer;
 static_assert(kScanTile == kCountScanTile, "tile size shared with the tickets' tile sums");
 
-__global__ void __launch_bounds__(256) k_cs_count(RebinArgs a) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t stride = gridDim.x * blockDim.x;
-  const uint32_t lane = threadIdx.x & 31;
-  if (i == 0) a.ctrl->big_count = 0u;  // the scan lists this rebin's large cells
-  // whole warps walk the particles, so every lane takes part in the match
-  for (uint32_t base = i - lane; base < a.n; base += stride) {
-    const uint32_t j = base + lane;
-    const uint32_t k = j < a.n ? a.keys[j] : a.ncells;
-    const uint32_t t = warp_ticket(k, a.ncells, a.counts, a.tile_sums, kCountScanShift, a.tp_cap,
-                                   a.tp_cap ? a.tile_sums_cap : nullptr);
-    if (j < a.n) a.ticket[j] = t;
+// Gives back the tickets of n particles: their cells' counters and all tile
+// sums are zero again.  Returns at once when *run_if reads 0.
+__global__ void __launch_bounds__(256)
+k_cs_untake(const uint32_t* __restrict__ run_if, const uint32_t* __restrict__ keys, uint32_t n,
+            CountDev c, uint32_t ntiles) {
+  if (*run_if == 0u) return;
+  const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  for (uint32_t i = i0; i < n; i += stride)
+    if (keys[i] < c.ncells) c.counts[keys[i]] = 0u;
+  for (uint32_t t = i0; t < ntiles; t += stride) {
+    c.tile_sums[t] = 0u;
+    if (c.tile_sums_cap) c.tile_sums_cap[t] = 0u;
   }
 }
 
@@ -661,18 +661,21 @@ __global__ void __launch_bounds__(kBigThreads, 8) k_cs_big(RebinArgs a) {
 
 }  // namespace
 
+cudaError_t launch_untake(const uint32_t* run_if, const uint32_t* keys, uint32_t n,
+                          const CountDev& c, int sms, cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  const uint32_t need = (n + 255) / 256, few = (uint32_t)(sms > 0 ? sms : 1) * 4u;
+  k_cs_untake<<<need < few ? need : few, 256, 0, st>>>(run_if, keys, n, c,
+                                                       (c.ncells + kScanTile - 1) / kScanTile);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_count_sort_step(const RebinArgs& a, int step, uint32_t big_blocks,
                                    cudaStream_t st, bool* launched) {
   const uint32_t ntiles = (a.ncells + kScanTile - 1) / kScanTile;
   const uint32_t nblk = (a.n + 255) / 256;
   *launched = true;
-  if (step == 0) {
-    if (!nblk) {
-      *launched = false;
-      return cudaSuccess;
-    }
-    k_cs_count<<<nblk, 256, 0, st>>>(a);
-  } else if (step == 1) {
+  if (step == 1) {
     RebinArgs b = a;
     b.prefixed_tiles = ntiles > kPrefixTiles ? ntiles : 0u;
     if (b.prefixed_tiles) {
@@ -704,15 +707,6 @@ cudaError_t launch_count_sort_step(const RebinArgs& a, int step, uint32_t big_bl
       k_cs_big<false><<<big_blocks ? big_blocks : 1u, kBigThreads, 0, st>>>(a);
   }
   return cudaGetLastError();
-}
-
-cudaError_t launch_count_sort(const RebinArgs& a, uint32_t big_blocks, cudaStream_t st) {
-  for (int step = 0; step < kCountSortSteps; ++step) {
-    bool launched;
-    const cudaError_t e = launch_count_sort_step(a, step, big_blocks, st, &launched);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
 }
 
 uint32_t count_sort_steps(uint32_t n) { return n ? 5u : 1u; }

@@ -968,10 +968,15 @@ k_gate(const float* __restrict__ part, uint32_t nparts, GateState* __restrict__ 
   if (mode == 1 && gs->fallback == 0u) return;
   float v[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
   // unrolled, so that the loads of several partials are in flight at once
-#pragma unroll 4
+#pragma unroll 8
   for (uint32_t b = threadIdx.x; b < nparts; b += blockDim.x) {
-#pragma unroll
-    for (int k = 0; k < 5; ++k) v[k] = k == 1 ? fmaxf(v[k], part[b * 8 + k]) : v[k] + part[b * 8 + k];
+    const float4 p = reinterpret_cast<const float4*>(part)[b * 2];
+    const float last = part[b * 8 + 4];
+    v[0] += p.x;
+    v[1] = fmaxf(v[1], p.y);
+    v[2] += p.z;
+    v[3] += p.w;
+    v[4] += last;
   }
   __shared__ float tot[8];
   block_partials(v, tot - blockIdx.x * 8);

@@ -64,28 +64,13 @@ int ensure_metrics(WrachContext* ctx) {
   return WRACH_OK;
 }
 
-// The rebin of a frame whose solve output is in pos_o / vel_o / keys.
-int enqueue_rebin(WrachContext* ctx) {
-  wrach::RebinArgs r = rebin_args(ctx);
-  r.n = ctx->n;
-  r.dst_capacity = ctx->total_cap;
-  r.pos_src = ctx->pos_o;
-  r.vel_src = ctx->vel_o;
-  r.pos_dst = ctx->pos;
-  r.vel_dst = ctx->vel;
-  r.cell_dst = ctx->cell_of[ctx->cur ^ 1];
-  r.force_general = 0;
-  CK(wrach::launch_count_sort(r, ctx->big_blocks, ctx->stream));
-  ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells);
-  ctx->cur ^= 1;
-  return WRACH_OK;
-}
-
 // The plain extended solve of the binned frame into pos_o / vel_o / keys;
-// the final pass writes the gate metrics when `a.part` is set.
+// the final pass writes the gate metrics when `a.part` is set, and takes the
+// rebin's tickets.
 int enqueue_plain_solve(WrachContext* ctx, const wrach::SolveArgs& a) {
   wrach::SolveArgs inner = a;
   inner.part = nullptr;
+  inner.count = wrach::CountDev{};
   const float2* q = nullptr;
   CK(enqueue_iterations(ctx, inner, ctx->ph.iterations - 1, ctx->stream, &q, []() {}));
   wrach::SolveArgs fin = a;
@@ -105,6 +90,7 @@ int enqueue_surrogate_frame(WrachContext* ctx, int calibration) {
   auto& S = ctx->sur;
   wrach::SolveArgs a = solve_args(ctx);
   a.part = S.part;
+  a.count = ticket_args(ctx);
   int rc;
   if (calibration) {
     // a plain frame: its metrics are the reference of the next frames
@@ -118,13 +104,16 @@ int enqueue_surrogate_frame(WrachContext* ctx, int calibration) {
     CK(wrach::launch_gate(S.part, wrach::solve_blocks(a), S.gate, 0, ctx->stream));
     // the plain solve of the same frame, run only when the gate failed it
     // (its launches stride over the frame with few blocks, so skipping them
-    // is cheap), and the gate again on its metrics
+    // is cheap), after the surrogate's tickets are given back, and the gate
+    // again on its metrics
     a.run_if = &S.gate->fallback;
+    CK(wrach::launch_untake(a.run_if, ctx->keys, ctx->n, a.count, ctx->sms, ctx->stream));
     if ((rc = enqueue_plain_solve(ctx, a))) return rc;
     CK(wrach::launch_gate(S.part, wrach::solve_blocks(a), S.gate, 1, ctx->stream));
-    ctx->launches += (ctx->n ? 2 : 0) + 2;
+    ctx->launches += (ctx->n ? 3 : 0) + 2;
   }
-  return enqueue_rebin(ctx);
+  CK(enqueue_rebin(ctx, true, []() {}));
+  return WRACH_OK;
 }
 
 }  // namespace

@@ -130,14 +130,16 @@ constexpr uint32_t kBigCell = 2048;
 // big_blocks: the grid of the large-cell step (its blocks loop over the
 // listed cells); kBigBlocksPerSm per SM unless a config sets it.
 constexpr uint32_t kBigBlocksPerSm = 8;
-cudaError_t launch_count_sort(const RebinArgs& a, uint32_t big_blocks, cudaStream_t st);
-// The same, one step at a time (steps 0 .. kCountSortSteps - 1: count, scan,
-// scatter, place, large cells); *launched is false for a step that has
-// nothing to do.  Step 0 is left out when the tickets were taken with the
-// keys (SolveArgs::count, launch_upload_keys).
+// One step of the sort: 1 scan, 2 scatter, 3 place, 4 large cells (step 0, the
+// tickets, is taken with the keys: SolveArgs::count, launch_upload_keys);
+// *launched is false for a step that has nothing to do.
 constexpr int kCountSortSteps = 5;
 cudaError_t launch_count_sort_step(const RebinArgs& a, int step, uint32_t big_blocks,
                                    cudaStream_t st, bool* launched);
+// Gives a pass's tickets back (its n keys): the counters and tile sums are zero
+// again; skipped when *run_if reads 0.
+cudaError_t launch_untake(const uint32_t* run_if, const uint32_t* keys, uint32_t n,
+                          const CountDev& c, int sms, cudaStream_t st);
 // Steps of one rebin (count, scan, scatter, place, large cells; the scan
 // alone when there are no particles) and its kernel launches (a large grid's
 // scan step is two launches).

@@ -298,24 +298,21 @@ int enqueue_frame(WrachContext* ctx) {
     mark(ctx);
     ctx->launches += ctx->n ? std::max<uint32_t>(K, 1) : 0u;
   }
-  // outside per-launch profiling the large cells' sort runs aside
-  CK(enqueue_rebin(ctx, !ctx->event_hook, [&]() { mark(ctx); }));
+  CK(enqueue_rebin(ctx, ctx->event_hook != nullptr, [&]() { mark(ctx); }));
   return WRACH_OK;
 }
 
-// Steps wrach_profile_frame times in one frame: each solve launch, then
-// each rebin launch (an empty frame's solve launches nothing, but still marks
-// its steps).
+// Steps wrach_profile_frame times in one frame: each solve launch, then the
+// scan and the scatter and place steps (an empty frame's solve launches
+// nothing, but still marks its steps).
 uint32_t frame_steps(const WrachContext* ctx) {
-  const uint32_t rebin = wrach::count_sort_steps(ctx->n);
-  return std::max<uint32_t>(ctx->ph.iterations, 1) + rebin - (ctx->n ? 1 : 0);
+  return std::max<uint32_t>(ctx->ph.iterations, 1) + (ctx->n ? 4u : 1u);
 }
 
 // Kernel launches of one frame.
 uint32_t frame_launches(const WrachContext* ctx) {
-  const uint32_t extra = wrach::count_sort_launches(ctx->n, ctx->ncells) - wrach::count_sort_steps(ctx->n);
-  if (!ctx->n) return wrach::count_sort_launches(0, ctx->ncells);
-  return frame_steps(ctx) + extra;
+  return (ctx->n ? std::max<uint32_t>(ctx->ph.iterations, 1) : 0u) +
+         wrach::count_sort_launches(ctx->n, ctx->ncells);
 }
 
 // One frame captured as a CUDA graph, instantiated once per table parity
@@ -644,7 +641,7 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
   r.cell_dst = ctx->cell_of[ctx->cur ^ 1];
   r.force_general = 1;
   bool launched;
-  CK(wrach::launch_count_sort_step(r, 1, ctx->big_blocks, ctx->stream, &launched));
+  CK(wrach::launch_count_sort_step(r, wrach::kScan, ctx->big_blocks, ctx->stream, &launched));
   // per-world counts from the new table, written to the host on a stream of
   // their own beside the place steps and the velocities' copy
   const uint32_t nw = ctx->nworlds;
@@ -654,13 +651,12 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
       ctx->table(ctx->cur ^ 1), ctx->gather_idx, nw + 1, ctx->gather_h);
   CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->counts_ev, ctx->back));
-  ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells) + (r.n ? 0 : 1);
+  ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells) + 1;
   auto place = [&]() {
-    for (int step = 2; step < wrach::kCountSortSteps; ++step) {
-      // the place steps (3, 4) are the first to read the velocities
-      if (vel_aside && step == 3) CK(cudaStreamWaitEvent(ctx->stream, ctx->join_ev, 0));
-      CK(wrach::launch_count_sort_step(r, step, ctx->big_blocks, ctx->stream, &launched));
-    }
+    CK(wrach::launch_count_sort_step(r, wrach::kScatter, ctx->big_blocks, ctx->stream, &launched));
+    // the place step is the first to read the velocities
+    if (vel_aside) CK(cudaStreamWaitEvent(ctx->stream, ctx->join_ev, 0));
+    CK(wrach::launch_count_sort_step(r, wrach::kPlace, ctx->big_blocks, ctx->stream, &launched));
     return (int)WRACH_OK;
   };
   if (direct && (rc = place())) return rc;

@@ -27,7 +27,7 @@ struct Store {
 struct WrachContext {
   int device = 0;
   cudaStream_t stream = nullptr;
-  // a frame's large-cell sort runs on `aux`, beside the small cells' pass
+  // uploads: the velocities' copy beside the positions' keys
   cudaStream_t aux = nullptr;
   // uploads: the counts' way to the host
   cudaStream_t back = nullptr;
@@ -159,11 +159,12 @@ wrach::RebinArgs rebin_args(WrachContext* ctx);
 // What a frame's last solve launch needs to take the rebin's tickets.
 wrach::CountDev ticket_args(WrachContext* ctx);
 // The rebin of a frame whose solve output is in pos_o / vel_o / keys and
-// whose tickets are taken.  `after` runs after each launch; with `fork` the
-// large cells' step runs on the second stream beside the small cells'.
+// whose tickets are taken.  `after` runs after each launch; `apart` launches
+// the small and the large cells' place steps on their own.
 template <typename After>
-cudaError_t enqueue_rebin(WrachContext* ctx, bool fork, After after) {
-  wrach::RebinArgs r = rebin_args(ctx);
+cudaError_t enqueue_rebin(WrachContext* ctx, bool apart, After after) {
+  using namespace wrach;
+  RebinArgs r = rebin_args(ctx);
   r.n = ctx->n;
   r.dst_capacity = ctx->total_cap;
   r.pos_src = ctx->pos_o;
@@ -172,29 +173,16 @@ cudaError_t enqueue_rebin(WrachContext* ctx, bool fork, After after) {
   r.vel_dst = ctx->vel;
   r.cell_dst = ctx->cell_of[ctx->cur ^ 1];
   r.force_general = 0;
-  cudaStream_t st = ctx->stream;
-  cudaError_t e;
-  bool launched;
-  for (int step = 1; step < wrach::kCountSortSteps; ++step) {
-    // the large cells' sort (the last step) writes other slots than the
-    // small cells' pass before it
-    if (fork && r.n && step == wrach::kCountSortSteps - 2) {
-      if ((e = cudaEventRecord(ctx->fork_ev, st)) != cudaSuccess ||
-          (e = cudaStreamWaitEvent(ctx->aux, ctx->fork_ev, 0)) != cudaSuccess ||
-          (e = wrach::launch_count_sort_step(r, step + 1, ctx->big_blocks, ctx->aux, &launched)) !=
-              cudaSuccess ||
-          (e = cudaEventRecord(ctx->join_ev, ctx->aux)) != cudaSuccess ||
-          (e = wrach::launch_count_sort_step(r, step, ctx->big_blocks, st, &launched)) !=
-              cudaSuccess ||
-          (e = cudaStreamWaitEvent(st, ctx->join_ev, 0)) != cudaSuccess)
-        return e;
-      break;
-    }
-    if ((e = wrach::launch_count_sort_step(r, step, ctx->big_blocks, st, &launched)) != cudaSuccess)
-      return e;
+  const CountSortStep together[] = {kScan, kScatter, kPlace};
+  const CountSortStep each[] = {kScan, kScatter, kPlaceSmall, kPlaceLarge};
+  for (int k = 0; k < (apart ? 4 : 3); ++k) {
+    bool launched;
+    const cudaError_t e = launch_count_sort_step(r, apart ? each[k] : together[k], ctx->big_blocks,
+                                                 ctx->stream, &launched);
+    if (e != cudaSuccess) return e;
     if (launched) after();
   }
-  ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells) - (r.n ? 1 : 0);
+  ctx->launches += count_sort_launches(r.n, ctx->ncells) + (apart && r.n ? 1 : 0);
   ctx->cur ^= 1;
   return cudaSuccess;
 }

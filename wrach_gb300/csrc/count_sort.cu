@@ -29,7 +29,7 @@
 //            the taking-part particles' positions, cells and (for the learned
 //            surrogate) velocities into the compacted arrays.  Cells of up to kSmallCell particles are
 //            ranked by one thread per slot
-//   cells    one block per listed cell: up to kBigCell particles ranked by a
+//   large    (with place, in blocks of their own) one block per listed cell: up to kBigCell particles ranked by a
 //            bitmap of their source indices (or a bitonic sort) in shared
 //            memory, more than that a block-wide LSD radix sort of them in
 //            global memory; then the gather.  It writes other slots than place, so the two may run
@@ -101,6 +101,7 @@ __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* red) {
 constexpr uint32_t kPrefixTiles = 2048, kRun = 256;
 
 __global__ void __launch_bounds__(kRun) k_cs_tile_prefix(RebinArgs a, uint32_t ntiles) {
+  begin_after();
   __shared__ uint32_t ws[kRun / 32], wc[kRun / 32];
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const uint32_t i = blockIdx.x * kRun + t;
@@ -151,6 +152,7 @@ __device__ __forceinline__ void list_large(const RebinArgs& a, uint32_t cell) {
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_cs_scan(RebinArgs a) {
+  begin_after();
   __shared__ uint32_t warp_sum[kScanThreads / 32], red[kScanThreads / 32];
   __shared__ uint32_t warp_cap[kScanThreads / 32];
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -268,6 +270,7 @@ __global__ void __launch_bounds__(kScanThreads) k_cs_scan(RebinArgs a) {
 constexpr uint32_t kGroupThreads = kScanTile / (2 * kGroup);
 
 __global__ void __launch_bounds__(kGroupThreads) k_cs_scan_groups(RebinArgs a) {
+  begin_after();
   __shared__ uint32_t warp_sum[kGroupThreads / 32], warp_cap[kGroupThreads / 32];
   constexpr uint32_t per = 2 * kGroup;
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -352,6 +355,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_cs_scan_groups(RebinArgs a) {
 
 template <bool GROUPED>
 __global__ void __launch_bounds__(256) k_cs_scatter(RebinArgs a, uint32_t ntiles) {
+  begin_after();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   // the scan has read the tile sums: clear them for the next rebin
   for (uint32_t u = i; u < ntiles; u += gridDim.x * blockDim.x) {
@@ -397,9 +401,9 @@ __device__ __forceinline__ void add_overflow(const RebinArgs& a, uint32_t overfl
   if ((threadIdx.x & 31) == 0 && wo) atomicAdd(&a.ctrl->overflow, wo);
 }
 
+// The small cells: one thread per slot q.
 template <bool GROUPED>
-__global__ void __launch_bounds__(256) k_cs_place(RebinArgs a) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void place_slot(const RebinArgs& a, uint32_t q) {
   const CellTable table = new_table<GROUPED>(a);
   const uint32_t total = table.start(a.ncells);
   uint32_t overflow = 0;
@@ -450,8 +454,13 @@ static_assert(kBigThreads == 256, "one radix digit per thread");
 // into src or alt (returned), in chunks of 256 values: inside a chunk a
 // value's slot is its digit's running offset, plus the counts of its digit
 // in the chunk's earlier warps, plus its rank among its warp's equal digits.
-__device__ uint32_t* block_radix_sort(uint32_t* src, uint32_t* alt, uint32_t m, uint32_t key_bits) {
-  __shared__ uint32_t hist[256], wcnt[kBigThreads / 32][256];
+struct RadixScratch {
+  uint32_t hist[256], wcnt[kBigThreads / 32][256];
+};
+__device__ uint32_t* block_radix_sort(RadixScratch& R, uint32_t* src, uint32_t* alt, uint32_t m,
+                                      uint32_t key_bits) {
+  auto& hist = R.hist;
+  auto& wcnt = R.wcnt;
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const uint32_t lanemask_lt = (1u << lane) - 1u;
   for (uint32_t shift = 0; shift < key_bits; shift += 8) {
@@ -597,19 +606,22 @@ __device__ bool page_ranks(PageRanks& P, const uint32_t* src, uint32_t s) {
 // in shared memory (bitonic, padded to a power of two, one compare-exchange
 // per pair index and stage); larger cells by the block-wide radix sort in
 // global memory; then the gather.
-// Eight blocks per SM (its grid), so at most 32 registers.
+union BigScratch {
+  uint32_t sv[kBigCell];
+  PageRanks pages;
+  RadixScratch radix;
+};
+
+// The large cells, by blocks block, block + blocks, ... of `blocks`.
 template <bool GROUPED>
-__global__ void __launch_bounds__(kBigThreads, 8) k_cs_big(RebinArgs a) {
-  __shared__ union {
-    uint32_t sv[kBigCell];
-    PageRanks pages;
-  } sh;
+__device__ __forceinline__ void place_large(const RebinArgs& a, BigScratch& sh, uint32_t block,
+                                            uint32_t blocks) {
   uint32_t* sv = sh.sv;
   const uint32_t nb = min(a.ctrl->big_count, a.big_cap);
   const CellTable table = new_table<GROUPED>(a);
   uint32_t overflow = 0;
   const uint32_t key_bits = a.n > 1 ? 32u - __clz(a.n - 1) : 1u;
-  for (uint32_t w = blockIdx.x; w < nb; w += gridDim.x) {
+  for (uint32_t w = block; w < nb; w += blocks) {
     const uint32_t k = a.big_list[w];
     uint32_t s0, s1;
     table.span(k, s0, s1);
@@ -617,7 +629,7 @@ __global__ void __launch_bounds__(kBigThreads, 8) k_cs_big(RebinArgs a) {
     if (threadIdx.x == 0) a.counts[k] = 0u;  // read by the scan; zero for the next rebin
     const uint32_t s = s1 > s0 ? s1 - s0 : 0u;
     if (s > kBigCell) {
-      const uint32_t* sorted = block_radix_sort(a.idx_tmp + s0, a.idx_alt + s0, s, key_bits);
+      const uint32_t* sorted = block_radix_sort(sh.radix, a.idx_tmp + s0, a.idx_alt + s0, s, key_bits);
       for (uint32_t r = threadIdx.x; r < s; r += kBigThreads) place_one<GROUPED>(a, s0 + r, r, sorted[r], k, overflow);
       if (threadIdx.x == 0) atomicAdd(&a.ctrl->huge_cells, 1u);
       __syncthreads();
@@ -659,6 +671,23 @@ __global__ void __launch_bounds__(kBigThreads, 8) k_cs_big(RebinArgs a) {
   add_overflow(a, overflow);
 }
 
+// The place steps: the first big_blocks blocks take the large cells, which
+// last longest, the others the small ones' slots.  In one launch the two run
+// side by side without a second stream's fork and join, and its blocks wait
+// their turn behind the scatter's (on a stream of their own the large cells'
+// blocks came after those of a place launch that overlaps the scatter: the
+// collapsed 1M lattice 101 -> 107 us).  Eight blocks per SM (kBigBlocksPerSm), so
+// at most 32 registers.
+template <bool GROUPED>
+__global__ void __launch_bounds__(kBigThreads, 8) k_cs_place(RebinArgs a, uint32_t big_blocks) {
+  __shared__ BigScratch sh;
+  begin_after();
+  if (blockIdx.x < big_blocks)
+    place_large<GROUPED>(a, sh, blockIdx.x, big_blocks);
+  else
+    place_slot<GROUPED>(a, (blockIdx.x - big_blocks) * kBigThreads + threadIdx.x);
+}
+
 }  // namespace
 
 cudaError_t launch_untake(const uint32_t* run_if, const uint32_t* keys, uint32_t n,
@@ -675,45 +704,36 @@ cudaError_t launch_count_sort_step(const RebinArgs& a, int step, uint32_t big_bl
   const uint32_t ntiles = (a.ncells + kScanTile - 1) / kScanTile;
   const uint32_t nblk = (a.n + 255) / 256;
   *launched = true;
-  if (step == 1) {
+  if (step == kScan) {
     RebinArgs b = a;
     b.prefixed_tiles = ntiles > kPrefixTiles ? ntiles : 0u;
     if (b.prefixed_tiles) {
-      k_cs_tile_prefix<<<(ntiles + kRun - 1) / kRun, kRun, 0, st>>>(b, ntiles);
-      const cudaError_t e = cudaGetLastError();
+      const cudaError_t e =
+          launch_after(k_cs_tile_prefix, (ntiles + kRun - 1) / kRun, kRun, st, b, ntiles);
       if (e != cudaSuccess) return e;
     }
-    if (a.groups_new)
-      k_cs_scan_groups<<<ntiles, kGroupThreads, 0, st>>>(b);
-    else
-      k_cs_scan<<<ntiles ? ntiles : 1u, kScanThreads, 0, st>>>(b);
+    return a.groups_new ? launch_after(k_cs_scan_groups, ntiles, kGroupThreads, st, b)
+                        : launch_after(k_cs_scan, ntiles ? ntiles : 1u, kScanThreads, st, b);
   } else if (!nblk) {
     *launched = false;
     return cudaSuccess;
-  } else if (step == 2) {
-    if (a.groups_new)
-      k_cs_scatter<true><<<nblk, 256, 0, st>>>(a, ntiles);
-    else
-      k_cs_scatter<false><<<nblk, 256, 0, st>>>(a, ntiles);
-  } else if (step == 3) {
-    if (a.groups_new)
-      k_cs_place<true><<<nblk, 256, 0, st>>>(a);
-    else
-      k_cs_place<false><<<nblk, 256, 0, st>>>(a);
+  } else if (step == kScatter) {
+    return launch_after(a.groups_new ? k_cs_scatter<true> : k_cs_scatter<false>, nblk, 256, st, a,
+                        ntiles);
   } else {
-    if (a.groups_new)
-      k_cs_big<true><<<big_blocks ? big_blocks : 1u, kBigThreads, 0, st>>>(a);
-    else
-      k_cs_big<false><<<big_blocks ? big_blocks : 1u, kBigThreads, 0, st>>>(a);
+    // at most n / (kSmallCell + 1) cells are large
+    const uint32_t large = min(big_blocks ? big_blocks : 1u, a.n / (kSmallCell + 1) + 1);
+    const uint32_t big = step == kPlaceSmall ? 0u : large;
+    const uint32_t small = step == kPlaceLarge ? 0u : nblk;
+    return launch_after(a.groups_new ? k_cs_place<true> : k_cs_place<false>, big + small,
+                        kBigThreads, st, a, big);
   }
   return cudaGetLastError();
 }
 
-uint32_t count_sort_steps(uint32_t n) { return n ? 5u : 1u; }
-
 uint32_t count_sort_launches(uint32_t n, uint32_t ncells) {
   const uint32_t ntiles = (ncells + kScanTile - 1) / kScanTile;
-  return count_sort_steps(n) + (ntiles > kPrefixTiles ? 1u : 0u);
+  return (n ? 3u : 1u) + (ntiles > kPrefixTiles ? 1u : 0u);
 }
 
 }  // namespace wrach

@@ -79,6 +79,7 @@ k_solve_reference(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32
                   const float2* __restrict__ pin, const float2* __restrict__ vin,
                   float2* __restrict__ pout, float2* __restrict__ vout,
                   uint32_t* __restrict__ keys, Ctrl* ctrl, CountDev count) {
+  begin_after();
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->big_count = 0u;  // listed afresh by the scan
@@ -306,8 +307,12 @@ k_jacobi_tp(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t nce
             const CellTable table, const uint32_t* __restrict__ tp_cell,
             const float2* __restrict__ qin, float2* __restrict__ qout,
             const uint32_t* __restrict__ run_if, uint4* __restrict__ rows) {
-  if (run_if && *run_if == 0u) return;
+  // the table is older than the kernel before: blocks without a particle
+  // (on a piled-up floor, most) end at once; block 0 always has one
   const uint32_t ntp = table.taking(ncells);
+  if (blockIdx.x * blockDim.x >= ntp && blockIdx.x != 0) return;
+  begin_after();
+  if (run_if && *run_if == 0u) return;
   const f32x2* __restrict__ q = reinterpret_cast<const f32x2*>(qin);
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ntp; t += gridDim.x * blockDim.x) {
     Rows R;
@@ -348,6 +353,7 @@ k_jacobi_final(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t 
                float2* __restrict__ pout, const float2* __restrict__ vin,
                float2* __restrict__ vout, uint32_t* __restrict__ keys, Ctrl* ctrl,
                const uint32_t* __restrict__ run_if, float* __restrict__ part, CountDev count) {
+  begin_after();
   if (run_if && *run_if == 0u) return;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // taking the tickets: the rebin's scan lists its large cells afresh
@@ -450,14 +456,12 @@ cudaError_t launch_solve_reference(const SolveArgs& a, cudaStream_t st) {
   const uint32_t own = (33u - a.ph.cap) * (threads / 32);
   const uint32_t blocks = (a.n + own - 1) / own;
   if (a.nworlds == 1)
-    k_solve_reference<true><<<blocks, threads, 0, st>>>(
-        Worlds<true>{a.world}, a.ph, a.n, a.table, a.cell_of, a.pos, a.vel, a.pos_out,
-        a.vel_out, a.keys, a.ctrl, a.count);
-  else
-    k_solve_reference<false><<<blocks, threads, 0, st>>>(
-        Worlds<false>{a.worlds, a.nworlds}, a.ph, a.n, a.table, a.cell_of, a.pos, a.vel,
-        a.pos_out, a.vel_out, a.keys, a.ctrl, a.count);
-  return cudaGetLastError();
+    return launch_after(k_solve_reference<true>, blocks, threads, st, Worlds<true>{a.world}, a.ph,
+                        a.n, a.table, a.cell_of, a.pos, a.vel, a.pos_out, a.vel_out, a.keys,
+                        a.ctrl, a.count);
+  return launch_after(k_solve_reference<false>, blocks, threads, st,
+                      Worlds<false>{a.worlds, a.nworlds}, a.ph, a.n, a.table, a.cell_of, a.pos,
+                      a.vel, a.pos_out, a.vel_out, a.keys, a.ctrl, a.count);
 }
 
 uint32_t solve_blocks(const SolveArgs& a) {
@@ -474,28 +478,26 @@ uint32_t solve_blocks(const SolveArgs& a) {
 static bool narrow_marks(const PhysDev& ph) { return 3 * ph.cap + 1 <= 32; }
 
 template <typename Mask, int ROWS>
-static void launch_iteration(const SolveArgs& a, uint32_t blocks, uint32_t threads,
-                             const float2* qin, float2* qout, cudaStream_t st) {
-  if (ROWS == 2 || a.nworlds == 1) {  // the rows read back need no world
-    k_jacobi_tp<Mask, ROWS, true><<<blocks, threads, 0, st>>>(
-        Worlds<true>{a.world}, a.ph, a.ncells, a.table, a.tp_cell, qin, qout, a.run_if, a.rows);
-  } else if constexpr (ROWS != 2) {
-    k_jacobi_tp<Mask, ROWS, false><<<blocks, threads, 0, st>>>(
-        Worlds<false>{a.worlds, a.nworlds}, a.ph, a.ncells, a.table, a.tp_cell, qin, qout, a.run_if,
-        a.rows);
+static cudaError_t launch_iteration(const SolveArgs& a, uint32_t blocks, uint32_t threads,
+                                    const float2* qin, float2* qout, cudaStream_t st) {
+  if constexpr (ROWS != 2) {
+    if (a.nworlds != 1)
+      return launch_after(k_jacobi_tp<Mask, ROWS, false>, blocks, threads, st,
+                          Worlds<false>{a.worlds, a.nworlds}, a.ph, a.ncells, a.table, a.tp_cell,
+                          qin, qout, a.run_if, a.rows);
   }
+  // the rows read back need no world
+  return launch_after(k_jacobi_tp<Mask, ROWS, true>, blocks, threads, st, Worlds<true>{a.world},
+                      a.ph, a.ncells, a.table, a.tp_cell, qin, qout, a.run_if, a.rows);
 }
 
 template <typename Mask>
-static void launch_iteration(const SolveArgs& a, uint32_t blocks, uint32_t threads,
-                             const float2* qin, float2* qout, cudaStream_t st) {
+static cudaError_t launch_iteration(const SolveArgs& a, uint32_t blocks, uint32_t threads,
+                                    const float2* qin, float2* qout, cudaStream_t st) {
   const int mode = a.rows ? a.rows_mode : 0;
-  if (mode == 1)
-    launch_iteration<Mask, 1>(a, blocks, threads, qin, qout, st);
-  else if (mode == 2)
-    launch_iteration<Mask, 2>(a, blocks, threads, qin, qout, st);
-  else
-    launch_iteration<Mask, 0>(a, blocks, threads, qin, qout, st);
+  if (mode == 1) return launch_iteration<Mask, 1>(a, blocks, threads, qin, qout, st);
+  if (mode == 2) return launch_iteration<Mask, 2>(a, blocks, threads, qin, qout, st);
+  return launch_iteration<Mask, 0>(a, blocks, threads, qin, qout, st);
 }
 
 cudaError_t launch_jacobi_iteration(const SolveArgs& a, const float2* qin, float2* qout,
@@ -503,38 +505,33 @@ cudaError_t launch_jacobi_iteration(const SolveArgs& a, const float2* qin, float
   if (a.n == 0) return cudaSuccess;
   const uint32_t threads = a.block ? a.block : 128;
   const uint32_t blocks = solve_blocks(a);
-  if (narrow_marks(a.ph))
-    launch_iteration<uint32_t>(a, blocks, threads, qin, qout, st);
-  else
-    launch_iteration<uint64_t>(a, blocks, threads, qin, qout, st);
-  return cudaGetLastError();
+  return narrow_marks(a.ph) ? launch_iteration<uint32_t>(a, blocks, threads, qin, qout, st)
+                            : launch_iteration<uint64_t>(a, blocks, threads, qin, qout, st);
 }
 
 template <typename Mask, int ROWS, bool METRICS>
-static void launch_final(const SolveArgs& a, uint32_t blocks, uint32_t threads, const float2* qtp,
-                         int do_push, cudaStream_t st) {
+static cudaError_t launch_final(const SolveArgs& a, uint32_t blocks, uint32_t threads,
+                                const float2* qtp, int do_push, cudaStream_t st) {
   if (a.nworlds == 1)
-    k_jacobi_final<Mask, ROWS, METRICS, true><<<blocks, threads, 0, st>>>(
-        Worlds<true>{a.world}, a.ph, a.n, do_push, a.table, a.tp_of, a.cell_of, a.rows, a.pos, qtp,
-        a.pos_out, a.vel, a.vel_out, a.keys, a.ctrl, a.run_if, a.part, a.count);
-  else
-    k_jacobi_final<Mask, ROWS, METRICS, false><<<blocks, threads, 0, st>>>(
-        Worlds<false>{a.worlds, a.nworlds}, a.ph, a.n, do_push, a.table, a.tp_of, a.cell_of, a.rows,
-        a.pos, qtp, a.pos_out, a.vel, a.vel_out, a.keys, a.ctrl, a.run_if, a.part, a.count);
+    return launch_after(k_jacobi_final<Mask, ROWS, METRICS, true>, blocks, threads, st,
+                        Worlds<true>{a.world}, a.ph, a.n, do_push, a.table, a.tp_of, a.cell_of,
+                        a.rows, a.pos, qtp, a.pos_out, a.vel, a.vel_out, a.keys, a.ctrl, a.run_if,
+                        a.part, a.count);
+  return launch_after(k_jacobi_final<Mask, ROWS, METRICS, false>, blocks, threads, st,
+                      Worlds<false>{a.worlds, a.nworlds}, a.ph, a.n, do_push, a.table, a.tp_of,
+                      a.cell_of, a.rows, a.pos, qtp, a.pos_out, a.vel, a.vel_out, a.keys, a.ctrl,
+                      a.run_if, a.part, a.count);
 }
 
 template <typename Mask>
-static void launch_final(const SolveArgs& a, uint32_t blocks, uint32_t threads, const float2* qtp,
-                         int do_push, cudaStream_t st) {
+static cudaError_t launch_final(const SolveArgs& a, uint32_t blocks, uint32_t threads,
+                                const float2* qtp, int do_push, cudaStream_t st) {
   const bool rows = a.rows && a.rows_mode == 2;
-  if (a.part && rows)
-    launch_final<Mask, 2, true>(a, blocks, threads, qtp, do_push, st);
-  else if (a.part)
-    launch_final<Mask, 0, true>(a, blocks, threads, qtp, do_push, st);
-  else if (rows)
-    launch_final<Mask, 2, false>(a, blocks, threads, qtp, do_push, st);
-  else
-    launch_final<Mask, 0, false>(a, blocks, threads, qtp, do_push, st);
+  if (a.part)
+    return rows ? launch_final<Mask, 2, true>(a, blocks, threads, qtp, do_push, st)
+                : launch_final<Mask, 0, true>(a, blocks, threads, qtp, do_push, st);
+  return rows ? launch_final<Mask, 2, false>(a, blocks, threads, qtp, do_push, st)
+              : launch_final<Mask, 0, false>(a, blocks, threads, qtp, do_push, st);
 }
 
 cudaError_t launch_jacobi_final(const SolveArgs& a, const float2* qtp, int do_push,
@@ -542,11 +539,8 @@ cudaError_t launch_jacobi_final(const SolveArgs& a, const float2* qtp, int do_pu
   if (a.n == 0) return cudaSuccess;
   const uint32_t threads = a.block ? a.block : 128;
   const uint32_t blocks = solve_blocks(a);
-  if (narrow_marks(a.ph))
-    launch_final<uint32_t>(a, blocks, threads, qtp, do_push, st);
-  else
-    launch_final<uint64_t>(a, blocks, threads, qtp, do_push, st);
-  return cudaGetLastError();
+  return narrow_marks(a.ph) ? launch_final<uint32_t>(a, blocks, threads, qtp, do_push, st)
+                            : launch_final<uint64_t>(a, blocks, threads, qtp, do_push, st);
 }
 
 }  // namespace wrach

@@ -112,7 +112,7 @@ int enqueue_surrogate_frame(WrachContext* ctx, int calibration) {
     CK(wrach::launch_gate(S.part, wrach::solve_blocks(a), S.gate, 1, ctx->stream));
     ctx->launches += (ctx->n ? 3 : 0) + 2;
   }
-  CK(enqueue_rebin(ctx, true, []() {}));
+  CK(enqueue_rebin(ctx, false, []() {}));
   return WRACH_OK;
 }
 

@@ -412,6 +412,17 @@ __device__ __forceinline__ uint64_t global_ns() {
   return t;
 }
 
+// Start of a kernel launched by launch_after: waits for the kernel before it
+// (its memory included), then lets the next one's blocks be scheduled, so that
+// their launch overlaps this kernel's end.  A kernel's launch overlaps only
+// its direct predecessor, which has itself waited.  Frames of eight launches
+// of 2 to 4 us (16,384 particles) 24.0 -> 21.4 us, 1M lattice 107.5 -> 104.5,
+// the reference physics 48.1 -> 45.2.
+__device__ __forceinline__ void begin_after() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Bounded device waits give up after this many nanoseconds and raise
 // kFlagTimeout instead of hanging the GPU.
 constexpr uint64_t kWaitLimitNs = 1000000000ull;

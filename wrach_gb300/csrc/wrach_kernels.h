@@ -8,6 +8,23 @@
 
 namespace wrach {
 
+// Launches a frame kernel that begins with begin_after: its blocks may be
+// scheduled before the stream's last kernel has ended.
+template <typename... Params, typename... Args>
+cudaError_t launch_after(void (*kernel)(Params...), uint32_t blocks, uint32_t threads,
+                         cudaStream_t st, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // Entries past their particle count that the compacted positions and the
 // iterates have room for (the iterations read candidates several at a time).
 constexpr uint32_t kRowPad = 4;
@@ -130,20 +147,19 @@ constexpr uint32_t kBigCell = 2048;
 // big_blocks: the grid of the large-cell step (its blocks loop over the
 // listed cells); kBigBlocksPerSm per SM unless a config sets it.
 constexpr uint32_t kBigBlocksPerSm = 8;
-// One step of the sort: 1 scan, 2 scatter, 3 place, 4 large cells (step 0, the
-// tickets, is taken with the keys: SolveArgs::count, launch_upload_keys);
-// *launched is false for a step that has nothing to do.
-constexpr int kCountSortSteps = 5;
+// One step of the sort (the tickets are taken with the keys: SolveArgs::count,
+// launch_upload_keys): the scan, the scatter, then the place steps in one
+// launch or, to be timed, the small and the large cells' apart.  *launched is
+// false for a step that has nothing to do.
+enum CountSortStep { kScan = 1, kScatter, kPlaceSmall, kPlaceLarge, kPlace };
 cudaError_t launch_count_sort_step(const RebinArgs& a, int step, uint32_t big_blocks,
                                    cudaStream_t st, bool* launched);
 // Gives a pass's tickets back (its n keys): the counters and tile sums are zero
 // again; skipped when *run_if reads 0.
 cudaError_t launch_untake(const uint32_t* run_if, const uint32_t* keys, uint32_t n,
                           const CountDev& c, int sms, cudaStream_t st);
-// Steps of one rebin (count, scan, scatter, place, large cells; the scan
-// alone when there are no particles) and its kernel launches (a large grid's
-// scan step is two launches).
-uint32_t count_sort_steps(uint32_t n);
+// Kernel launches of one rebin (a large grid's scan step is two; the scan
+// alone when there are no particles).
 uint32_t count_sort_launches(uint32_t n, uint32_t ncells);
 
 // Keys for an upload re-pack: the first n_keep sources are particles of the

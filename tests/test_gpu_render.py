@@ -43,3 +43,21 @@ def test_msaa_resolves_the_union_of_covered_samples(W):
         img = sim.render(48, 36)
     assert np.array_equal(img, R.render(p, dims[0], dims[1], 48, 36))
     assert img[0, 0] == 255
+
+
+def test_render_of_changing_sizes(W):
+    # widths at the edges of the 8-pixel words, quads from a fraction of a
+    # pixel to several words, one context drawing one size after the other
+    rng = np.random.default_rng(8)
+    dims = (48.0, 36.0)
+    pos = rng.uniform((0, 0), dims, size=(120, 2)).astype(np.float32)
+    pos[:3] = [[0.0, 0.0], [48.0, 36.0], [24.0, 0.0]]
+    with W.Simulation(W.WrachConfig(dimensions=dims, cell_size=3, capacity=200)) as sim:
+        sim.add_particles(pos, np.zeros_like(pos))
+        p, _, _ = sim.read_frame()
+        for w, h in [(48, 36), (1, 1), (7, 90), (8, 8), (9, 300), (1200, 17), (65, 64), (48, 36), (3, 500)]:
+            assert np.array_equal(sim.render(w, h), R.render(p, dims[0], dims[1], w, h)), (w, h)
+        # other particles on the same scratch
+        sim.set_particles(pos[:5], np.zeros((5, 2), np.float32))
+        p, _, _ = sim.read_frame()
+        assert np.array_equal(sim.render(65, 64), R.render(p, dims[0], dims[1], 65, 64))

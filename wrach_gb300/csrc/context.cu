@@ -1026,15 +1026,20 @@ int wrach_render(WrachContext* ctx, uint32_t world, uint32_t width_px, uint32_t 
   if (world >= ctx->nworlds) return fail(ctx, WRACH_ERR_INVALID_ARGUMENT, "world out of range");
   DeviceGuard guard(ctx->device);
   const size_t npix = (size_t)width_px * height_px;
-  if (npix > ctx->render_cap) {
+  const size_t words = wrach::render_words(width_px, height_px);
+  // a narrow image takes more words per pixel than a wide one
+  if (npix > ctx->render_cap || words > ctx->cover_cap) {
+    const size_t pixels = std::max(npix, ctx->render_cap), cover = std::max(words, ctx->cover_cap);
     dfree(ctx->render_cover);
     dfree(ctx->render_image);
     ctx->render_cover = nullptr;
     ctx->render_image = nullptr;
-    ctx->render_cap = 0;
-    CK(dalloc(&ctx->render_cover, npix));
-    CK(dalloc(&ctx->render_image, npix));
-    ctx->render_cap = npix;
+    ctx->render_cap = ctx->cover_cap = 0;
+    CK(dalloc(&ctx->render_cover, cover));
+    CK(dalloc(&ctx->render_image, pixels));
+    CK(cudaMemsetAsync(ctx->render_cover, 0, cover * sizeof(uint32_t), ctx->stream));
+    ctx->render_cap = pixels;
+    ctx->cover_cap = cover;
   }
   const WorldDev& w = ctx->worlds_h[world];
   CK(wrach::launch_render(ctx->pos + ctx->poff_h[world], ctx->n_h[world], w.dim_x, w.dim_y, width_px,

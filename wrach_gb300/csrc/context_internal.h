@@ -92,7 +92,7 @@ struct WrachContext {
   uint32_t last_n = 0xFFFFFFFFu;      // particle count of the last frame stepped
   uint32_t* render_cover = nullptr;   // wrach_render scratch and image
   uint8_t* render_image = nullptr;
-  size_t render_cap = 0;
+  size_t render_cap = 0, cover_cap = 0;  // pixels, words of coverage
   cudaEvent_t* event_hook = nullptr;  // wrach_profile_frame: one event per launch boundary
   uint32_t event_count = 0;
   // the learned surrogate (wrach_surrogate_*)

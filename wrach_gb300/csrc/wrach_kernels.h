@@ -283,8 +283,9 @@ cudaError_t launch_keep_outside(const uint32_t* keys, uint32_t ncells, uint32_t 
                                 float2* dst_vel, uint32_t* tile_sums, uint32_t* count,
                                 cudaStream_t st);
 
-// Headless point rasteriser (render.cu): `cover` holds width_px * height_px
-// u32 scratch, `image` the 8-bit result.
+// Headless point rasteriser (render.cu): `cover` is render_words words of
+// scratch, zero before and after, `image` (8-byte aligned) the 8-bit result.
+size_t render_words(uint32_t width_px, uint32_t height_px);
 cudaError_t launch_render(const float2* pos, uint32_t n, float world_w, float world_h,
                           uint32_t width_px, uint32_t height_px, uint32_t* cover,
                           uint8_t* image, cudaStream_t st);

@@ -110,7 +110,6 @@ void release(WrachContext* ctx) {
   if (ctx->join_ev) cudaEventDestroy(ctx->join_ev);
   if (ctx->counts_ev) cudaEventDestroy(ctx->counts_ev);
   if (ctx->aux) cudaStreamDestroy(ctx->aux);
-  if (ctx->back) cudaStreamDestroy(ctx->back);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
 }
 
@@ -471,7 +470,6 @@ int create_impl(const WrachConfig* config, uint32_t nworlds, const float* dims,
   cudaError_t e;
   if ((e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess) return oom(e);
   if ((e = cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking)) != cudaSuccess) return oom(e);
-  if ((e = cudaStreamCreateWithFlags(&ctx->back, cudaStreamNonBlocking)) != cudaSuccess) return oom(e);
   if ((e = cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming)) != cudaSuccess) return oom(e);
   if ((e = cudaEventCreateWithFlags(&ctx->join_ev, cudaEventDisableTiming)) != cudaSuccess) return oom(e);
   if ((e = cudaEventCreateWithFlags(&ctx->counts_ev, cudaEventDisableTiming)) != cudaSuccess) return oom(e);
@@ -642,15 +640,13 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
   r.force_general = 1;
   bool launched;
   CK(wrach::launch_count_sort_step(r, wrach::kScan, ctx->big_blocks, ctx->stream, &launched));
-  // per-world counts from the new table, written to the host on a stream of
-  // their own beside the place steps and the velocities' copy
+  // per-world counts from the new table, written to the host ahead of the
+  // place steps
   const uint32_t nw = ctx->nworlds;
-  CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
-  CK(cudaStreamWaitEvent(ctx->back, ctx->fork_ev, 0));
-  k_gather_starts<<<(nw + 1 + 255) / 256, 256, 0, ctx->back>>>(
+  k_gather_starts<<<(nw + 1 + 255) / 256, 256, 0, ctx->stream>>>(
       ctx->table(ctx->cur ^ 1), ctx->gather_idx, nw + 1, ctx->gather_h);
   CK(cudaGetLastError());
-  CK(cudaEventRecord(ctx->counts_ev, ctx->back));
+  CK(cudaEventRecord(ctx->counts_ev, ctx->stream));
   ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells) + 1;
   auto place = [&]() {
     CK(wrach::launch_count_sort_step(r, wrach::kScatter, ctx->big_blocks, ctx->stream, &launched));
@@ -802,7 +798,6 @@ int wrach_destroy(WrachContext* ctx) {
     // a frame's work on `aux` is joined into `stream`, unless its enqueue
     // failed between the fork and the join
     if (ctx->aux) cudaStreamSynchronize(ctx->aux);
-    if (ctx->back) cudaStreamSynchronize(ctx->back);
     release(ctx);
   }
   delete ctx;

@@ -29,8 +29,6 @@ struct WrachContext {
   cudaStream_t stream = nullptr;
   // uploads: the velocities' copy beside the positions' keys
   cudaStream_t aux = nullptr;
-  // uploads: the counts' way to the host
-  cudaStream_t back = nullptr;
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   // uploads: the per-world counts read back (the call waits for them only)
   cudaEvent_t counts_ev = nullptr;

@@ -27,13 +27,14 @@
 //            of the cell's particles with a smaller source index; then the
 //            gather of positions, velocities and cells into that slot, and of
 //            the taking-part particles' positions, cells and (for the learned
-//            surrogate) velocities into the compacted arrays.  Cells of up to kSmallCell particles are
-//            ranked by one thread per slot
-//   large    (with place, in blocks of their own) one block per listed cell: up to kBigCell particles ranked by a
-//            bitmap of their source indices (or a bitonic sort) in shared
-//            memory, more than that a block-wide LSD radix sort of them in
-//            global memory; then the gather.  It writes other slots than place, so the two may run
-//            at the same time
+//            surrogate) velocities into the compacted arrays.  Cells of up
+//            to kSmallCell particles are ranked by one thread per slot
+//   large    (with place, in blocks of their own) one block per listed cell:
+//            up to kBigCell particles ranked by a bitmap of their source
+//            indices (or a bitonic sort) in shared memory, more than that a
+//            block-wide LSD radix sort of them in global memory; then the
+//            gather.  It writes other slots than place, so the two may run at
+//            the same time
 //
 // The result is the stable order (a cell's particles keep their source
 // order), the order of the oracle's counting sort and of rebin.cu's radix
@@ -77,27 +78,16 @@ k_cs_untake(const uint32_t* __restrict__ run_if, const uint32_t* __restrict__ ke
   }
 }
 
-__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* red) {
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  v = __reduce_add_sync(0xffffffffu, v);
-  __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  uint32_t s = 0;
-#pragma unroll
-  for (uint32_t w = 0; w < kScanThreads / 32; ++w) s += red[w];
-  return s;
-}
-
 // Scans: one block per tile of 2048 cells.  The tile's prefix is the sum of the
 // earlier tiles' counts, which the tickets' pass has already totalled, so no
-// block waits for another.
-// Past this many tiles of the table, k_cs_tile_prefix first turns the tile
-// sums into prefixes, one block per kRun tiles: a tile's sum becomes that of
-// the run's earlier tiles, and the run's own sum goes behind the tile sums.
-// A scan block then adds up the earlier runs instead of the earlier tiles (one
-// block that scanned all tiles by itself took 134 us for the 44,775 tiles of
-// 92M cells; 2.5 us now).
+// block waits for another.  Past this many tiles of the table,
+// k_cs_tile_prefix first turns the tile sums into prefixes, one block per kRun
+// tiles: a tile's sum becomes that of the run's earlier tiles, and the run's
+// own sum goes behind the tile sums.  A scan block then adds up the earlier
+// runs instead of the earlier tiles (one block that scanned all tiles by
+// itself took 134 us for the 44,775 tiles of 92M cells; 2.5 us now).  1,013
+// tiles are still better summed by each block (a frame 103.9 us, 105.8 with
+// the launch).
 constexpr uint32_t kPrefixTiles = 2048, kRun = 256;
 
 __global__ void __launch_bounds__(kRun) k_cs_tile_prefix(RebinArgs a, uint32_t ntiles) {
@@ -153,8 +143,7 @@ __device__ __forceinline__ void list_large(const RebinArgs& a, uint32_t cell) {
 
 __global__ void __launch_bounds__(kScanThreads) k_cs_scan(RebinArgs a) {
   begin_after();
-  __shared__ uint32_t warp_sum[kScanThreads / 32], red[kScanThreads / 32];
-  __shared__ uint32_t warp_cap[kScanThreads / 32];
+  __shared__ uint4 sums[kScanThreads / 32];
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const uint32_t tile = blockIdx.x, n = a.ncells;
   if (tile == 0 && t == 0 && !a.force_general) a.ctrl->frames += 1;
@@ -179,19 +168,19 @@ __global__ void __launch_bounds__(kScanThreads) k_cs_scan(RebinArgs a) {
     sum += v[u];
     csum += min(v[u], cap);
   }
-  // the earlier tiles' totals
-  uint32_t prefix, cprefix;
-  if (a.prefixed_tiles) {
-    prefix = before_tile(a.tile_sums, tile, a.prefixed_tiles);
-    cprefix = cap ? before_tile(a.tile_sums_cap, tile, a.prefixed_tiles) : 0u;
-  } else {
-    uint32_t pre = 0, cpre = 0;
+  // the earlier tiles' totals: the tickets' pass has them ready.  Their sum
+  // goes through the same barrier as the block's own scans below
+  uint32_t pre = 0, cpre = 0;
+  if (!a.prefixed_tiles) {
     for (uint32_t u = t; u < tile; u += kScanThreads) {
       pre += __ldcg(a.tile_sums + u);
       if (cap) cpre += __ldcg(a.tile_sums_cap + u);
     }
-    prefix = block_sum(pre, red);
-    cprefix = cap ? block_sum(cpre, red) : 0u;
+    pre = __reduce_add_sync(0xffffffffu, pre);
+    if (cap) cpre = __reduce_add_sync(0xffffffffu, cpre);
+  } else if (warp == 0) {
+    pre = before_tile(a.tile_sums, tile, a.prefixed_tiles);
+    if (cap) cpre = before_tile(a.tile_sums_cap, tile, a.prefixed_tiles);
   }
   // block-wide exclusive scans of the per-thread sums
   uint32_t x = sum, cx = csum;
@@ -204,18 +193,18 @@ __global__ void __launch_bounds__(kScanThreads) k_cs_scan(RebinArgs a) {
       cx += cy;
     }
   }
-  if (lane == 31) {
-    warp_sum[warp] = x;
-    warp_cap[warp] = cx;
-  }
+  if (lane == 31) sums[warp] = make_uint4(x, cx, pre, cpre);
   __syncthreads();
-  uint32_t before = 0, total = 0, cbefore = 0, ctotal = 0;
+  uint32_t before = 0, total = 0, cbefore = 0, ctotal = 0, prefix = 0, cprefix = 0;
 #pragma unroll
   for (uint32_t w = 0; w < kScanThreads / 32; ++w) {
-    before += w < warp ? warp_sum[w] : 0u;
-    total += warp_sum[w];
-    cbefore += w < warp ? warp_cap[w] : 0u;
-    ctotal += warp_cap[w];
+    const uint4 s = sums[w];
+    before += w < warp ? s.x : 0u;
+    total += s.x;
+    cbefore += w < warp ? s.y : 0u;
+    ctotal += s.y;
+    prefix += s.z;
+    cprefix += s.w;
   }
   uint32_t run = prefix + before + x - sum;
   uint32_t crun = cprefix + cbefore + cx - csum;
@@ -353,6 +342,10 @@ __global__ void __launch_bounds__(kGroupThreads) k_cs_scan_groups(RebinArgs a) {
     a.groups_new[n / kGroup] = make_uint4(run, crun, 0u, 0u);
 }
 
+// Bound by its chain of loads: the key and the ticket together, then the cell's
+// span.  The span also tells the large cells apart, whose slots the next launch
+// then leaves at their first load (4M particles in 256 worlds, this and the
+// place step's loads side by side: 391 -> 387 us a frame).
 template <bool GROUPED>
 __global__ void __launch_bounds__(256) k_cs_scatter(RebinArgs a, uint32_t ntiles) {
   begin_after();
@@ -363,12 +356,15 @@ __global__ void __launch_bounds__(256) k_cs_scatter(RebinArgs a, uint32_t ntiles
     if (a.tp_cap) a.tile_sums_cap[u] = 0u;
   }
   if (i >= a.n) return;
-  const uint32_t k = a.keys[i];
+  const uint32_t k = a.keys[i], ticket = a.ticket[i];
   if (k >= a.ncells) return;
-  const uint32_t dst = new_table<GROUPED>(a).start(k) + a.ticket[i];
+  uint32_t s0, s1;
+  new_table<GROUPED>(a).span(k, s0, s1);
+  const uint32_t dst = s0 + ticket;
   if (dst < a.n) {  // always true unless the scan timed out
     a.idx_tmp[dst] = i;
-    a.cell_tmp[dst] = k;
+    // a large cell's slots are not place_slot's
+    a.cell_tmp[dst] = s1 - s0 > kSmallCell ? a.ncells : k;
   }
 }
 
@@ -408,15 +404,14 @@ __device__ __forceinline__ void place_slot(const RebinArgs& a, uint32_t q) {
   const uint32_t total = table.start(a.ncells);
   uint32_t overflow = 0;
   // the guards below only matter if the scan timed out (table inconsistent)
-  const uint32_t k = q < total && q < a.n ? a.cell_tmp[q] : a.ncells;
-  uint32_t c0 = 0u, c1 = 0u;
-  if (k < a.ncells) table.span(k, c0, c1);
-  // larger cells are the scan's work list, placed by k_cs_big
-  if (k < a.ncells && c1 - c0 <= kSmallCell) {
+  const bool in = q < total && q < a.n;
+  const uint32_t k = in ? a.cell_tmp[q] : a.ncells, me = in ? a.idx_tmp[q] : a.n;
+  if (k < a.ncells) {
+    uint32_t c0, c1;
+    table.span(k, c0, c1);
     const uint32_t s1 = min(c1, min(total, a.n));
-    const uint32_t me = a.idx_tmp[q];
     // the particle's data and its cell's compacted start do not depend on
-    // its rank: their loads go out before the rank's
+    // its rank: their loads go out with the cell's span
     const bool src_ok = me < a.n;
     const float2 p = src_ok ? a.pos_src[me] : make_float2(0.f, 0.f);
     const float2 v = src_ok ? a.vel_src[me] : make_float2(0.f, 0.f);

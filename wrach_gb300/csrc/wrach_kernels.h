@@ -184,10 +184,17 @@ cudaError_t launch_wait_probe(const uint32_t* word, uint32_t value, uint64_t lim
 cudaError_t launch_local_keys(const uint32_t* cell_of, uint32_t n, uint32_t cell_off,
                               uint32_t* out, cudaStream_t st);
 
-// Reference-layout table of one world (cells + 2 entries) from the cell
-// table.
-cudaError_t launch_world_table(const CellTable& table, uint32_t cell_off,
-                               uint32_t cells, uint32_t* out, cudaStream_t st);
+// A world's readback: n particles' positions and velocities (as words) and its
+// table in the reference's layout (cells + 2 entries), each null or written
+// where its pointer says, in device memory or in pinned host memory.
+struct WorldRead {
+  const uint32_t *pos, *vel;
+  uint32_t *pos_out, *vel_out, *table_out;
+  uint32_t n;
+  CellTable table;
+  uint32_t cell_off, cells;
+};
+cudaError_t launch_read_world(const WorldRead& r, int sms, cudaStream_t st);
 
 // The surrogate network (surrogate.cu): FP32 master parameters in the order
 // w1 [64 in][64 out], b1 [64], w2 [64][64], b2 [64], w3 [64][8], b3 [8]

@@ -99,3 +99,27 @@ def test_a_move_that_changes_the_grid_is_refused(W):
         assert tuple(sim.settings().view_anchor) == (3.0, 0.0)
     finally:
         sim.close()
+
+
+@pytest.mark.parametrize("n", [0, 1, 31, 33, 1023, 1024, 1025, 2049])
+@pytest.mark.parametrize("outside", ["none", "all", "mixed", "last"])
+def test_write_back_at_tile_edges(W, O, n, outside):
+    """The store's rebuild moves 1024 items a block by a bit an item: its
+    edges, with no item, every item, some or the last one outside."""
+    dims = (16.0, 9.0)
+    pos, vel = _field(n, n, (0.0, 0.0), (15.9, 8.9))
+    out = {"none": np.zeros(n, bool), "all": np.ones(n, bool),
+           "mixed": np.arange(n) % 7 < 3, "last": np.arange(n) == n - 1}[outside]
+    pos[out] += np.float32([32.0, 0.0])
+    sim = make_sim(W, dims, 1, 1, 2, 0.1, capacity=max(n, 1))
+    try:
+        w, ph = O.world(dims[0], dims[1], 1), oracle_physics(O, 1, 2, 0.1)
+        sim.set_particles(pos, vel)
+        frame = O.pack(w, pos, vel, capacity=sim.capacity())
+        sim.step(1)
+        frame = O.step(w, ph, frame[0], frame[1], frame[2], 1)[:3]
+        sim.write_back()
+        _store_equal(sim, O.write_back(w, pos, vel, frame[1], frame[2]), "n %d %s" % (n, outside))
+        assert_frame_equal(sim.read_frame(), frame, "the frame stays")
+    finally:
+        sim.close()

@@ -734,9 +734,9 @@ int write_back_impl(WrachContext* ctx, uint32_t world) {
   Store& s = ctx->stores[world];
   const uint32_t nf = ctx->n_h[world], off = ctx->poff_h[world];
   int rc;
-  if ((rc = ensure_sort_capacity(ctx, (size_t)s.n + 1))) return rc;
+  const uint32_t ntiles = wrach::store_tiles(s.n);
+  if ((rc = ensure_sort_capacity(ctx, std::max((size_t)s.n + 1, (size_t)ntiles * 32)))) return rc;
   if ((rc = ensure_stage(ctx, (size_t)s.n + nf))) return rc;
-  const uint32_t ntiles = wrach::keep_outside_tiles(s.n);
   if (ntiles + 1 > ctx->compact_cap) {
     dfree(ctx->compact_sums);
     ctx->compact_sums = nullptr;
@@ -744,26 +744,28 @@ int write_back_impl(WrachContext* ctx, uint32_t world) {
     CK(dalloc(&ctx->compact_sums, (size_t)ntiles + 1));
     ctx->compact_cap = (size_t)ntiles + 1;
   }
-  uint32_t kept = 0;
-  if (s.n) {
-    CK(wrach::launch_upload_keys(ctx->worlds_d, (int)ctx->nworlds, ctx->ncells, world, 0, nullptr,
-                                 s.n, s.pos, ctx->keys, ctx->ctrl, wrach::CountDev{},
-                                 ctx->stream));
-    CK(wrach::launch_keep_outside(ctx->keys, ctx->ncells, s.n, s.pos, s.vel, ctx->stage_pos,
-                                  ctx->stage_vel, ctx->compact_sums, ctx->compact_sums + ntiles,
-                                  ctx->stream));
-    ctx->launches += ntiles ? 4 : 2;
-    CK(cudaMemcpyAsync(ctx->gather_h, ctx->compact_sums + ntiles, 4, cudaMemcpyDeviceToHost,
-                       ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    kept = ctx->gather_h[0];
-  }
-  if (nf) {
-    CK(cudaMemcpyAsync(ctx->stage_pos + kept, ctx->pos + off, (size_t)nf * sizeof(float2),
-                       cudaMemcpyDeviceToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->stage_vel + kept, ctx->vel + off, (size_t)nf * sizeof(float2),
-                       cudaMemcpyDeviceToDevice, ctx->stream));
-  }
+  wrach::StoreRebuild r{};
+  r.worlds = ctx->worlds_d;
+  r.target = world;
+  r.n = s.n;
+  r.nf = nf;
+  r.pos = s.pos;
+  r.vel = s.vel;
+  r.frame_pos = ctx->pos + off;
+  r.frame_vel = ctx->vel + off;
+  r.dst_pos = ctx->stage_pos;
+  r.dst_vel = ctx->stage_vel;
+  r.outside = ctx->keys;
+  r.tile_sums = ctx->compact_sums;
+  r.kept = ctx->compact_sums + ntiles;
+  r.kept_host = ctx->gather_h;
+  CK(wrach::launch_outside(r, ctx->stream));
+  CK(cudaEventRecord(ctx->counts_ev, ctx->stream));
+  CK(wrach::launch_rebuild(r, ctx->stream));
+  ctx->launches += (ntiles ? 2 : 1) + (s.n + nf ? 1 : 0);
+  // the store is rebuilt while the host learns its size
+  CK(cudaEventSynchronize(ctx->counts_ev));
+  const uint32_t kept = ctx->gather_h[0];
   if (ctx->nworlds == 1) {
     // the rebuilt store takes the place of the old one, whose buffers serve
     // the next rebuild (with more worlds the staging buffers are larger than

@@ -24,7 +24,8 @@
 // The cell-start table comes from per-cell counts (atomics during the first
 // pass): tile sums are taken between two barriers of the first pass, and after
 // the gather every block scans them and writes its own tiles' starts.
-#include <limits.h>
+#include <algorithm>
+
 
 #include "wrach_internal.cuh"
 #include "wrach_kernels.h"
@@ -379,19 +380,6 @@ cudaError_t launch_rebin(const RebinArgs& a, int grid, cudaStream_t st) {
 
 namespace {
 
-// SpatialBin::get_cell_coord (runners/bevy/src/spatial_bin.rs:48-64):
-// Rust's f32::div_euclid then a saturating `as i32` (NaN -> 0).
-__device__ __forceinline__ int32_t cell_coord_euclid(float x, uint32_t cs) {
-  const float d = (float)cs;
-  float q = truncf(__fdiv_rn(x, d));
-  // the remainder has the sign of x
-  if (x < 0.0f && fmodf(x, d) < 0.0f) q = __fsub_rn(q, 1.0f);
-  if (q != q) return 0;
-  if (q >= 2147483648.0f) return INT_MAX;
-  if (q <= -2147483648.0f) return INT_MIN;
-  return (int32_t)q;
-}
-
 // Keys of the sources, and the counting sort's tickets with them when
 // count.ticket is set (every lane of a warp takes part): the keys never wait
 // in memory for a launch of their own (1M particles: 7.4 us + 16.6 us apart,
@@ -408,12 +396,7 @@ k_upload_keys(const WorldDev* __restrict__ worlds, int nworlds, uint32_t ncells,
     const uint32_t k = cell_of[i];
     if ((uint32_t)world_of_cell(worlds, nworlds, k) != target) key = k;
   } else if (live) {
-    const WorldDev w = worlds[target];
-    const float2 p = new_pos[i - n_keep];
-    const int64_t cx = (int64_t)cell_coord_euclid(p.x, w.cs) - w.blx;
-    const int64_t cy = (int64_t)cell_coord_euclid(p.y, w.cs) - w.bly;
-    if (!(cx < 0 || cy < 0 || cx >= (int64_t)w.gx || cy >= (int64_t)w.gy))
-      key = w.cell_off + (uint32_t)cy * w.gx + (uint32_t)cx;
+    key = upload_key(worlds[target], new_pos[i - n_keep], ncells);
   }
   if (live) keys[i] = key;
   if (count.ticket) {

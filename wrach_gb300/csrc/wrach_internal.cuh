@@ -7,6 +7,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdint.h>
 
 namespace wrach {
@@ -384,6 +385,28 @@ __device__ __forceinline__ void neighbour_rows(const WorldDev& w, const CellTabl
 // (kNoTp: takes no part).  Every neighbour row of the 3x3 search is then one
 // contiguous compacted range, over-full cells or not.
 constexpr uint32_t kNoTp = 0xFFFFFFFFu;
+
+// SpatialBin::get_cell_coord (runners/bevy/src/spatial_bin.rs:48-64):
+// Rust's f32::div_euclid then a saturating `as i32` (NaN -> 0).
+__device__ __forceinline__ int32_t cell_coord_euclid(float x, uint32_t cs) {
+  const float d = (float)cs;
+  float q = truncf(__fdiv_rn(x, d));
+  // the remainder has the sign of x
+  if (x < 0.0f && fmodf(x, d) < 0.0f) q = __fsub_rn(q, 1.0f);
+  if (q != q) return 0;
+  if (q >= 2147483648.0f) return INT_MAX;
+  if (q <= -2147483648.0f) return INT_MIN;
+  return (int32_t)q;
+}
+
+// The cell of world w that an uploaded particle belongs to; `none` outside its
+// viewport.
+__device__ __forceinline__ uint32_t upload_key(const WorldDev& w, float2 p, uint32_t none) {
+  const int64_t cx = (int64_t)cell_coord_euclid(p.x, w.cs) - w.blx;
+  const int64_t cy = (int64_t)cell_coord_euclid(p.y, w.cs) - w.bly;
+  if (cx < 0 || cy < 0 || cx >= (int64_t)w.gx || cy >= (int64_t)w.gy) return none;
+  return w.cell_off + (uint32_t)cy * w.gx + (uint32_t)cx;
+}
 
 __device__ __forceinline__ uint64_t ld_acquire_u64(const uint64_t* p) {
   uint64_t v;

@@ -281,14 +281,23 @@ cudaError_t launch_errors(const SolveArgs& a, const float2* corr, const float2* 
 cudaError_t launch_penetration(const SolveArgs& a, const float2* pos, const float2* vel,
                                float* part, float* out, cudaStream_t st);
 
-// Viewport streaming (viewport.cu): the n items whose key is >= ncells
-// (outside the viewport), in order, into dst; *count receives how many.
-// `tile_sums` holds keep_outside_tiles(n) words of scratch.
-uint32_t keep_outside_tiles(uint32_t n);
-cudaError_t launch_keep_outside(const uint32_t* keys, uint32_t ncells, uint32_t n,
-                                const float2* pos, const float2* vel, float2* dst_pos,
-                                float2* dst_vel, uint32_t* tile_sums, uint32_t* count,
-                                cudaStream_t st);
+// Viewport streaming (viewport.cu): the n store items outside world `target`'s
+// viewport, in order, into dst, and the frame's nf items after them.  *kept and
+// *kept_host (pinned) receive how many were outside.  launch_outside finds
+// them, launch_rebuild moves them.
+struct StoreRebuild {
+  const WorldDev* worlds;
+  uint32_t target, n, nf;
+  const float2 *pos, *vel;              // the store
+  const float2 *frame_pos, *frame_vel;
+  float2 *dst_pos, *dst_vel;
+  uint32_t* outside;                    // store_tiles(n) * 32 words of scratch
+  uint32_t* tile_sums;                  // store_tiles(n) words of scratch
+  uint32_t *kept, *kept_host;
+};
+uint32_t store_tiles(uint32_t n);
+cudaError_t launch_outside(const StoreRebuild& r, cudaStream_t st);
+cudaError_t launch_rebuild(const StoreRebuild& r, cudaStream_t st);
 
 // Headless point rasteriser (render.cu): `cover` is render_words words of
 // scratch, zero before and after, `image` (8-byte aligned) the 8-bit result.

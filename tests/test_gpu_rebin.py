@@ -116,3 +116,34 @@ def test_profiled_frames_match_graph_frames(W, O):
             assert_frame_equal(sim.read_frame(), ref, "frame %d" % (f + 1))
     finally:
         sim.close()
+
+
+@pytest.mark.parametrize("dims", [(31.5, 63.5), (32.5, 63.5), (40.0, 30.0)])
+@pytest.mark.parametrize("add", [False, True])
+def test_an_upload_past_the_capacity_places_nothing(W, O, dims, add):
+    """One world's place steps do not wait for the host to know the count (the
+    scan writes it; at a tile's edge, one cell row past it and inside one):
+    a count that just fits is placed, one more leaves frame, cell table and
+    counters as they are, large cells or not."""
+    pos, vel = _clustered(5, dims, [(3, 4, 63), (9, 9, 64), (9, 10, 65), (20, 20, 700)], 900)
+    n = len(pos)
+    more = np.full((1, 2), 20.5, np.float32)
+    sim = make_sim(W, dims, 1, 1, 4, 0.1, capacity=n)
+    try:
+        w, ph = O.world(dims[0], dims[1], 1), oracle_physics(O, 1, 4, 0.1)
+        sim.set_particles(pos, vel)
+        ref = O.pack(w, pos, vel, capacity=n)
+        assert_frame_equal(sim.read_frame(), ref, "a count that just fits")
+        sim.step(1)
+        ref = O.step(w, ph, ref[0], ref[1], ref[2], 1)[:3]
+        with pytest.raises(W.WrachError):
+            if add:
+                sim.add_particles(more, more * 0)
+            else:
+                sim.set_particles(np.concatenate([pos, more]), np.concatenate([vel, more * 0]))
+        assert_frame_equal(sim.read_frame(), ref, "refused")
+        sim.step(2)
+        ref = O.step(w, ph, ref[0], ref[1], ref[2], 2)[:3]
+        assert_frame_equal(sim.read_frame(), ref, "two frames later")
+    finally:
+        sim.close()

@@ -615,13 +615,13 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
   if (replace) s.n = 0;
   int rc = ensure_store(ctx, s, (size_t)s.n + n_add);
   if (rc) return rc;
-  // The sort places straight into the frame buffers.  For one world re-packed
-  // from a store that holds no more particles than its frame (`direct`) the
-  // capacity check below cannot fail, so the place steps follow the scan at
-  // once, and the velocities are copied on the second stream while the
-  // positions' keys are counted, scanned and scattered (only the place steps
-  // read them); otherwise the place steps wait for the counts.
-  const bool direct = ctx->nworlds == 1 && replace && n_add <= ctx->cap_h[world];
+  // The sort places straight into the frame buffers.  One world's place steps
+  // follow the scan at once (they place nothing when the frame's capacity is
+  // exceeded, which the host then reports), and its velocities are copied on
+  // the second stream while the positions' keys are counted, scanned and
+  // scattered (only the place steps read them).  Of several worlds each has
+  // its own capacity: their place steps wait for the counts.
+  const bool direct = ctx->nworlds == 1;
   const bool vel_aside = direct && n_add;
   if (n_add) {
     CK(cudaMemcpyAsync(s.pos + s.n, pos, (size_t)n_add * sizeof(float2), kind, ctx->stream));
@@ -673,16 +673,23 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
   r.vel_dst = ctx->vel;
   r.cell_dst = ctx->cell_of[ctx->cur ^ 1];
   r.force_general = 1;
+  // per-world counts from the new table, written to the host ahead of the
+  // place steps: one world's by the scan itself
+  const uint32_t nw = ctx->nworlds;
+  if (direct) {
+    r.fits_only = 1;
+    r.total_out = ctx->gather_h + 1;
+  }
   bool launched;
   CK(wrach::launch_count_sort_step(r, wrach::kScan, ctx->big_blocks, ctx->stream, &launched));
-  // per-world counts from the new table, written to the host ahead of the
-  // place steps
-  const uint32_t nw = ctx->nworlds;
-  k_gather_starts<<<(nw + 1 + 255) / 256, 256, 0, ctx->stream>>>(
-      ctx->table(ctx->cur ^ 1), ctx->gather_idx, nw + 1, ctx->gather_h);
-  CK(cudaGetLastError());
+  if (!direct) {
+    k_gather_starts<<<(nw + 1 + 255) / 256, 256, 0, ctx->stream>>>(
+        ctx->table(ctx->cur ^ 1), ctx->gather_idx, nw + 1, ctx->gather_h);
+    CK(cudaGetLastError());
+    ctx->launches += 1;
+  }
   CK(cudaEventRecord(ctx->counts_ev, ctx->stream));
-  ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells) + 1;
+  ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells);
   auto place = [&]() {
     CK(wrach::launch_count_sort_step(r, wrach::kScatter, ctx->big_blocks, ctx->stream, &launched));
     // the place step is the first to read the velocities
@@ -696,6 +703,7 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
   // caller enqueues next on the context's stream
   CK(cudaEventSynchronize(ctx->counts_ev));
   if (vel_aside) CK(cudaEventSynchronize(ctx->join_ev));
+  if (direct) ctx->gather_h[0] = 0u;
   const std::vector<uint32_t> starts(ctx->gather_h, ctx->gather_h + nw + 1);
   for (uint32_t w = 0; w < nw; ++w) {
     const uint32_t cnt = starts[w + 1] - starts[w];

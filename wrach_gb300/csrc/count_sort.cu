@@ -250,7 +250,10 @@ __global__ void __launch_bounds__(kScanThreads) k_cs_scan(RebinArgs a) {
       run += v[u];
     }
   }
-  if (t == 0 && (tile + 1) * kScanTile >= n) a.cs_new[n] = prefix + total;
+  if (t == 0 && (tile + 1) * kScanTile >= n) {
+    a.cs_new[n] = prefix + total;
+    if (a.total_out) *a.total_out = prefix + total;
+  }
 }
 
 // The same for a grouped table: a thread takes 16 cells, two records.  It
@@ -340,6 +343,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_cs_scan_groups(RebinArgs a) {
   }
   if (t == kGroupThreads - 1 && (tile + 1) * kScanTile == n)
     a.groups_new[n / kGroup] = make_uint4(run, crun, 0u, 0u);
+  if (a.total_out && t == kGroupThreads - 1 && tile == gridDim.x - 1) *a.total_out = run;
 }
 
 // Bound by its chain of loads: the key and the ticket together, then the cell's
@@ -677,6 +681,8 @@ template <bool GROUPED>
 __global__ void __launch_bounds__(kBigThreads, 8) k_cs_place(RebinArgs a, uint32_t big_blocks) {
   __shared__ BigScratch sh;
   begin_after();
+  // an upload that is refused leaves the frame as it is
+  if (a.fits_only && new_table<GROUPED>(a).start(a.ncells) > a.dst_capacity) return;
   if (blockIdx.x < big_blocks)
     place_large<GROUPED>(a, sh, blockIdx.x, big_blocks);
   else

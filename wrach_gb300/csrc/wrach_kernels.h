@@ -112,6 +112,8 @@ struct RebinArgs {
   // the starts), the taking-part particles' starts of a dense one
   uint4* groups_new;
   uint32_t* ct_new;
+  uint32_t* total_out;          // the scan also writes the particles' total here (optional)
+  int fits_only;                // place nothing when they are more than dst_capacity
   uint32_t prefixed_tiles;      // scan step: tiles whose sums are prefixes (set by it; 0: none)
   // the taking-part particles, compacted (extended physics; tp_cap == 0: none)
   uint32_t tp_cap;              // cell capacity: the first tp_cap of a cell take part

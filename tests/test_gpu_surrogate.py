@@ -83,6 +83,39 @@ def test_forward_and_gradients_match_oracle(W):
             assert err < 3e-2, (name, err)
 
 
+@pytest.mark.parametrize("n", [1, 300, 20011])
+def test_a_batch_leaves_no_sums_behind(W, n):
+    """The launch that reads a batch's sums clears them: batches before (one of
+    them with NaN inputs) and training steps between (of learning rate 0, so
+    the network stays) do not change a batch's gradients.  The sums' order is
+    free: at most 152 blocks' FP32 partial sums per parameter, 152 * 2^-24 of
+    the sum of their magnitudes, which for sums of either sign is taken as 100
+    times the largest gradient."""
+    torch = _torch()
+    rng = np.random.default_rng(n)
+    with _sim(W, (30.0, 30.0), 900) as sim:
+        sim.add_particles(rng.uniform(0, 30, (800, 2)).astype(np.float32), np.zeros((800, 2), np.float32))
+        sim.surrogate_init(0, 4096)
+        sim.surrogate_set_params(_random_net(rng))
+        assert sim.surrogate_collect() > 0
+        x = torch.randn((n, 64), device="cuda").to(torch.bfloat16)
+        t = torch.randn((n, 2), device="cuda")
+        bad = torch.full((n, 64), float("nan"), device="cuda").to(torch.bfloat16)
+        torch.cuda.synchronize()
+        first, loss = sim.surrogate_gradients(x.data_ptr(), t.data_ptr(), n)
+        tol = 152 * 2.0 ** -24 * 100 * np.abs(first).max()
+        again = []
+        again.append(sim.surrogate_gradients(x.data_ptr(), t.data_ptr(), n))
+        trained = sim.surrogate_train(1, 256, 0.0)
+        again.append(sim.surrogate_gradients(x.data_ptr(), t.data_ptr(), n))
+        assert np.isnan(sim.surrogate_gradients(bad.data_ptr(), t.data_ptr(), n)[1])
+        again.append(sim.surrogate_gradients(x.data_ptr(), t.data_ptr(), n))
+        for g, l in again:
+            assert np.abs(g - first).max() <= tol and abs(l - loss) <= 152 * 2.0 ** -24 * abs(loss)
+        # a training step reports its own batch's loss
+        assert np.isfinite(trained) and trained > 0
+
+
 @pytest.mark.parametrize("n,shift", [(1, 0), (17, 0), (128, 0), (129, 2), (300, 4), (20011, 0), (40001, 2)])
 def test_gradients_over_tiles(W, n, shift):
     # tiles of 128 rows, one or several per block, ragged last tiles, and rows

@@ -149,8 +149,9 @@ int wrach_surrogate_init(WrachContext* ctx, uint32_t seed, uint32_t max_samples)
   if (!S.ready) {
     const size_t nbf = (size_t)2 * (2 * kMlpIn * kMlpHidden + kMlpHidden * kMlpOutPad);
     CK(dalloc(&S.params, kMlpParams));
-    // the gradients and, behind them, the loss: cleared and read back as one
-    CK(dalloc(&S.grad, kMlpParams + 1));
+    // the gradients, the loss and the last batch's loss
+    CK(dalloc(&S.grad, kMlpParams + 2));
+    CK(cudaMemsetAsync(S.grad, 0, (kMlpParams + 2) * sizeof(float), ctx->stream));
     S.loss = S.grad + kMlpParams;
     CK(cudaMallocHost(reinterpret_cast<void**>(&S.grad_h), (kMlpParams + 1) * sizeof(float)));
     CK(dalloc(&S.mom1, kMlpParams));
@@ -268,12 +269,10 @@ int wrach_surrogate_gradients(WrachContext* ctx, const uint16_t* d_x, const floa
   if (!n || !d_x || !d_t || !grad || !loss) return WRACH_ERR_INVALID_ARGUMENT;
   DeviceGuard guard(ctx->device);
   auto& S = ctx->sur;
-  CK(cudaMemsetAsync(S.grad, 0, (wrach::kMlpParams + 1) * 4, ctx->stream));
   CK(wrach::launch_mlp_backward(S.m, d_x, reinterpret_cast<const float2*>(d_t), n, 1.0f / n, S.grad,
                                 S.loss, ctx->sms, ctx->stream));
-  ctx->launches += 1;
-  CK(cudaMemcpyAsync(S.grad_h, S.grad, (wrach::kMlpParams + 1) * 4, cudaMemcpyDeviceToHost,
-                     ctx->stream));
+  CK(wrach::launch_take_gradients(S.grad, S.grad_h, ctx->stream));
+  ctx->launches += 2;
   CK(cudaStreamSynchronize(ctx->stream));
   std::memcpy(grad, S.grad_h, wrach::kMlpParams * 4);
   *loss = S.grad_h[wrach::kMlpParams];
@@ -385,7 +384,6 @@ int wrach_surrogate_train(WrachContext* ctx, uint32_t steps, uint32_t batch, flo
     // a window of the sample buffer, spread over it by a multiplicative hash
     const uint32_t span = S.nsamples - b + 1;
     const uint32_t off = (uint32_t)(((uint64_t)(S.step + 1) * 2654435761ull) % span);
-    CK(cudaMemsetAsync(S.grad, 0, (wrach::kMlpParams + 1) * 4, ctx->stream));
     CK(wrach::launch_mlp_backward(S.m, S.tx + (size_t)off * wrach::kMlpIn, S.tt + off, b, 1.0f / b,
                                   S.grad, S.loss, ctx->sms, ctx->stream));
     ++S.step;
@@ -393,7 +391,7 @@ int wrach_surrogate_train(WrachContext* ctx, uint32_t steps, uint32_t batch, flo
     ctx->launches += 2;
   }
   if (loss) {
-    CK(cudaMemcpyAsync(loss, S.loss, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaMemcpyAsync(loss, S.loss + 1, 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
   }
   return WRACH_OK;

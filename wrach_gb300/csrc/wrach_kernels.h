@@ -11,11 +11,12 @@ namespace wrach {
 // Launches a frame kernel that begins with begin_after: its blocks may be
 // scheduled before the stream's last kernel has ended.
 template <typename... Params, typename... Args>
-cudaError_t launch_after(void (*kernel)(Params...), uint32_t blocks, uint32_t threads,
-                         cudaStream_t st, const Args&... args) {
+cudaError_t launch_after_with(size_t smem, void (*kernel)(Params...), uint32_t blocks,
+                              uint32_t threads, cudaStream_t st, const Args&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -23,6 +24,11 @@ cudaError_t launch_after(void (*kernel)(Params...), uint32_t blocks, uint32_t th
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+template <typename... Params, typename... Args>
+cudaError_t launch_after(void (*kernel)(Params...), uint32_t blocks, uint32_t threads,
+                         cudaStream_t st, const Args&... args) {
+  return launch_after_with(0, kernel, blocks, threads, st, args...);
 }
 
 // Entries past their particle count that the compacted positions and the
@@ -270,7 +276,11 @@ bool train_setup();
 cudaError_t launch_mlp_backward(const MlpDev& m, const uint16_t* x, const float2* target,
                                 uint32_t n, float inv_rows, float* grad, float* loss,
                                 int sms, cudaStream_t st);
-cudaError_t launch_adam(const MlpDev& m, const float* grad, float* mom1, float* mom2, float lr,
+// The sums of launch_mlp_backward's batches (kMlpParams gradients, the loss
+// behind them, then the last batch's loss) are zero between batches: the launch
+// that reads them clears them.
+cudaError_t launch_take_gradients(float* grad, float* out, cudaStream_t st);
+cudaError_t launch_adam(const MlpDev& m, float* grad, float* mom1, float* mom2, float lr,
                         uint32_t step, cudaStream_t st);
 // target[i] = q_t - p_i for the first n frame particles, q compacted (zero
 // for a particle that takes no part).

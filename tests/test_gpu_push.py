@@ -68,3 +68,58 @@ def test_rows_of_every_length(W, O, cap, cell_size):
             sim.step(1)
             ref = O.step(w, ph, ref[0], ref[1], ref[2], 1)[:3]
             assert_frame_equal(sim.read_frame(), ref, "frame %d" % frame)
+
+
+@pytest.mark.parametrize("many", [-1, 0, 1])
+@pytest.mark.parametrize("cap", [1, 9, 10])
+def test_both_sides_of_the_few_particles_rule(W, O, cap, many):
+    """Up to 256 particles per SM the solve kernels keep more loads and pushes
+    in flight: rows of every parity and length, below, at and past that count."""
+    import torch
+    rng = np.random.default_rng(100 * cap)
+    few = 256 * torch.cuda.get_device_properties(0).multi_processor_count
+    n = few + many if many >= 0 else few // 8 + 1
+    gx, gy = 211, 197
+    pos = np.empty((0, 2))
+    while len(pos) < n:
+        counts = rng.integers(0, cap + 3, gx * gy)
+        cell = np.repeat(np.arange(gx * gy), counts)
+        more = np.stack([cell % gx, cell // gx], 1) + rng.uniform(0.01, 0.99, (len(cell), 2))
+        pos = np.concatenate([pos, more])
+    pos = pos[:n].astype(np.float32)
+    vel = rng.normal(0, 0.5, pos.shape).astype(np.float32)
+    dims = (gx - 0.5, gy - 0.5)
+    cfg = W.WrachConfig(dimensions=dims, cell_size=1, mode=1, iterations=4, gravity=0.1,
+                        cell_capacity=cap, capacity=n)
+    ph = O.Physics(1, 4, 0.1, 1.0, 1.0, cap)
+    w = O.world(dims[0], dims[1], 1)
+    with W.Simulation(cfg) as sim:
+        sim.set_particles(pos, vel)
+        ref = O.pack(w, pos, vel, n)
+        for frame in range(3):
+            sim.step(1)
+            ref = O.step(w, ph, ref[0], ref[1], ref[2], 1)[:3]
+            assert_frame_equal(sim.read_frame(), ref, "frame %d" % frame)
+
+
+@pytest.mark.parametrize("filler", [0, 60_000])
+def test_push_of_one_pair_among_many(W, O, filler):
+    # the same separations, with and without a full world that takes the
+    # launches past the few-particles rule
+    sep = _separations(1.0, np.random.default_rng(5))
+    cfg = W.WrachConfig(cell_size=1, mode=1, iterations=3, gravity=0.0, capacity=max(filler, 4))
+    dims = (6.0, 6.0)
+    ph = O.Physics(1, 3, 0.0, 1.0, 1.0, 9)
+    w = O.world(dims[0], dims[1], 1)
+    vel = np.zeros((2, 2), np.float32)
+    rng = np.random.default_rng(9)
+    with W.Simulation(cfg, worlds=[dims] * len(sep) + [(300.0, 300.0)]) as sim:
+        for k, d in enumerate(sep):
+            sim.set_particles(np.array([(0, 0), d], np.float32), vel, world=k)
+        sim.set_particles(rng.uniform(0, 300, (filler, 2)).astype(np.float32),
+                          np.zeros((filler, 2), np.float32), world=len(sep))
+        sim.step(1)
+        for k, d in enumerate(sep):
+            pos = np.array([(0, 0), d], np.float32)
+            ref = O.step(w, ph, *O.pack(w, pos, vel, cfg.capacity), 1)[:3]
+            assert_frame_equal(sim.read_frame(world=k), ref, "separation %r" % (d,))

@@ -199,12 +199,14 @@ struct RowStep {
 
 // The marks of the three rows' candidates.  Mask holds the bits of a row:
 // 3 * cap + 1.  The rows' first steps are loaded together; few rows of sparse
-// frames need a second.
+// frames need a second.  FEW: the further steps of the three rows side by
+// side, two of each at a time, for grids so small that a scheduler has a warp
+// or two and every wait for a load shows.
 template <typename Mask>
 struct Marks {
   Mask m[3];
 };
-template <typename Mask>
+template <typename Mask, bool FEW>
 __device__ __forceinline__ Marks<Mask> all_marks(const PhysDev& ph, const f32x2* __restrict__ q,
                                                  f32x2 qi2, const Rows& R) {
   Marks<Mask> M;
@@ -213,13 +215,36 @@ __device__ __forceinline__ Marks<Mask> all_marks(const PhysDev& ph, const f32x2*
   for (int r = 0; r < 3; ++r) first[r].load(q + (R.start(r) & ~1u));
 #pragma unroll
   for (int r = 0; r < 3; ++r) M.m[r] = first[r].marks(ph, qi2);
+  if constexpr (FEW) {
+    uint32_t end[3], most = 0;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      end[r] = (R.start(r) & 1u) + R.length(r);
+      most = max(most, end[r]);
+    }
+    for (uint32_t k0 = kStep; k0 < most; k0 += 2 * kStep) {
+      RowStep more[3][2];
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (uint32_t k = k0; k < k0 + 2 * kStep; k += kStep)
+          if (k < end[r]) more[r][(k - k0) / kStep].load(q + ((R.start(r) & ~1u) + k));
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (uint32_t k = k0; k < k0 + 2 * kStep; k += kStep)
+          if (k < end[r]) M.m[r] |= (Mask)more[r][(k - k0) / kStep].marks(ph, qi2) << k;
+    }
+  }
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
     const uint32_t s = R.start(r), n = R.length(r), odd = s & 1u;
-    for (uint32_t k = kStep; k < odd + n; k += kStep) {
-      RowStep more;
-      more.load(q + (s - odd + k));
-      M.m[r] |= (Mask)more.marks(ph, qi2) << k;
+    if constexpr (!FEW) {
+      for (uint32_t k = kStep; k < odd + n; k += kStep) {
+        RowStep more;
+        more.load(q + (s - odd + k));
+        M.m[r] |= (Mask)more.marks(ph, qi2) << k;
+      }
     }
     // the row alone, without the particle itself
     M.m[r] &= (((Mask)1 << n) - 1) << odd;
@@ -267,28 +292,42 @@ struct MarkWalk {
 // current one.  Two marks a turn: their factors are paired arithmetic, and the
 // loop's own instructions serve both (4M particles in dense clusters, frame
 // 8: the three iterations 203, 176 and 227 us with one mark a turn and the
-// general square root and division, 181, 157 and 135 us now).  METRICS: pen =
-// the deepest overlap min_d - distance with a pushing neighbour.
-template <typename Mask, bool METRICS>
+// general square root and division, 181, 157 and 135 us now).  FEW: four a
+// turn, whose chains of arithmetic run side by side.  METRICS: pen = the
+// deepest overlap min_d - distance with a pushing neighbour.
+template <typename Mask, bool METRICS, bool FEW>
 __device__ __forceinline__ void push_marked(const PhysDev& ph, const f32x2* __restrict__ q,
                                             f32x2 qi2, const Rows& R, const Marks<Mask>& M,
                                             float& ax, float& ay, float& pen) {
   MarkWalk<Mask> walk(R, M);
+  constexpr int turn = FEW ? 4 : 2;
   while (walk.cur) {
-    const uint32_t j0 = walk.take();
-    const bool two = walk.cur != 0;
-    const uint32_t j1 = two ? walk.take() : j0;
-    const f32x2 d0 = f2_sub(q[j0], qi2), d1 = f2_sub(q[j1], qi2);
-    float f0, f1, e0, e1;
-    push_factors_near(f2_len2(d0), f2_len2(d1), ph, f0, f1, e0, e1);
-    if (METRICS) pen = fmaxf(pen, __fsub_rn(ph.min_d, e0));
-    // scalar: a paired multiply feeding a paired add may be fused
-    ax = __fadd_rn(ax, __fmul_rn(f2_x(d0), f0));
-    ay = __fadd_rn(ay, __fmul_rn(f2_y(d0), f0));
-    if (two) {
-      if (METRICS) pen = fmaxf(pen, __fsub_rn(ph.min_d, e1));
-      ax = __fadd_rn(ax, __fmul_rn(f2_x(d1), f1));
-      ay = __fadd_rn(ay, __fmul_rn(f2_y(d1), f1));
+    uint32_t j[turn];
+    int many = 1;
+    j[0] = walk.take();
+#pragma unroll
+    for (int u = 1; u < turn; ++u) {
+      j[u] = j[0];
+      if (walk.cur) {
+        j[u] = walk.take();
+        ++many;
+      }
+    }
+    f32x2 d[turn];
+    float s[turn], f[turn], e[turn];
+#pragma unroll
+    for (int u = 0; u < turn; ++u) d[u] = f2_sub(q[j[u]], qi2);
+#pragma unroll
+    for (int u = 0; u < turn; ++u) s[u] = f2_len2(d[u]);
+    push_factors_near<turn>(s, ph, f, e);
+#pragma unroll
+    for (int u = 0; u < turn; ++u) {
+      if (u == 0 || u < many) {
+        if (METRICS) pen = fmaxf(pen, __fsub_rn(ph.min_d, e[u]));
+        // scalar: a paired multiply feeding a paired add may be fused
+        ax = __fadd_rn(ax, __fmul_rn(f2_x(d[u]), f[u]));
+        ay = __fadd_rn(ay, __fmul_rn(f2_y(d[u]), f[u]));
+      }
     }
   }
 }
@@ -303,8 +342,8 @@ __device__ __forceinline__ void push_marked(const PhysDev& ph, const f32x2* __re
 // At most 42 registers (three blocks of 512): the loads' latency needs the
 // warps.  On the 1M lattice an iteration issues about 60% of the time and
 // waits for its gathers through L1 for the rest.
-template <typename Mask, int ROWS, bool ONE>
-__global__ void __launch_bounds__(512, 3)
+template <typename Mask, int ROWS, bool ONE, bool FEW>
+__global__ void __launch_bounds__(512, FEW ? 1 : 3)
 k_jacobi_tp(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t ncells,
             const CellTable table, const uint32_t* __restrict__ tp_cell,
             const float2* __restrict__ qin, float2* __restrict__ qout,
@@ -328,7 +367,7 @@ k_jacobi_tp(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t nce
     }
     const f32x2 qi2 = q[t];
     float ax = 0.f, ay = 0.f, pen = 0.f;
-    push_marked<Mask, false>(ph, q, qi2, R, all_marks<Mask>(ph, q, qi2, R), ax, ay, pen);
+    push_marked<Mask, false, FEW>(ph, q, qi2, R, all_marks<Mask, FEW>(ph, q, qi2, R), ax, ay, pen);
     qout[t] = make_float2(__fsub_rn(f2_x(qi2), ax), __fsub_rn(f2_y(qi2), ay));
   }
 }
@@ -346,8 +385,8 @@ k_jacobi_tp(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t nce
 // [4] the kinetic energy a plain frame gives (gravity, the clamp and wall
 // reflections only change the velocity).  A launch whose `run_if` flag reads
 // 0 returns at once.
-template <typename Mask, int ROWS, bool METRICS, bool ONE>
-__global__ void __launch_bounds__(512, METRICS ? 2 : 3)
+template <typename Mask, int ROWS, bool METRICS, bool ONE, bool FEW>
+__global__ void __launch_bounds__(512, FEW ? 1 : METRICS ? 2 : 3)
 k_jacobi_final(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t n,
                int do_push, const CellTable table, const uint32_t* __restrict__ tp_of,
                const uint32_t* __restrict__ cell_of, const uint4* __restrict__ rows,
@@ -392,7 +431,7 @@ k_jacobi_final(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t 
           } else {
             R = tp_rows(w, table, c, t);
           }
-          push_marked<Mask, METRICS>(ph, q, qi2, R, all_marks<Mask>(ph, q, qi2, R), ax, ay, pen);
+          push_marked<Mask, METRICS, FEW>(ph, q, qi2, R, all_marks<Mask, FEW>(ph, q, qi2, R), ax, ay, pen);
         }
         qx = __fsub_rn(f2_x(qi2), ax);
         qy = __fsub_rn(f2_y(qi2), ay);
@@ -479,27 +518,36 @@ uint32_t solve_blocks(const SolveArgs& a) {
 // A row's marks fit 32 bits: its candidates and one more for an odd start.
 static bool narrow_marks(const PhysDev& ph) { return 3 * ph.cap + 1 <= 32; }
 
-template <typename Mask, int ROWS>
+template <typename Mask, int ROWS, bool FEW>
 static cudaError_t launch_iteration(const SolveArgs& a, uint32_t blocks, uint32_t threads,
                                     const float2* qin, float2* qout, cudaStream_t st) {
   if constexpr (ROWS != 2) {
     if (a.nworlds != 1)
-      return launch_after(k_jacobi_tp<Mask, ROWS, false>, blocks, threads, st,
+      return launch_after(k_jacobi_tp<Mask, ROWS, false, FEW>, blocks, threads, st,
                           Worlds<false>{a.worlds, a.nworlds}, a.ph, a.ncells, a.table, a.tp_cell,
                           qin, qout, a.run_if, a.rows);
   }
   // the rows read back need no world
-  return launch_after(k_jacobi_tp<Mask, ROWS, true>, blocks, threads, st, Worlds<true>{a.world},
+  return launch_after(k_jacobi_tp<Mask, ROWS, true, FEW>, blocks, threads, st, Worlds<true>{a.world},
                       a.ph, a.ncells, a.table, a.tp_cell, qin, qout, a.run_if, a.rows);
 }
 
-template <typename Mask>
+// Up to two blocks of 128 per SM, the kernels with more loads and pushes in
+// flight per thread (their 108 registers leave 16 warps an SM): 16,384
+// particles piled up, 35.0 -> 31.0 us a frame, 32,768 39.0 -> 34.8, and no
+// difference while they are spread out (20.7 and 24.0).  65,536 42.8 -> 40.2,
+// but spread out 26.8 -> 28.3, and 262,144 52 -> 62.
+static bool few_particles(const SolveArgs& a) {
+  return narrow_marks(a.ph) && !a.part && a.n <= (uint32_t)(a.sms > 0 ? a.sms : 1) * 256u;
+}
+
+template <typename Mask, bool FEW>
 static cudaError_t launch_iteration(const SolveArgs& a, uint32_t blocks, uint32_t threads,
                                     const float2* qin, float2* qout, cudaStream_t st) {
   const int mode = a.rows ? a.rows_mode : 0;
-  if (mode == 1) return launch_iteration<Mask, 1>(a, blocks, threads, qin, qout, st);
-  if (mode == 2) return launch_iteration<Mask, 2>(a, blocks, threads, qin, qout, st);
-  return launch_iteration<Mask, 0>(a, blocks, threads, qin, qout, st);
+  if (mode == 1) return launch_iteration<Mask, 1, FEW>(a, blocks, threads, qin, qout, st);
+  if (mode == 2) return launch_iteration<Mask, 2, FEW>(a, blocks, threads, qin, qout, st);
+  return launch_iteration<Mask, 0, FEW>(a, blocks, threads, qin, qout, st);
 }
 
 cudaError_t launch_jacobi_iteration(const SolveArgs& a, const float2* qin, float2* qout,
@@ -512,19 +560,20 @@ cudaError_t launch_jacobi_iteration(const SolveArgs& a, const float2* qin, float
   // 771 -> 765 us spread out, 326 -> 304 us piled up; with 54 per SM 786 and 295.
   const uint32_t most = (uint32_t)(a.sms > 0 ? a.sms : 1) * (13824u / threads);
   const uint32_t blocks = std::min(solve_blocks(a), most);
-  return narrow_marks(a.ph) ? launch_iteration<uint32_t>(a, blocks, threads, qin, qout, st)
-                            : launch_iteration<uint64_t>(a, blocks, threads, qin, qout, st);
+  if (few_particles(a)) return launch_iteration<uint32_t, true>(a, blocks, threads, qin, qout, st);
+  return narrow_marks(a.ph) ? launch_iteration<uint32_t, false>(a, blocks, threads, qin, qout, st)
+                            : launch_iteration<uint64_t, false>(a, blocks, threads, qin, qout, st);
 }
 
-template <typename Mask, int ROWS, bool METRICS>
+template <typename Mask, int ROWS, bool METRICS, bool FEW>
 static cudaError_t launch_final(const SolveArgs& a, uint32_t blocks, uint32_t threads,
                                 const float2* qtp, int do_push, cudaStream_t st) {
   if (a.nworlds == 1)
-    return launch_after(k_jacobi_final<Mask, ROWS, METRICS, true>, blocks, threads, st,
+    return launch_after(k_jacobi_final<Mask, ROWS, METRICS, true, FEW>, blocks, threads, st,
                         Worlds<true>{a.world}, a.ph, a.n, do_push, a.table, a.tp_of, a.cell_of,
                         a.rows, a.pos, qtp, a.pos_out, a.vel, a.vel_out, a.keys, a.ctrl, a.run_if,
                         a.part, a.count);
-  return launch_after(k_jacobi_final<Mask, ROWS, METRICS, false>, blocks, threads, st,
+  return launch_after(k_jacobi_final<Mask, ROWS, METRICS, false, FEW>, blocks, threads, st,
                       Worlds<false>{a.worlds, a.nworlds}, a.ph, a.n, do_push, a.table, a.tp_of,
                       a.cell_of, a.rows, a.pos, qtp, a.pos_out, a.vel, a.vel_out, a.keys, a.ctrl,
                       a.run_if, a.part, a.count);
@@ -535,10 +584,15 @@ static cudaError_t launch_final(const SolveArgs& a, uint32_t blocks, uint32_t th
                                 const float2* qtp, int do_push, cudaStream_t st) {
   const bool rows = a.rows && a.rows_mode == 2;
   if (a.part)
-    return rows ? launch_final<Mask, 2, true>(a, blocks, threads, qtp, do_push, st)
-                : launch_final<Mask, 0, true>(a, blocks, threads, qtp, do_push, st);
-  return rows ? launch_final<Mask, 2, false>(a, blocks, threads, qtp, do_push, st)
-              : launch_final<Mask, 0, false>(a, blocks, threads, qtp, do_push, st);
+    return rows ? launch_final<Mask, 2, true, false>(a, blocks, threads, qtp, do_push, st)
+                : launch_final<Mask, 0, true, false>(a, blocks, threads, qtp, do_push, st);
+  if constexpr (sizeof(Mask) == 4) {
+    if (few_particles(a))
+      return rows ? launch_final<Mask, 2, false, true>(a, blocks, threads, qtp, do_push, st)
+                  : launch_final<Mask, 0, false, true>(a, blocks, threads, qtp, do_push, st);
+  }
+  return rows ? launch_final<Mask, 2, false, false>(a, blocks, threads, qtp, do_push, st)
+              : launch_final<Mask, 0, false, false>(a, blocks, threads, qtp, do_push, st);
 }
 
 cudaError_t launch_jacobi_final(const SolveArgs& a, const float2* qtp, int do_push,

@@ -217,8 +217,8 @@ __device__ __forceinline__ float push_factor_general(float s, const PhysDev& ph,
 __device__ __forceinline__ bool push_special(float s, float d, const PhysDev& ph) {
   return !(s >= ph.slow_below) || (__float_as_uint(d) | 0xFF800000u) == 0xFFFFFFFFu;
 }
-__device__ __forceinline__ void push_factors_near(float s0, float s1, const PhysDev& ph, float& f0,
-                                                  float& f1, float& dist0, float& dist1) {
+__device__ __forceinline__ void push_factors_plain(float s0, float s1, const PhysDev& ph, float& f0,
+                                                   float& f1, float& dist0, float& dist1) {
   const f32x2 s = f2_pack(s0, s1), y = f2_pack(rsqrt_approx(s0), rsqrt_approx(s1));
   const f32x2 g = f2_mul(s, y), minus = f2_both(-1.0f), one = f2_both(1.0f);
   const f32x2 d = f2_fma(f2_fma(g, g, f2_mul(s, minus)), f2_mul(y, f2_both(-0.5f)), g);
@@ -232,9 +232,20 @@ __device__ __forceinline__ void push_factors_near(float s0, float s1, const Phys
   f1 = f2_y(f);
   dist0 = f2_x(d);
   dist1 = f2_y(d);
-  if (push_special(s0, dist0, ph) || push_special(s1, dist1, ph)) {
-    f0 = push_factor_general(s0, ph, dist0);
-    f1 = push_factor_general(s1, ph, dist1);
+}
+// N (even) pairs at once, so that their chains interleave.
+template <int N>
+__device__ __forceinline__ void push_factors_near(const float (&s)[N], const PhysDev& ph,
+                                                  float (&f)[N], float (&dist)[N]) {
+#pragma unroll
+  for (int u = 0; u < N; u += 2)
+    push_factors_plain(s[u], s[u + 1], ph, f[u], f[u + 1], dist[u], dist[u + 1]);
+  bool special = false;
+#pragma unroll
+  for (int u = 0; u < N; ++u) special = special || push_special(s[u], dist[u], ph);
+  if (special) {
+#pragma unroll
+    for (int u = 0; u < N; ++u) f[u] = push_factor_general(s[u], ph, dist[u]);
   }
 }
 

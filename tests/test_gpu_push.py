@@ -123,3 +123,36 @@ def test_push_of_one_pair_among_many(W, O, filler):
             pos = np.array([(0, 0), d], np.float32)
             ref = O.step(w, ph, *O.pack(w, pos, vel, cfg.capacity), 1)[:3]
             assert_frame_equal(sim.read_frame(world=k), ref, "separation %r" % (d,))
+
+
+@pytest.mark.parametrize("cap", [11, 16])
+def test_rows_around_32_marks(W, O, cap):
+    """Where rows may hold more than 32 marks, a warp whose rows do not takes
+    the 32-bit walk: rows of 28 to 36 candidates at odd and even starts, in
+    warps of their own and mixed with longer and shorter ones."""
+    rng = np.random.default_rng(cap)
+    gx, gy = 160, 24
+    counts = np.zeros((gy, gx), np.int64)
+    for y in range(0, gy, 3):
+        # runs of 16 cells whose rows hold `rows` candidates, then empty cells
+        for k, rows in enumerate(rng.permutation(np.arange(28, 37))[:8]):
+            three = np.array([rows // 3, rows // 3, rows - 2 * (rows // 3)]).clip(0, cap)
+            counts[y, 20 * k:20 * k + 15] = np.tile(three, 5)
+            counts[y, 20 * k + 15:20 * k + 18] = rng.integers(0, cap + 3, 3)
+    counts = counts.ravel()
+    cell = np.repeat(np.arange(gx * gy), counts)
+    pos = (np.stack([cell % gx, cell // gx], 1) + rng.uniform(0.01, 0.99, (len(cell), 2))) * 2
+    pos = pos.astype(np.float32)
+    vel = rng.normal(0, 0.5, pos.shape).astype(np.float32)
+    dims = (gx * 2 - 0.5, gy * 2 - 0.5)
+    cfg = W.WrachConfig(dimensions=dims, cell_size=2, mode=1, iterations=3, gravity=0.1,
+                        cell_capacity=cap, capacity=len(pos))
+    ph = O.Physics(1, 3, 0.1, 1.0, 1.0, cap)
+    w = O.world(dims[0], dims[1], 2)
+    with W.Simulation(cfg) as sim:
+        sim.set_particles(pos, vel)
+        ref = O.pack(w, pos, vel, len(pos))
+        for frame in range(3):
+            sim.step(1)
+            ref = O.step(w, ph, ref[0], ref[1], ref[2], 1)[:3]
+            assert_frame_equal(sim.read_frame(), ref, "frame %d" % frame)

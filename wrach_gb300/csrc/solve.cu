@@ -332,6 +332,27 @@ __device__ __forceinline__ void push_marked(const PhysDev& ph, const f32x2* __re
   }
 }
 
+// An iteration's push by all candidates in reach.  Where the cell capacity
+// allows rows of more marks than 32 bits, most warps have none: they take the
+// 32-bit walk (300,000 particles, capacity 16, six passes: 67.7 us a frame
+// with 64-bit marks throughout, 63.2 now; at 5 a cell 94.7 and 87.9; with all
+// cells past 10, where nearly no warp does, 139.7 and 141.0).  The last pass
+// keeps its one walk: it gains nothing from a second.
+template <typename Mask, bool FEW>
+__device__ __forceinline__ void push_all(const PhysDev& ph, const f32x2* __restrict__ q, f32x2 qi2,
+                                         const Rows& R, float& ax, float& ay) {
+  float pen = 0.f;
+  if constexpr (sizeof(Mask) > 4) {
+    // no length has bit 5: 31 candidates and an odd start are 32 marks
+    if (!__any_sync(__activemask(), (R.len & 0x20820u) != 0u)) {
+      push_marked<uint32_t, false, FEW>(ph, q, qi2, R, all_marks<uint32_t, FEW>(ph, q, qi2, R), ax,
+                                        ay, pen);
+      return;
+    }
+  }
+  push_marked<Mask, false, FEW>(ph, q, qi2, R, all_marks<Mask, FEW>(ph, q, qi2, R), ax, ay, pen);
+}
+
 // One Jacobi iteration but the last, one thread per compacted (taking-part)
 // particle: q' = q - push sum, over the compacted count (a
 // grid-stride loop; the plain frames' grid covers every particle of the
@@ -366,8 +387,8 @@ k_jacobi_tp(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t nce
       if (ROWS == 1) rows[t] = make_uint4(R.s0, R.s1, R.s2, R.len);
     }
     const f32x2 qi2 = q[t];
-    float ax = 0.f, ay = 0.f, pen = 0.f;
-    push_marked<Mask, false, FEW>(ph, q, qi2, R, all_marks<Mask, FEW>(ph, q, qi2, R), ax, ay, pen);
+    float ax = 0.f, ay = 0.f;
+    push_all<Mask, FEW>(ph, q, qi2, R, ax, ay);
     qout[t] = make_float2(__fsub_rn(f2_x(qi2), ax), __fsub_rn(f2_y(qi2), ay));
   }
 }
@@ -431,7 +452,8 @@ k_jacobi_final(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t 
           } else {
             R = tp_rows(w, table, c, t);
           }
-          push_marked<Mask, METRICS, FEW>(ph, q, qi2, R, all_marks<Mask, FEW>(ph, q, qi2, R), ax, ay, pen);
+          push_marked<Mask, METRICS, FEW>(ph, q, qi2, R, all_marks<Mask, FEW>(ph, q, qi2, R), ax, ay,
+                                          pen);
         }
         qx = __fsub_rn(f2_x(qi2), ax);
         qy = __fsub_rn(f2_y(qi2), ay);

@@ -98,7 +98,7 @@ struct WrachContext {
     bool ready = false;
     wrach::MlpDev m{};
     float *params = nullptr, *grad = nullptr, *mom1 = nullptr, *mom2 = nullptr;
-    float *loss = nullptr;           // behind the gradients, and the last batch's behind it
+    float* loss = nullptr;           // the last batch's, behind the gradients
     float *grad_h = nullptr;         // pinned: the gradients and the loss read back
     float *metrics = nullptr;
     float* part = nullptr;           // per-block metrics of a solve launch (8 floats a block)

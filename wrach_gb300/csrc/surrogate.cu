@@ -383,13 +383,20 @@ __device__ __forceinline__ void add_tile(float* w, uint32_t ld, uint32_t m0, uin
   atomicAdd(reinterpret_cast<float2*>(p + 8 * ld), make_float2(c[2], c[3]));
 }
 
+// The loss, a 64-bit sum behind the gradients: with 32 bits it turned with the
+// order of the warps' shares by up to 2e-6 of itself.
+__device__ __forceinline__ double* loss_of(float* grad) {
+  return reinterpret_cast<double*>(grad + kMlpParams);
+}
+static_assert(kMlpParams % 2 == 0, "the loss is 8-byte aligned");
+
 // Gradients of L = 0.5 * sum over rows and the 2 outputs of (y - target)^2 /
 // `scale_rows` with respect to every parameter, added into `grad` (FP32,
 // the MlpDev parameter order: w1 [in][out], b1, w2, b2, w3 [in][8], b3).
-// Also adds the loss into *loss.
+// Also adds the loss into the 64-bit sum behind them.
 __global__ void __launch_bounds__(kTrainThreads, 1)
 k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restrict__ target,
-               uint32_t n, float inv_rows, float* __restrict__ grad, float* __restrict__ loss) {
+               uint32_t n, float inv_rows, float* __restrict__ grad) {
   extern __shared__ __align__(16) uint8_t dyn[];
   begin_after();
   SmemTrain& sm = *reinterpret_cast<SmemTrain*>(dyn);
@@ -537,7 +544,8 @@ k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restric
   }
   if (lane == 0) {
     atomicAdd(reinterpret_cast<float2*>(grad + o_b3), make_float2(sb3[0], sb3[1]));
-    if (lsum != 0.f) atomicAdd(loss, lsum * inv_rows);
+    // (in 64 bits: a sum of up to 1216 warps' shares)
+    if (lsum != 0.f) atomicAdd(loss_of(grad), (double)lsum * (double)inv_rows);
   }
 }
 
@@ -548,9 +556,14 @@ k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restric
 // a copy to the host and its gap replaced by k_take_gradients: 44 -> 34 us).
 // Behind the gradients lie the loss and the last batch's loss, which stays.
 __device__ __forceinline__ float take_sum(float* grad, uint32_t i, uint32_t nparams) {
+  if (i == nparams) {
+    const float loss = (float)*loss_of(grad);
+    *loss_of(grad) = 0.0;
+    grad[nparams + 2] = loss;
+    return loss;
+  }
   const float g = grad[i];
   grad[i] = 0.f;
-  if (i == nparams) grad[nparams + 1] = g;
   return g;
 }
 
@@ -1132,12 +1145,12 @@ bool train_setup() {
 }
 
 cudaError_t launch_mlp_backward(const MlpDev& m, const uint16_t* x, const float2* target,
-                                uint32_t n, float inv_rows, float* grad, float* loss, int sms,
+                                uint32_t n, float inv_rows, float* grad, int sms,
                                 cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   const uint32_t tiles = (n + kTrainRows - 1) / kTrainRows, most = sms > 0 ? sms : 1;
   return launch_after_with(sizeof(SmemTrain), k_mlp_backward, tiles < most ? tiles : most,
-                           kTrainThreads, st, m, x, target, n, inv_rows, grad, loss);
+                           kTrainThreads, st, m, x, target, n, inv_rows, grad);
 }
 
 cudaError_t launch_take_gradients(float* grad, float* out, cudaStream_t st) {

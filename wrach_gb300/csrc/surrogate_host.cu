@@ -150,9 +150,9 @@ int wrach_surrogate_init(WrachContext* ctx, uint32_t seed, uint32_t max_samples)
     const size_t nbf = (size_t)2 * (2 * kMlpIn * kMlpHidden + kMlpHidden * kMlpOutPad);
     CK(dalloc(&S.params, kMlpParams));
     // the gradients, the loss and the last batch's loss
-    CK(dalloc(&S.grad, kMlpParams + 2));
-    CK(cudaMemsetAsync(S.grad, 0, (kMlpParams + 2) * sizeof(float), ctx->stream));
-    S.loss = S.grad + kMlpParams;
+    CK(dalloc(&S.grad, kMlpParams + 3));
+    CK(cudaMemsetAsync(S.grad, 0, (kMlpParams + 3) * sizeof(float), ctx->stream));
+    S.loss = S.grad + kMlpParams + 2;
     CK(cudaMallocHost(reinterpret_cast<void**>(&S.grad_h), (kMlpParams + 1) * sizeof(float)));
     CK(dalloc(&S.mom1, kMlpParams));
     CK(dalloc(&S.mom2, kMlpParams));
@@ -270,7 +270,7 @@ int wrach_surrogate_gradients(WrachContext* ctx, const uint16_t* d_x, const floa
   DeviceGuard guard(ctx->device);
   auto& S = ctx->sur;
   CK(wrach::launch_mlp_backward(S.m, d_x, reinterpret_cast<const float2*>(d_t), n, 1.0f / n, S.grad,
-                                S.loss, ctx->sms, ctx->stream));
+                                ctx->sms, ctx->stream));
   CK(wrach::launch_take_gradients(S.grad, S.grad_h, ctx->stream));
   ctx->launches += 2;
   CK(cudaStreamSynchronize(ctx->stream));
@@ -385,13 +385,13 @@ int wrach_surrogate_train(WrachContext* ctx, uint32_t steps, uint32_t batch, flo
     const uint32_t span = S.nsamples - b + 1;
     const uint32_t off = (uint32_t)(((uint64_t)(S.step + 1) * 2654435761ull) % span);
     CK(wrach::launch_mlp_backward(S.m, S.tx + (size_t)off * wrach::kMlpIn, S.tt + off, b, 1.0f / b,
-                                  S.grad, S.loss, ctx->sms, ctx->stream));
+                                  S.grad, ctx->sms, ctx->stream));
     ++S.step;
     CK(wrach::launch_adam(S.m, S.grad, S.mom1, S.mom2, lr, S.step, ctx->stream));
     ctx->launches += 2;
   }
   if (loss) {
-    CK(cudaMemcpyAsync(loss, S.loss + 1, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaMemcpyAsync(loss, S.loss, 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
   }
   return WRACH_OK;

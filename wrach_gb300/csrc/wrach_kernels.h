@@ -274,11 +274,11 @@ cudaError_t launch_mlp_forward_tc(const MlpDev& m, const uint16_t* x, uint32_t n
 // memory size).
 bool train_setup();
 cudaError_t launch_mlp_backward(const MlpDev& m, const uint16_t* x, const float2* target,
-                                uint32_t n, float inv_rows, float* grad, float* loss,
-                                int sms, cudaStream_t st);
-// The sums of launch_mlp_backward's batches (kMlpParams gradients, the loss
-// behind them, then the last batch's loss) are zero between batches: the launch
-// that reads them clears them.
+                                uint32_t n, float inv_rows, float* grad, int sms,
+                                cudaStream_t st);
+// The sums of launch_mlp_backward's batches (kMlpParams gradients, the 64-bit
+// loss behind them, then the last batch's loss) are zero between batches: the
+// launch that reads them clears them.
 cudaError_t launch_take_gradients(float* grad, float* out, cudaStream_t st);
 cudaError_t launch_adam(const MlpDev& m, float* grad, float* mom1, float* mom2, float lr,
                         uint32_t step, cudaStream_t st);

@@ -73,7 +73,7 @@ __device__ __forceinline__ void publish_flags(Ctrl* ctrl, uint32_t flags) {
 // the cells that start in its first W particles (all their m particles are in
 // its lanes), and integrates the particles past a cell's capacity among its
 // first W.  1M particles, cell size 1: 36 us and a separate ticket launch of
-// 14 us before, 23 us with the tickets now.
+// 14 us before, 21 us with the tickets now.
 template <bool ONE>
 __global__ void __launch_bounds__(512, 3)
 k_solve_reference(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t n,

@@ -145,7 +145,7 @@ int rebin_grid_size(int device, uint32_t digit_bits);
 cudaError_t launch_rebin(const RebinArgs& a, int grid, cudaStream_t st);
 
 // The same rebin as a stable counting sort over the cells (count_sort.cu),
-// five plain launches: cells of up to kSmallCell particles are ranked per
+// short launches: cells of up to kSmallCell particles are ranked per
 // slot, cells of up to kBigCell in shared memory, larger ones in global
 // memory by one block each.
 constexpr uint32_t kCountScanShift = 11;

@@ -51,6 +51,7 @@ __device__ __forceinline__ uint32_t samples_in(const float (&offset)[4], int px,
 __global__ void __launch_bounds__(256)
 k_raster(const float2* __restrict__ pos, uint32_t n, float sx, float sy, uint32_t width_px,
          uint32_t height_px, uint32_t row_words, uint32_t* __restrict__ cover) {
+  begin_after();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float2 p = pos[i];
@@ -93,6 +94,7 @@ k_raster(const float2* __restrict__ pos, uint32_t n, float sx, float sy, uint32_
 __global__ void __launch_bounds__(256)
 k_resolve(uint32_t* __restrict__ cover, uint32_t width_px, uint32_t height_px, uint32_t row_words,
           uint8_t* __restrict__ image) {
+  begin_after();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)row_words * height_px) return;
   const uint32_t mask = cover[i];
@@ -122,13 +124,12 @@ cudaError_t launch_render(const float2* pos, uint32_t n, float world_w, float wo
   const uint32_t row_words = (width_px + 7) / 8;
   const float sx = (float)width_px / world_w, sy = (float)height_px / world_h;
   if (n) {
-    k_raster<<<(n + 255) / 256, 256, 0, st>>>(pos, n, sx, sy, width_px, height_px, row_words, cover);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_after(k_raster, (n + 255) / 256, 256, st, pos, n, sx, sy, width_px,
+                                       height_px, row_words, cover);
     if (e != cudaSuccess) return e;
   }
-  k_resolve<<<(unsigned)((render_words(width_px, height_px) + 255) / 256), 256, 0, st>>>(
-      cover, width_px, height_px, row_words, image);
-  return cudaGetLastError();
+  return launch_after(k_resolve, (uint32_t)((render_words(width_px, height_px) + 255) / 256), 256, st,
+                      cover, width_px, height_px, row_words, image);
 }
 
 }  // namespace wrach

@@ -660,7 +660,8 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
     src_pos = ctx->stage_pos;
     src_vel = ctx->stage_vel;
   }
-  CK(wrach::launch_upload_keys(ctx->worlds_d, (int)ctx->nworlds, ctx->ncells, world, n_keep,
+  CK(wrach::launch_upload_keys(ctx->worlds_d, (int)ctx->nworlds, ctx->ncells, world,
+                               ctx->worlds_h[world], n_keep,
                                ctx->cell_of[ctx->cur], n_new, s.pos, ctx->keys, ctx->ctrl,
                                ticket_args(ctx), ctx->stream));
   ctx->launches += nsrc ? 1 : 0;
@@ -737,8 +738,10 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
 // The world's store becomes: its particles outside the viewport (store
 // order), then the world's frame particles (frame order) -- per cell the
 // reference's write-back of the GPU's particles into its store
-// (particle_store.rs:71-85, a TODO there).
-int write_back_impl(WrachContext* ctx, uint32_t world) {
+// (particle_store.rs:71-85, a TODO there).  With `moved` the world's settings
+// on the device become those, for the re-packing that follows (a copy from the
+// host would stand between the two).
+int write_back_impl(WrachContext* ctx, uint32_t world, const WorldDev* moved = nullptr) {
   Store& s = ctx->stores[world];
   const uint32_t nf = ctx->n_h[world], off = ctx->poff_h[world];
   int rc;
@@ -754,6 +757,8 @@ int write_back_impl(WrachContext* ctx, uint32_t world) {
   }
   wrach::StoreRebuild r{};
   r.worlds = ctx->worlds_d;
+  r.moves = moved != nullptr;
+  if (moved) r.moved = *moved;
   r.target = world;
   r.n = s.n;
   r.nf = nf;
@@ -1025,13 +1030,15 @@ int wrach_set_viewport(WrachContext* ctx, uint32_t world, float anchor_x, float 
     return fail(ctx, WRACH_ERR_INVALID_ARGUMENT,
                 "the viewport at this anchor has a different grid size; move it by whole cells "
                 "or use a size that is a multiple of the cell size");
-  int rc = write_back_impl(ctx, world);
-  if (rc) return rc;
   w.cell_off = old.cell_off;
+  const int rc = write_back_impl(ctx, world, &w);
+  if (rc) {
+    // out of memory: the device keeps the settings that the host keeps
+    cudaMemcpyAsync(ctx->worlds_d + world, &old, sizeof(WorldDev), cudaMemcpyHostToDevice, ctx->stream);
+    return rc;
+  }
   ctx->worlds_h[world] = w;
   drop_graphs(ctx);  // a single world's settings are among its launches' arguments
-  CK(cudaMemcpyAsync(ctx->worlds_d + world, &ctx->worlds_h[world], sizeof(WorldDev),
-                     cudaMemcpyHostToDevice, ctx->stream));
   // the frame, packed from the store under the new viewport
   return upload_impl(ctx, world, nullptr, nullptr, 0, cudaMemcpyDeviceToDevice, false);
 }

@@ -386,9 +386,10 @@ namespace {
 // 18 us together).
 __global__ void __launch_bounds__(256)
 k_upload_keys(const WorldDev* __restrict__ worlds, int nworlds, uint32_t ncells, uint32_t target,
-              uint32_t n_keep, const uint32_t* __restrict__ cell_of, uint32_t n_new,
+              const __grid_constant__ WorldDev world, uint32_t n_keep, const uint32_t* __restrict__ cell_of, uint32_t n_new,
               const float2* __restrict__ new_pos, uint32_t* __restrict__ keys, Ctrl* ctrl,
               CountDev count) {
+  begin_after();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = i < n_keep + n_new;
   uint32_t key = ncells;
@@ -396,7 +397,7 @@ k_upload_keys(const WorldDev* __restrict__ worlds, int nworlds, uint32_t ncells,
     const uint32_t k = cell_of[i];
     if ((uint32_t)world_of_cell(worlds, nworlds, k) != target) key = k;
   } else if (live) {
-    key = upload_key(worlds[target], new_pos[i - n_keep], ncells);
+    key = upload_key(world, new_pos[i - n_keep], ncells);
   }
   if (live) keys[i] = key;
   if (count.ticket) {
@@ -429,6 +430,7 @@ __device__ __forceinline__ void copy_words(const uint32_t* __restrict__ src,
 // and without the turn from copies to the table's kernel and back: 256 worlds
 // of 1.7 MB 10.4 -> 7.7 ms, one of 2.3 MB with its frame 47.3 -> 41.1 us.
 __global__ void __launch_bounds__(512) k_read_world(const WorldRead r) {
+  begin_after();
   if (r.pos_out) copy_words(r.pos, r.pos_out, 2 * r.n);
   if (r.vel_out) copy_words(r.vel, r.vel_out, 2 * r.n);
   if (r.table_out) {
@@ -462,15 +464,14 @@ cudaError_t launch_wait_probe(const uint32_t* word, uint32_t value, uint64_t lim
 
 cudaError_t launch_upload_keys(const WorldDev* worlds, int nworlds,
                                uint32_t ncells, uint32_t target,
-                               uint32_t n_keep, const uint32_t* cell_of,
+                               const WorldDev& world, uint32_t n_keep, const uint32_t* cell_of,
                                uint32_t n_new, const float2* new_pos,
                                uint32_t* keys, Ctrl* ctrl, const CountDev& count,
                                cudaStream_t st) {
   const uint32_t n = n_keep + n_new;
   if (n == 0) return cudaSuccess;
-  k_upload_keys<<<(n + 255) / 256, 256, 0, st>>>(worlds, nworlds, ncells, target, n_keep, cell_of,
-                                                 n_new, new_pos, keys, ctrl, count);
-  return cudaGetLastError();
+  return launch_after(k_upload_keys, (n + 255) / 256, 256, st, worlds, nworlds, ncells, target,
+                      world, n_keep, cell_of, n_new, new_pos, keys, ctrl, count);
 }
 
 namespace {
@@ -495,8 +496,7 @@ cudaError_t launch_read_world(const WorldRead& r, int sms, cudaStream_t st) {
   if (words == 0) return cudaSuccess;
   // two blocks per SM keep the link full
   const uint32_t most = (uint32_t)(sms > 0 ? sms : 1) * 2u;
-  k_read_world<<<std::min((words + 511) / 512, most), 512, 0, st>>>(r);
-  return cudaGetLastError();
+  return launch_after(k_read_world, std::min((words + 511) / 512, most), 512, st, r);
 }
 
 }  // namespace wrach

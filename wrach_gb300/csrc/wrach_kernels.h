@@ -177,7 +177,7 @@ uint32_t count_sort_launches(uint32_t n, uint32_t ncells);
 // count.ticket set, also the counting sort's tickets (its step 0).
 cudaError_t launch_upload_keys(const WorldDev* worlds, int nworlds,
                                uint32_t ncells, uint32_t target,
-                               uint32_t n_keep, const uint32_t* cell_of,
+                               const WorldDev& world, uint32_t n_keep, const uint32_t* cell_of,
                                uint32_t n_new, const float2* new_pos,
                                uint32_t* keys, Ctrl* ctrl, const CountDev& count,
                                cudaStream_t st);
@@ -297,8 +297,12 @@ cudaError_t launch_penetration(const SolveArgs& a, const float2* pos, const floa
 // viewport, in order, into dst, and the frame's nf items after them.  *kept and
 // *kept_host (pinned) receive how many were outside.  launch_outside finds
 // them, launch_rebuild moves them.
+// With `moves` the target's settings become `moved` once the particles outside
+// are found.
 struct StoreRebuild {
-  const WorldDev* worlds;
+  WorldDev* worlds;
+  WorldDev moved;
+  int moves;
   uint32_t target, n, nf;
   const float2 *pos, *vel;              // the store
   const float2 *frame_pos, *frame_vel;

@@ -57,9 +57,9 @@ int32_t cell_coord(float x, uint32_t cs) {
 }
 
 // The device's view of `bytes` of host memory at p when all of them lie in one
-// allocation of the CUDA runtime (pinned, so kernels may write there), or
-// null: pageable memory and memory that was registered afterwards (its flags
-// may forbid writes) go through the copy engine.
+// pinned allocation that kernels may write to, or null: pageable memory, and
+// pinned memory with other flags than portable and mapped (write-combined,
+// read-only or I/O memory), go through the copy engine.
 uint32_t* device_view(void* p, size_t bytes) {
   if (!p || (uintptr_t)p % 4) return nullptr;
   using GetAttribute = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
@@ -77,7 +77,8 @@ uint32_t* device_view(void* p, size_t bytes) {
   CUdeviceptr start = 0;
   size_t size = 0;
   if (!get || cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != cudaMemoryTypeHost ||
-      !at.devicePointer || cudaHostGetFlags(&flags, p) != cudaSuccess) {
+      !at.devicePointer || cudaHostGetFlags(&flags, p) != cudaSuccess ||
+      (flags & ~(cudaHostAllocPortable | cudaHostAllocMapped)) != 0) {
     cudaGetLastError();
     return nullptr;
   }
@@ -940,8 +941,9 @@ int wrach_read(WrachContext* ctx, uint32_t world, float* positions, float* veloc
   r.cells = cells;
   // Two arrays or more in the host's pinned memory are written by one launch:
   // three copies of 1/3 MB each take 17.0 us, one of 1 MB 13.7 and the launch
-  // 14.1; for one array alone the copy engine's start is the cheaper one.
-  if (!!positions + !!velocities + !!indices >= 2) {
+  // 14.1.  For one array alone the copy engine's start is the cheaper one,
+  // except for a table that a launch has to lay out anyway.
+  if (!!positions + !!velocities + !!indices >= 2 || (indices && !whole)) {
     r.pos_out = device_view(positions, (size_t)n * 8);
     r.vel_out = device_view(velocities, (size_t)n * 8);
     r.table_out = device_view(indices, ((size_t)cells + 2) * 4);

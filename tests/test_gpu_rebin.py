@@ -147,3 +147,21 @@ def test_an_upload_past_the_capacity_places_nothing(W, O, dims, add):
         assert_frame_equal(sim.read_frame(), ref, "two frames later")
     finally:
         sim.close()
+
+
+@pytest.mark.parametrize("gx,gy", [(1, 3), (11, 93), (32, 32), (25, 41), (13, 79), (23, 89), (32, 64),
+                                   (683, 3), (37, 83), (1024, 3), (439, 7), (4096, 1), (17, 241)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_cells_at_the_edges_of_half_tiles(W, O, gx, gy, mode):
+    """The scan's threads take four cells of either half of a 2048-cell tile:
+    grids whose last cells are just before, at and past a half's and a tile's
+    end, with counts above the capacity and above 64 in the last cells."""
+    rng = np.random.default_rng(gx * gy)
+    dims = (gx - 0.5, gy - 0.5)
+    piles = [(gx - 1, gy - 1, 70), (max(gx - 2, 0), gy - 1, 11), (0, 0, 66), (gx // 2, gy // 2, 9)]
+    parts = [rng.uniform((0, 0), dims, size=(3 * gx * gy // 4 + 5, 2))]
+    for cx, cy, m in piles:
+        parts.append(np.column_stack([cx + rng.uniform(0.02, 0.45, m), cy + rng.uniform(0.02, 0.45, m)]))
+    pos = rng.permutation(np.concatenate(parts)).astype(np.float32)
+    vel = rng.normal(0, 0.4, size=pos.shape).astype(np.float32)
+    _run(W, O, dims, pos, vel, mode, 3, 0.1 if mode else 0.0)

@@ -47,6 +47,7 @@ namespace wrach {
 namespace {
 
 constexpr uint32_t kScanThreads = 256, kScanPer = 8;
+static_assert(kScanPer == 8, "a scan thread takes 4 cells of each half tile");
 // Without taking-part particles (reference physics) a grouped table's records
 // count up to this many particles of a cell; cells with more are wide.
 constexpr uint32_t kPlainCap = 31;
@@ -141,40 +142,40 @@ __device__ __forceinline__ void list_large(const RebinArgs& a, uint32_t cell) {
   if (w < a.big_cap) a.big_list[w] = cell;
 }
 
+// A thread takes four cells of either half of the tile, so that a warp's 16-byte
+// loads and stores are contiguous: with eight cells in a row per thread every
+// sector moved in two halves, and each count crossed from L2 twice (2.1M cells
+// 8.2 -> 6.1 us, 8.4M 24.6 -> 20.5; a frame of 262,144 particles 52.8 -> 49.0).
 __global__ void __launch_bounds__(kScanThreads) k_cs_scan(RebinArgs a) {
   begin_after();
   __shared__ uint4 sums[kScanThreads / 32];
+  __shared__ uint2 earlier[kScanThreads / 32];
+  constexpr uint32_t kHalf = kScanTile / 2;
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const uint32_t tile = blockIdx.x, n = a.ncells;
   if (tile == 0 && t == 0 && !a.force_general) a.ctrl->frames += 1;
-  const uint32_t c0 = tile * kScanTile + t * kScanPer;
-  uint32_t v[kScanPer];
-  if (c0 + kScanPer <= n) {
-    const uint4* src = reinterpret_cast<const uint4*>(a.counts + c0);
+  const uint32_t c0 = tile * kScanTile + t * 4;
+  uint32_t v[2][4];
 #pragma unroll
-    for (uint32_t u = 0; u < kScanPer / 4; ++u) {
-      const uint4 q = __ldcg(src + u);
-      v[4 * u] = q.x; v[4 * u + 1] = q.y; v[4 * u + 2] = q.z; v[4 * u + 3] = q.w;
+  for (uint32_t h = 0; h < 2; ++h) {
+    const uint32_t c = c0 + h * kHalf;
+    if (c + 4 <= n) {
+      const uint4 q = *reinterpret_cast<const uint4*>(a.counts + c);
+      v[h][0] = q.x; v[h][1] = q.y; v[h][2] = q.z; v[h][3] = q.w;
+    } else {
+#pragma unroll
+      for (uint32_t u = 0; u < 4; ++u) v[h][u] = c + u < n ? a.counts[c + u] : 0u;
     }
-  } else {
-#pragma unroll
-    for (uint32_t u = 0; u < kScanPer; ++u) v[u] = c0 + u < n ? __ldcg(a.counts + c0 + u) : 0u;
   }
   // the capped counts (the taking-part particles) when the capped table is wanted
   const uint32_t cap = a.tp_cap;
-  uint32_t sum = 0, csum = 0;
-#pragma unroll
-  for (uint32_t u = 0; u < kScanPer; ++u) {
-    sum += v[u];
-    csum += min(v[u], cap);
-  }
   // the earlier tiles' totals: the tickets' pass has them ready.  Their sum
   // goes through the same barrier as the block's own scans below
   uint32_t pre = 0, cpre = 0;
   if (!a.prefixed_tiles) {
     for (uint32_t u = t; u < tile; u += kScanThreads) {
-      pre += __ldcg(a.tile_sums + u);
-      if (cap) cpre += __ldcg(a.tile_sums_cap + u);
+      pre += a.tile_sums[u];
+      if (cap) cpre += a.tile_sums_cap[u];
     }
     pre = __reduce_add_sync(0xffffffffu, pre);
     if (cap) cpre = __reduce_add_sync(0xffffffffu, cpre);
@@ -182,75 +183,78 @@ __global__ void __launch_bounds__(kScanThreads) k_cs_scan(RebinArgs a) {
     pre = before_tile(a.tile_sums, tile, a.prefixed_tiles);
     if (cap) cpre = before_tile(a.tile_sums_cap, tile, a.prefixed_tiles);
   }
+  uint32_t x[2], cx[2];
+#pragma unroll
+  for (uint32_t h = 0; h < 2; ++h) {
+    x[h] = v[h][0] + v[h][1] + v[h][2] + v[h][3];
+    cx[h] = min(v[h][0], cap) + min(v[h][1], cap) + min(v[h][2], cap) + min(v[h][3], cap);
+  }
+  const uint32_t own[2] = {x[0], x[1]}, cown[2] = {cx[0], cx[1]};
   // block-wide exclusive scans of the per-thread sums
-  uint32_t x = sum, cx = csum;
 #pragma unroll
   for (uint32_t o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    const uint32_t cy = __shfl_up_sync(0xffffffffu, cx, o);
-    if (lane >= o) {
-      x += y;
-      cx += cy;
+#pragma unroll
+    for (uint32_t h = 0; h < 2; ++h) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x[h], o);
+      const uint32_t cy = __shfl_up_sync(0xffffffffu, cx[h], o);
+      if (lane >= o) {
+        x[h] += y;
+        cx[h] += cy;
+      }
     }
   }
-  if (lane == 31) sums[warp] = make_uint4(x, cx, pre, cpre);
+  if (lane == 31) {
+    sums[warp] = make_uint4(x[0], cx[0], x[1], cx[1]);
+    earlier[warp] = make_uint2(pre, cpre);
+  }
   __syncthreads();
-  uint32_t before = 0, total = 0, cbefore = 0, ctotal = 0, prefix = 0, cprefix = 0;
+  uint32_t run[2] = {0u, 0u}, crun[2] = {0u, 0u}, first = 0, cfirst = 0, total = 0, ctotal = 0;
+  uint32_t prefix = 0, cprefix = 0;
 #pragma unroll
   for (uint32_t w = 0; w < kScanThreads / 32; ++w) {
     const uint4 s = sums[w];
-    before += w < warp ? s.x : 0u;
-    total += s.x;
-    cbefore += w < warp ? s.y : 0u;
-    ctotal += s.y;
-    prefix += s.z;
-    cprefix += s.w;
+    const uint2 e = earlier[w];
+    run[0] += w < warp ? s.x : 0u;
+    crun[0] += w < warp ? s.y : 0u;
+    run[1] += w < warp ? s.z : 0u;
+    crun[1] += w < warp ? s.w : 0u;
+    first += s.x;
+    cfirst += s.y;
+    total += s.x + s.z;
+    ctotal += s.y + s.w;
+    prefix += e.x;
+    cprefix += e.y;
   }
-  uint32_t run = prefix + before + x - sum;
-  uint32_t crun = cprefix + cbefore + cx - csum;
+  run[0] += prefix + x[0] - own[0];
+  crun[0] += cprefix + cx[0] - cown[0];
+  run[1] += prefix + first + x[1] - own[1];
+  crun[1] += cprefix + cfirst + cx[1] - cown[1];
 #pragma unroll
-  for (uint32_t u = 0; u < kScanPer; ++u)
-    if (v[u] > kSmallCell) list_large(a, c0 + u);
-  if (cap) {
-    if (c0 + kScanPer <= n) {
-      uint4* dst = reinterpret_cast<uint4*>(a.ct_new + c0);
+  for (uint32_t h = 0; h < 2; ++h) {
+    const uint32_t c = c0 + h * kHalf;
+    uint32_t at[4], cat[4];
 #pragma unroll
-      for (uint32_t u = 0; u < kScanPer / 4; ++u) {
-        uint4 q;
-        q.x = crun; crun += min(v[4 * u], cap);
-        q.y = crun; crun += min(v[4 * u + 1], cap);
-        q.z = crun; crun += min(v[4 * u + 2], cap);
-        q.w = crun; crun += min(v[4 * u + 3], cap);
-        dst[u] = q;
-      }
+    for (uint32_t u = 0; u < 4; ++u) {
+      if (v[h][u] > kSmallCell) list_large(a, c + u);
+      at[u] = run[h];
+      cat[u] = crun[h];
+      run[h] += v[h][u];
+      crun[h] += min(v[h][u], cap);
+    }
+    if (c + 4 <= n) {
+      *reinterpret_cast<uint4*>(a.cs_new + c) = make_uint4(at[0], at[1], at[2], at[3]);
+      if (cap) *reinterpret_cast<uint4*>(a.ct_new + c) = make_uint4(cat[0], cat[1], cat[2], cat[3]);
     } else {
 #pragma unroll
-      for (uint32_t u = 0; u < kScanPer; ++u) {
-        if (c0 + u < n) a.ct_new[c0 + u] = crun;
-        crun += min(v[u], cap);
+      for (uint32_t u = 0; u < 4; ++u) {
+        if (c + u >= n) break;
+        a.cs_new[c + u] = at[u];
+        if (cap) a.ct_new[c + u] = cat[u];
       }
-    }
-    if (t == 0 && (tile + 1) * kScanTile >= n) a.ct_new[n] = cprefix + ctotal;
-  }
-  if (c0 + kScanPer <= n) {
-    uint4* dst = reinterpret_cast<uint4*>(a.cs_new + c0);
-#pragma unroll
-    for (uint32_t u = 0; u < kScanPer / 4; ++u) {
-      uint4 q;
-      q.x = run; run += v[4 * u];
-      q.y = run; run += v[4 * u + 1];
-      q.z = run; run += v[4 * u + 2];
-      q.w = run; run += v[4 * u + 3];
-      dst[u] = q;
-    }
-  } else {
-#pragma unroll
-    for (uint32_t u = 0; u < kScanPer; ++u) {
-      if (c0 + u < n) a.cs_new[c0 + u] = run;
-      run += v[u];
     }
   }
   if (t == 0 && (tile + 1) * kScanTile >= n) {
+    if (cap) a.ct_new[n] = cprefix + ctotal;
     a.cs_new[n] = prefix + total;
     if (a.total_out) *a.total_out = prefix + total;
   }

@@ -116,6 +116,49 @@ def test_a_batch_leaves_no_sums_behind(W, n):
         assert np.isfinite(trained) and trained > 0
 
 
+def _glorot_net(rng):
+    """Glorot-uniform hidden layers, small biases, outputs of a few tenths."""
+    p = np.zeros(M.N_PARAMS, np.float32)
+    w1, b1, w2, b2, w3, b3 = M.unpack(p)
+    a = (6.0 / 128.0) ** 0.5
+    w1[:], w2[:] = rng.uniform(-a, a, (64, 64)), rng.uniform(-a, a, (64, 64))
+    b1[:], b2[:] = rng.uniform(-0.1, 0.1, 64), rng.uniform(-0.1, 0.1, 64)
+    w3[:, :2], b3[:2] = rng.uniform(-0.3, 0.3, (64, 2)), rng.uniform(-0.1, 0.1, 2)
+    return M.pack(w1, b1, w2, b2, w3, b3)
+
+
+@pytest.mark.parametrize("n,batches", [(1000, 16), (16384, 16), (40001, 8)])
+def test_loss_against_64_bits(W, n, batches):
+    """The loss is the 64-bit network's but for activations whose FP32 error
+    turns their BF16 rounding.  With an error of 2^-21 (four products of 16
+    inputs, their sum, the GELU) and neighbours 2^-8.5 apart on average, 1 in
+    3000 activations turn, 0.044 of a row's 128; each moves one output by 2^-8.5
+    of about 0.3 * 0.17 (activation times weight) at an error of about 0.45, so
+    by 6.5e-5 of a loss of about 0.2 per row, of either sign: 4.2e-6 per row
+    over sqrt(n) rows, 6.8e-5 / sqrt(n).  The FP32 outputs and the FP32 result
+    add 2^-23.  Of `batches` root mean squares 3 standard deviations are allowed.
+    With a hardware tanh (an error of 2^-11) it is 9.7e-6 of 1,000 rows and
+    2.4e-6 of 16,384."""
+    torch = _torch()
+    off = []
+    with _sim(W, (30.0, 30.0), 100) as sim:
+        sim.surrogate_init(0, 16)
+        for k in range(batches):
+            rng = np.random.default_rng(1000 + k)
+            params = _glorot_net(rng)
+            sim.surrogate_set_params(params)
+            x = M.bf16(rng.normal(0, 1, (n, 64)).astype(np.float32))
+            x[:, 50:] = 0
+            t = rng.normal(0, 0.3, (n, 2)).astype(np.float32)
+            dx = torch.from_numpy(M.bf16_bits(x).astype(np.uint16).view(np.int16)).cuda()
+            dt = torch.from_numpy(t).cuda()
+            torch.cuda.synchronize()
+            want = M.loss(params, x, t)
+            off.append((sim.surrogate_gradients(dx.data_ptr(), dt.data_ptr(), n)[1] - want) / want)
+    rms = np.sqrt(np.mean(np.square(off)))
+    assert rms <= (6.8e-5 / np.sqrt(n) + 2.0 ** -23) * (1 + 3 / np.sqrt(2 * batches)), off
+
+
 @pytest.mark.parametrize("n,shift", [(1, 0), (17, 0), (128, 0), (129, 2), (300, 4), (20011, 0), (40001, 2)])
 def test_gradients_over_tiles(W, n, shift):
     # tiles of 128 rows, one or several per block, ragged last tiles, and rows

@@ -63,6 +63,10 @@ __device__ __forceinline__ float gelu_and_grad(float& x) {
   x = 0.5f * (1.0f + t) + h * (1.0f - t * t) * kGeluC * (1.0f + 3.0f * kGeluA * x2);
   return h * (1.0f + t);
 }
+// GELU for the loss, to some FP32 ulps: 0.5 (1 + tanh(u)) = 1 / (1 + exp(-2 u)).
+__device__ __forceinline__ float gelu_full(float x) {
+  return __fdividef(x, 1.0f + __expf(-2.0f * kGeluC * x * (1.0f + kGeluA * x * x)));
+}
 
 // Shared-memory copy of the network for the forward pass: the weights as
 // BF16 in the [out][in] layout (the B operand, k = in contiguous) and the
@@ -405,14 +409,61 @@ __device__ __forceinline__ double* loss_of(float* grad) {
   return reinterpret_cast<double*>(grad + kMlpParams);
 }
 static_assert(kMlpParams % 2 == 0, "the loss is 8-byte aligned");
+__device__ __forceinline__ double half_square(float e0, float e1) {
+  return 0.5 * ((double)e0 * e0 + (double)e1 * e1);
+}
+
+// The network's outputs for the loss.  An activation that is rounded to the
+// other BF16 neighbour shifts the loss, and the hardware tanh (and, less, sums
+// that the tensor cores round towards zero along a chain) does that to many:
+// here each product of 16 inputs starts from zero, the four are added to nearest
+// and the GELU is gelu_full.  Root mean square error of the loss against 64
+// bits over 50 batches of 1,000 and 16,384 and 20 of 65,536 rows, as the
+// gradients' forward pass has it 9.7e-6, 2.4e-6 and 1.5e-6, this way 1.0e-6,
+// 4.7e-7 and 2.9e-7; the batches' times 27.1, 33.5 and 45.8 us without a second
+// pass, 29.5, 35.2 and 54.5 with it, so that it runs only for a loss that is
+// read.  (Exact sums of the four and an FP32-exact GELU: 9.9e-7, 3.6e-7 and
+// 2.2e-7 in 34.5, 40.0 and 74.3 us.)
+__device__ __forceinline__ void loss_layer(const uint32_t* wt, const float* b, uint32_t lane,
+                                           const uint32_t (&in)[4][4], uint32_t (&out)[4][4]) {
+  const uint32_t g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (uint32_t nt = 0; nt < 8; ++nt) {
+    const uint32_t* row = wt + (nt * 8 + g) * kRow + t;
+    float p[4][4] = {}, h[4];
+#pragma unroll
+    for (uint32_t kk = 0; kk < 4; ++kk)
+      mma_bf16(p[kk], in[kk], lds_keep(row + kk * 8), lds_keep(row + kk * 8 + 4));
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q)
+      h[q] = gelu_full((p[0][q] + p[1][q]) + (p[2][q] + p[3][q]) + b[nt * 8 + 2 * t + (q & 1)]);
+    out[nt / 2][2 * (nt & 1)] = pack_bf16(h[0], h[1]);
+    out[nt / 2][2 * (nt & 1) + 1] = pack_bf16(h[2], h[3]);
+  }
+}
+__device__ __forceinline__ void loss_forward(const SmemNet& s, uint32_t lane,
+                                             const uint32_t (&ax)[4][4], float (&y)[4]) {
+  const uint32_t g = lane >> 2, t = lane & 3;
+  uint32_t h1[4][4], h2[4][4];
+  loss_layer(s.w1t, s.b1, lane, ax, h1);
+  loss_layer(s.w2t, s.b2, lane, h1, h2);
+  const uint32_t* row = s.w3t + g * kRow + t;
+  float p[4][4] = {};
+#pragma unroll
+  for (uint32_t kk = 0; kk < 4; ++kk)
+    mma_bf16(p[kk], h2[kk], lds_keep(row + kk * 8), lds_keep(row + kk * 8 + 4));
+#pragma unroll
+  for (uint32_t q = 0; q < 4; ++q)
+    y[q] = (p[0][q] + p[1][q]) + (p[2][q] + p[3][q]) + s.b3[2 * t + (q & 1)];
+}
 
 // Gradients of L = 0.5 * sum over rows and the 2 outputs of (y - target)^2 /
 // `scale_rows` with respect to every parameter, added into `grad` (FP32,
 // the MlpDev parameter order: w1 [in][out], b1, w2, b2, w3 [in][8], b3).
-// Also adds the loss into the 64-bit sum behind them.
+// With `want_loss` also adds the loss into the 64-bit sum behind them.
 __global__ void __launch_bounds__(kTrainThreads, 1)
 k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restrict__ target,
-               uint32_t n, float inv_rows, float* __restrict__ grad) {
+               uint32_t n, float inv_rows, float* __restrict__ grad, int want_loss) {
   extern __shared__ __align__(16) uint8_t dyn[];
   begin_after();
   SmemTrain& sm = *reinterpret_cast<SmemTrain*>(dyn);
@@ -421,7 +472,8 @@ k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restric
   const uint32_t g = lane >> 2, t = lane & 3;
   const uint32_t row0 = warp * 16, m0 = (warp & 3) * 16, n0 = (warp >> 2) * 32;
   float acc1[4][4] = {}, acc2[4][4] = {}, acc3[4] = {};
-  float sb1[8][2] = {}, sb2[8][2] = {}, sb3[2] = {}, lsum = 0.f;
+  float sb1[8][2] = {}, sb2[8][2] = {}, sb3[2] = {};
+  double lsum = 0.0;
   const uint32_t tiles = (n + kTrainRows - 1) / kTrainRows;
   // a caller's rows may start at any 4-byte boundary
   const bool x16 = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
@@ -458,6 +510,11 @@ k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restric
 #pragma unroll
     for (uint32_t kk = 0; kk < 4; ++kk)
       ldsm4(a[kk], st.x + (row0 + (lane & 15)) * kRow + kk * 8 + (lane >> 4) * 4);
+    if (want_loss) {
+      loss_forward(sm.net, lane, a, y);
+      if (t == 0 && r0 < n) lsum += half_square(y[0] - tg0.x, y[1] - tg0.y);
+      if (t == 0 && r1 < n) lsum += half_square(y[2] - tg1.x, y[3] - tg1.y);
+    }
     mlp_tile_forward(sm.net, lane, a, z1, h1, z2, h2, y);
     store_a(st.h1, row0, lane, h1);
     store_a(st.h2, row0, lane, h2);
@@ -466,13 +523,11 @@ k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restric
     if (t == 0) {
       if (r0 < n) {
         const float e0 = y[0] - tg0.x, e1 = y[1] - tg0.y;
-        lsum += 0.5f * (e0 * e0 + e1 * e1);
         dy[0] = e0 * inv_rows;
         dy[1] = e1 * inv_rows;
       }
       if (r1 < n) {
         const float e0 = y[2] - tg1.x, e1 = y[3] - tg1.y;
-        lsum += 0.5f * (e0 * e0 + e1 * e1);
         dy[2] = e0 * inv_rows;
         dy[3] = e1 * inv_rows;
       }
@@ -562,13 +617,10 @@ k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restric
   }
   if (lane == 0) {
     atomicAdd(reinterpret_cast<float2*>(grad + o_b3), make_float2(sb3[0], sb3[1]));
-    // (in 64 bits: a sum of up to 1216 warps' shares)
-    if (lsum != 0.f) atomicAdd(loss_of(grad), (double)lsum * (double)inv_rows);
+    if (want_loss) atomicAdd(loss_of(grad), lsum * (double)inv_rows);
   }
 }
 
-// Adam on the FP32 master parameters (the order above), then the BF16
-// copies in both layouts.
 // A batch's sums end with the launch that reads them: it leaves zeros for the
 // next batch's, so that no clear stands between two batches (16,384 rows, with
 // a copy to the host and its gap replaced by k_take_gradients: 44 -> 34 us).
@@ -594,6 +646,8 @@ __global__ void __launch_bounds__(256) k_take_gradients(float* __restrict__ grad
   if (i <= nparams) out[i] = take_sum(grad, i, nparams);
 }
 
+// Adam on the FP32 master parameters (the order above), then the BF16
+// copies in both layouts.
 __global__ void k_adam(MlpDev m, float* __restrict__ grad, float* __restrict__ mom1,
                        float* __restrict__ mom2, float lr, float b1, float b2, float eps,
                        float bc1, float bc2, uint32_t nparams) {
@@ -1163,12 +1217,12 @@ bool train_setup() {
 }
 
 cudaError_t launch_mlp_backward(const MlpDev& m, const uint16_t* x, const float2* target,
-                                uint32_t n, float inv_rows, float* grad, int sms,
+                                uint32_t n, float inv_rows, float* grad, bool want_loss, int sms,
                                 cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   const uint32_t tiles = (n + kTrainRows - 1) / kTrainRows, most = sms > 0 ? sms : 1;
   return launch_after_with(sizeof(SmemTrain), k_mlp_backward, tiles < most ? tiles : most,
-                           kTrainThreads, st, m, x, target, n, inv_rows, grad);
+                           kTrainThreads, st, m, x, target, n, inv_rows, grad, (int)want_loss);
 }
 
 cudaError_t launch_take_gradients(float* grad, float* out, cudaStream_t st) {

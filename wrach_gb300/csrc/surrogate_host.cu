@@ -270,7 +270,7 @@ int wrach_surrogate_gradients(WrachContext* ctx, const uint16_t* d_x, const floa
   DeviceGuard guard(ctx->device);
   auto& S = ctx->sur;
   CK(wrach::launch_mlp_backward(S.m, d_x, reinterpret_cast<const float2*>(d_t), n, 1.0f / n, S.grad,
-                                ctx->sms, ctx->stream));
+                                true, ctx->sms, ctx->stream));
   CK(wrach::launch_take_gradients(S.grad, S.grad_h, ctx->stream));
   ctx->launches += 2;
   CK(cudaStreamSynchronize(ctx->stream));
@@ -385,7 +385,7 @@ int wrach_surrogate_train(WrachContext* ctx, uint32_t steps, uint32_t batch, flo
     const uint32_t span = S.nsamples - b + 1;
     const uint32_t off = (uint32_t)(((uint64_t)(S.step + 1) * 2654435761ull) % span);
     CK(wrach::launch_mlp_backward(S.m, S.tx + (size_t)off * wrach::kMlpIn, S.tt + off, b, 1.0f / b,
-                                  S.grad, ctx->sms, ctx->stream));
+                                  S.grad, s + 1 == steps, ctx->sms, ctx->stream));
     ++S.step;
     CK(wrach::launch_adam(S.m, S.grad, S.mom1, S.mom2, lr, S.step, ctx->stream));
     ctx->launches += 2;

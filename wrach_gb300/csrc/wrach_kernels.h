@@ -273,8 +273,9 @@ cudaError_t launch_mlp_forward_tc(const MlpDev& m, const uint16_t* x, uint32_t n
 // One-time set-up of the training kernel on the current device (its shared
 // memory size).
 bool train_setup();
+// A batch's gradients, and its loss if that will be read, into the sums.
 cudaError_t launch_mlp_backward(const MlpDev& m, const uint16_t* x, const float2* target,
-                                uint32_t n, float inv_rows, float* grad, int sms,
+                                uint32_t n, float inv_rows, float* grad, bool want_loss, int sms,
                                 cudaStream_t st);
 // The sums of launch_mlp_backward's batches (kMlpParams gradients, the 64-bit
 // loss behind them, then the last batch's loss) are zero between batches: the

@@ -35,3 +35,22 @@ def test_cells_across_warps(W, O, cap, n, block):
             sim.step(1)
             ref = O.step(w, ph, ref[0], ref[1], ref[2], 1)[:3]
             assert_frame_equal(sim.read_frame(), ref, "frame %d" % frame)
+
+
+@pytest.mark.parametrize("zeros", [(-0.0, -0.0), (0.0, -0.0), (-0.0, 0.0), (0.0, 0.0)])
+@pytest.mark.parametrize("axis", [0, 1])
+def test_signed_zeros(W, O, zeros, axis):
+    """Coordinates that are equal zeros: a push leaves the first -0 and turns
+    the second into +0, and a velocity of -0 carries the sign to the output."""
+    pos = np.zeros((4, 2), np.float32)
+    pos[:2, axis], pos[:2, 1 - axis] = zeros, (1.0, 1.25)
+    pos[2:, axis], pos[2:, 1 - axis] = zeros, (7.0, 7.0)  # coincident
+    vel = np.full((4, 2), -0.0, np.float32)
+    w, ph = O.world(12.0, 12.0, 3), O.Physics(0, 1, 0.0, 1.0, 1.0, 9)
+    with W.Simulation(W.WrachConfig(dimensions=(12.0, 12.0), cell_size=3, mode=0, capacity=8)) as sim:
+        sim.set_particles(pos, vel)
+        ref = O.pack(w, pos, vel, 8)
+        for frame in range(2):
+            sim.step(1)
+            ref = O.step(w, ph, ref[0], ref[1], ref[2], 1)[:3]
+            assert_frame_equal(sim.read_frame(), ref, "frame %d" % frame)

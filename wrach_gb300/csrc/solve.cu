@@ -66,8 +66,9 @@ __device__ __forceinline__ void publish_flags(Ctrl* ctrl, uint32_t flags) {
 // serve m (m - 1) / 2 pairs, with a particle's position in its lane's
 // registers (one thread per cell held them in indexed arrays, in local
 // memory, and swept them one by one).  A pair's two lanes both compute its
-// push: p_i - (p_j - p_i) f and p_j - (p_i - p_j) f round like the
-// reference's p_j + (p_j - p_i) f.
+// push, from the same difference as the reference: p_i - (p_j - p_i) f and
+// p_j + (p_j - p_i) f (with the other difference, two coordinates of -0 would
+// both stay -0, where the reference's j becomes +0).
 //
 // Warp w covers the particles [W w, W w + 32), W = 33 - capacity: it solves
 // the cells that start in its first W particles (all their m particles are in
@@ -117,11 +118,14 @@ k_solve_reference(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32
     const bool pair = other < m && other != rank;
     const uint32_t from = (lane + other - rank) & 31u;
     const float qx = __shfl_sync(0xffffffffu, px, from), qy = __shfl_sync(0xffffffffu, py, from);
-    const float dx = __fsub_rn(qx, px), dy = __fsub_rn(qy, py);
+    const bool second = rank > other;
+    const float dx = second ? __fsub_rn(px, qx) : __fsub_rn(qx, px);
+    const float dy = second ? __fsub_rn(py, qy) : __fsub_rn(qy, py);
     float f;
     if (pair && push_factor(dx, dy, ph.min_d, ph.skip_d2, f)) {
-      px = __fsub_rn(px, __fmul_rn(dx, f));
-      py = __fsub_rn(py, __fmul_rn(dy, f));
+      const float mx = __fmul_rn(dx, f), my = __fmul_rn(dy, f);
+      px = __fadd_rn(px, second ? mx : -mx);
+      py = __fadd_rn(py, second ? my : -my);
     }
   }
   if (mine) {

@@ -159,6 +159,37 @@ def test_loss_against_64_bits(W, n, batches):
     assert rms <= (6.8e-5 / np.sqrt(n) + 2.0 ** -23) * (1 + 3 / np.sqrt(2 * batches)), off
 
 
+@pytest.mark.parametrize("parts", [2, 128])
+def test_gradients_of_a_large_batch(W, parts):
+    """One batch of `parts` * 2^14 rows against the mean of the parts' gradients
+    taken one by one.  The tiles are the same, and 1 / rows differs by a power of
+    two, so only the tiles' sums differ.  A block adds parts * 128 / SMs of them
+    and the blocks' sums follow, each addition off by 0.29 * 2^-23 of a sum that
+    grows with the square root of its terms: root mean square
+    0.29 * 2^-23 * sqrt(terms / 2) of the gradients' norm; four times that is
+    allowed."""
+    torch = _torch()
+    rows, sms = 1 << 14, torch.cuda.get_device_properties(0).multi_processor_count
+    gen = torch.Generator(device="cuda").manual_seed(parts)
+    x = torch.randn((parts * rows, 64), generator=gen, device="cuda").to(torch.bfloat16)
+    t = 0.3 * torch.randn((parts * rows, 2), generator=gen, device="cuda")
+    torch.cuda.synchronize()
+    with _sim(W, (30.0, 30.0), 100) as sim:
+        sim.surrogate_init(0, 16)
+        sim.surrogate_set_params(_glorot_net(np.random.default_rng(parts)))
+        whole, loss = sim.surrogate_gradients(x.data_ptr(), t.data_ptr(), parts * rows)
+        mean, mean_loss = np.zeros(M.N_PARAMS), 0.0
+        for k in range(parts):
+            g, l = sim.surrogate_gradients(x[k * rows:].data_ptr(), t[k * rows:].data_ptr(), rows)
+            mean += np.float64(g) / parts
+            mean_loss += l / parts
+    terms = parts * 128 / sms + 2 * sms
+    tol = 4 * 0.29 * 2.0 ** -23 * np.sqrt(terms / 2)
+    assert np.linalg.norm(whole - mean) <= tol * np.linalg.norm(mean)
+    # the loss: FP32 results of a 64-bit sum
+    assert abs(loss - mean_loss) <= 2.0 ** -23 * mean_loss
+
+
 @pytest.mark.parametrize("n,shift", [(1, 0), (17, 0), (128, 0), (129, 2), (300, 4), (20011, 0), (40001, 2)])
 def test_gradients_over_tiles(W, n, shift):
     # tiles of 128 rows, one or several per block, ragged last tiles, and rows

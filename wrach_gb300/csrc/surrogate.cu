@@ -371,9 +371,12 @@ __device__ __forceinline__ void to_a(uint32_t (&a)[4][4], const float (&c)[8][4]
   }
 }
 
-// acc (4 n-tiles from column n0) += AT^T BT over the tile's rows, AT the
-// columns m0 .. m0 + 15 of `at`.
-__device__ __forceinline__ void rows_product(float (&acc)[4][4], const uint32_t* at,
+// sum (4 n-tiles from column n0) += AT^T BT over the tile's rows, AT the
+// columns m0 .. m0 + 15 of `at`.  The product of a tile's 128 rows starts from
+// zero and is added to nearest: sums that stayed in the tensor cores'
+// accumulators over all of a block's tiles were rounded towards zero at every
+// 16 rows (2M rows, 108 tiles a block: 1.5e-5 of the gradients' norm, 2.2e-7 now).
+__device__ __forceinline__ void rows_product(float (&sum)[4][4], const uint32_t* at,
                                              const uint32_t* bt, uint32_t m0, uint32_t n0,
                                              uint32_t lane) {
   const uint32_t mi = lane >> 3, r = lane & 7;
@@ -381,6 +384,7 @@ __device__ __forceinline__ void rows_product(float (&acc)[4][4], const uint32_t*
   const uint32_t* pa = at + ((mi >> 1) * 8 + r) * kRow + (m0 + (mi & 1) * 8) / 2;
   // B: matrices (k 0-7, n 0-7), (k 8-15, n 0-7), (k 0-7, n 8-15), (k 8-15, n 8-15)
   const uint32_t* pb = bt + ((mi & 1) * 8 + r) * kRow + (n0 + (mi >> 1) * 8) / 2;
+  float acc[4][4] = {};
 #pragma unroll
   for (uint32_t ks = 0; ks < kTrainRows / 16; ++ks) {
     uint32_t a[4], b[4], c[4];
@@ -392,6 +396,10 @@ __device__ __forceinline__ void rows_product(float (&acc)[4][4], const uint32_t*
     mma_bf16(acc[2], a, c[0], c[1]);
     mma_bf16(acc[3], a, c[2], c[3]);
   }
+#pragma unroll
+  for (uint32_t u = 0; u < 4; ++u)
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) sum[u][q] += acc[u][q];
 }
 
 // A 16x8 tile of sums (C layout) into the row-major matrix w of `ld` columns.
@@ -471,7 +479,7 @@ k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restric
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t g = lane >> 2, t = lane & 3;
   const uint32_t row0 = warp * 16, m0 = (warp & 3) * 16, n0 = (warp >> 2) * 32;
-  float acc1[4][4] = {}, acc2[4][4] = {}, acc3[4] = {};
+  float sum1[4][4] = {}, sum2[4][4] = {}, sum3[4] = {};
   float sb1[8][2] = {}, sb2[8][2] = {}, sb3[2] = {};
   double lsum = 0.0;
   const uint32_t tiles = (n + kTrainRows - 1) / kTrainRows;
@@ -569,17 +577,20 @@ k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restric
     store_a(st.dz1, row0, lane, a);
     __syncthreads();
     // the weight gradients' products over the tile's rows
-    rows_product(acc1, st.x, st.dz1, m0, n0, lane);
-    rows_product(acc2, st.h1, st.dz2, m0, n0, lane);
+    rows_product(sum1, st.x, st.dz1, m0, n0, lane);
+    rows_product(sum2, st.h1, st.dz2, m0, n0, lane);
     if (n0 == 0) {
       const uint32_t mi = lane >> 3, r = lane & 7;
+      float acc[4] = {};
 #pragma unroll
       for (uint32_t ks = 0; ks < kTrainRows / 16; ++ks) {
         uint32_t b[4], b0, b1;
         ldsm4t(b, st.h2 + (ks * 16 + (mi >> 1) * 8 + r) * kRow + (m0 + (mi & 1) * 8) / 2);
         ldsm2t(b0, b1, st.dy + (ks * 16 + (mi & 1) * 8 + r) * (kOutPad / 2));
-        mma_bf16(acc3, b, b0, b1);
+        mma_bf16(acc, b, b0, b1);
       }
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) sum3[q] += acc[q];
     }
     __syncthreads();
   }
@@ -588,10 +599,10 @@ k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restric
   const uint32_t o_w3 = o_b2 + kHid, o_b3 = o_w3 + kHid * kOutPad;
 #pragma unroll
   for (uint32_t u = 0; u < 4; ++u) {
-    add_tile(grad, kHid, m0, n0 + u * 8, acc1[u], lane);
-    add_tile(grad + o_w2, kHid, m0, n0 + u * 8, acc2[u], lane);
+    add_tile(grad, kHid, m0, n0 + u * 8, sum1[u], lane);
+    add_tile(grad + o_w2, kHid, m0, n0 + u * 8, sum2[u], lane);
   }
-  if (n0 == 0) add_tile(grad + o_w3, kOutPad, m0, 0, acc3, lane);
+  if (n0 == 0) add_tile(grad + o_w3, kOutPad, m0, 0, sum3, lane);
   // bias gradients: the columns' sums over the rows a warp's lanes hold
 #pragma unroll
   for (uint32_t o = 4; o < 32; o <<= 1) {

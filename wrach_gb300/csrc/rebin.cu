@@ -408,11 +408,13 @@ k_upload_keys(const WorldDev* __restrict__ worlds, int nworlds, uint32_t ncells,
   }
 }
 
-// `count` words from src to dst, four in flight per thread of the grid.
+// `count` words from src to dst, four in flight per thread of the grid.  Counts
+// reach 2^32 - 2 (the largest frame capacity), and the indices pass them by up
+// to four strides: 64 bits.
 __device__ __forceinline__ void copy_words(const uint32_t* __restrict__ src,
-                                           uint32_t* __restrict__ dst, uint32_t count) {
-  const uint32_t stride = gridDim.x * blockDim.x;
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+                                           uint32_t* __restrict__ dst, size_t count) {
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   for (; i + 3 * stride < count; i += 4 * stride) {
     uint32_t v[4];
 #pragma unroll
@@ -431,8 +433,8 @@ __device__ __forceinline__ void copy_words(const uint32_t* __restrict__ src,
 // of 1.7 MB 10.4 -> 7.7 ms, one of 2.3 MB with its frame 47.3 -> 41.1 us.
 __global__ void __launch_bounds__(512) k_read_world(const WorldRead r) {
   begin_after();
-  if (r.pos_out) copy_words(r.pos, r.pos_out, 2 * r.n);
-  if (r.vel_out) copy_words(r.vel, r.vel_out, 2 * r.n);
+  if (r.pos_out) copy_words(r.pos, r.pos_out, (size_t)2 * r.n);
+  if (r.vel_out) copy_words(r.vel, r.vel_out, (size_t)2 * r.n);
   if (r.table_out) {
     const uint32_t stride = gridDim.x * blockDim.x, base = r.table.start(r.cell_off);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < r.cells + 2; i += stride)
@@ -496,7 +498,7 @@ cudaError_t launch_read_world(const WorldRead& r, int sms, cudaStream_t st) {
   if (words == 0) return cudaSuccess;
   // two blocks per SM keep the link full
   const uint32_t most = (uint32_t)(sms > 0 ? sms : 1) * 2u;
-  return launch_after(k_read_world, std::min((words + 511) / 512, most), 512, st, r);
+  return launch_after(k_read_world, std::min(words / 512 + 1, most), 512, st, r);
 }
 
 }  // namespace wrach

@@ -187,10 +187,13 @@ int ensure_stage(WrachContext* ctx, size_t need) {
   return WRACH_OK;
 }
 
+// Particles of one sort: their number is a 32-bit count.
+constexpr size_t kMaxStore = 0xFFFFFFF0u;
+
 int ensure_store(WrachContext* ctx, Store& s, size_t need) {
   if (need <= s.cap) return WRACH_OK;
   size_t cap = std::max<size_t>(need, (size_t)s.cap * 2);
-  if (cap > 0xFFFFFFF0ull) return fail(ctx, WRACH_ERR_CAPACITY, "store too large");
+  if (cap > kMaxStore) return fail(ctx, WRACH_ERR_CAPACITY, "store too large");
   float2 *np = nullptr, *nv = nullptr;
   CK(dalloc(&np, cap));
   CK(dalloc(&nv, cap));
@@ -641,7 +644,7 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
   // belong to the world being re-packed from its store, so none are
   const uint32_t n_keep = ctx->nworlds > 1 ? ctx->n : 0u, n_new = s.n;
   const size_t nsrc = (size_t)n_keep + n_new;
-  if (nsrc > 0xFFFFFFF0ull) {
+  if (nsrc > kMaxStore) {
     s.n = old_n;
     return fail(ctx, WRACH_ERR_CAPACITY, "too many particles");
   }
@@ -780,6 +783,7 @@ int write_back_impl(WrachContext* ctx, uint32_t world, const WorldDev* moved = n
   // the store is rebuilt while the host learns its size
   CK(cudaEventSynchronize(ctx->counts_ev));
   const uint32_t kept = ctx->gather_h[0];
+  if ((size_t)kept + nf > kMaxStore) return fail(ctx, WRACH_ERR_CAPACITY, "store too large");
   if (ctx->nworlds == 1) {
     // the rebuilt store takes the place of the old one, whose buffers serve
     // the next rebuild (with more worlds the staging buffers are larger than
@@ -787,7 +791,7 @@ int write_back_impl(WrachContext* ctx, uint32_t world, const WorldDev* moved = n
     std::swap(s.pos, ctx->stage_pos);
     std::swap(s.vel, ctx->stage_vel);
     const size_t cap = s.cap;
-    s.cap = (uint32_t)std::min<size_t>(ctx->stage_cap, 0xFFFFFFF0u);
+    s.cap = (uint32_t)std::min(ctx->stage_cap, kMaxStore);
     ctx->stage_cap = cap;
     s.n = kept + nf;
     return WRACH_OK;

@@ -122,7 +122,8 @@ __global__ void __launch_bounds__(kThreads) k_rebuild(const StoreRebuild r, uint
     }
     return;
   }
-  const uint32_t j0 = (blockIdx.x - ntiles) * kTile + threadIdx.x, kept = *r.kept;
+  const uint32_t j0 = (blockIdx.x - ntiles) * kTile + threadIdx.x;
+  const size_t kept = *r.kept;
 #pragma unroll
   for (uint32_t u = 0; u < kPer; ++u) {
     const uint32_t j = j0 + u * kThreads;

@@ -269,6 +269,12 @@ int wrach_stats(WrachContext *ctx, WrachStats *out);
 int wrach_selftest_wait(WrachContext *ctx, uint32_t limit_us,
                         uint32_t *timed_out, uint32_t *waited_us);
 
+/* Self-test of a failed growth: the nth allocation from here on that grows
+ * the context's store, staging or sort buffers (0: none) fails on the host as
+ * if the device were out of memory.  The context stays usable.  No
+ * counterpart in the reference. */
+int wrach_selftest_alloc(WrachContext *ctx, uint32_t nth);
+
 /* The last error message of the context ("" if none). */
 const char *wrach_last_error(WrachContext *ctx);
 

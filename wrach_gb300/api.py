@@ -287,6 +287,10 @@ class Simulation:
                                                 ctypes.byref(us)))
         return bool(t.value), int(us.value)
 
+    def selftest_alloc(self, nth):
+        """Make the nth allocation from here on that grows a buffer fail (0: none)."""
+        self._check(self._L.wrach_selftest_alloc(self._ctx, int(nth)))
+
     # -- viewport streaming -------------------------------------------------
     def write_back(self, world=0):
         """Write the world's frame back into its store."""

@@ -152,37 +152,17 @@ void release(WrachContext* ctx) {
 // The buffers below may still be in use by work queued on the context's
 // streams (a frame, or the last steps of an upload), so a reallocation waits
 // for that work before freeing them.
-int ensure_sort_capacity(WrachContext* ctx, size_t need) {
-  if (need <= ctx->sort_cap) return WRACH_OK;
-  size_t cap = std::max(need, ctx->sort_cap * 2);
-  CK(cudaStreamSynchronize(ctx->stream));
-  CK(cudaStreamSynchronize(ctx->aux));
-  uint32_t** bufs[] = {&ctx->keys, &ctx->kA, &ctx->kB, &ctx->iA, &ctx->iB};
-  for (auto b : bufs) {
-    dfree(*b);
-    *b = nullptr;
-  }
-  for (auto b : bufs) CK(dalloc(b, cap));
-  dfree(ctx->big_list);
-  ctx->big_list = nullptr;
-  // at most cap / (kSmallCell + 1) cells can be larger than kSmallCell
-  ctx->big_cap = (uint32_t)(cap / (wrach::kSmallCell + 1) + 2);
-  CK(dalloc(&ctx->big_list, ctx->big_cap));
-  ctx->sort_cap = cap;
-  drop_graphs(ctx);
-  return WRACH_OK;
-}
-
 int ensure_stage(WrachContext* ctx, size_t need) {
   if (need <= ctx->stage_cap) return WRACH_OK;
   size_t cap = std::max(need, ctx->stage_cap * 2);
   CK(cudaStreamSynchronize(ctx->stream));
   CK(cudaStreamSynchronize(ctx->aux));
+  ctx->stage_cap = 0;  // until both are there
   dfree(ctx->stage_pos);
   dfree(ctx->stage_vel);
   ctx->stage_pos = ctx->stage_vel = nullptr;
-  CK(dalloc(&ctx->stage_pos, cap));
-  CK(dalloc(&ctx->stage_vel, cap));
+  CK(dalloc(ctx, &ctx->stage_pos, cap));
+  CK(dalloc(ctx, &ctx->stage_vel, cap));
   ctx->stage_cap = cap;
   return WRACH_OK;
 }
@@ -195,8 +175,12 @@ int ensure_store(WrachContext* ctx, Store& s, size_t need) {
   size_t cap = std::max<size_t>(need, (size_t)s.cap * 2);
   if (cap > kMaxStore) return fail(ctx, WRACH_ERR_CAPACITY, "store too large");
   float2 *np = nullptr, *nv = nullptr;
-  CK(dalloc(&np, cap));
-  CK(dalloc(&nv, cap));
+  CK(dalloc(ctx, &np, cap));
+  const cudaError_t e = dalloc(ctx, &nv, cap);
+  if (e != cudaSuccess) {
+    dfree(np);
+    CK(e);
+  }
   if (s.n) {
     CK(cudaMemcpyAsync(np, s.pos, s.n * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
     CK(cudaMemcpyAsync(nv, s.vel, s.n * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
@@ -228,6 +212,25 @@ void drop_graphs(WrachContext* ctx) {
         cudaGraphExecDestroy(g);
         g = nullptr;
       }
+}
+
+int ensure_sort_capacity(WrachContext* ctx, size_t need) {
+  if (need <= ctx->sort_cap) return WRACH_OK;
+  size_t cap = std::max(need, ctx->sort_cap * 2);
+  CK(cudaStreamSynchronize(ctx->stream));
+  CK(cudaStreamSynchronize(ctx->aux));
+  drop_graphs(ctx);
+  ctx->sort_cap = 0;  // until all of them are there
+  uint32_t** bufs[] = {&ctx->keys, &ctx->kA, &ctx->kB, &ctx->iA, &ctx->iB, &ctx->big_list};
+  for (auto b : bufs) {
+    dfree(*b);
+    *b = nullptr;
+  }
+  // at most cap / (kSmallCell + 1) cells can be larger than kSmallCell
+  ctx->big_cap = (uint32_t)(cap / (wrach::kSmallCell + 1) + 2);
+  for (auto b : bufs) CK(dalloc(ctx, b, b == &ctx->big_list ? ctx->big_cap : cap));
+  ctx->sort_cap = cap;
+  return WRACH_OK;
 }
 
 int fail(WrachContext* c, int code, const std::string& msg) {
@@ -877,6 +880,7 @@ int wrach_add_particles_device(WrachContext* ctx, uint32_t world, const float* d
 int wrach_step(WrachContext* ctx, uint32_t nsteps) {
   if (!ctx) return WRACH_ERR_INVALID_ARGUMENT;
   DeviceGuard guard(ctx->device);
+  if (int rc = ensure_sort_capacity(ctx, ctx->total_cap)) return rc;
   for (uint32_t s = 0; s < nsteps; ++s) {
     // a graph holds the particle count (grid sizes) it was captured with;
     // buffer reallocations drop the graphs.  Capturing one takes about as long
@@ -909,11 +913,13 @@ int wrach_profile_frame(WrachContext* ctx, float* ms, uint32_t cap, uint32_t* co
   const uint32_t nl = frame_steps(ctx);
   *count = nl;
   if (!ms || cap < nl) return fail(ctx, WRACH_ERR_INVALID_ARGUMENT, "profile buffer too small");
+  int rc = ensure_sort_capacity(ctx, ctx->total_cap);
+  if (rc) return rc;
   std::vector<cudaEvent_t> ev(nl + 1);
   for (auto& e : ev) CK(cudaEventCreate(&e));
   ctx->event_hook = ev.data();
   ctx->event_count = 0;
-  int rc = enqueue_frame(ctx);
+  rc = enqueue_frame(ctx);
   ctx->event_hook = nullptr;
   if (rc == WRACH_OK) {
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1062,6 +1068,12 @@ int wrach_selftest_wait(WrachContext* ctx, uint32_t limit_us, uint32_t* timed_ou
   CK(cudaStreamSynchronize(ctx->stream));
   *timed_out = h[0];
   *waited_us = h[1];
+  return WRACH_OK;
+}
+
+int wrach_selftest_alloc(WrachContext* ctx, uint32_t nth) {
+  if (!ctx) return WRACH_ERR_INVALID_ARGUMENT;
+  ctx->fail_alloc = nth;
   return WRACH_OK;
 }
 

@@ -83,6 +83,7 @@ struct WrachContext {
   uint32_t* gather_out = nullptr;
   uint32_t* gather_h = nullptr;   // pinned, written by the device (nworlds + 1)
   std::string err;
+  uint32_t fail_alloc = 0;  // wrach_selftest_alloc: the growth's allocation that fails (0: none)
   uint64_t launches = 0;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   uint32_t graph_n[2] = {0, 0};       // particle count each graph was captured with
@@ -132,7 +133,22 @@ cudaError_t dalloc(T** p, size_t count) {
   return cudaMalloc((void**)p, count * sizeof(T));
 }
 
+// The same for a buffer that grows with the context's use.
+template <typename T>
+cudaError_t dalloc(WrachContext* ctx, T** p, size_t count) {
+  if (ctx->fail_alloc && --ctx->fail_alloc == 0) {
+    *p = nullptr;
+    return cudaErrorMemoryAllocation;
+  }
+  return dalloc(p, count);
+}
+
 void dfree(void* p);
+
+// The sort's scratch for `need` sources.  A growth that fails leaves none, and
+// the captured frames, which hold its address, are dropped: every call that
+// uses the scratch asks for it first.
+int ensure_sort_capacity(WrachContext* ctx, size_t need);
 
 // Destroys the captured frames (their launches' arguments are out of date).
 void drop_graphs(WrachContext* ctx);

@@ -403,6 +403,7 @@ int wrach_surrogate_step(WrachContext* ctx, uint32_t nsteps, float max_penetrati
   if (rc) return rc;
   DeviceGuard guard(ctx->device);
   if ((rc = ensure_metrics(ctx))) return rc;
+  if ((rc = ensure_sort_capacity(ctx, ctx->total_cap))) return rc;
   auto& S = ctx->sur;
   wrach::GateState g0{};
   g0.tol = max_penetration;

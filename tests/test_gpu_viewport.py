@@ -123,3 +123,67 @@ def test_write_back_at_tile_edges(W, O, n, outside):
         assert_frame_equal(sim.read_frame(), frame, "the frame stays")
     finally:
         sim.close()
+
+
+@pytest.mark.parametrize("worlds", [1, 3])
+@pytest.mark.parametrize("add", [False, True])
+@pytest.mark.parametrize("why", ["capacity", 1, 2, 3, 7])
+def test_a_refused_upload_leaves_the_store(W, O, worlds, add, why):
+    """More particles than the frame takes, or (a number) that allocation of a
+    growth failing: frame and store stay as they are, and what follows works
+    from them."""
+    dims, cap, at = (40.0, 30.0), 800, worlds - 1
+    pos, vel = _field(21, 1000, (0.0, 0.0), (39.9, 29.9))
+    pos[700:] += np.float32([64.0, 0.0])  # outside the viewport
+    if why == "capacity":
+        more = _field(22, 900, (0.0, 0.0), (39.9, 29.9))
+    else:
+        more = _field(22, 20000, (100.0, 0.0), (140.0, 29.9))
+    cfg = W.WrachConfig(dimensions=dims, cell_size=1, mode=1, iterations=2, gravity=0.1, capacity=cap)
+    w, ph = O.world(dims[0], dims[1], 1), O.extended_physics(2, 0.1)
+    with W.Simulation(cfg, worlds=[dims] * worlds if worlds > 1 else None) as sim:
+        for k in range(worlds):
+            sim.set_particles(pos, vel, world=k)
+        sim.step(2)
+        frame = O.step(w, ph, *O.pack(w, pos, vel, cap), 2)[:3]
+        with pytest.raises(W.WrachError) as e:
+            if why != "capacity":
+                sim.selftest_alloc(why)
+            (sim.add_particles if add else sim.set_particles)(*more, world=at)
+        sim.selftest_alloc(0)
+        assert e.value.code == (2 if why == "capacity" else 4)
+        _store_equal(sim, (pos, vel), "after the refusal", world=at)
+        assert_frame_equal(sim.read_frame(world=at), frame, "after the refusal")
+        extra = _field(23, 20, (0.0, 0.0), (39.9, 29.9))
+        sim.add_particles(*extra, world=at)
+        store = np.concatenate([pos, extra[0]]), np.concatenate([vel, extra[1]])
+        _store_equal(sim, store, "a further upload", world=at)
+        frame = O.pack(w, *store, cap)
+        assert_frame_equal(sim.read_frame(world=at), frame, "a further upload")
+        sim.step(1)
+        frame = O.step(w, ph, *frame, 1)[:3]
+        sim.set_viewport((64.0, 0.0), world=at)
+        store = O.write_back(w, store[0], store[1], frame[1], frame[2])
+        w = O.world(dims[0], dims[1], 1, anchor=(64.0, 0.0))
+        _store_equal(sim, store, "a move", world=at)
+        assert_frame_equal(sim.read_frame(world=at), O.pack(w, *store, cap), "a move")
+        sim.set_particles(*extra, world=at)
+        _store_equal(sim, extra, "a replacing upload", world=at)
+
+
+@pytest.mark.parametrize("worlds", [1, 2])
+def test_replacing_uploads_of_every_size(W, O, worlds):
+    # from none to more and back: a replacing upload's particles are staged, and
+    # its buffers and the store's change places
+    dims = (40.0, 30.0)
+    cfg = W.WrachConfig(dimensions=dims, cell_size=1, mode=1, iterations=2, gravity=0.1, capacity=3000)
+    w, ph = O.world(dims[0], dims[1], 1), O.extended_physics(2, 0.1)
+    with W.Simulation(cfg, worlds=[dims] * worlds if worlds > 1 else None) as sim:
+        for k, n in enumerate([0, 5, 0, 900, 2900, 1, 2900, 0, 30]):
+            pos, vel = _field(40 + k, n, (-10.0, 0.0), (39.9, 29.9))
+            sim.set_particles(pos, vel, world=worlds - 1)
+            _store_equal(sim, (pos, vel), "%d particles" % n, world=worlds - 1)
+            ref = O.pack(w, pos, vel, 3000)
+            assert_frame_equal(sim.read_frame(world=worlds - 1), ref, "%d particles" % n)
+            sim.step(2)
+            assert_frame_equal(sim.read_frame(world=worlds - 1), O.step(w, ph, *ref, 2)[:3], "frames of %d" % n)

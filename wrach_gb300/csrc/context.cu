@@ -610,70 +610,56 @@ int create_impl(const WrachConfig* config, uint32_t nworlds, const float* dims,
   return WRACH_OK;
 }
 
-int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
-                const float* vel, uint32_t n_add, cudaMemcpyKind kind,
-                bool replace) {
-  if (!ctx) return WRACH_ERR_INVALID_ARGUMENT;
-  if (world >= ctx->nworlds) return fail(ctx, WRACH_ERR_INVALID_ARGUMENT, "world out of range");
-  if (n_add && (!pos || !vel)) return fail(ctx, WRACH_ERR_INVALID_ARGUMENT, "null particle arrays");
-  DeviceGuard guard(ctx->device);
+// The particles of the other worlds' frames, which a re-pack of one world
+// sorts again; with one world there are none.
+uint32_t kept_particles(const WrachContext* ctx) { return ctx->nworlds > 1 ? ctx->n : 0u; }
+
+// One world's staged particles become its store, whose buffers serve the next
+// staging.
+void swap_stage(WrachContext* ctx, Store& s) {
+  std::swap(s.pos, ctx->stage_pos);
+  std::swap(s.vel, ctx->stage_vel);
+  const size_t cap = s.cap;
+  s.cap = (uint32_t)std::min(ctx->stage_cap, kMaxStore);
+  ctx->stage_cap = cap;
+}
+
+// Packs the frame of `world` from n_new particles: its store's or, `staged`,
+// those in the staging buffers behind the kept ones, which then become the
+// store.  The caller has made room in the store (of several worlds), the staging
+// buffers (kept and new) and the sort's scratch.  Frame, table, counters and
+// store stay as they are when the frame's capacity is exceeded.  vel_aside: the
+// new velocities are on their way on the second stream.
+int repack(WrachContext* ctx, uint32_t world, uint32_t n_new, bool staged, bool vel_aside) {
   Store& s = ctx->stores[world];
-  const uint32_t old_n = s.n;
-  if (replace) s.n = 0;
-  int rc = ensure_store(ctx, s, (size_t)s.n + n_add);
-  if (rc) return rc;
+  const uint32_t n_keep = kept_particles(ctx), nsrc = n_keep + n_new;
   // The sort places straight into the frame buffers.  One world's place steps
   // follow the scan at once (they place nothing when the frame's capacity is
-  // exceeded, which the host then reports), and its velocities are copied on
-  // the second stream while the positions' keys are counted, scanned and
-  // scattered (only the place steps read them).  Of several worlds each has
-  // its own capacity: their place steps wait for the counts.
+  // exceeded, which the host then reports), and its velocities are copied
+  // while the positions' keys are counted, scanned and scattered (only the
+  // place steps read them).  Of several worlds each has its own capacity: their
+  // place steps wait for the counts.
   const bool direct = ctx->nworlds == 1;
-  const bool vel_aside = direct && n_add;
-  if (n_add) {
-    CK(cudaMemcpyAsync(s.pos + s.n, pos, (size_t)n_add * sizeof(float2), kind, ctx->stream));
-    if (vel_aside) {
-      CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
-      CK(cudaStreamWaitEvent(ctx->aux, ctx->fork_ev, 0));
-      CK(cudaMemcpyAsync(s.vel + s.n, vel, (size_t)n_add * sizeof(float2), kind, ctx->aux));
-      CK(cudaEventRecord(ctx->join_ev, ctx->aux));
-    } else {
-      CK(cudaMemcpyAsync(s.vel + s.n, vel, (size_t)n_add * sizeof(float2), kind, ctx->stream));
-    }
-  }
-  s.n += n_add;
-
-  // the frame's particles of other worlds are kept; with one world they all
-  // belong to the world being re-packed from its store, so none are
-  const uint32_t n_keep = ctx->nworlds > 1 ? ctx->n : 0u, n_new = s.n;
-  const size_t nsrc = (size_t)n_keep + n_new;
-  if (nsrc > kMaxStore) {
-    s.n = old_n;
-    return fail(ctx, WRACH_ERR_CAPACITY, "too many particles");
-  }
-  if ((rc = ensure_stage(ctx, nsrc))) return rc;
-  if ((rc = ensure_sort_capacity(ctx, nsrc))) return rc;
-  // the sort's source: [kept frame particles, store]; without kept
+  // the sort's source: [kept frame particles, new particles]; without kept
   // particles the store itself
-  const float2* src_pos = s.pos;
-  const float2* src_vel = s.vel;
+  const bool from_stage = staged || n_keep;
+  const float2* src_pos = from_stage ? ctx->stage_pos : s.pos;
+  const float2* src_vel = from_stage ? ctx->stage_vel : s.vel;
   if (n_keep) {
     CK(cudaMemcpyAsync(ctx->stage_pos, ctx->pos, n_keep * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->stage_vel, ctx->vel, n_keep * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
-    if (n_new) {
+    if (n_new && !staged) {
       CK(cudaMemcpyAsync(ctx->stage_pos + n_keep, s.pos, n_new * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
       CK(cudaMemcpyAsync(ctx->stage_vel + n_keep, s.vel, n_new * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
     }
-    src_pos = ctx->stage_pos;
-    src_vel = ctx->stage_vel;
   }
   CK(wrach::launch_upload_keys(ctx->worlds_d, (int)ctx->nworlds, ctx->ncells, world,
-                               ctx->worlds_h[world], n_keep,
-                               ctx->cell_of[ctx->cur], n_new, s.pos, ctx->keys, ctx->ctrl,
-                               ticket_args(ctx), ctx->stream));
+                               ctx->worlds_h[world], n_keep, ctx->cell_of[ctx->cur], n_new,
+                               src_pos + n_keep, ctx->keys, ctx->ctrl, ticket_args(ctx),
+                               ctx->stream));
   ctx->launches += nsrc ? 1 : 0;
   wrach::RebinArgs r = rebin_args(ctx);
-  r.n = (uint32_t)nsrc;
+  r.n = nsrc;
   r.dst_capacity = ctx->total_cap;
   r.pos_src = src_pos;
   r.vel_src = src_vel;
@@ -705,6 +691,7 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
     CK(wrach::launch_count_sort_step(r, wrach::kPlace, ctx->big_blocks, ctx->stream, &launched));
     return (int)WRACH_OK;
   };
+  int rc;
   if (direct && (rc = place())) return rc;
   // the call returns once the counts are known and the source arrays have
   // been read; the place steps may still be running, ahead of whatever the
@@ -717,7 +704,6 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
     const uint32_t cnt = starts[w + 1] - starts[w];
     if (cnt > ctx->cap_h[w]) {
       // nothing is placed; the counters are left as the place steps leave them
-      s.n = old_n;
       CK(cudaMemsetAsync(ctx->counts, 0, ((size_t)ctx->ncells + 1) * 4, ctx->stream));
       CK(cudaMemsetAsync(ctx->tile_sums, 0, (size_t)ctx->ntiles * 4, ctx->stream));
       if (ctx->tile_sums_cap)
@@ -728,6 +714,13 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
     }
   }
   if (!direct && (rc = place())) return rc;
+  if (staged && direct) {
+    swap_stage(ctx, s);
+  } else if (staged && n_new) {
+    CK(cudaMemcpyAsync(s.pos, src_pos + n_keep, n_new * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(s.vel, src_vel + n_keep, n_new * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
+  }
+  s.n = n_new;
   ctx->cur ^= 1;
   ctx->n = starts[nw];
   for (uint32_t w = 0; w < nw; ++w) {
@@ -736,6 +729,40 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
   }
   ctx->graph_ok = true;
   return WRACH_OK;
+}
+
+int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
+                const float* vel, uint32_t n_add, cudaMemcpyKind kind,
+                bool replace) {
+  if (!ctx) return WRACH_ERR_INVALID_ARGUMENT;
+  if (world >= ctx->nworlds) return fail(ctx, WRACH_ERR_INVALID_ARGUMENT, "world out of range");
+  if (n_add && (!pos || !vel)) return fail(ctx, WRACH_ERR_INVALID_ARGUMENT, "null particle arrays");
+  DeviceGuard guard(ctx->device);
+  Store& s = ctx->stores[world];
+  const uint32_t n_keep = kept_particles(ctx);
+  const size_t n_new = (size_t)(replace ? 0u : s.n) + n_add, nsrc = n_keep + n_new;
+  if (nsrc > kMaxStore) return fail(ctx, WRACH_ERR_CAPACITY, "too many particles");
+  // A replacing upload is staged, any other goes behind the store's particles:
+  // the store keeps what it holds until the frame is known to fit.
+  const bool one = ctx->nworlds == 1;
+  int rc;
+  if ((rc = ensure_stage(ctx, nsrc))) return rc;
+  if (!(one && replace) && (rc = ensure_store(ctx, s, n_new))) return rc;
+  if ((rc = ensure_sort_capacity(ctx, nsrc))) return rc;
+  const bool vel_aside = one && n_add;
+  if (n_add) {
+    float2* to_pos = replace ? ctx->stage_pos + n_keep : s.pos + s.n;
+    float2* to_vel = replace ? ctx->stage_vel + n_keep : s.vel + s.n;
+    CK(cudaMemcpyAsync(to_pos, pos, (size_t)n_add * sizeof(float2), kind, ctx->stream));
+    if (vel_aside) {
+      CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
+      CK(cudaStreamWaitEvent(ctx->aux, ctx->fork_ev, 0));
+    }
+    cudaStream_t st = vel_aside ? ctx->aux : ctx->stream;
+    CK(cudaMemcpyAsync(to_vel, vel, (size_t)n_add * sizeof(float2), kind, st));
+    if (vel_aside) CK(cudaEventRecord(ctx->join_ev, ctx->aux));
+  }
+  return repack(ctx, world, (uint32_t)n_new, replace, vel_aside);
 }
 
 // ---------------------------------------------------------------------------
@@ -788,14 +815,8 @@ int write_back_impl(WrachContext* ctx, uint32_t world, const WorldDev* moved = n
   const uint32_t kept = ctx->gather_h[0];
   if ((size_t)kept + nf > kMaxStore) return fail(ctx, WRACH_ERR_CAPACITY, "store too large");
   if (ctx->nworlds == 1) {
-    // the rebuilt store takes the place of the old one, whose buffers serve
-    // the next rebuild (with more worlds the staging buffers are larger than
-    // any world's store)
-    std::swap(s.pos, ctx->stage_pos);
-    std::swap(s.vel, ctx->stage_vel);
-    const size_t cap = s.cap;
-    s.cap = (uint32_t)std::min(ctx->stage_cap, kMaxStore);
-    ctx->stage_cap = cap;
+    // (with more worlds the staging buffers are larger than any world's store)
+    swap_stage(ctx, s);
     s.n = kept + nf;
     return WRACH_OK;
   }

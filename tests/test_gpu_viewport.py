@@ -187,3 +187,66 @@ def test_replacing_uploads_of_every_size(W, O, worlds):
             assert_frame_equal(sim.read_frame(world=worlds - 1), ref, "%d particles" % n)
             sim.step(2)
             assert_frame_equal(sim.read_frame(world=worlds - 1), O.step(w, ph, *ref, 2)[:3], "frames of %d" % n)
+
+
+@pytest.mark.parametrize("worlds", [1, 3])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_a_refused_move_leaves_the_viewport(W, O, worlds, mode):
+    """A move to where the store holds more particles than the frame takes, and
+    one that each of its allocations fails in turn: settings, frame, the next
+    steps' walls and the store stay, and the moves after it start from them."""
+    dims, cap, at, K = (40.0, 30.0), 800, worlds - 1, 4 if mode else 1
+    pos, vel = _field(31, 1700, (0.0, 0.0), (39.9, 29.9))
+    pos[700:1600] += np.float32([64.0, 0.0])  # too many there
+    pos[1600:] += np.float32([128.0, 0.0])
+    cfg = W.WrachConfig(dimensions=dims, cell_size=1, mode=mode, iterations=K, gravity=0.1 if mode else 0.0,
+                        capacity=cap)
+    w, ph = O.world(dims[0], dims[1], 1), oracle_physics(O, mode, K, 0.1 if mode else 0.0)
+    store = pos, vel
+    with W.Simulation(cfg, worlds=[dims] * worlds if worlds > 1 else None) as sim:
+        for k in range(worlds):
+            sim.set_particles(pos, vel, world=k)
+        sim.step(3)
+        frame = O.step(w, ph, *O.pack(w, pos, vel, cap), 3)[:3]
+
+        def unmoved(what):
+            nonlocal frame
+            assert tuple(sim.settings(at).view_anchor) == (0.0, 0.0), what
+            _store_equal(sim, store, what, world=at)
+            assert_frame_equal(sim.read_frame(world=at), frame, what)
+            sim.step(2)
+            frame = O.step(w, ph, *frame, 2)[:3]
+            assert_frame_equal(sim.read_frame(world=at), frame, what + ", two frames later")
+
+        with pytest.raises(W.CapacityError):
+            sim.set_viewport((64.0, 0.0), world=at)
+        unmoved("after the refusal")
+        sim.write_back(world=at)
+        store = O.write_back(w, store[0], store[1], frame[1], frame[2])
+        _store_equal(sim, store, "write-back", world=at)
+        grown = np.concatenate([store[0], pos[700:] + np.float32([96.0, 0.0])])
+        store = grown, np.concatenate([store[1], vel[700:]])
+        sim.set_particles(*store, world=at)
+        frame = O.pack(w, *store, cap)
+        nth = 1
+        while True:
+            sim.selftest_alloc(nth)
+            try:
+                sim.set_viewport((128.0, 0.0), world=at)
+                break
+            except W.WrachError as e:
+                assert e.code == W._lib.WRACH_ERR_OUT_OF_MEMORY and nth < 12
+                unmoved("allocation %d" % nth)
+            nth += 1
+        sim.selftest_alloc(0)
+        for anchor in [(128.0, 0.0), (0.0, 0.0)]:
+            if anchor[0] == 0.0:
+                sim.set_viewport(anchor, world=at)
+            store = O.write_back(w, store[0], store[1], frame[1], frame[2])
+            w = O.world(dims[0], dims[1], 1, anchor=anchor)
+            frame = O.pack(w, *store, cap)
+            _store_equal(sim, store, "moved to %s" % (anchor,), world=at)
+            assert_frame_equal(sim.read_frame(world=at), frame, "moved to %s" % (anchor,))
+            sim.step(2)
+            frame = O.step(w, ph, *frame, 2)[:3]
+            assert_frame_equal(sim.read_frame(world=at), frame, "two frames at %s" % (anchor,))

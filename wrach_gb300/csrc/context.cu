@@ -614,14 +614,22 @@ int create_impl(const WrachConfig* config, uint32_t nworlds, const float* dims,
 // sorts again; with one world there are none.
 uint32_t kept_particles(const WrachContext* ctx) { return ctx->nworlds > 1 ? ctx->n : 0u; }
 
-// One world's staged particles become its store, whose buffers serve the next
-// staging.
-void swap_stage(WrachContext* ctx, Store& s) {
-  std::swap(s.pos, ctx->stage_pos);
-  std::swap(s.vel, ctx->stage_vel);
-  const size_t cap = s.cap;
-  s.cap = (uint32_t)std::min(ctx->stage_cap, kMaxStore);
-  ctx->stage_cap = cap;
+// The n particles staged behind the first `at` places become the store `s`.
+// With one world (at = 0) its buffers serve the next staging; with more the
+// staging buffers are larger than any world's store, which has room for n.
+int take_staged(WrachContext* ctx, Store& s, uint32_t at, uint32_t n) {
+  if (ctx->nworlds == 1) {
+    std::swap(s.pos, ctx->stage_pos);
+    std::swap(s.vel, ctx->stage_vel);
+    const size_t cap = s.cap;
+    s.cap = (uint32_t)std::min(ctx->stage_cap, kMaxStore);
+    ctx->stage_cap = cap;
+  } else if (n) {
+    CK(cudaMemcpyAsync(s.pos, ctx->stage_pos + at, (size_t)n * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(s.vel, ctx->stage_vel + at, (size_t)n * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
+  }
+  s.n = n;
+  return WRACH_OK;
 }
 
 // Packs the frame of `world` from n_new particles: its store's or, `staged`,
@@ -714,12 +722,7 @@ int repack(WrachContext* ctx, uint32_t world, uint32_t n_new, bool staged, bool 
     }
   }
   if (!direct && (rc = place())) return rc;
-  if (staged && direct) {
-    swap_stage(ctx, s);
-  } else if (staged && n_new) {
-    CK(cudaMemcpyAsync(s.pos, src_pos + n_keep, n_new * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(s.vel, src_vel + n_keep, n_new * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
-  }
+  if (staged && (rc = take_staged(ctx, s, n_keep, n_new))) return rc;
   s.n = n_new;
   ctx->cur ^= 1;
   ctx->n = starts[nw];
@@ -769,19 +772,21 @@ int upload_impl(WrachContext* ctx, uint32_t world, const float* pos,
 // Viewport streaming
 // ---------------------------------------------------------------------------
 
-// The world's store becomes: its particles outside the viewport (store
-// order), then the world's frame particles (frame order) -- per cell the
-// reference's write-back of the GPU's particles into its store
-// (particle_store.rs:71-85, a TODO there).  With `moved` the world's settings
-// on the device become those, for the re-packing that follows (a copy from the
-// host would stand between the two).
-int write_back_impl(WrachContext* ctx, uint32_t world, const WorldDev* moved = nullptr) {
+// The world's store as it becomes, staged behind the first `at` places: its
+// particles outside the viewport (store order), then the world's frame
+// particles (frame order) -- per cell the reference's write-back of the GPU's
+// particles into its store (particle_store.rs:71-85, a TODO there).  *count is
+// its size, for which the store of a batch has room then.  With `moved` the
+// world's settings on the device become those, for the re-packing that follows
+// (a copy from the host would stand between the two).
+int rebuild_store(WrachContext* ctx, uint32_t world, uint32_t at, const WorldDev* moved,
+                  uint32_t* count) {
   Store& s = ctx->stores[world];
   const uint32_t nf = ctx->n_h[world], off = ctx->poff_h[world];
   int rc;
   const uint32_t ntiles = wrach::store_tiles(s.n);
   if ((rc = ensure_sort_capacity(ctx, std::max((size_t)s.n + 1, (size_t)ntiles * 32)))) return rc;
-  if ((rc = ensure_stage(ctx, (size_t)s.n + nf))) return rc;
+  if ((rc = ensure_stage(ctx, (size_t)at + s.n + nf))) return rc;
   if (ntiles + 1 > ctx->compact_cap) {
     dfree(ctx->compact_sums);
     ctx->compact_sums = nullptr;
@@ -800,8 +805,8 @@ int write_back_impl(WrachContext* ctx, uint32_t world, const WorldDev* moved = n
   r.vel = s.vel;
   r.frame_pos = ctx->pos + off;
   r.frame_vel = ctx->vel + off;
-  r.dst_pos = ctx->stage_pos;
-  r.dst_vel = ctx->stage_vel;
+  r.dst_pos = ctx->stage_pos + at;
+  r.dst_vel = ctx->stage_vel + at;
   r.outside = ctx->keys;
   r.tile_sums = ctx->compact_sums;
   r.kept = ctx->compact_sums + ntiles;
@@ -812,22 +817,10 @@ int write_back_impl(WrachContext* ctx, uint32_t world, const WorldDev* moved = n
   ctx->launches += (ntiles ? 2 : 1) + (s.n + nf ? 1 : 0);
   // the store is rebuilt while the host learns its size
   CK(cudaEventSynchronize(ctx->counts_ev));
-  const uint32_t kept = ctx->gather_h[0];
-  if ((size_t)kept + nf > kMaxStore) return fail(ctx, WRACH_ERR_CAPACITY, "store too large");
-  if (ctx->nworlds == 1) {
-    // (with more worlds the staging buffers are larger than any world's store)
-    swap_stage(ctx, s);
-    s.n = kept + nf;
-    return WRACH_OK;
-  }
-  if ((rc = ensure_store(ctx, s, (size_t)kept + nf))) return rc;
-  if (kept + nf) {
-    CK(cudaMemcpyAsync(s.pos, ctx->stage_pos, ((size_t)kept + nf) * sizeof(float2),
-                       cudaMemcpyDeviceToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(s.vel, ctx->stage_vel, ((size_t)kept + nf) * sizeof(float2),
-                       cudaMemcpyDeviceToDevice, ctx->stream));
-  }
-  s.n = kept + nf;
+  const size_t size = (size_t)ctx->gather_h[0] + nf;
+  if (at + size > kMaxStore) return fail(ctx, WRACH_ERR_CAPACITY, "store too large");
+  if (ctx->nworlds > 1 && (rc = ensure_store(ctx, s, size))) return rc;
+  *count = (uint32_t)size;
   return WRACH_OK;
 }
 
@@ -1046,8 +1039,9 @@ int wrach_write_back(WrachContext* ctx, uint32_t world) {
   if (!ctx) return WRACH_ERR_INVALID_ARGUMENT;
   if (world >= ctx->nworlds) return fail(ctx, WRACH_ERR_INVALID_ARGUMENT, "world out of range");
   DeviceGuard guard(ctx->device);
-  const int rc = write_back_impl(ctx, world);
-  if (rc) return rc;
+  uint32_t count = 0;
+  int rc = rebuild_store(ctx, world, 0, nullptr, &count);
+  if (rc || (rc = take_staged(ctx, ctx->stores[world], 0, count))) return rc;
   CK(cudaStreamSynchronize(ctx->stream));
   return WRACH_OK;
 }
@@ -1064,16 +1058,24 @@ int wrach_set_viewport(WrachContext* ctx, uint32_t world, float anchor_x, float 
                 "the viewport at this anchor has a different grid size; move it by whole cells "
                 "or use a size that is a multiple of the cell size");
   w.cell_off = old.cell_off;
-  const int rc = write_back_impl(ctx, world, &w);
+  // the rebuilt store is staged and the frame packed from it under the new
+  // viewport; both are taken when the frame fits
+  uint32_t count = 0;
+  const uint32_t n_keep = kept_particles(ctx);
+  int rc = rebuild_store(ctx, world, n_keep, &w, &count);
+  if (!rc) {
+    ctx->worlds_h[world] = w;
+    rc = ensure_sort_capacity(ctx, (size_t)n_keep + count);
+    if (!rc) rc = repack(ctx, world, count, true, false);
+  }
   if (rc) {
-    // out of memory: the device keeps the settings that the host keeps
+    // refused: host and device keep the viewport
+    ctx->worlds_h[world] = old;
     cudaMemcpyAsync(ctx->worlds_d + world, &old, sizeof(WorldDev), cudaMemcpyHostToDevice, ctx->stream);
     return rc;
   }
-  ctx->worlds_h[world] = w;
   drop_graphs(ctx);  // a single world's settings are among its launches' arguments
-  // the frame, packed from the store under the new viewport
-  return upload_impl(ctx, world, nullptr, nullptr, 0, cudaMemcpyDeviceToDevice, false);
+  return WRACH_OK;
 }
 
 int wrach_selftest_wait(WrachContext* ctx, uint32_t limit_us, uint32_t* timed_out,

@@ -250,3 +250,35 @@ def test_a_refused_move_leaves_the_viewport(W, O, worlds, mode):
             sim.step(2)
             frame = O.step(w, ph, *frame, 2)[:3]
             assert_frame_equal(sim.read_frame(world=at), frame, "two frames at %s" % (anchor,))
+
+
+@pytest.mark.parametrize("surrogate", [False, True])
+def test_a_batch_moves_between_captured_frames(W, O, surrogate):
+    """A batch keeps its captured frames over a move (they read the worlds'
+    settings from the device): the frames after it have the new walls."""
+    dims = [(40.0, 30.0), (50.0, 20.0)]
+    cfg = W.WrachConfig(cell_size=1, mode=1, iterations=4, gravity=0.1, capacity=2000)
+    fields = [_field(70 + k, 1200, (2.0, 2.0), (d[0] - 8.0, d[1] - 8.0)) for k, d in enumerate(dims)]
+    ph = O.extended_physics(4, 0.1)
+    worlds = [O.world(d[0], d[1], 1) for d in dims]
+    ref = [O.pack(w, p, v, 2000) for w, (p, v) in zip(worlds, fields)]
+    with W.Simulation(cfg, worlds=dims) as sim:
+        for k, (p, v) in enumerate(fields):
+            sim.set_particles(p, v, world=k)
+        if surrogate:
+            sim.surrogate_init(0, 1)
+        # an impossible bound on the overlap: every surrogate frame falls back
+        step = (lambda n: sim.surrogate_step(n, max_penetration=-1e9)) if surrogate else sim.step
+        for anchor in [(1.0, 1.0), (0.0, 0.0)]:
+            step(6)
+            ref = [O.step(w, ph, *r, 6)[:3] for w, r in zip(worlds, ref)]
+            sim.set_viewport(anchor, world=1)
+            store = O.write_back(worlds[1], *fields[1], ref[1][1], ref[1][2])
+            fields[1] = store
+            worlds[1] = O.world(dims[1][0], dims[1][1], 1, anchor=anchor)
+            ref[1] = O.pack(worlds[1], *store, 2000)
+            for frames in (1, 5):
+                step(frames)
+                ref = [O.step(w, ph, *r, frames)[:3] for w, r in zip(worlds, ref)]
+                for k in (0, 1):
+                    assert_frame_equal(sim.read_frame(world=k), ref[k], "world %d at %s" % (k, anchor))

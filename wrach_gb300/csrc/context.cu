@@ -898,8 +898,8 @@ int wrach_step(WrachContext* ctx, uint32_t nsteps) {
   for (uint32_t s = 0; s < nsteps; ++s) {
     // a graph holds the particle count (grid sizes) it was captured with;
     // buffer reallocations drop the graphs.  Capturing one takes about as long
-    // as a 1M-particle frame, so the first frame of a new count runs eagerly
-    // (a viewport on the move never steps a count twice).
+    // as a 1M-particle frame, so the first frame of a new count, or of a single
+    // world's new viewport, runs eagerly.
     cudaGraphExec_t& graph = ctx->graph[ctx->cur];
     const bool again = ctx->last_n == ctx->n;
     ctx->last_n = ctx->n;
@@ -1074,7 +1074,12 @@ int wrach_set_viewport(WrachContext* ctx, uint32_t world, float anchor_x, float 
     cudaMemcpyAsync(ctx->worlds_d + world, &old, sizeof(WorldDev), cudaMemcpyHostToDevice, ctx->stream);
     return rc;
   }
-  drop_graphs(ctx);  // a single world's settings are among its launches' arguments
+  if (ctx->nworlds == 1) {
+    // its settings are among its launches' arguments; a batch's launches read
+    // them from the device and are captured no more often than its counts change
+    drop_graphs(ctx);
+    ctx->last_n = 0xFFFFFFFFu;
+  }
   return WRACH_OK;
 }
 

@@ -269,6 +269,15 @@ int wrach_stats(WrachContext *ctx, WrachStats *out);
 int wrach_selftest_wait(WrachContext *ctx, uint32_t limit_us,
                         uint32_t *timed_out, uint32_t *waited_us);
 
+/* Self-test of the short push factor: for every binary32 squared distance
+ * that it serves at this minimum distance, its root and factor against the
+ * general square root and division.  *compared is their number (0 for
+ * distances that always take the general code), *wrong how many have other
+ * bits: none.  The context's own distance is not touched.  Blocks.  No
+ * counterpart in the reference. */
+int wrach_selftest_push(WrachContext *ctx, float min_distance,
+                        uint64_t *compared, uint64_t *wrong);
+
 /* Self-test of a failed growth: the nth allocation from here on that grows
  * the context's store, staging or sort buffers (0: none) fails on the host as
  * if the device were out of memory.  The context stays usable.  No

@@ -156,3 +156,24 @@ def test_rows_around_32_marks(W, O, cap):
             sim.step(1)
             ref = O.step(w, ph, ref[0], ref[1], ref[2], 1)[:3]
             assert_frame_equal(sim.read_frame(), ref, "frame %d" % frame)
+
+
+def test_the_short_push_factor_everywhere(W):
+    """Root and factor of every binary32 squared distance that the short code
+    serves, against the general square root and division: the distances of the
+    other tests, powers of two and their neighbours, significands of all ones,
+    both ends of the range, and random ones over it."""
+    rng = np.random.default_rng(17)
+    two = np.float32(2.0) ** np.arange(-20, 21, dtype=np.float32)
+    near = np.concatenate([np.nextafter(two[1:], np.float32(0)), np.nextafter(two[:-1], np.float32(4e9))])
+    rand = np.exp2(rng.uniform(-20, 20, 180)).astype(np.float32)
+    with W.Simulation(W.WrachConfig(dimensions=(4.0, 4.0), cell_size=1, mode=1, capacity=4)) as sim:
+        for d in np.concatenate([[1.0, 0.37, 2.5, 0.1, 0.9], two, near, rand]).astype(np.float32):
+            compared, wrong = sim.selftest_push(float(d))
+            # all from 2^-60 to the distance's square but roots of all ones
+            binades = 60 + 2 * np.log2(float(d))
+            assert compared > 0.99 * (binades - 1) * 2 ** 23 and wrong == 0, (float(d), compared, wrong)
+        for d in (2.0 ** -21, 2.0 ** 21):
+            assert sim.selftest_push(d) == (0, 0)
+        with pytest.raises(W.WrachError):
+            sim.selftest_push(0.0)

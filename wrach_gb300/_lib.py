@@ -131,6 +131,8 @@ SIGNATURES = {
     "wrach_write_back": (ctypes.c_int, [_P, ctypes.c_uint32]),
     "wrach_read_keys": (ctypes.c_int, [_P, ctypes.c_uint32, _U, ctypes.c_uint32]),
     "wrach_selftest_wait": (ctypes.c_int, [_P, ctypes.c_uint32, _U, _U]),
+    "wrach_selftest_push": (ctypes.c_int, [_P, ctypes.c_float, ctypes.POINTER(ctypes.c_uint64),
+                                           ctypes.POINTER(ctypes.c_uint64)]),
     "wrach_selftest_alloc": (ctypes.c_int, [_P, ctypes.c_uint32]),
     "wrach_set_viewport": (ctypes.c_int, [_P, ctypes.c_uint32, ctypes.c_float, ctypes.c_float]),
     "wrach_store_size": (ctypes.c_int, [_P, ctypes.c_uint32, _U]),

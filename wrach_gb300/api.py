@@ -287,6 +287,14 @@ class Simulation:
                                                 ctypes.byref(us)))
         return bool(t.value), int(us.value)
 
+    def selftest_push(self, min_distance):
+        """(compared, wrong): the squared distances that the short push factor
+        serves, and how many of them have other bits than the general one."""
+        n, bad = ctypes.c_uint64(0), ctypes.c_uint64(0)
+        self._check(self._L.wrach_selftest_push(self._ctx, float(min_distance), ctypes.byref(n),
+                                                ctypes.byref(bad)))
+        return int(n.value), int(bad.value)
+
     def selftest_alloc(self, nth):
         """Make the nth allocation from here on that grows a buffer fail (0: none)."""
         self._check(self._L.wrach_selftest_alloc(self._ctx, int(nth)))

@@ -108,6 +108,15 @@ float skip_threshold(float min_d) {
   return s;
 }
 
+// The push factor's constants for a minimum distance.  Far from the ends of the
+// exponent range every intermediate value of the short push factor is normal;
+// other distances take the general code.
+void set_push(PhysDev& ph, float min_d) {
+  ph.min_d = min_d;
+  ph.skip_d2 = skip_threshold(min_d);
+  ph.slow_below = min_d >= 0x1p-20f && min_d <= 0x1p20f ? 0x1p-60f : INFINITY;
+}
+
 uint32_t bits_for(uint32_t v) {
   uint32_t b = 0;
   while (b < 32 && (v >> b) != 0) ++b;
@@ -465,13 +474,9 @@ int create_impl(const WrachConfig* config, uint32_t nworlds, const float* dims,
   ctx->ph.mode = c.mode;
   ctx->ph.iterations = c.mode == WRACH_MODE_REFERENCE ? 1u : c.iterations;
   ctx->ph.gravity = c.mode == WRACH_MODE_REFERENCE ? 0.0f : c.gravity;
-  ctx->ph.min_d = c.min_distance;
+  set_push(ctx->ph, c.min_distance);
   ctx->ph.vmax = c.max_velocity;
   ctx->ph.cap = c.cell_capacity;
-  ctx->ph.skip_d2 = skip_threshold(c.min_distance);
-  // far from the ends of the exponent range every intermediate value of the
-  // fast push factor is normal; other distances take the general code
-  ctx->ph.slow_below = c.min_distance >= 0x1p-20f && c.min_distance <= 0x1p20f ? 0x1p-60f : INFINITY;
 
   ctx->nworlds = nworlds;
   ctx->worlds_h.resize(nworlds);
@@ -1096,6 +1101,32 @@ int wrach_selftest_wait(WrachContext* ctx, uint32_t limit_us, uint32_t* timed_ou
   CK(cudaStreamSynchronize(ctx->stream));
   *timed_out = h[0];
   *waited_us = h[1];
+  return WRACH_OK;
+}
+
+int wrach_selftest_push(WrachContext* ctx, float min_distance, uint64_t* compared,
+                        uint64_t* wrong) {
+  if (!ctx || !compared || !wrong) return WRACH_ERR_INVALID_ARGUMENT;
+  if (!(min_distance > 0.0f) || std::isinf(min_distance))
+    return fail(ctx, WRACH_ERR_INVALID_ARGUMENT, "bad minimum distance");
+  DeviceGuard guard(ctx->device);
+  PhysDev ph{};
+  set_push(ph, min_distance);
+  // positive binary32 values order like their bits
+  uint32_t first, end;
+  std::memcpy(&first, &ph.slow_below, 4);
+  std::memcpy(&end, &ph.skip_d2, 4);
+  unsigned long long *d = nullptr, h[2] = {0, 0};
+  CK(dalloc(&d, 2));
+  cudaError_t e = cudaMemsetAsync(d, 0, sizeof(h), ctx->stream);
+  if (e == cudaSuccess) e = wrach::launch_push_check(ph, first, end, ctx->sms, d, ctx->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  dfree(d);
+  CK(e);
+  ctx->launches += first < end ? 1 : 0;
+  *compared = h[0];
+  *wrong = h[1];
   return WRACH_OK;
 }
 

@@ -517,7 +517,39 @@ k_jacobi_final(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t 
   }
 }
 
+// Every squared distance that the short push factor serves, two at a time,
+// against the general square root and division: counts[0] += compared,
+// counts[1] += of them, root or factor with other bits.
+__global__ void __launch_bounds__(256) k_push_check(PhysDev ph, uint32_t first, uint32_t end,
+                                                    unsigned long long* __restrict__ counts) {
+  unsigned long long compared = 0, wrong = 0;
+  const uint64_t stride = 2ull * gridDim.x * blockDim.x;
+  for (uint64_t i = first + 2ull * (blockIdx.x * blockDim.x + threadIdx.x); i < end; i += stride) {
+    const float s[2] = {__uint_as_float((uint32_t)i), __uint_as_float((uint32_t)i + 1u)};
+    float f[2], d[2];
+    push_factors_plain(s[0], s[1], ph, f[0], f[1], d[0], d[1]);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (i + u >= end || push_special(s[u], d[u], ph)) continue;
+      float dist;
+      const float want = push_factor_general(s[u], ph, dist);
+      ++compared;
+      wrong += __float_as_uint(want) != __float_as_uint(f[u]) ||
+               __float_as_uint(dist) != __float_as_uint(d[u]);
+    }
+  }
+  atomicAdd(&counts[0], compared);
+  if (wrong) atomicAdd(&counts[1], wrong);
+}
+
 }  // namespace
+
+cudaError_t launch_push_check(const PhysDev& ph, uint32_t first, uint32_t end, int sms,
+                              unsigned long long* counts, cudaStream_t st) {
+  if (first >= end) return cudaSuccess;
+  k_push_check<<<(sms > 0 ? sms : 1) * 8, 256, 0, st>>>(ph, first, end, counts);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_solve_reference(const SolveArgs& a, cudaStream_t st) {
   if (a.n == 0) return cudaSuccess;

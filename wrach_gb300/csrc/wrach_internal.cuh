@@ -205,9 +205,9 @@ __device__ __forceinline__ bool push_factor(float ex, float ey, float min_d,
 //   quotient  f = q + (a - d q) y with q ~ a / d and y = RN(1 / d)
 // y takes two Newton steps from the root's estimate and is RN(1 / d) for
 // every d whose significand is not all ones; those, and s below
-// ph.slow_below (zero among them) or NaN, take the general code.  d and y
-// were compared with the correctly rounded root and reciprocal for every
-// binary32 s in [2^-60, 2^60].
+// ph.slow_below (zero among them) or NaN, take the general code.  No theorem
+// covers the hardware's reciprocal root: d and f are compared with the general
+// code's for every s that comes here at some 300 distances (launch_push_check).
 __device__ __forceinline__ float push_factor_general(float s, const PhysDev& ph, float& dist) {
   float d = __fsqrt_rn(s);
   dist = d;

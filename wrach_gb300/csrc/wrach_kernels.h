@@ -68,6 +68,11 @@ struct SolveArgs {
   int rows_mode;
 };
 
+// Compares the short push factor (push_factors_plain) with the general one for
+// the squared distances whose bits lie in [first, end): counts[0] grows by
+// those compared, counts[1] by those that differ.
+cudaError_t launch_push_check(const PhysDev& ph, uint32_t first, uint32_t end, int sms,
+                              unsigned long long* counts, cudaStream_t st);
 cudaError_t launch_solve_reference(const SolveArgs& a, cudaStream_t st);
 // One extended-mode iteration but the last, over the compacted taking-part
 // particles: qin and qout are compacted (the first iteration reads

@@ -268,8 +268,6 @@ def launch_bytes(kind, n, c, n_tp=None):
         return 36 * n + 4 * c       # pos, vel in; pos, vel, key out
     if kind == "rebin":
         return 40 * n + 8 * c       # key, pos, vel in; pos, vel, cell_of out; table in + out
-    if kind == "rebin_count":
-        return 8 * n                # keys in, tickets out
     if kind == "rebin_scan":
         return 12 * c               # counts in; cell-start and capped tables out
     if kind == "rebin_scatter":
@@ -279,9 +277,9 @@ def launch_bytes(kind, n, c, n_tp=None):
     return 0
 
 
-# the launches of the rebin (a stable counting sort), in order; the first is
-# left out of frames, whose last solve launch takes the tickets
-REBIN_STEPS = ["count", "scan", "scatter", "place", "large_cells"]
+# the launches of the rebin (a stable counting sort), in order; its tickets are
+# taken by the frame's last solve launch
+REBIN_STEPS = ["scan", "scatter", "place", "large_cells"]
 
 
 def run_ours(args):
@@ -352,9 +350,7 @@ def run_ours(args):
     # (frames 1..K of the trajectory), the frames the line's value covers
     solve_kinds = (["jacobi"] * (cfg["iterations"] - 1) + ["jacobi_final"] if cfg["mode"] else
                    ["solve_reference"])
-    # frames take the rebin's tickets in their last solve launch
-    rebin_kinds = REBIN_STEPS[1:]
-    kinds = solve_kinds + ["rebin_" + s for s in rebin_kinds]
+    kinds = solve_kinds + ["rebin_" + s for s in REBIN_STEPS]
     sim.set_particles(pos, vel)
     window = min(args.steps, args.trajectory)
     every_prof = max(1, window // max(1, args.profile_frames))
@@ -386,7 +382,7 @@ def run_ours(args):
     per_kind = {}
     for k, ms in zip(solve_kinds, prof):
         per_kind.setdefault(k, []).append(ms)
-    rebin_steps = {s: float(ms) for s, ms in zip(rebin_kinds, prof[len(solve_kinds):])}
+    rebin_steps = {s: float(ms) for s, ms in zip(REBIN_STEPS, prof[len(solve_kinds):])}
     # the dominant kernel: the most time per frame of one kernel (the
     # rebin's launches each count on their own)
     for step, ms in rebin_steps.items():

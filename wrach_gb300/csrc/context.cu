@@ -699,7 +699,7 @@ int repack(WrachContext* ctx, uint32_t world, uint32_t n_new, bool staged, bool 
   ctx->launches += wrach::count_sort_launches(r.n, ctx->ncells);
   auto place = [&]() {
     CK(wrach::launch_count_sort_step(r, wrach::kScatter, ctx->big_blocks, ctx->stream, &launched));
-    // the place step is the first to read the velocities
+    // the place step is the first to read the velocities (the order is RebinOrder's)
     if (vel_aside) CK(cudaStreamWaitEvent(ctx->stream, ctx->join_ev, 0));
     CK(wrach::launch_count_sort_step(r, wrach::kPlace, ctx->big_blocks, ctx->stream, &launched));
     return (int)WRACH_OK;
@@ -872,7 +872,7 @@ int wrach_destroy(WrachContext* ctx) {
   {
     DeviceGuard guard(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    // a frame's work on `aux` is joined into `stream`, unless its enqueue
+    // an upload's copy on `aux` is joined into `stream`, unless its enqueue
     // failed between the fork and the join
     if (ctx->aux) cudaStreamSynchronize(ctx->aux);
     release(ctx);

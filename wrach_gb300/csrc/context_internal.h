@@ -174,7 +174,8 @@ wrach::RebinArgs rebin_args(WrachContext* ctx);
 wrach::CountDev ticket_args(WrachContext* ctx);
 // The rebin of a frame whose solve output is in pos_o / vel_o / keys and
 // whose tickets are taken.  `after` runs after each launch; `apart` launches
-// the small and the large cells' place steps on their own.
+// the small and the large cells' place steps on their own.  The order of the
+// launches is RebinOrder's.
 template <typename After>
 cudaError_t enqueue_rebin(WrachContext* ctx, bool apart, After after) {
   using namespace wrach;

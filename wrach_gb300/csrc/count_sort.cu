@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(256) k_cs_scatter(RebinArgs a, uint32_t ntiles
   uint32_t s0, s1;
   new_table<GROUPED>(a).span(k, s0, s1);
   const uint32_t dst = s0 + ticket;
-  if (dst < a.n) {  // always true unless the scan timed out
+  if (dst < a.n) {  // (always: the tickets number what the scan counted)
     a.idx_tmp[dst] = i;
     // a large cell's slots are not place_slot's
     a.cell_tmp[dst] = s1 - s0 > kSmallCell ? a.ncells : k;
@@ -411,7 +411,6 @@ __device__ __forceinline__ void place_slot(const RebinArgs& a, uint32_t q) {
   const CellTable table = new_table<GROUPED>(a);
   const uint32_t total = table.start(a.ncells);
   uint32_t overflow = 0;
-  // the guards below only matter if the scan timed out (table inconsistent)
   const bool in = q < total && q < a.n;
   const uint32_t k = in ? a.cell_tmp[q] : a.ncells, me = in ? a.idx_tmp[q] : a.n;
   if (k < a.ncells) {

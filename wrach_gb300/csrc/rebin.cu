@@ -26,7 +26,6 @@
 // the gather every block scans them and writes its own tiles' starts.
 #include <algorithm>
 
-
 #include "wrach_internal.cuh"
 #include "wrach_kernels.h"
 
@@ -386,7 +385,8 @@ namespace {
 // 18 us together).
 __global__ void __launch_bounds__(256)
 k_upload_keys(const WorldDev* __restrict__ worlds, int nworlds, uint32_t ncells, uint32_t target,
-              const __grid_constant__ WorldDev world, uint32_t n_keep, const uint32_t* __restrict__ cell_of, uint32_t n_new,
+              const __grid_constant__ WorldDev world, uint32_t n_keep,
+              const uint32_t* __restrict__ cell_of, uint32_t n_new,
               const float2* __restrict__ new_pos, uint32_t* __restrict__ keys, Ctrl* ctrl,
               CountDev count) {
   begin_after();

@@ -373,8 +373,8 @@ k_jacobi_tp(const __grid_constant__ Worlds<ONE> worlds, PhysDev ph, uint32_t nce
             const CellTable table, const uint32_t* __restrict__ tp_cell,
             const float2* __restrict__ qin, float2* __restrict__ qout,
             const uint32_t* __restrict__ run_if, uint4* __restrict__ rows) {
-  // the table is older than the kernel before: blocks without a particle
-  // (on a piled-up floor, most) end at once; block 0 always has one
+  // the table is older than the kernel before (RebinOrder): blocks without a
+  // particle (on a piled-up floor, most) end at once; block 0 always has one
   const uint32_t ntp = table.taking(ncells);
   if (blockIdx.x * blockDim.x >= ntp && blockIdx.x != 0) return;
   begin_after();
@@ -594,9 +594,11 @@ static cudaError_t launch_iteration(const SolveArgs& a, uint32_t blocks, uint32_
 
 // Up to two blocks of 128 per SM, the kernels with more loads and pushes in
 // flight per thread (their 108 registers leave 16 warps an SM): 16,384
-// particles piled up, 35.0 -> 31.0 us a frame, 32,768 39.0 -> 34.8, and no
-// difference while they are spread out (20.7 and 24.0).  65,536 42.8 -> 40.2,
-// but spread out 26.8 -> 28.3, and 262,144 52 -> 62.
+// particles piled up, 35.0 -> 31.0 us a frame, 32,768 39.0 -> 34.8, spread out
+// 20.7 and 24.0 either way.  From 2,000 to 38,900 particles (the rule's end on
+// 152 SMs), 0.06 and 0.48 of them per px^2 and two to six iterations, frames take
+// 0 to 13% less spread out and 0 to 16% less piled up.  65,536 42.8 -> 40.2, but
+// spread out 26.8 -> 28.3, and 262,144 52 -> 62.
 static bool few_particles(const SolveArgs& a) {
   return narrow_marks(a.ph) && !a.part && a.n <= (uint32_t)(a.sms > 0 ? a.sms : 1) * 256u;
 }
@@ -618,6 +620,8 @@ cudaError_t launch_jacobi_iteration(const SolveArgs& a, const float2* qin, float
   // block without one still costs its launch: past 9 waves of blocks (108 of
   // 128 threads per SM) the blocks stride instead.  4M particles, 31,250 blocks:
   // 771 -> 765 us spread out, 326 -> 304 us piled up; with 54 per SM 786 and 295.
+  // It begins to act at 2.1M on 152 SMs, and from there to 4M frames take 0 to 2%
+  // less spread out and 0.5 to 7% less piled up (2.6M: 254 -> 251, 222 -> 216).
   const uint32_t most = (uint32_t)(a.sms > 0 ? a.sms : 1) * (13824u / threads);
   const uint32_t blocks = std::min(solve_blocks(a), most);
   if (few_particles(a)) return launch_iteration<uint32_t, true>(a, blocks, threads, qin, qout, st);

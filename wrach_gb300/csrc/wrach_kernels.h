@@ -164,6 +164,13 @@ constexpr uint32_t kBigBlocksPerSm = 8;
 // launch_upload_keys): the scan, the scatter, then the place steps in one
 // launch or, to be timed, the small and the large cells' apart.  *launched is
 // false for a step that has nothing to do.
+//
+// RebinOrder: a rebin of any particles ends with a place launch behind a scatter
+// launch behind the scan that writes the table, each waiting for the one before
+// it.  So a launch after the rebin may read the table ahead of its own wait
+// (k_jacobi_tp does): when its blocks start, the place launch's have passed
+// their wait for the scatter, which had waited for the scan.  A rebin whose last
+// launch writes the table itself would make that read a race.
 enum CountSortStep { kScan = 1, kScatter, kPlaceSmall, kPlaceLarge, kPlace };
 cudaError_t launch_count_sort_step(const RebinArgs& a, int step, uint32_t big_blocks,
                                    cudaStream_t st, bool* launched);

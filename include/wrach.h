@@ -118,7 +118,8 @@ int wrach_destroy(WrachContext *ctx);
 int wrach_add_particles(WrachContext *ctx, uint32_t world, const float *pos,
                         const float *vel, uint32_t n);
 
-/* Replaces the world's store with these n particles and re-packs the frame
+/* Replaces the world's store with these n particles (a refused call leaves
+ * store and frame as they are) and re-packs the frame
  * from them (ParticleStore::add_particles_to_cell followed by
  * create_packed_data, runners/bevy/src/particle_store.rs:62-65,103-149,
  * for the whole store at once).  The host arrays are read before the call
@@ -245,7 +246,8 @@ int wrach_write_back(WrachContext *ctx, uint32_t world);
  * store under the new viewport (its walls move with it).  The grid size must
  * stay the same (always so for a move by whole cells, or for a viewport whose
  * sides are multiples of the cell size); otherwise
- * WRACH_ERR_INVALID_ARGUMENT.  Blocks until the new frame's particles are
+ * WRACH_ERR_INVALID_ARGUMENT.  A refused move leaves viewport, frame and store
+ * as they are.  Blocks until the new frame's particles are
  * counted.  No counterpart in the reference. */
 int wrach_set_viewport(WrachContext *ctx, uint32_t world, float anchor_x,
                        float anchor_y);

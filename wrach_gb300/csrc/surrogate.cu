@@ -306,13 +306,13 @@ __global__ void __launch_bounds__(128) k_mlp_forward(MlpDev m, const uint16_t* _
 // shared memory as BF16, [row][feature] in padded rows.  Then the warps share
 // out the weight gradients X^T dZ1, H1^T dZ2 and H2^T dY, contractions over
 // the tile's rows: warp w owns input features 16 (w mod 4) .. + 15 and one
-// half of the outputs of each product, and keeps those sums in its registers
+// half of the outputs of each product, and adds them to sums in its registers
 // over all of the block's tiles (the transposed operands come from
 // ldmatrix.trans).  What it waits for is latency (of the weights' loads, the
 // two layers and the final sums into global memory): 16,384 rows are 128
 // blocks of one tile.  Before, each warp added every 16-row product into
 // shared memory with atomics, 272 of them a tile, and 4 warps filled an SM's
-// shared memory: 61 us then, 15 us now (16,384 rows).
+// shared memory: 61 us then, 15 us now, 17 with the loss (16,384 rows).
 constexpr uint32_t kTrainRows = 128, kTrainThreads = 256;
 
 struct SmemTile {
@@ -906,8 +906,9 @@ k_samples(const WorldDev* __restrict__ worlds, int nworlds, uint32_t ncells,
 // block, and a warp waits for none of the others afterwards (its rows are its
 // own lanes').  1M lattice: 130 us with one 16-row tile at a time, 4-byte row
 // stores (8 lanes to a bank) and every candidate inserted, 95 us now; it
-// issues 43% of the time and waits for the candidates' loads for most of the
-// rest, with 4 warps a scheduler (128 registers; 3 blocks an SM spill: 118).
+// issues 57% of the time and waits for the candidates' loads and the products
+// for the rest, with 4 warps a scheduler (128 registers; 3 blocks an SM spill:
+// 118).
 constexpr uint32_t kFuseThreads = 256;
 
 __global__ void __launch_bounds__(kFuseThreads, 2)

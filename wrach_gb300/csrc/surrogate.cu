@@ -139,19 +139,44 @@ __device__ __forceinline__ void bfrag(const uint32_t* wt, uint32_t kk, uint32_t 
 // fragment of the input (4 k-tiles).  Writes the A fragments h1, h2 of the
 // activations, the GELU's derivatives z1, z2 at the pre-activations (C
 // layout, 8 n-tiles) and the output y (one n-tile).
+//
+// LOSS: the outputs for the loss, yl, by activations of their own from the same
+// weight fragments.  An activation that is rounded to the other BF16 neighbour
+// shifts the loss, and the hardware tanh (and, less, sums that the tensor cores
+// round towards zero along a chain) does that to many: here each product of 16
+// inputs starts from zero, the four are added to nearest and the GELU is
+// gelu_full.  Root mean square error of the loss against 64 bits over 50 batches
+// of 1,000 and 16,384 and 20 of 65,536 rows, as the gradients' activations have
+// it 9.7e-6, 2.4e-6 and 1.5e-6, this way 1.0e-6, 4.7e-7 and 2.9e-7; the batches'
+// times 27.1, 33.5 and 45.8 us without, 29.3, 35.2 and 52.7 with it, so that it is
+// done only for a loss that is read.  (A pass of its own: 29.5, 35.2 and 54.5;
+// with exact sums of the four and an FP32-exact GELU 9.9e-7, 3.6e-7 and 2.2e-7
+// in 34.5, 40.0 and 74.3 us.)
+template <bool LOSS>
 __device__ __forceinline__ void hidden_layer(const uint32_t* wt, const float* b, uint32_t lane,
-                                             const uint32_t (&in)[4][4], float (&z)[8][4],
-                                             uint32_t (&h)[4][4]) {
+                                             const uint32_t (&in)[4][4],
+                                             const uint32_t (&inl)[4][4], float (&z)[8][4],
+                                             uint32_t (&h)[4][4], uint32_t (&hl)[4][4]) {
   const uint32_t t = lane & 3;
 #pragma unroll
   for (uint32_t nt = 0; nt < 8; ++nt) {
     const float bl = b[nt * 8 + 2 * t], bh = b[nt * 8 + 2 * t + 1];
     z[nt][0] = bl; z[nt][1] = bh; z[nt][2] = bl; z[nt][3] = bh;
+    float p[4][4] = {};
 #pragma unroll
     for (uint32_t kk = 0; kk < 4; ++kk) {
       uint32_t b0, b1;
       bfrag(wt, kk, nt, lane, b0, b1);
       mma_bf16(z[nt], in[kk], b0, b1);
+      if (LOSS) mma_bf16(p[kk], inl[kk], b0, b1);
+    }
+    if (LOSS) {
+      float g[4];
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q)
+        g[q] = gelu_full((p[0][q] + p[1][q]) + (p[2][q] + p[3][q]) + (q & 1 ? bh : bl));
+      hl[nt / 2][2 * (nt & 1)] = pack_bf16(g[0], g[1]);
+      hl[nt / 2][2 * (nt & 1) + 1] = pack_bf16(g[2], g[3]);
     }
   }
 #pragma unroll
@@ -162,21 +187,30 @@ __device__ __forceinline__ void hidden_layer(const uint32_t* wt, const float* b,
     h[nt / 2][2 * (nt & 1) + 1] = pack_bf16(g2, g3);
   }
 }
+template <bool LOSS>
 __device__ __forceinline__ void mlp_tile_forward(const SmemNet& s, uint32_t lane,
                                                  const uint32_t (&ax)[4][4],
                                                  float (&z1)[8][4], uint32_t (&h1)[4][4],
                                                  float (&z2)[8][4], uint32_t (&h2)[4][4],
-                                                 float (&y)[4]) {
+                                                 float (&y)[4], float (&yl)[4]) {
   const uint32_t t = lane & 3;
-  hidden_layer(s.w1t, s.b1, lane, ax, z1, h1);
-  hidden_layer(s.w2t, s.b2, lane, h1, z2, h2);
+  uint32_t l1[4][4], l2[4][4];
+  hidden_layer<LOSS>(s.w1t, s.b1, lane, ax, ax, z1, h1, l1);
+  hidden_layer<LOSS>(s.w2t, s.b2, lane, h1, l1, z2, h2, l2);
   const float bl = s.b3[2 * t], bh = s.b3[2 * t + 1];
   y[0] = bl; y[1] = bh; y[2] = bl; y[3] = bh;
+  float p[4][4] = {};
 #pragma unroll
   for (uint32_t kk = 0; kk < 4; ++kk) {
     uint32_t b0, b1;
     bfrag(s.w3t, kk, 0, lane, b0, b1);
     mma_bf16(y, h2[kk], b0, b1);
+    if (LOSS) mma_bf16(p[kk], l2[kk], b0, b1);
+  }
+  if (LOSS) {
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q)
+      yl[q] = (p[0][q] + p[1][q]) + (p[2][q] + p[3][q]) + (q & 1 ? bh : bl);
   }
 }
 
@@ -421,57 +455,14 @@ __device__ __forceinline__ double half_square(float e0, float e1) {
   return 0.5 * ((double)e0 * e0 + (double)e1 * e1);
 }
 
-// The network's outputs for the loss.  An activation that is rounded to the
-// other BF16 neighbour shifts the loss, and the hardware tanh (and, less, sums
-// that the tensor cores round towards zero along a chain) does that to many:
-// here each product of 16 inputs starts from zero, the four are added to nearest
-// and the GELU is gelu_full.  Root mean square error of the loss against 64
-// bits over 50 batches of 1,000 and 16,384 and 20 of 65,536 rows, as the
-// gradients' forward pass has it 9.7e-6, 2.4e-6 and 1.5e-6, this way 1.0e-6,
-// 4.7e-7 and 2.9e-7; the batches' times 27.1, 33.5 and 45.8 us without a second
-// pass, 29.5, 35.2 and 54.5 with it, so that it runs only for a loss that is
-// read.  (Exact sums of the four and an FP32-exact GELU: 9.9e-7, 3.6e-7 and
-// 2.2e-7 in 34.5, 40.0 and 74.3 us.)
-__device__ __forceinline__ void loss_layer(const uint32_t* wt, const float* b, uint32_t lane,
-                                           const uint32_t (&in)[4][4], uint32_t (&out)[4][4]) {
-  const uint32_t g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (uint32_t nt = 0; nt < 8; ++nt) {
-    const uint32_t* row = wt + (nt * 8 + g) * kRow + t;
-    float p[4][4] = {}, h[4];
-#pragma unroll
-    for (uint32_t kk = 0; kk < 4; ++kk)
-      mma_bf16(p[kk], in[kk], lds_keep(row + kk * 8), lds_keep(row + kk * 8 + 4));
-#pragma unroll
-    for (uint32_t q = 0; q < 4; ++q)
-      h[q] = gelu_full((p[0][q] + p[1][q]) + (p[2][q] + p[3][q]) + b[nt * 8 + 2 * t + (q & 1)]);
-    out[nt / 2][2 * (nt & 1)] = pack_bf16(h[0], h[1]);
-    out[nt / 2][2 * (nt & 1) + 1] = pack_bf16(h[2], h[3]);
-  }
-}
-__device__ __forceinline__ void loss_forward(const SmemNet& s, uint32_t lane,
-                                             const uint32_t (&ax)[4][4], float (&y)[4]) {
-  const uint32_t g = lane >> 2, t = lane & 3;
-  uint32_t h1[4][4], h2[4][4];
-  loss_layer(s.w1t, s.b1, lane, ax, h1);
-  loss_layer(s.w2t, s.b2, lane, h1, h2);
-  const uint32_t* row = s.w3t + g * kRow + t;
-  float p[4][4] = {};
-#pragma unroll
-  for (uint32_t kk = 0; kk < 4; ++kk)
-    mma_bf16(p[kk], h2[kk], lds_keep(row + kk * 8), lds_keep(row + kk * 8 + 4));
-#pragma unroll
-  for (uint32_t q = 0; q < 4; ++q)
-    y[q] = (p[0][q] + p[1][q]) + (p[2][q] + p[3][q]) + s.b3[2 * t + (q & 1)];
-}
-
 // Gradients of L = 0.5 * sum over rows and the 2 outputs of (y - target)^2 /
 // `scale_rows` with respect to every parameter, added into `grad` (FP32,
 // the MlpDev parameter order: w1 [in][out], b1, w2, b2, w3 [in][8], b3).
-// With `want_loss` also adds the loss into the 64-bit sum behind them.
+// LOSS: also adds the loss into the 64-bit sum behind them.
+template <bool LOSS>
 __global__ void __launch_bounds__(kTrainThreads, 1)
 k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restrict__ target,
-               uint32_t n, float inv_rows, float* __restrict__ grad, int want_loss) {
+               uint32_t n, float inv_rows, float* __restrict__ grad) {
   extern __shared__ __align__(16) uint8_t dyn[];
   begin_after();
   SmemTrain& sm = *reinterpret_cast<SmemTrain*>(dyn);
@@ -518,12 +509,12 @@ k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restric
 #pragma unroll
     for (uint32_t kk = 0; kk < 4; ++kk)
       ldsm4(a[kk], st.x + (row0 + (lane & 15)) * kRow + kk * 8 + (lane >> 4) * 4);
-    if (want_loss) {
-      loss_forward(sm.net, lane, a, y);
-      if (t == 0 && r0 < n) lsum += half_square(y[0] - tg0.x, y[1] - tg0.y);
-      if (t == 0 && r1 < n) lsum += half_square(y[2] - tg1.x, y[3] - tg1.y);
+    float yl[4];
+    mlp_tile_forward<LOSS>(sm.net, lane, a, z1, h1, z2, h2, y, yl);
+    if (LOSS && t == 0) {
+      if (r0 < n) lsum += half_square(yl[0] - tg0.x, yl[1] - tg0.y);
+      if (r1 < n) lsum += half_square(yl[2] - tg1.x, yl[3] - tg1.y);
     }
-    mlp_tile_forward(sm.net, lane, a, z1, h1, z2, h2, y);
     store_a(st.h1, row0, lane, h1);
     store_a(st.h2, row0, lane, h2);
     // dY (C layout, one n-tile; only columns 0 and 1 are real outputs)
@@ -615,7 +606,7 @@ k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restric
       }
 #pragma unroll
     for (uint32_t u = 0; u < 2; ++u) sb3[u] += __shfl_xor_sync(0xffffffffu, sb3[u], o);
-    lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+    if (LOSS) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
   }
   if (g == 0) {
 #pragma unroll
@@ -628,7 +619,7 @@ k_mlp_backward(MlpDev m, const uint16_t* __restrict__ x, const float2* __restric
   }
   if (lane == 0) {
     atomicAdd(reinterpret_cast<float2*>(grad + o_b3), make_float2(sb3[0], sb3[1]));
-    if (want_loss) atomicAdd(loss_of(grad), lsum * (double)inv_rows);
+    if (LOSS) atomicAdd(loss_of(grad), lsum * (double)inv_rows);
   }
 }
 
@@ -1224,8 +1215,11 @@ cudaError_t launch_mlp_forward(const MlpDev& m, const uint16_t* x, uint32_t n, f
 }
 
 bool train_setup() {
-  return cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)sizeof(SmemTrain)) == cudaSuccess;
+  for (auto k : {k_mlp_backward<false>, k_mlp_backward<true>})
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(SmemTrain)) != cudaSuccess)
+      return false;
+  return true;
 }
 
 cudaError_t launch_mlp_backward(const MlpDev& m, const uint16_t* x, const float2* target,
@@ -1233,8 +1227,9 @@ cudaError_t launch_mlp_backward(const MlpDev& m, const uint16_t* x, const float2
                                 cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   const uint32_t tiles = (n + kTrainRows - 1) / kTrainRows, most = sms > 0 ? sms : 1;
-  return launch_after_with(sizeof(SmemTrain), k_mlp_backward, tiles < most ? tiles : most,
-                           kTrainThreads, st, m, x, target, n, inv_rows, grad, (int)want_loss);
+  return launch_after_with(sizeof(SmemTrain), want_loss ? k_mlp_backward<true> : k_mlp_backward<false>,
+                           tiles < most ? tiles : most, kTrainThreads, st, m, x, target, n, inv_rows,
+                           grad);
 }
 
 cudaError_t launch_take_gradients(float* grad, float* out, cudaStream_t st) {
